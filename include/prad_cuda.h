@@ -109,6 +109,8 @@ const char* prad_version(void);
  *    the values are the same bit for bit;
  *  "tc_panel_n" = n: column tiles per panel of the persistent GEMM's tile walk (0 = automatic: two
  *    panels when the column operand exceeds 40 MB, so that a panel of it stays in L2);
+ *  "pool_bytes" = n: most bytes of freed device blocks (prad_free) the context keeps for later prad_alloc calls
+ *    (default 1/16 of the device memory; "0" gives the kept blocks back and keeps none);
  *  "tc_pipeline" = "16x4" | "32x2" | "8x8" (k-block floats x stages of the tf32x3 kernel) */
 prad_status prad_set_option(prad_ctx* ctx, const char* key, const char* value);
 /* wait for everything enqueued on the context (what the managed code gets for free
@@ -169,6 +171,9 @@ prad_status prad_get_timings(prad_ctx* ctx, prad_timing_t* out, int capacity, in
  * Stand in for accelerator.Allocate2DDenseX / CopyFromCPU / GetAsArray2D
  * (src/RMAD/GpuMatrixMultiplyOperation.cs:190-201) and for the jagged<->flat
  * conversion (:210-271), but buffers persist across operations. */
+/* prad_free does not wait: the block is kept (see the option "pool_bytes") and a later prad_alloc of this context
+ * may return it; its new work runs behind everything enqueued so far on the context's stream and on the legacy
+ * default stream.  A caller that used the block on a non-blocking stream of its own waits for that before the free. */
 prad_status prad_alloc(prad_ctx* ctx, size_t bytes, void** out_dptr);
 prad_status prad_free(prad_ctx* ctx, void* dptr);
 prad_status prad_zero(prad_ctx* ctx, void* dptr, size_t bytes);

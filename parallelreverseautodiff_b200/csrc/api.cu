@@ -30,7 +30,7 @@ static prad_status grow(prad_ctx* ctx, void** p, size_t* have, size_t need, bool
     *p = nullptr;
     *have = 0;
   }
-  e = host ? cudaMallocHost(p, want) : cudaMalloc(p, want);
+  e = host ? cudaMallocHost(p, want) : device_malloc(p, want);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     set_error("scratch allocation of %zu bytes failed: %s", want, cudaGetErrorString(e));
@@ -85,6 +85,7 @@ prad_status prad_init(int device, prad_ctx** out_ctx) {
   prad_ctx* c = new prad_ctx();
   c->device = device;
   c->sm_count = prop.multiProcessorCount;
+  c->total_mem = prop.totalGlobalMem;
   e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     set_error("prad_init: cudaStreamCreate: %s", cudaGetErrorString(e));
@@ -110,6 +111,7 @@ prad_status prad_shutdown(prad_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   dp_destroy(ctx);
   runtime_destroy(ctx);
+  pool_destroy(ctx);
   if (ctx->ws) cudaFree(ctx->ws);
   if (ctx->tc_err) cudaFree(ctx->tc_err);
   for (void* r : ctx->retired) cudaFree(r);
@@ -162,6 +164,13 @@ prad_status prad_set_option(prad_ctx* ctx, const char* key, const char* value) {
   if (!strcmp(key, "gemm_small")) {
     PRAD_REQUIRE(!strcmp(value, "0") || !strcmp(value, "1"), PRAD_ERR_INVALID, "prad_set_option: gemm_small must be 0 or 1, got '%s'", value);
     ctx->gemm_small = atoi(value);
+    return PRAD_OK;
+  }
+  if (!strcmp(key, "pool_bytes")) {   // most bytes of freed device blocks the context keeps for reuse
+    char* end = nullptr;
+    const unsigned long long n = strtoull(value, &end, 10);
+    PRAD_REQUIRE(end != value && *end == 0 && value[0] != '-', PRAD_ERR_INVALID, "prad_set_option: pool_bytes must be a number of bytes, got '%s'", value);
+    pool_limit(ctx, (size_t)n);
     return PRAD_OK;
   }
   if (!strcmp(key, "tc_pair")) {
@@ -243,22 +252,14 @@ prad_status prad_alloc(prad_ctx* ctx, size_t bytes, void** out_dptr) {
   PRAD_REQUIRE(out_dptr, PRAD_ERR_INVALID, "prad_alloc: null output");
   *out_dptr = nullptr;
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc(out_dptr, bytes);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    set_error("prad_alloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
-    return e == cudaErrorMemoryAllocation ? PRAD_ERR_OOM : PRAD_ERR_CUDA;
-  }
-  return PRAD_OK;
+  return pool_alloc(ctx, bytes, out_dptr);
 }
 
 prad_status prad_free(prad_ctx* ctx, void* dptr) {
   PRAD_CHECK_CTX(ctx);
   PRAD_NOT_CAPTURING(ctx, "prad_free");
   if (!dptr) return PRAD_OK;
-  PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
-  PRAD_CUDA(cudaFree(dptr));
-  return PRAD_OK;
+  return pool_free(ctx, dptr);
 }
 
 prad_status prad_alloc_host(prad_ctx* ctx, size_t bytes, void** out_hptr) {

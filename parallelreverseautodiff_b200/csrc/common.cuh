@@ -19,6 +19,7 @@ enum class GemmF32 { Auto, Simt, SimtFma, Tf32x3, Tf32B16, Bf16x3, Fp16x3 };
 enum class GemmF64 { Auto, Simt, SimtFma, Dmma };
 
 struct DpState;  // data-parallel state (dp.cu)
+struct DevicePool;  // freed device blocks kept for reuse (pool.cu)
 
 }  // namespace prad
 
@@ -42,6 +43,8 @@ struct prad_ctx {
   void* stage = nullptr;
   size_t stage_bytes = 0;
   prad::DpState* dp = nullptr;
+  prad::DevicePool* pool = nullptr;
+  size_t total_mem = 0;               // device memory in bytes
   // give-up flag of the tensor-core GEMMs (device int, sticky until the host reads it)
   int* tc_err = nullptr;
   bool tc_pending_check = false;
@@ -138,6 +141,14 @@ prad_status ensure_workspace(prad_ctx* ctx, size_t bytes);
 // grows the pinned host scratch
 prad_status ensure_host_workspace(prad_ctx* ctx, size_t bytes);
 prad_status ensure_stage(prad_ctx* ctx, size_t bytes);
+
+// device memory with a bounded cache of freed blocks (pool.cu)
+prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out);
+prad_status pool_free(prad_ctx* ctx, void* p);
+void pool_limit(prad_ctx* ctx, size_t cap);   // most bytes this context keeps
+// cudaMalloc; when memory is short every context's cached blocks go back to the device first
+cudaError_t device_malloc(void** out, size_t bytes);
+void pool_destroy(prad_ctx* ctx);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

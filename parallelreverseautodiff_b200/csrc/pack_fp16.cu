@@ -501,8 +501,8 @@ static bool packed_ok(const prad_packed* p) { return p && p->magic == 0x50414b44
   PRAD_REQUIRE(prad::packed_ok(p), PRAD_ERR_INVALID, who ": the packed operand is null or destroyed")
 
 static prad_status alloc_form(PackedForm& f) {
-  cudaError_t e = cudaMalloc((void**)&f.h, f.h_bytes() ? f.h_bytes() : 16);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&f.blk, f.blk_bytes() ? f.blk_bytes() : 16);
+  cudaError_t e = device_malloc((void**)&f.h, f.h_bytes() ? f.h_bytes() : 16);
+  if (e == cudaSuccess) e = device_malloc((void**)&f.blk, f.blk_bytes() ? f.blk_bytes() : 16);
   if (e == cudaSuccess) e = cudaMemset(f.blk, 0, f.blk_bytes());     // rows beyond the matrix keep exponent 0
   if (e != cudaSuccess) {
     (void)cudaGetLastError();

@@ -188,7 +188,7 @@ prad_status prad_slot_store(prad_ctx* ctx, const void* guid_16_bytes, const void
     void* p = const_cast<void*>(ptrs_host[i]);
     if (copy && p && bytes_host[i]) {
       void* q = nullptr;
-      cudaError_t e = cudaMalloc(&q, bytes_host[i]);
+      cudaError_t e = device_malloc(&q, bytes_host[i]);
       if (e != cudaSuccess) {
         (void)cudaGetLastError();
         free_slot(fresh);

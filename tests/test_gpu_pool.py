@@ -1,0 +1,58 @@
+"""Reuse of freed device blocks (prad_alloc / prad_free): contents, size classes, recordings, limits."""
+import numpy as np
+import pytest
+
+from parallelreverseautodiff_b200 import engine as E
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 1000, 4097, 262145])
+def test_blocks_are_reused_and_hold_what_is_written_last(n):
+    with E.Engine(0) as eng:
+        a = np.arange(n, dtype=np.float32)
+        for k in range(20):
+            m = eng.upload(a + k)
+            s = eng.scale(m, 2.0)
+            m.free()
+            t = eng.scale(s, 0.5)            # may live in m's block
+            np.testing.assert_array_equal(t.numpy(), a + k)
+
+
+def test_a_freed_block_comes_back_and_the_limit_holds():
+    with E.Engine(0) as eng:
+        m = eng.empty((1000,), np.float32)
+        p = m.ptr
+        m.free()
+        assert eng.empty((1001,), np.float32).ptr == p          # the same size class
+        eng.set_option("pool_bytes", "0")
+        free0 = eng.device_info()["free_bytes"]
+        big = eng.empty((64 << 20,), np.float32)
+        big.free()
+        assert eng.device_info()["free_bytes"] == free0         # given back at once
+        eng.set_option("pool_bytes", str(4 << 30))
+        big = eng.empty((64 << 20,), np.float32)
+        big.free()
+        assert eng.device_info()["free_bytes"] < free0          # kept
+        eng.set_option("pool_bytes", "0")
+        assert eng.device_info()["free_bytes"] == free0
+        with pytest.raises(Exception):
+            eng.set_option("pool_bytes", "-1")
+
+
+def test_blocks_cross_contexts_and_recordings():
+    a = np.arange(5000, dtype=np.float64)
+    with E.Engine(0) as e1, E.Engine(0) as e2:
+        m = e1.upload(a)
+        e1.sync()
+        E.check(e2.lib.prad_free(e2.ctx, m.ptr))                 # freed by another context
+        m.ptr = 0
+        x = e1.upload(a)
+        seq_out = []
+        e1.scale(x, 3.0)
+        seq = e1.record(lambda: seq_out.append(e1.scale(x, 3.0)))   # a block born in a recording is not from the cache
+        junk = [e1.scale(x, float(k)) for k in range(8)]
+        seq.launch()
+        np.testing.assert_array_equal(seq_out[0].numpy(), 3.0 * a)
+        np.testing.assert_array_equal(junk[5].numpy(), 5.0 * a)
+        seq.close()
