@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -158,6 +159,20 @@ inline int stream_grid(const prad_ctx* ctx, int64_t work_items, int per_block, i
   int64_t cap = (int64_t)ctx->sm_count * ctas_per_sm;
   if (need < 1) need = 1;
   return (int)(need < cap ? need : cap);
+}
+
+// Lets `Kernel` use `bytes` of dynamic shared memory on the context's device (needed above 48 KB): asked for once per
+// kernel and device.
+template <auto Kernel> inline prad_status allow_smem(prad_ctx* ctx, int bytes) {
+  if (bytes <= 48 * 1024) return PRAD_OK;
+  static std::atomic<uint64_t> done{0};
+  const uint64_t bit = 1ull << (ctx->device & 63);
+  if (!(done.load(std::memory_order_acquire) & bit)) {
+    const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    PRAD_REQUIRE(e == cudaSuccess, PRAD_ERR_CUDA, "cannot reserve %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+    done.fetch_or(bit, std::memory_order_release);
+  }
+  return PRAD_OK;
 }
 
 // ---- internal entry points shared between translation units -------------------------------

@@ -13,6 +13,10 @@ prad_status gemm_simt(prad_ctx* ctx, bool exact, bool tA, bool tB, int M, int N,
                       void* C, int ldc, int batch, int64_t sA, int64_t sB, int64_t sC,
                       const GemmEpilogue& e);
 
+template <typename T>
+prad_status gemm_simt_backward(prad_ctx* ctx, bool exact, const void* A, const void* B, const void* dC, void* dA, void* dB, int M,
+                               int K, int N, bool accumulate_dB, double dB_scale, const GemmEpilogue& e_dA);
+
 // tensor-core variants (return PRAD_ERR_UNSUPPORTED when a shape does not fit them)
 prad_status gemm_tf32x3(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, double alpha,
                         const void* A, int lda, const void* B, int ldb, double beta, void* C,
@@ -23,35 +27,30 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
                           int ldc, int batch, int64_t sA, int64_t sB, int64_t sC,
                           const GemmEpilogue& e, bool probe_only);
 
+// whether a product runs on a tensor-core kernel
+static bool wants_tensor_cores(prad_ctx* ctx, prad_dtype dt, bool tA, bool tB, int M, int N, int K, double alpha, const void* A,
+                               int lda, const void* B, int ldb, double beta, void* C, int ldc, int batch, int64_t sA, int64_t sB,
+                               int64_t sC, const GemmEpilogue& epi) {
+  if (dt == PRAD_F32)
+    return ctx->gemm_f32 != GemmF32::Simt && ctx->gemm_f32 != GemmF32::SimtFma &&
+           gemm_tf32x3(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, true) == PRAD_OK;
+  return (ctx->gemm_f64 == GemmF64::Auto || ctx->gemm_f64 == GemmF64::Dmma) &&
+         gemm_f64_dmma(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, true) == PRAD_OK;
+}
+
 prad_status gemm_dispatch(prad_ctx* ctx, prad_dtype dt, bool tA, bool tB, int M, int N, int K,
                           double alpha, const void* A, int lda, const void* B, int ldb,
                           double beta, void* C, int ldc, int batch, int64_t sA, int64_t sB,
                           int64_t sC, const GemmEpilogue& epi) {
   if (M == 0 || N == 0 || batch == 0) return PRAD_OK;
-  if (dt == PRAD_F32) {
-    const bool want_tc = ctx->gemm_f32 == GemmF32::Auto || ctx->gemm_f32 == GemmF32::Tf32x3 ||
-                         ctx->gemm_f32 == GemmF32::Tf32B16 || ctx->gemm_f32 == GemmF32::Bf16x3 ||
-                         ctx->gemm_f32 == GemmF32::Fp16x3;
-    if (want_tc) {
-      prad_status p = gemm_tf32x3(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
-                                  batch, sA, sB, sC, epi, true);
-      if (p == PRAD_OK)
-        return gemm_tf32x3(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA,
-                           sB, sC, epi, false);
-    }
-    return gemm_simt<float>(ctx, ctx->gemm_f32 != GemmF32::SimtFma, tA, tB, M, N, K, alpha, A, lda,
-                            B, ldb, beta, C, ldc, batch, sA, sB, sC, epi);
-  }
-  const bool want_dmma = ctx->gemm_f64 == GemmF64::Auto || ctx->gemm_f64 == GemmF64::Dmma;
-  if (want_dmma) {
-    prad_status p = gemm_f64_dmma(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
-                                  batch, sA, sB, sC, epi, true);
-    if (p == PRAD_OK)
-      return gemm_f64_dmma(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA,
-                           sB, sC, epi, false);
-  }
-  return gemm_simt<double>(ctx, ctx->gemm_f64 != GemmF64::SimtFma, tA, tB, M, N, K, alpha, A, lda,
-                           B, ldb, beta, C, ldc, batch, sA, sB, sC, epi);
+  const bool tc = wants_tensor_cores(ctx, dt, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi);
+  if (dt == PRAD_F32)
+    return tc ? gemm_tf32x3(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, false)
+              : gemm_simt<float>(ctx, ctx->gemm_f32 != GemmF32::SimtFma, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
+                                 batch, sA, sB, sC, epi);
+  return tc ? gemm_f64_dmma(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, false)
+            : gemm_simt<double>(ctx, ctx->gemm_f64 != GemmF64::SimtFma, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch,
+                                sA, sB, sC, epi);
 }
 
 // ---- MultiplyAndSum ------------------------------------------------------------------------
@@ -105,20 +104,24 @@ static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void
                                         prad_act act_below, const void* saved_below,
                                         double act_alpha) {
   prad_status s;
+  GemmEpilogue e_dA, e_dB;
+  e_dA.dact = act_below;
+  e_dA.saved = saved_below;
+  e_dA.act_alpha = act_alpha;
+  // dA (MxK) = dC (MxN) * B^T  (B is KxN) ; dB (KxN) = A^T (A is MxK) * dC (MxN)
+  if (dA && dB && M > 0 && K > 0 && N > 0 &&
+      !wants_tensor_cores(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA) &&
+      !wants_tensor_cores(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0, 0, 0, e_dB))
+    return dt == PRAD_F32 ? gemm_simt_backward<float>(ctx, ctx->gemm_f32 != GemmF32::SimtFma, A, B, dC, dA, dB, M, K, N,
+                                                      accumulate_dB != 0, dB_scale, e_dA)
+                          : gemm_simt_backward<double>(ctx, ctx->gemm_f64 != GemmF64::SimtFma, A, B, dC, dA, dB, M, K, N,
+                                                       accumulate_dB != 0, dB_scale, e_dA);
   if (dA) {
-    GemmEpilogue e;
-    e.dact = act_below;
-    e.saved = saved_below;
-    e.act_alpha = act_alpha;
-    // dA (MxK) = dC (MxN) * B^T  (B is KxN)
-    s = gemm_dispatch(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e);
+    s = gemm_dispatch(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA);
     if (s) return s;
   }
   if (dB) {
-    GemmEpilogue e;
-    // dB (KxN) = A^T (A is MxK) * dC (MxN)
-    s = gemm_dispatch(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N,
-                      accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0, 0, 0, e);
+    s = gemm_dispatch(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0, 0, 0, e_dB);
     if (s) return s;
   }
   return PRAD_OK;

@@ -363,6 +363,17 @@ class FeedForwardNetwork:
         if self.acts[L - 1] != E.ACT_NONE:
             e.act_backward(self.acts[L - 1], self._saved(L), cur, alpha, out=cur)
         for l in range(L, 0, -1):
+            if self.world == 1 and not probe and (l > 1 or need_dx):
+                # nothing to reduce between the two products: one call, which can run them side by side
+                below = self.acts[l - 2] if l > 1 else E.ACT_NONE
+                nxt = self.dZ[1].view((rows, self.sizes[l - 1]))
+                e.matmul_backward(self.A[l - 1], self.W[l - 1], cur, dA=nxt, dB=self.dW[l - 1], act_below=below,
+                                  saved_below=self._saved(l - 1) if below != E.ACT_NONE else None, act_alpha=alpha)
+                if self.use_bias:
+                    e.add_broadcast_backward(cur, dbias=self.db[l - 1])
+                self.dZ.reverse()
+                cur = nxt
+                continue
             if probe:
                 probe("gemm", True)
             e.matmul_backward(self.A[l - 1], None, cur, dB=self.dW[l - 1], need_dA=False)
