@@ -384,6 +384,20 @@ prad_status prad_lstm_cell_backward(prad_ctx* ctx, prad_dtype dt, int64_t n, con
                                     double loss_scale, const void* const* dh_contrib_host, int n_contrib,
                                     const void* dc_next, const void* const* gates_ifgo_host, const void* tanh_c,
                                     const void* c_prev, void* const* dpre_ifgo_host, void* dc_prev);
+/* The recurrent part of an LSTM layer over a whole sequence in one call: one row per sample, time steps stacked along the
+ * rows (steps * batch rows of `hidden` values), the four gates i, f, g, o stacked as matrices where one pointer stands for
+ * all (U: four hidden x hidden matrices; pre, dpre: four matrices of steps * batch rows).
+ * prad_lstm_forward: pre holds W_g x_t on entry and W_g x_t + U_g h_{t-1} + b_g on exit; gates, C, tanh(C), H, H_prev (H one
+ * step earlier, h_{-1} = 0), FC = f (.) c_{t-1} and IG = i (.) g are written for every step.
+ * prad_lstm_backward: per step prad_lstm_cell_backward with a target at every step and the four gradients dpre_g(t+1) U_g as
+ * its contributions; dpre receives the gradients w.r.t. the gate pre-activations.  scratch: 6 * batch * hidden values.
+ * The values are bit-identical to the calls one by one. */
+prad_status prad_lstm_forward(prad_ctx* ctx, prad_dtype dt, int steps, int batch, int hidden, const void* U,
+                              const void* const* bias_ifgo_host, void* pre, void* const* gates_ifgo_host, void* C,
+                              void* tanh_c, void* H, void* H_prev, void* FC, void* IG);
+prad_status prad_lstm_backward(prad_ctx* ctx, prad_dtype dt, int steps, int batch, int hidden, const void* U,
+                               const void* H, const void* target, double loss_scale, const void* const* gates_ifgo_host,
+                               const void* tanh_c, const void* C, void* dpre, void* scratch);
 /* MatrixAddOperation.cs:29-68 / MatrixAddThreeOperation.cs:30-67 (c may be NULL).  Their
  * Backward returns copies of dOut; prad_copy (or simply aliasing dOut) provides that. */
 prad_status prad_add_forward(prad_ctx* ctx, prad_dtype dt, const void* a, const void* b,

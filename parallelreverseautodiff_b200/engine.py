@@ -490,6 +490,16 @@ class Engine:
                                                loss_scale, contrib, len(dh_contrib), self._p(dc_next), gates, tanh_c.ptr,
                                                self._p(c_prev), dpre, self._p(dc_prev)))
 
+    def lstm_forward(self, steps, batch, U, bias_ifgo, pre, gates_ifgo, C_, tanh_c, H, H_prev, FC, IG):
+        """The recurrent part of an LSTM layer's Forward, all time steps (prad_lstm_forward)."""
+        check(self.lib.prad_lstm_forward(self.ctx, dtype_code(H.dtype), steps, batch, H.shape[1], U.ptr, self._ptr_list(bias_ifgo),
+                                         pre.ptr, self._ptr_list(gates_ifgo), C_.ptr, tanh_c.ptr, H.ptr, H_prev.ptr, FC.ptr, IG.ptr))
+
+    def lstm_backward(self, steps, batch, U, H, target, loss_scale, gates_ifgo, tanh_c, C_, dpre, scratch):
+        """The recurrent part of backpropagation through time, all time steps (prad_lstm_backward)."""
+        check(self.lib.prad_lstm_backward(self.ctx, dtype_code(H.dtype), steps, batch, H.shape[1], U.ptr, H.ptr, target.ptr,
+                                          loss_scale, self._ptr_list(gates_ifgo), tanh_c.ptr, C_.ptr, dpre.ptr, scratch.ptr))
+
     def add_forward(self, a, b, c=None, out=None):
         out = out or self.empty(a.shape, a.dtype)
         check(self.lib.prad_add_forward(self.ctx, dtype_code(a.dtype), a.ptr, b.ptr, self._p(c),

@@ -545,6 +545,7 @@ class LstmNetwork:
         self.dX = z(TB, n_in)
         self._tmp = [z(batch, n_hidden) for _ in range(18)]
         self._rec_all, rec = stacked(batch, n_hidden)             # dZ_g(t) U_g for the four gates
+        self._seq_scratch = z(6 * batch, n_hidden)
         for k, g in enumerate(self.GATES):
             self._tmp[8 + k] = rec[g]
 
@@ -562,35 +563,14 @@ class LstmNetwork:
         e, T, B = self.eng, self.T, self.B
         e.upload(np.ascontiguousarray(x_host, self.dtype).reshape(T * B, -1), out=self.X)
         e.upload(np.ascontiguousarray(y_host, self.dtype).reshape(T * B, -1), out=self.Y)
-        e.zero_(self.Hprev)
         nh, n_in, TB, G = self.n_h, self.n_in, T * B, len(self.GATES)
         first = self.GATES[0]
         # input contribution of all steps and gates: X_all * W_g^T, one strided-batched product
         e.gemm(self.X, self.W[first], self.pre[first], transB=True, batch=G, strideA=0, strideB=nh * n_in,
                strideC=TB * nh)
-        acts = {"i": E.ACT_SIGMOID, "f": E.ACT_SIGMOID, "g": E.ACT_TANH, "o": E.ACT_SIGMOID}
-        for t in range(T):
-            hp = self._step(self.Hprev, t)
-            if t > 0:           # + h_{t-1} * U_g^T for the four gates (MatrixAddThree: (Wx + Uh) + b)
-                e.gemm(hp, self.U[first], self._step(self.pre[first], t), transB=True, beta=1.0, batch=G,
-                       strideA=0, strideB=nh * nh, strideC=TB * nh)
-            for g in self.GATES:
-                p = self._step(self.pre[g], t)
-                e.add_broadcast_forward(p, self.b[g], out=p)
-                e.act_forward(acts[g], p, out=self._step(self.gate[g], t))
-            c, fc, ig = self._step(self.C, t), self._step(self.FC, t), self._step(self.IG, t)
-            e.hadamard_forward(self._step(self.gate["i"], t), self._step(self.gate["g"], t), out=ig)
-            if t > 0:
-                e.hadamard_forward(self._step(self.gate["f"], t), self._step(self.C, t - 1), out=fc)
-            else:
-                e.zero_(fc)
-            e.add_forward(fc, ig, out=c)
-            tc = self._step(self.tanhC, t)
-            e.act_forward(E.ACT_TANH, c, out=tc)
-            h = self._step(self.H, t)
-            e.hadamard_forward(self._step(self.gate["o"], t), tc, out=h)
-            if t + 1 < T:
-                e.copy(self._step(self.Hprev, t + 1), h)
+        # per step + h_{t-1} * U_g^T + b_g (MatrixAddThree: (Wx + Uh) + b), the gates and the cell
+        e.lstm_forward(T, B, self._U_all, [self.b[g] for g in self.GATES], self._pre_all, [self.gate[g] for g in self.GATES],
+                       self.C, self.tanhC, self.H, self.Hprev, self.FC, self.IG)
         return self.H
 
     def backward(self):
@@ -601,22 +581,9 @@ class LstmNetwork:
         if not self.fused_cell:
             self._backward_steps_by_operation()
         else:
-            # one launch per time step for everything elementwise (prad_lstm_cell_backward), one strided-batched
-            # product for the four recurrent gradients; bit-identical to the operation-by-operation path
-            dh_rec, dc_next = [], None
-            g0 = self.GATES[0]
-            for t in range(T - 1, -1, -1):
-                st = lambda m: self._step(m, t)        # noqa: E731
-                dc_prev = tmp[15 + (t & 1)] if t > 0 else None
-                e.lstm_cell_backward(st(self.H), st(self.Y), 2.0 / nh, dh_rec, dc_next,
-                                     [st(self.gate[k]) for k in ("i", "f", "g", "o")], st(self.tanhC),
-                                     self._step(self.C, t - 1) if t > 0 else None,
-                                     [st(self.dpre[k]) for k in ("i", "f", "g", "o")], dc_prev)
-                dc_next = dc_prev
-                if t > 0:           # gradient w.r.t. h_{t-1}: one product per gate, summed by the next call
-                    e.gemm(st(self.dpre[g0]), self.U[g0], tmp[8], batch=len(self.GATES),
-                           strideA=T * B * nh, strideB=nh * nh, strideC=B * nh)
-                    dh_rec = [tmp[8 + k] for k in range(len(self.GATES))]
+            # all time steps in one call, bit-identical to the operation-by-operation path
+            e.lstm_backward(T, B, self._U_all, self.H, self.Y, 2.0 / nh, [self.gate[g] for g in self.GATES], self.tanhC, self.C,
+                            self._dpre_all, self._seq_scratch)
         inv_b = 1.0 / B
         first = True
         g0, G, TB = self.GATES[0], len(self.GATES), T * B
