@@ -4,7 +4,7 @@
 // values, and the next step needs all of it.  As 16 launches forward and 2 backward per step, a 64-step sequence took
 // 5.1 ms of kernels and 8 ms with the calls that launch them; the arithmetic of a step is 1 us.
 //
-// Here the batch is cut into tiles of at most 4 rows, and a CLUSTER of CTAs owns one tile for all time steps: CTA r of the
+// Here the batch is cut into tiles of at most 5 rows, and a CLUSTER of CTAs owns one tile for all time steps: CTA r of the
 // cluster owns JJ hidden units (all four gates of them), keeps their rows of the recurrent weights in shared memory from the
 // first step to the last, and hands what it computed in a step (h_t forward, the four dpre_t backward) to its cluster
 // neighbours' shared memory with one bulk copy each, which the receiver waits for on an mbarrier.  Clusters never talk to
@@ -21,7 +21,6 @@
 namespace prad {
 namespace lstm {
 
-constexpr int NT = 128;              // threads of a CTA: [0, 4 JP) multiply, [64, 64 + BB JP) do the cell
 constexpr int WAIT_LIMIT = 1 << 18;  // polls
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -62,13 +61,19 @@ template <typename T, int N> __device__ __forceinline__ void lds16(const T* p, T
 template <typename T, int JP, int BB, int NG>
 struct Tile {
   static constexpr int VEC = 16 / sizeof(T);
-  static constexpr int TR = BB == 1 ? 1 : 2, TC = BB == 4 ? 2 : 1;     // outputs per multiplying thread: rows x columns
+  static constexpr int TR = BB == 4 ? 2 : BB, TC = BB == 4 ? 2 : 1;    // outputs per multiplying thread: rows x columns
   static constexpr int COLS = 4 * JP;                                   // (gate, hidden unit)
   static constexpr int BLOCK = NG * BB * JP;                            // what one CTA hands over per step
-  static_assert(JP % VEC == 0 && JP / VEC % 2 == 0 && COLS <= 64 && BB * JP <= 64, "tile");
+  static constexpr int G = JP / VEC;                                     // 16-byte groups of k per block
+  static constexpr int DEPTH = G % 4 == 0 ? 4 : G % 3 == 0 ? 3 : 2;     // groups in registers
+  // Forward: a thread per gate value (their exponentials are most of a step outside the product), backward: per cell
+  static constexpr int MUL = (COLS + 31) / 32 * 32;                      // the first warps multiply, those behind do the cell
+  static constexpr int CELL = ((NG == 1 ? COLS : JP) * BB + 31) / 32 * 32;
+  static constexpr int NT = MUL + CELL;
+  static_assert(JP % VEC == 0 && G % DEPTH == 0 && COLS <= MUL && BB * JP <= CELL, "tile");
   static int pitch(int cs) { const int v = cs * JP / VEC; return (v % 2 ? v : v + 1) * VEC; }   // of a column's weights
   static size_t smem(int cs) {
-    return 128 + sizeof(T) * ((size_t)COLS * pitch(cs) + 2 * (size_t)cs * BLOCK + 2 * BLOCK + (size_t)BB * COLS);
+    return 128 + sizeof(T) * ((size_t)COLS * pitch(cs) + 2 * (size_t)cs * BLOCK + 2 * BLOCK + (size_t)BB * COLS * (NG == 1 ? 2 : 1));
   }
 
   T *u, *buf, *src, *res;
@@ -98,15 +103,16 @@ struct Tile {
     cluster_barrier();
   }
   // exchange e (0, 1, ...): everything in src[e & 1] goes to every CTA of the cluster, this one included.  Called by the
-  // 64 cell threads after they have written it.
+  // cell threads after they have written it.
   __device__ void send(int e) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("bar.sync 1, 64;" ::: "memory");
+    cell_sync();
     const uint32_t b = bar + 8 * (e & 1), bytes = BLOCK * sizeof(T);
-    const int r = (int)threadIdx.x - 64;
+    const int r = (int)threadIdx.x - MUL;
     if (r == 0) mbar_expect(b, (uint32_t)cs * bytes);
     if (r < cs) push(in_cta(saddr(buf + ((e & 1) * cs + rank) * BLOCK), (uint32_t)r), saddr(src + (e & 1) * BLOCK), bytes, in_cta(b, (uint32_t)r));
   }
+  __device__ void cell_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CELL) : "memory"); }
   __device__ void wait(int e, int* err) {
     if (dead) return;
     for (int i = 0; i < WAIT_LIMIT; ++i)
@@ -131,12 +137,18 @@ struct Tile {
     const T* ap = buf + (e & 1) * cs * BLOCK + (gate * BB + row0) * JP;
     const T* up = u + col0 * ps;
     constexpr int CSTEP = JP / 2;      // a thread's second column is of the same gate
+    // DEPTH - 1 groups of k are on their way from shared memory while one is multiplied (a group is 16 cycles of double
+    // arithmetic, half of what a load takes), and the products of the next k are formed before the sums of this one.  What
+    // is read behind the last block is memory that is there and never used.
     T acc[TR][TC], pr[TR][TC];
-    alignas(16) T a[2][TR][VEC], b[2][TC][VEC];
+    alignas(16) T a[DEPTH][TR][VEC], b[DEPTH][TC][VEC];
 #pragma unroll
-    for (int i = 0; i < TR; ++i) lds16(ap + i * JP, a[0][i]);
+    for (int g = 0; g < DEPTH - 1; ++g) {
 #pragma unroll
-    for (int j = 0; j < TC; ++j) lds16(up + j * CSTEP * ps, b[0][j]);
+      for (int i = 0; i < TR; ++i) lds16(ap + g * VEC + i * JP, a[g][i]);
+#pragma unroll
+      for (int j = 0; j < TC; ++j) lds16(up + g * VEC + j * CSTEP * ps, b[g][j]);
+    }
 #pragma unroll
     for (int i = 0; i < TR; ++i)
 #pragma unroll
@@ -146,14 +158,14 @@ struct Tile {
       }
     for (int p = 0; p < cs; ++p) {
 #pragma unroll
-      for (int g = 0; g < JP / VEC; ++g) {
-        const int h = g & 1;
-        // the next 16 bytes of k (after the last block: memory that is there, never used)
-        const T* an = g + 1 < JP / VEC ? ap + (g + 1) * VEC : ap + BLOCK;
+      for (int g = 0; g < G; ++g) {
+        constexpr int D1 = DEPTH - 1;
+        const T* an = g + D1 < G ? ap + (g + D1) * VEC : ap + BLOCK + (g + D1 - G) * VEC;
 #pragma unroll
-        for (int i = 0; i < TR; ++i) lds16(an + i * JP, a[h ^ 1][i]);
+        for (int i = 0; i < TR; ++i) lds16(an + i * JP, a[(g + D1) % DEPTH][i]);
 #pragma unroll
-        for (int j = 0; j < TC; ++j) lds16(up + (g + 1) * VEC + j * CSTEP * ps, b[h ^ 1][j]);
+        for (int j = 0; j < TC; ++j) lds16(up + (g + D1) * VEC + j * CSTEP * ps, b[(g + D1) % DEPTH][j]);
+        const int h = g % DEPTH, h1 = (g + 1) % DEPTH;
 #pragma unroll
         for (int kk = 0; kk < VEC; ++kk) {
           T pn[TR][TC];
@@ -161,7 +173,7 @@ struct Tile {
           for (int i = 0; i < TR; ++i)
 #pragma unroll
             for (int j = 0; j < TC; ++j)
-              pn[i][j] = kk + 1 < VEC ? mul_rn(a[h][i][kk + 1], b[h][j][kk + 1]) : mul_rn(a[h ^ 1][i][0], b[h ^ 1][j][0]);
+              pn[i][j] = kk + 1 < VEC ? mul_rn(a[h][i][kk + 1], b[h][j][kk + 1]) : mul_rn(a[h1][i][0], b[h1][j][0]);
 #pragma unroll
           for (int i = 0; i < TR; ++i)
 #pragma unroll
@@ -192,7 +204,7 @@ template <typename T> struct ForwardArgs {
 };
 
 template <typename T, int JP, int BB>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(Tile<T, JP, BB, 1>::NT)
 forward_kernel(const __grid_constant__ ForwardArgs<T> p) {
   using L = Tile<T, JP, BB, 1>;
   extern __shared__ __align__(128) unsigned char lstm_smem[];
@@ -200,50 +212,50 @@ forward_kernel(const __grid_constant__ ForwardArgs<T> p) {
   const int nh = p.nh;
   const int64_t plane = (int64_t)p.steps * p.batch * nh;
   const int kp = s.cs * JP;
-  for (int i = threadIdx.x; i < L::COLS * kp; i += NT) {     // this CTA's rows of U_g
+  for (int i = threadIdx.x; i < L::COLS * kp; i += L::NT) {     // this CTA's rows of U_g
     const int c = i / kp, k = i % kp, q = k % JP, unit = s.rank * p.jj + c % JP, kg = k / JP * p.jj + q;
     T v = (T)0;
     if (c % JP < p.jj && unit < nh && q < p.jj && kg < nh) v = p.U[((int64_t)(c / JP) * nh + unit) * nh + kg];
     s.u[c * s.ps + k] = v;
   }
   s.begin();
-  const int e = (int)threadIdx.x - 64, row = e / JP, jl = e % JP, unit = s.rank * p.jj + jl;
-  const int brow = (int)(blockIdx.x / s.cs) * BB + row;
-  const bool cell_thread = e >= 0, cell = cell_thread && row < BB && jl < p.jj && unit < nh && brow < p.batch;
-  T bias[4], c_prev = (T)0;
-  if (cell)
-#pragma unroll
-    for (int g = 0; g < 4; ++g) bias[g] = p.b[g][unit];
+  const int q = (int)threadIdx.x - L::MUL;
+  const bool cell_thread = q >= 0;
+  // as a gate thread: row q / COLS, column q % COLS
+  const int grow = q / L::COLS, gcol = q % L::COLS, gate = gcol / JP, gunit = s.rank * p.jj + gcol % JP;
+  const int tile0 = (int)(blockIdx.x / s.cs) * BB;
+  const bool gate_on = cell_thread && grow < BB && gcol % JP < p.jj && gunit < nh && tile0 + grow < p.batch;
+  // as a cell thread: row q / JP, hidden unit q % JP
+  const int row = q / JP, jl = q % JP, unit = s.rank * p.jj + jl;
+  const bool cell = cell_thread && row < BB && jl < p.jj && unit < nh && tile0 + row < p.batch;
+  const T bias = gate_on ? p.b[gate][gunit] : (T)0;
+  T* gates = s.res + BB * L::COLS;
+  T c_prev = (T)0;
 
   for (int t = 0; t < p.steps; ++t) {
-    const int64_t at = ((int64_t)t * p.batch + brow) * nh + unit;
-    T pre[4];
-    if (cell)
-#pragma unroll
-      for (int g = 0; g < 4; ++g) pre[g] = p.pre[g * plane + at];
+    const int64_t gat = ((int64_t)t * p.batch + tile0 + grow) * nh + gunit;
+    T pre = gate_on ? p.pre[gate * plane + gat] : (T)0;
     if (t > 0 && !cell_thread) {
       s.wait(t - 1, p.err);
       s.multiply(t - 1);
     }
     __syncthreads();
+    if (gate_on) {
+      if (t > 0) pre = add_rn(pre, s.res[grow * L::COLS + gcol]);
+      pre = add_rn(pre, bias);
+      p.pre[gate * plane + gat] = pre;
+      const T v = act_value<T>(gate == 2 ? PRAD_ACT_TANH : PRAD_ACT_SIGMOID, pre, (T)0);      // i, f, g, o
+      gates[grow * L::COLS + gcol] = v;
+      p.gate[gate][gat] = v;
+    }
+    if (cell_thread) s.cell_sync();
     if (cell) {
-      T v[4];
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        if (t > 0) pre[g] = add_rn(pre[g], s.res[row * L::COLS + g * JP + jl]);
-        pre[g] = add_rn(pre[g], bias[g]);
-        p.pre[g * plane + at] = pre[g];
-      }
-      v[0] = act_value<T>(PRAD_ACT_SIGMOID, pre[0], (T)0);      // i, f, g, o
-      v[1] = act_value<T>(PRAD_ACT_SIGMOID, pre[1], (T)0);
-      v[2] = act_value<T>(PRAD_ACT_TANH, pre[2], (T)0);
-      v[3] = act_value<T>(PRAD_ACT_SIGMOID, pre[3], (T)0);
-      const T ig = mul_rn(v[0], v[2]), fc = t > 0 ? mul_rn(v[1], c_prev) : (T)0;
-      const T c = add_rn(fc, ig), tc = act_value<T>(PRAD_ACT_TANH, c, (T)0), h = mul_rn(v[3], tc);
+      const int64_t at = ((int64_t)t * p.batch + tile0 + row) * nh + unit;
+      const T* v = gates + row * L::COLS + jl;
+      const T ig = mul_rn(v[0], v[2 * JP]), fc = t > 0 ? mul_rn(v[JP], c_prev) : (T)0;
+      const T c = add_rn(fc, ig), tc = act_value<T>(PRAD_ACT_TANH, c, (T)0), h = mul_rn(v[3 * JP], tc);
       c_prev = c;
       s.src[(t & 1) * L::BLOCK + row * JP + jl] = h;
-#pragma unroll
-      for (int g = 0; g < 4; ++g) p.gate[g][at] = v[g];
       p.IG[at] = ig;
       p.FC[at] = fc;
       p.C[at] = c;
@@ -268,7 +280,7 @@ template <typename T> struct BackwardArgs {
 };
 
 template <typename T, int JP, int BB>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(Tile<T, JP, BB, 4>::NT)
 backward_kernel(const __grid_constant__ BackwardArgs<T> p) {
   using L = Tile<T, JP, BB, 4>;
   extern __shared__ __align__(128) unsigned char lstm_smem[];
@@ -276,14 +288,14 @@ backward_kernel(const __grid_constant__ BackwardArgs<T> p) {
   const int nh = p.nh;
   const int64_t plane = (int64_t)p.steps * p.batch * nh;
   const int kp = s.cs * JP;
-  for (int i = threadIdx.x; i < L::COLS * kp; i += NT) {     // this CTA's columns of U_g; neighbouring threads: neighbouring columns
+  for (int i = threadIdx.x; i < L::COLS * kp; i += L::NT) {     // this CTA's columns of U_g; neighbouring threads: neighbouring columns
     const int jl = i % JP, k = i / JP % kp, g = i / (JP * kp), q = k % JP, unit = s.rank * p.jj + jl, kg = k / JP * p.jj + q;
     T v = (T)0;
     if (jl < p.jj && unit < nh && q < p.jj && kg < nh) v = p.U[((int64_t)g * nh + kg) * nh + unit];
     s.u[(g * JP + jl) * s.ps + k] = v;
   }
   s.begin();
-  const int e = (int)threadIdx.x - 64, row = e / JP, jl = e % JP, unit = s.rank * p.jj + jl;
+  const int e = (int)threadIdx.x - L::MUL, row = e / JP, jl = e % JP, unit = s.rank * p.jj + jl;
   const int brow = (int)(blockIdx.x / s.cs) * BB + row;
   const bool cell_thread = e >= 0, cell = cell_thread && row < BB && jl < p.jj && unit < nh && brow < p.batch;
   T dc_next = (T)0;
@@ -349,7 +361,7 @@ template <typename T> static Plan plan_of(int nh) {
 }
 
 // Clusters of this kernel that fit the device at once; 0 if none does.  Asked once per kernel, cluster size and device.
-template <auto Kernel> static int clusters_at_once(prad_ctx* ctx, int cs, size_t smem) {
+template <auto Kernel> static int clusters_at_once(prad_ctx* ctx, int cs, int nt, size_t smem) {
   static std::atomic<int> known[64][5];
   int lg = 0;
   while ((1 << lg) < cs) ++lg;
@@ -366,7 +378,7 @@ template <auto Kernel> static int clusters_at_once(prad_ctx* ctx, int cs, size_t
     at[0].val.clusterDim.x = cs;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)cs);
-    cfg.blockDim = dim3(NT);
+    cfg.blockDim = dim3((unsigned)nt);
     cfg.dynamicSmemBytes = smem;
     cfg.attrs = at;
     cfg.numAttrs = 1;
@@ -378,14 +390,14 @@ template <auto Kernel> static int clusters_at_once(prad_ctx* ctx, int cs, size_t
 }
 
 template <auto Kernel, typename Args>
-static prad_status launch(prad_ctx* ctx, int cs, size_t smem, int tiles, const Args& args) {
+static prad_status launch(prad_ctx* ctx, int cs, int nt, size_t smem, int tiles, const Args& args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = cs;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3((unsigned)(cs * tiles));
-  cfg.blockDim = dim3(NT);
+  cfg.blockDim = dim3((unsigned)nt);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
   cfg.attrs = at;
@@ -396,29 +408,49 @@ static prad_status launch(prad_ctx* ctx, int cs, size_t smem, int tiles, const A
   return PRAD_OK;
 }
 
-// The smallest batch tile with which all clusters run at once (a step takes the same time for one row as for four);
-// more than four rows per cluster would not fit next to the weights, larger batches run in turns, as many as one launch per
-// operation would cost.  PRAD_ERR_UNSUPPORTED: too many turns, or too many hidden units for a cluster's shared memory.
+// The batch tile.  A step takes a cluster little longer for four rows than for one (double, 256 units: 3.5 .. 5.7 us), and a
+// B200 runs 7 clusters of 16 at once, 15 of 8: so the smallest tile
+// with which all clusters run at once -- five rows exist for a batch of 29 .. 35 on those 7 -- or else five or four rows in the
+// fewest turns.  PRAD_ERR_UNSUPPORTED: more turns than one launch per operation is worth, or too many hidden units for a
+// cluster's shared memory.
 constexpr int MAX_TURNS = 8;
 template <typename T, bool FORWARD, int JP, typename Args>
 static prad_status run_jp(prad_ctx* ctx, const Plan& pl, Args& a) {
   constexpr int NG = FORWARD ? 1 : 4;
   const int B = a.batch;
   a.jj = pl.jj;
-#define PRAD_LSTM_TRY(BB_)                                                                                             \
+  int rows = 0, turns = 0;
+#define PRAD_LSTM_TILE(BB_, DO)                                                                                        \
   do {                                                                                                                 \
     constexpr auto K = [] {                                                                                            \
       if constexpr (FORWARD) return &forward_kernel<T, JP, BB_>;                                                       \
       else return &backward_kernel<T, JP, BB_>;                                                                        \
     }();                                                                                                               \
-    const size_t smem = Tile<T, JP, BB_, NG>::smem(pl.cs);                                                             \
-    const int tiles = (int)ceil_div(B, BB_), fit = smem <= 227 * 1024 ? clusters_at_once<K>(ctx, pl.cs, smem) : 0;     \
-    if (fit > 0 && (tiles <= fit || (BB_ == 4 && tiles <= MAX_TURNS * fit))) return launch<K>(ctx, pl.cs, smem, tiles, a);                           \
+    using L = Tile<T, JP, BB_, NG>;                                                                                    \
+    const size_t smem = L::smem(pl.cs);                                                                                \
+    const int tiles = (int)ceil_div(B, BB_);                                                                           \
+    DO;                                                                                                                \
   } while (0)
-  PRAD_LSTM_TRY(1);
-  PRAD_LSTM_TRY(2);
-  PRAD_LSTM_TRY(4);
-#undef PRAD_LSTM_TRY
+#define PRAD_LSTM_WEIGH(BB_)                                                                                           \
+  PRAD_LSTM_TILE(BB_, {                                                                                                \
+    const int fit = smem <= 227 * 1024 ? clusters_at_once<K>(ctx, pl.cs, L::NT, smem) : 0;                             \
+    const int n = fit > 0 ? (int)ceil_div(tiles, fit) : 0;                                                             \
+    if (n && (!turns || n < turns)) { turns = n; rows = BB_; }                                                         \
+  })
+#define PRAD_LSTM_RUN(BB_) \
+  PRAD_LSTM_TILE(BB_, if (rows == BB_) return launch<K>(ctx, pl.cs, L::NT, smem, tiles, a))
+  PRAD_LSTM_WEIGH(1);
+  PRAD_LSTM_WEIGH(2);
+  PRAD_LSTM_WEIGH(4);
+  PRAD_LSTM_WEIGH(5);
+  if (!turns || turns > MAX_TURNS) return PRAD_ERR_UNSUPPORTED;
+  PRAD_LSTM_RUN(1);
+  PRAD_LSTM_RUN(2);
+  PRAD_LSTM_RUN(4);
+  PRAD_LSTM_RUN(5);
+#undef PRAD_LSTM_RUN
+#undef PRAD_LSTM_WEIGH
+#undef PRAD_LSTM_TILE
   return PRAD_ERR_UNSUPPORTED;
 }
 
