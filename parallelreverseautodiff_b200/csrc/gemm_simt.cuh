@@ -43,10 +43,10 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // One operand's ROWS x BK tile in shared memory.  KC: k is contiguous in memory, layout [row][k]; otherwise [k][row].
-template <typename T, int ROWS, int BK, int NT, bool KC>
+template <typename T, int ROWS, int BK, int NT, bool KC, int PAD = 16 / sizeof(T)>
 struct OperandTile {
   static constexpr int VEC = 16 / sizeof(T);
-  static constexpr int PITCH = (KC ? BK : ROWS) + VEC;
+  static constexpr int PITCH = (KC ? BK : ROWS) + PAD;
   static constexpr int FAST = KC ? BK : ROWS, SLOW = KC ? ROWS : BK;
   static constexpr int SIZE = SLOW * PITCH;
 

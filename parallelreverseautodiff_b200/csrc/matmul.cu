@@ -38,6 +38,9 @@ static bool wants_tensor_cores(prad_ctx* ctx, prad_dtype dt, bool tA, bool tB, i
          gemm_f64_dmma(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, true) == PRAD_OK;
 }
 
+prad_status gemm_f64_dmma_backward(prad_ctx* ctx, const void* A, const void* B, const void* dC, void* dA, void* dB, int M, int K, int N,
+                                   bool accumulate_dB, double dB_scale, const GemmEpilogue& e_dA);
+
 prad_status gemm_dispatch(prad_ctx* ctx, prad_dtype dt, bool tA, bool tB, int M, int N, int K,
                           double alpha, const void* A, int lda, const void* B, int ldb,
                           double beta, void* C, int ldc, int batch, int64_t sA, int64_t sB,
@@ -109,13 +112,19 @@ static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void
   e_dA.saved = saved_below;
   e_dA.act_alpha = act_alpha;
   // dA (MxK) = dC (MxN) * B^T  (B is KxN) ; dB (KxN) = A^T (A is MxK) * dC (MxN)
-  if (dA && dB && M > 0 && K > 0 && N > 0 &&
-      !wants_tensor_cores(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA) &&
-      !wants_tensor_cores(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0, 0, 0, e_dB))
+  const bool both = dA && dB && M > 0 && K > 0 && N > 0;
+  const bool tc_A = both && wants_tensor_cores(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA);
+  const bool tc_B = both && wants_tensor_cores(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0,
+                                               0, 0, e_dB);
+  if (both && !tc_A && !tc_B)
     return dt == PRAD_F32 ? gemm_simt_backward<float>(ctx, ctx->gemm_f32 != GemmF32::SimtFma, A, B, dC, dA, dB, M, K, N,
                                                       accumulate_dB != 0, dB_scale, e_dA)
                           : gemm_simt_backward<double>(ctx, ctx->gemm_f64 != GemmF64::SimtFma, A, B, dC, dA, dB, M, K, N,
                                                        accumulate_dB != 0, dB_scale, e_dA);
+  // one launch where neither would be cut into k slices
+  if (both && tc_A && tc_B && dt == PRAD_F64 &&
+      (ceil_div(M, 64) * ceil_div(K, 64) * 2 > ctx->sm_count || N < 512) && (ceil_div(K, 64) * ceil_div(N, 64) * 2 > ctx->sm_count || M < 512))
+    return gemm_f64_dmma_backward(ctx, A, B, dC, dA, dB, M, K, N, accumulate_dB != 0, dB_scale, e_dA);
   if (dA) {
     s = gemm_dispatch(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA);
     if (s) return s;
