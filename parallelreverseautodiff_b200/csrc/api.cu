@@ -95,6 +95,7 @@ prad_status prad_init(int device, prad_ctx** out_ctx) {
   c->stream = c->own_stream;
   e = cudaMalloc((void**)&c->tc_err, 256);
   if (e == cudaSuccess) e = cudaMemset(c->tc_err, 0, 256);
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->host_flag, 64);
   if (e != cudaSuccess) {
     set_error("prad_init: flag allocation: %s", cudaGetErrorString(e));
     cudaStreamDestroy(c->own_stream);
@@ -114,6 +115,7 @@ prad_status prad_shutdown(prad_ctx* ctx) {
   pool_destroy(ctx);
   if (ctx->ws) cudaFree(ctx->ws);
   if (ctx->tc_err) cudaFree(ctx->tc_err);
+  if (ctx->host_flag) cudaFreeHost(ctx->host_flag);
   for (void* r : ctx->retired) cudaFree(r);
   if (ctx->stage) cudaFree(ctx->stage);
   if (ctx->host_ws) cudaFreeHost(ctx->host_ws);

@@ -46,6 +46,7 @@ struct prad_ctx {
   prad::DpState* dp = nullptr;
   prad::DevicePool* pool = nullptr;
   size_t total_mem = 0;               // device memory in bytes
+  int* host_flag = nullptr;   // page-locked int that kernels write and the host reads after a wait
   // give-up flag of the tensor-core GEMMs (device int, sticky until the host reads it)
   int* tc_err = nullptr;
   bool tc_pending_check = false;
@@ -164,7 +165,7 @@ inline int stream_grid(const prad_ctx* ctx, int64_t work_items, int per_block, i
 // Lets `Kernel` use `bytes` of dynamic shared memory on the context's device (needed above 48 KB): asked for once per
 // kernel and device.
 template <auto Kernel> inline prad_status allow_smem(prad_ctx* ctx, int bytes) {
-  if (bytes <= 48 * 1024) return PRAD_OK;
+  if (bytes <= 32 * 1024) return PRAD_OK;     // (48 KB less what a kernel declares itself)
   static std::atomic<uint64_t> done{0};
   const uint64_t bit = 1ull << (ctx->device & 63);
   if (!(done.load(std::memory_order_acquire) & bit)) {
@@ -194,7 +195,7 @@ prad_status gemm_dispatch(prad_ctx* ctx, prad_dtype dt, bool transA, bool transB
                           double beta, void* C, int ldc, int batch, int64_t sA, int64_t sB,
                           int64_t sC, const GemmEpilogue& epi);
 
-// dW[idx[i]][:] += dOut[i][:] for i ascending (bit-identical to the sequential loop); loss_embedding.cu
+// dW[idx[i]][:] += dOut[i][:] for i ascending (bit-identical to the sequential loop); embedding.cu
 prad_status embedding_scatter_ordered(prad_ctx* ctx, prad_dtype dt, const void* index_col, const void* dOut,
                                       void* dW, int n, int vocab, int dim, int* bad);
 

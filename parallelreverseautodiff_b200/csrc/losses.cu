@@ -1,5 +1,5 @@
-// Loss values and loss gradients (MSE, categorical cross-entropy) and the embedding
-// gather / ordered scatter-add.  (Compiled with -fmad=false.)
+// Loss values and loss gradients (MSE, categorical cross-entropy), Swish, SwigLU and BatchNormalization.
+// (Compiled with -fmad=false.)
 #include "act_math.cuh"
 #include "common.cuh"
 #include "reduce.cuh"
@@ -14,6 +14,13 @@ constexpr int LOSS_THREADS = 256;
 
 // kind 0: MSE term (o-t)^2 (MeanSquaredErrorLossOperation.cs:50-55)
 // kind 1: CCE term -t*log(o+eps) (CategoricalCrossEntropyLossOperation.cs:53-59)
+template <typename T> __device__ __forceinline__ T loss_term(T o, T t, int kind) {
+  if (kind == 0) {
+    const T d = sub_rn(o, t);
+    return mul_rn(d, d);
+  }
+  return mul_rn(-t, t_log(add_rn(o, Eps15<T>::v())));
+}
 template <typename T>
 __global__ void __launch_bounds__(LOSS_THREADS)
 loss_partial_kernel(const T* __restrict__ o, const T* __restrict__ t, double* __restrict__ partial,
@@ -21,17 +28,20 @@ loss_partial_kernel(const T* __restrict__ o, const T* __restrict__ t, double* __
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   double acc = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    T term;
-    if (kind == 0) {
-      T d = sub_rn(o[i], t[i]);
-      term = mul_rn(d, d);
-    } else {
-      term = mul_rn(-t[i], t_log(add_rn(o[i], Eps15<T>::v())));
-    }
-    acc += (double)term;
+    acc += (double)loss_term<T>(o[i], t[i], kind);
   }
   double s = block_sum_d<LOSS_THREADS>(acc);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+// A small loss in one launch: one CTA adds every term.
+constexpr int LOSS_SMALL_THREADS = 1024, LOSS_SMALL = 16 * LOSS_SMALL_THREADS;
+template <typename T>
+__global__ void __launch_bounds__(LOSS_SMALL_THREADS)
+loss_small_kernel(const T* __restrict__ o, const T* __restrict__ t, T* loss, int n, int kind, T divisor) {
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < n; i += LOSS_SMALL_THREADS) acc += (double)loss_term<T>(o[i], t[i], kind);
+  const double s = block_sum_d<LOSS_SMALL_THREADS>(acc);
+  if (threadIdx.x == 0) loss[0] = div_rn((T)s, divisor);
 }
 template <typename T>
 __global__ void loss_final_kernel(const double* __restrict__ partial, int nblocks, T* loss,
@@ -66,13 +76,18 @@ template <typename T>
 static prad_status loss_forward_t(prad_ctx* ctx, const void* o, const void* t, void* loss,
                                   int64_t rows, int cols, int kind) {
   int64_t n = rows * cols;
+  const T divisor = kind == 0 ? (T)(rows * cols) : (T)rows;
+  if (n <= LOSS_SMALL) {
+    loss_small_kernel<T><<<1, LOSS_SMALL_THREADS, 0, ctx->stream>>>((const T*)o, (const T*)t, (T*)loss, (int)n, kind, divisor);
+    PRAD_LAUNCHED(ctx);
+    return PRAD_OK;
+  }
   int grid = stream_grid(ctx, n, LOSS_THREADS * 4, 4);
   prad_status s = ensure_workspace(ctx, (size_t)grid * sizeof(double));
   if (s) return s;
   loss_partial_kernel<T><<<grid, LOSS_THREADS, 0, ctx->stream>>>((const T*)o, (const T*)t,
                                                                   (double*)ctx->ws, n, kind);
   PRAD_LAUNCHED(ctx);
-  T divisor = kind == 0 ? (T)(rows * cols) : (T)rows;
   loss_final_kernel<T><<<1, 32, 0, ctx->stream>>>((const double*)ctx->ws, grid, (T*)loss, divisor);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
@@ -256,192 +271,6 @@ bn_backward_kernel(const T* __restrict__ x, const double* __restrict__ stats, co
   }
 }
 
-// ---------------------------------------------------------------- embedding
-// EmbeddingOperation.cs:56-60: out[i] = W[(int)input[i,0]]
-template <typename T>
-__global__ void __launch_bounds__(256)
-embedding_gather_kernel(const T* __restrict__ index_col, const T* __restrict__ W,
-                        T* __restrict__ out, int n, int vocab, int dim, int* __restrict__ bad) {
-  for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    int idx = (int)index_col[i];
-    if (idx < 0 || idx >= vocab) {  // the managed code would throw IndexOutOfRange
-      if (threadIdx.x == 0) atomicExch(bad, i + 1);
-      continue;
-    }
-    for (int j = threadIdx.x; j < dim; j += blockDim.x)
-      out[(int64_t)i * dim + j] = W[(int64_t)idx * dim + j];
-  }
-}
-
-// EmbeddingOperation.cs:69-76: dW[idx[i]][j] += dOut[i][j] for i = 0..n-1 IN THAT ORDER.
-// Vocabulary rows are dealt to CTAs round-robin.  A CTA scans the index column in tiles,
-// compacts (stably) the positions whose row it owns, and adds those rows of dOut one after
-// the other; column j is always handled by the same thread, so every dW element sees its
-// contributions in input-row order and the sum is bit-identical to the sequential loop.
-// No floating-point atomics anywhere.
-template <typename T> struct EmbVec;
-template <> struct EmbVec<float> { using type = float4; static constexpr int N = 4; };
-template <> struct EmbVec<double> { using type = double2; static constexpr int N = 2; };
-
-constexpr int EMB_THREADS = 256;
-constexpr int EMB_ITEMS = 4;
-constexpr int EMB_TILE = EMB_THREADS * EMB_ITEMS;
-constexpr int EMB_CAP = 2048;       // positions a CTA keeps in shared memory before it falls back to adding in place
-
-// One tile of the index list: the positions whose vocabulary row this CTA owns (row % B == b), appended to
-// `list` in input order (thread order == element order).  Returns how many; all threads get the same count.
-template <typename T>
-__device__ __forceinline__ int emb_compact_tile(const T* __restrict__ index_col, int tile, int n, int vocab, int B, int b,
-                                                int* list, int cap_left, int* warp_cnt, int* tile_cnt, int* bad) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int mine[EMB_ITEMS];
-  int c = 0;
-#pragma unroll
-  for (int q = 0; q < EMB_ITEMS; ++q) {
-    const int i = tile + threadIdx.x * EMB_ITEMS + q;
-    mine[q] = -1;
-    if (i < n) {
-      const int idx = (int)index_col[i];
-      if (idx < 0 || idx >= vocab) {
-        if (b == 0) atomicExch(bad, i + 1);
-      } else if (idx % B == b) {
-        mine[q] = i;
-        ++c;
-      }
-    }
-  }
-  int incl = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += u;
-  }
-  if (lane == 31) warp_cnt[w] = incl;
-  __syncthreads();
-  int base = 0;
-  for (int k = 0; k < w; ++k) base += warp_cnt[k];
-  if (threadIdx.x == EMB_THREADS - 1) *tile_cnt = base + incl;
-  int pos = base + incl - c;
-#pragma unroll
-  for (int q = 0; q < EMB_ITEMS; ++q)
-    if (mine[q] >= 0) {
-      if (pos < cap_left) list[pos] = mine[q];
-      ++pos;
-    }
-  __syncthreads();
-  return *tile_cnt;
-}
-
-// dW[idx[i]] += dOut[i] for i ascending (EmbeddingOperation.cs:70-86), without float atomics: vocabulary rows are
-// dealt to the CTAs round-robin and a CTA adds the rows of dOut that hit one of its rows in input order.
-// Usual case: all positions a CTA owns fit in shared memory; then every owned row is summed in registers and
-// written exactly once (rows nobody hit are written as zeros), so dOut is read once and the table written once.
-// Otherwise (more than EMB_CAP hits on one CTA's rows) the CTA zeroes its rows and adds tile by tile in place.
-template <typename T>
-__global__ void __launch_bounds__(EMB_THREADS)
-embedding_scatter_ordered_kernel(const T* __restrict__ index_col, const T* __restrict__ dOut,
-                                 T* __restrict__ dW, int n, int vocab, int dim,
-                                 int* __restrict__ bad) {
-  __shared__ int list[EMB_CAP];
-  __shared__ int match[EMB_CAP];
-  __shared__ int warp_cnt[EMB_THREADS / 32];
-  __shared__ int tile_cnt, match_cnt;
-  const int B = gridDim.x, b = blockIdx.x;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-
-  // ---- collect the owned positions
-  int total = 0;
-  bool fits = true;
-  for (int tile = 0; tile < n && fits; tile += EMB_TILE) {
-    const int cnt = emb_compact_tile<T>(index_col, tile, n, vocab, B, b, list + total, EMB_CAP - total, warp_cnt, &tile_cnt, bad);
-    if (total + cnt > EMB_CAP) fits = false;
-    else total += cnt;
-    __syncthreads();
-  }
-
-  if (fits) {
-    using V = typename EmbVec<T>::type;
-    constexpr int VEC = EmbVec<T>::N;
-    const bool vec = dim % VEC == 0 && (((uintptr_t)dOut | (uintptr_t)dW) & 15) == 0;
-    for (int v = b; v < vocab; v += B) {
-      // positions that hit row v, in input order (warp 0: ordered compaction of 32 list entries per trip)
-      if (w == 0) {
-        int mc = 0;
-        for (int e0 = 0; e0 < total; e0 += 32) {
-          const int e = e0 + lane;
-          const int i = e < total ? list[e] : -1;
-          const bool hit = i >= 0 && (int)index_col[i] == v;
-          const unsigned m = __ballot_sync(0xffffffffu, hit);
-          if (hit) match[mc + __popc(m & ((1u << lane) - 1u))] = i;
-          mc += __popc(m);
-        }
-        if (lane == 0) match_cnt = mc;
-      }
-      __syncthreads();
-      const int mc = match_cnt;
-      T* row = dW + (int64_t)v * dim;
-      if (vec) {
-        for (int j = threadIdx.x; j < dim / VEC; j += EMB_THREADS) {
-          T acc[VEC];
-#pragma unroll
-          for (int q = 0; q < VEC; ++q) acc[q] = (T)0;
-          for (int k = 0; k < mc; ++k) {
-            const V x = __ldcs(reinterpret_cast<const V*>(dOut + (int64_t)match[k] * dim) + j);
-#pragma unroll
-            for (int q = 0; q < VEC; ++q) acc[q] = add_rn(acc[q], reinterpret_cast<const T*>(&x)[q]);
-          }
-          __stcs(reinterpret_cast<V*>(row) + j, *reinterpret_cast<const V*>(acc));
-        }
-      } else {
-        for (int j = threadIdx.x; j < dim; j += EMB_THREADS) {
-          T acc = (T)0;
-          for (int k = 0; k < mc; ++k) acc = add_rn(acc, dOut[(int64_t)match[k] * dim + j]);
-          row[j] = acc;
-        }
-      }
-      __syncthreads();
-    }
-    return;
-  }
-
-  // ---- more hits than the list holds: zero the owned rows, then add tile by tile in place
-  for (int v = b; v < vocab; v += B)
-    for (int j = threadIdx.x; j < dim; j += EMB_THREADS) dW[(int64_t)v * dim + j] = (T)0;
-  __syncthreads();
-  for (int tile = 0; tile < n; tile += EMB_TILE) {
-    const int cnt = emb_compact_tile<T>(index_col, tile, n, vocab, B, b, list, EMB_CAP, warp_cnt, &tile_cnt, bad);
-    for (int e = 0; e < cnt; ++e) {
-      const int i = list[e];
-      const int idx = (int)index_col[i];
-      for (int j = threadIdx.x; j < dim; j += EMB_THREADS) {
-        const int64_t o = (int64_t)idx * dim + j;
-        dW[o] = add_rn(dW[o], dOut[(int64_t)i * dim + j]);
-      }
-    }
-    __syncthreads();
-  }
-}
-
-static prad_status check_bad_index(prad_ctx* ctx, int* d_bad, const char* who) {
-  PRAD_NOT_CAPTURING(ctx, who);   // the index check reads a flag back
-  int h = 0;
-  PRAD_CUDA(cudaMemcpyAsync(&h, d_bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
-  PRAD_REQUIRE(h == 0, PRAD_ERR_INVALID, "%s: index at input row %d is outside [0, vocab)", who, h - 1);
-  return PRAD_OK;
-}
-
-// Ordered scatter-add for other translation units (the PRAD Tensor gather reverse): dW[idx[i]] += dOut[i]
-// for i ascending; `bad` is a device int that receives 1 + the first offending position.
-prad_status embedding_scatter_ordered(prad_ctx* ctx, prad_dtype dt, const void* index_col, const void* dOut,
-                                      void* dW, int n, int vocab, int dim, int* bad) {
-  int grid = vocab < ctx->sm_count * 8 ? vocab : ctx->sm_count * 8;
-  if (dt == PRAD_F32) embedding_scatter_ordered_kernel<float><<<grid, EMB_THREADS, 0, ctx->stream>>>((const float*)index_col, (const float*)dOut, (float*)dW, n, vocab, dim, bad);
-  else embedding_scatter_ordered_kernel<double><<<grid, EMB_THREADS, 0, ctx->stream>>>((const double*)index_col, (const double*)dOut, (double*)dW, n, vocab, dim, bad);
-  PRAD_LAUNCHED(ctx);
-  return PRAD_OK;
-}
-
 }  // namespace prad
 
 using namespace prad;
@@ -498,43 +327,6 @@ prad_status prad_cce_backward(prad_ctx* ctx, prad_dtype dt, const void* out, con
     cce_backward_kernel<double><<<grid, 256, 0, ctx->stream>>>((const double*)out, (const double*)target, (double*)grad, n, 1.0 / (double)rows_total);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
-}
-
-prad_status prad_embedding_forward(prad_ctx* ctx, prad_dtype dt, const void* index_col,
-                                   const void* W, void* out, int n, int vocab, int dim) {
-  PRAD_CHECK_CTX(ctx);
-  PRAD_REQUIRE(dtype_ok(dt) && n >= 0 && vocab >= 0 && dim >= 0, PRAD_ERR_INVALID,
-               "prad_embedding_forward: bad argument");
-  if (n == 0 || dim == 0) return PRAD_OK;
-  PRAD_REQUIRE(index_col && W && out, PRAD_ERR_INVALID, "prad_embedding_forward: null pointer");
-  prad_status s = ensure_workspace(ctx, 256);
-  if (s) return s;
-  int* bad = (int*)ctx->ws;
-  PRAD_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
-  int grid = stream_grid(ctx, n, 1, 8);
-  if (dt == PRAD_F32) embedding_gather_kernel<float><<<grid, 256, 0, ctx->stream>>>((const float*)index_col, (const float*)W, (float*)out, n, vocab, dim, bad);
-  else embedding_gather_kernel<double><<<grid, 256, 0, ctx->stream>>>((const double*)index_col, (const double*)W, (double*)out, n, vocab, dim, bad);
-  PRAD_LAUNCHED(ctx);
-  return check_bad_index(ctx, bad, "prad_embedding_forward");
-}
-
-prad_status prad_embedding_backward(prad_ctx* ctx, prad_dtype dt, const void* index_col,
-                                    const void* dOut, void* dW, int n, int vocab, int dim) {
-  PRAD_CHECK_CTX(ctx);
-  PRAD_REQUIRE(dtype_ok(dt) && n >= 0 && vocab >= 0 && dim >= 0, PRAD_ERR_INVALID,
-               "prad_embedding_backward: bad argument");
-  if (vocab == 0 || dim == 0) return PRAD_OK;
-  PRAD_REQUIRE(dW && (n == 0 || (index_col && dOut)), PRAD_ERR_INVALID,
-               "prad_embedding_backward: null pointer");
-  prad_status s = ensure_workspace(ctx, 256);
-  if (s) return s;
-  int* bad = (int*)ctx->ws;
-  PRAD_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
-  int grid = vocab < ctx->sm_count * 8 ? vocab : ctx->sm_count * 8;
-  if (dt == PRAD_F32) embedding_scatter_ordered_kernel<float><<<grid, EMB_THREADS, 0, ctx->stream>>>((const float*)index_col, (const float*)dOut, (float*)dW, n, vocab, dim, bad);
-  else embedding_scatter_ordered_kernel<double><<<grid, EMB_THREADS, 0, ctx->stream>>>((const double*)index_col, (const double*)dOut, (double*)dW, n, vocab, dim, bad);
-  PRAD_LAUNCHED(ctx);
-  return check_bad_index(ctx, bad, "prad_embedding_backward");
 }
 
 prad_status prad_swish_forward(prad_ctx* ctx, prad_dtype dt, const void* x, const void* beta, void* y, int64_t n) {

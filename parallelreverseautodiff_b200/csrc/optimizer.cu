@@ -12,7 +12,11 @@ namespace prad {
 
 constexpr int MT_MAX = 48;          // tensors per launch (table is a kernel argument)
 constexpr int MT_THREADS = 256;
-constexpr int MT_CHUNK = 256 * 32;  // elements a CTA covers
+constexpr int MT_CHUNK = 256 * 32;  // most elements a CTA covers
+// A CTA covers fewer where that many would leave SMs idle: an MLP's 670 000 parameters are 82 chunks of 8192, and a double
+// network's 46 000 are 12 of them (45 us for the update alone, one division and one square root after another), now 4
+// elements per thread at the least in float, 2 in double.
+constexpr int MT_FOLD = 256;        // partial sums a CTA adds up by itself instead of leaving them to a launch in between
 
 template <typename T> struct MtVec;
 template <> struct MtVec<float> { using type = float4; };
@@ -27,6 +31,8 @@ struct MultiTensor {
   int64_t size[MT_MAX];
   int blk_start[MT_MAX + 1];
   int count;
+  int chunk;  // elements a CTA covers, a multiple of MT_THREADS 16-byte vectors
+  bool fold;  // few partial sums per tensor: every CTA adds them up itself, in the order of mt_finalize_kernel
 };
 
 __device__ __forceinline__ int find_tensor(const MultiTensor& t, int blk) {
@@ -42,17 +48,30 @@ __device__ __forceinline__ int find_tensor(const MultiTensor& t, int blk) {
 // [2*MT_MAX] global sum of squares, then the per-CTA partials.
 constexpr int ST_MEAN = 0, ST_STD = MT_MAX, ST_SS = 2 * MT_MAX, ST_PART = 2 * MT_MAX + 8;
 
+// Sum of a tensor's partial sums, in CTA order by a fixed tree; all threads get it.
+__device__ __forceinline__ double add_partials(const MultiTensor& t, int ti, const double* part) {
+  double acc = 0.0;
+  for (int b = t.blk_start[ti] + threadIdx.x; b < t.blk_start[ti + 1]; b += MT_THREADS) acc += part[b];
+  return block_sum_d<MT_THREADS>(acc);
+}
+template <typename T> __device__ __forceinline__ T mean_of(double s, int64_t size) { return div_rn((T)s, (T)size); }            // sum / count
+template <typename T> __device__ __forceinline__ T sigma_of(double s, int64_t size) { return sqrt_rn(div_rn((T)s, (T)size)); }  // Sqrt(varianceSum / count)
+
+// The partial sums of kind 1 follow those of kind 0 (the other kinds use the first place).
+__device__ __forceinline__ int part_at(const MultiTensor& t, int kind) { return ST_PART + (kind == 1 ? t.blk_start[t.count] : 0); }
+
 // pass kinds: 0 = sum g ; 1 = sum (g-mean)^2 (T arithmetic for the square, as Pow(v-mean,2)
 // rounds to T in the float build) ; 2 = sum g^2 in double (global norm)
 template <typename T>
 __global__ void __launch_bounds__(MT_THREADS)
 mt_partial_kernel(MultiTensor t, double* __restrict__ stats, int kind) {
   const int ti = find_tensor(t, blockIdx.x);
-  const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * MT_CHUNK;
-  int64_t end = start + MT_CHUNK;
+  const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
+  int64_t end = start + t.chunk;
   if (end > t.size[ti]) end = t.size[ti];
   const T* g = (const T*)t.g[ti];
-  const T mean = kind == 1 ? (T)stats[ST_MEAN + ti] : (T)0;
+  T mean = (T)0;
+  if (kind == 1) mean = t.fold ? mean_of<T>(add_partials(t, ti, stats + ST_PART), t.size[ti]) : (T)stats[ST_MEAN + ti];
   double acc = 0.0;
   auto term = [&](T x) {
     if (kind == 0) acc += (double)x;
@@ -73,7 +92,7 @@ mt_partial_kernel(MultiTensor t, double* __restrict__ stats, int kind) {
   }
   for (int64_t i = i0 + threadIdx.x; i < end; i += MT_THREADS) term(g[i]);
   double s = block_sum_d<MT_THREADS>(acc);
-  if (threadIdx.x == 0) stats[ST_PART + blockIdx.x] = s;
+  if (threadIdx.x == 0) stats[part_at(t, kind) + blockIdx.x] = s;
 }
 
 // one CTA per tensor adds that tensor's partials in CTA order (fixed tree)
@@ -81,14 +100,10 @@ template <typename T>
 __global__ void __launch_bounds__(MT_THREADS)
 mt_finalize_kernel(MultiTensor t, double* __restrict__ stats, int kind) {
   const int ti = blockIdx.x;
-  double acc = 0.0;
-  for (int b = t.blk_start[ti] + threadIdx.x; b < t.blk_start[ti + 1]; b += MT_THREADS)
-    acc += stats[ST_PART + b];
-  double s = block_sum_d<MT_THREADS>(acc);
+  const double s = add_partials(t, ti, stats + part_at(t, kind));
   if (threadIdx.x == 0) {
-    const T n = (T)t.size[ti];
-    if (kind == 0) stats[ST_MEAN + ti] = (double)div_rn((T)s, n);           // mean = sum / count
-    else stats[ST_STD + ti] = (double)sqrt_rn(div_rn((T)s, n));             // Sqrt(varianceSum / count)
+    if (kind == 0) stats[ST_MEAN + ti] = (double)mean_of<T>(s, t.size[ti]);
+    else stats[ST_STD + ti] = (double)sigma_of<T>(s, t.size[ti]);
   }
 }
 // global norm: every partial of every tensor, one CTA
@@ -159,8 +174,8 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
   // host learns of it at its next prad_sync / prad_download, which returns PRAD_ERR_TIMEOUT).
   if (gemm_gave_up && *gemm_gave_up != 0) return;
   const int ti = find_tensor(t, blockIdx.x);
-  const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * MT_CHUNK;
-  int64_t end = start + MT_CHUNK;
+  const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
+  int64_t end = start + t.chunk;
   if (end > t.size[ti]) end = t.size[ti];
   T* g = (T*)t.g[ti];
   T* w = (T*)t.w[ti];
@@ -168,7 +183,15 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
   T* v = (T*)t.v[ti];
   T mean = 0, sd = 1, gscale = 1;
   bool scale_on = false;
-  if (clip_mode == 1) { mean = (T)stats[ST_MEAN + ti]; sd = (T)stats[ST_STD + ti]; }
+  if (clip_mode == 1) {
+    if (t.fold) {
+      mean = mean_of<T>(add_partials(t, ti, stats + ST_PART), t.size[ti]);
+      sd = sigma_of<T>(add_partials(t, ti, stats + part_at(t, 1)), t.size[ti]);
+    } else {
+      mean = (T)stats[ST_MEAN + ti];
+      sd = (T)stats[ST_STD + ti];
+    }
+  }
   if (clip_mode == 2) {
     double norm = sqrt(stats[ST_SS]);
     if (norm > max_norm) { gscale = (T)(max_norm / norm); scale_on = true; }
@@ -241,9 +264,16 @@ static AdamScalars<T> adam_scalars(double lr, double b1, double b2, double eps, 
 }
 
 // builds the table for tensors [first, first+cnt) ; returns the CTA count
-static int build_table(MultiTensor& t, void* const* w, void* const* g, void* const* m,
+template <typename T>
+static int build_table(const prad_ctx* ctx, MultiTensor& t, void* const* w, void* const* g, void* const* m,
                        void* const* v, const int64_t* sizes, int first, int cnt) {
   int blk = 0;
+  int64_t total = 0;
+  for (int k = 0; k < cnt; ++k) total += sizes[first + k];
+  constexpr int least = MT_THREADS * 16 / (int)sizeof(T);
+  t.chunk = MT_CHUNK;
+  while (t.chunk > least && total < (int64_t)t.chunk * 2 * ctx->sm_count) t.chunk /= 2;
+  t.fold = true;
   t.count = cnt;
   t.vec = true;
   auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
@@ -256,7 +286,8 @@ static int build_table(MultiTensor& t, void* const* w, void* const* g, void* con
     t.v[k] = v ? v[first + k] : nullptr;
     t.size[k] = sizes[first + k];
     t.blk_start[k] = blk;
-    int64_t nb = ceil_div(sizes[first + k], MT_CHUNK);
+    int64_t nb = ceil_div(sizes[first + k], t.chunk);
+    if (nb > MT_FOLD) t.fold = false;
     blk += (int)(nb < 1 ? 1 : nb);
   }
   t.blk_start[cnt] = blk;
@@ -275,17 +306,17 @@ static prad_status clip_adam_t(prad_ctx* ctx, void* const* w, void* const* g, vo
   MultiTensor t;
   for (int first = 0; first < count; first += MT_MAX) {
     int cnt = count - first < MT_MAX ? count - first : MT_MAX;
-    int nb = build_table(t, w, g, m, v, sizes, first, cnt);
+    int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
     if (nb > max_blocks) max_blocks = nb;
   }
-  prad_status s = ensure_workspace(ctx, (size_t)(ST_PART + max_blocks) * sizeof(double));
+  prad_status s = ensure_workspace(ctx, (size_t)(ST_PART + 2 * max_blocks) * sizeof(double));
   if (s) return s;
   double* stats = (double*)ctx->ws;
 
   if (clip_mode == 2) {  // the norm spans every tensor: first all partial sums, then apply
     for (int first = 0; first < count; first += MT_MAX) {
       int cnt = count - first < MT_MAX ? count - first : MT_MAX;
-      int nb = build_table(t, w, g, m, v, sizes, first, cnt);
+      int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
       mt_partial_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, 2);
       PRAD_LAUNCHED(ctx);
       mt_finalize_ss_kernel<<<1, MT_THREADS, 0, ctx->stream>>>(nb, stats, first > 0);
@@ -294,16 +325,15 @@ static prad_status clip_adam_t(prad_ctx* ctx, void* const* w, void* const* g, vo
   }
   for (int first = 0; first < count; first += MT_MAX) {
     int cnt = count - first < MT_MAX ? count - first : MT_MAX;
-    int nb = build_table(t, w, g, m, v, sizes, first, cnt);
+    int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
     if (clip_mode == 1) {
-      mt_partial_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, 0);
-      PRAD_LAUNCHED(ctx);
-      mt_finalize_kernel<T><<<cnt, MT_THREADS, 0, ctx->stream>>>(t, stats, 0);
-      PRAD_LAUNCHED(ctx);
-      mt_partial_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, 1);
-      PRAD_LAUNCHED(ctx);
-      mt_finalize_kernel<T><<<cnt, MT_THREADS, 0, ctx->stream>>>(t, stats, 1);
-      PRAD_LAUNCHED(ctx);
+      for (int kind = 0; kind < 2; ++kind) {
+        mt_partial_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, kind);
+        PRAD_LAUNCHED(ctx);
+        if (t.fold) continue;
+        mt_finalize_kernel<T><<<cnt, MT_THREADS, 0, ctx->stream>>>(t, stats, kind);
+        PRAD_LAUNCHED(ctx);
+      }
     }
     mt_apply_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, clip_mode, (T)clip_value,
                                                            (T)min_value, clip_value, do_adam, a,

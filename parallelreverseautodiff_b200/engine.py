@@ -25,6 +25,10 @@ _DT = {np.dtype(np.float32): F32, np.dtype(np.float64): F64}
 
 def dtype_code(dtype) -> int:
     try:
+        return _DT[dtype]              # a matrix' own dtype: no conversion
+    except (KeyError, TypeError):
+        pass
+    try:
         return _DT[np.dtype(dtype)]
     except KeyError:
         raise TypeError(f"only float32 (PRADLite) and float64 (PRAD) are supported, got {dtype}")
@@ -329,7 +333,7 @@ class Engine:
     # ------------------------------------------------------------ helpers
     @staticmethod
     def _p(m: Optional[DeviceMatrix]):
-        return C.c_void_p(m.ptr) if m is not None else None
+        return m.ptr if m is not None else None
 
     @staticmethod
     def _ptr_list(ms: Iterable[DeviceMatrix]):
