@@ -109,6 +109,8 @@ const char* prad_version(void);
  *    the values are the same bit for bit;
  *  "tc_panel_n" = n: column tiles per panel of the persistent GEMM's tile walk (0 = automatic: two
  *    panels when the column operand exceeds 40 MB, so that a panel of it stays in L2);
+ *  "graph_plan" = "1" (default) | "0": prad_graph_forward / _backward of a graph of many small operations run as one kernel
+ *    planned at the first call, or as one launch per operation; elementwise values and products are the same bit for bit;
  *  "pool_bytes" = n: most bytes of freed device blocks (prad_free) the context keeps for later prad_alloc calls
  *    (default 1/16 of the device memory; "0" gives the kept blocks back and keeps none);
  *  "tc_pipeline" = "16x4" | "32x2" | "8x8" (k-block floats x stages of the tf32x3 kernel) */

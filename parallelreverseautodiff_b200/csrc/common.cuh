@@ -53,6 +53,7 @@ struct prad_ctx {
   int tc_variant = 0;  // pipeline shape of the tensor-core GEMM (option "tc_pipeline")
   bool tc_split_k = true;  // option "tc_split_k": cut k across CTAs when the tile count wastes SMs
   int tc_prefetch = 0;     // option "tc_prefetch": k-blocks of 32 by which the packed FP16 product prefetches its row operand into L2
+  int graph_plan = 1;      // option "graph_plan": graphs of small operations run as one kernel per walk
   int gemm_small = 1;      // option "gemm_small": batches of products of at most 64 x 64 outputs on one CTA per product
   int tc_pair = 1;         // option "tc_pair": packed FP16 products on CTA pairs (tcgen05 cta_group::2, 256-row tiles): 0 never, 1 for k or N >= 1024, 2 always
   int tc_panel_n = 0;      // option "tc_panel_n": column tiles per panel of the persistent GEMM's tile walk (0 = automatic)
@@ -165,7 +166,7 @@ inline int stream_grid(const prad_ctx* ctx, int64_t work_items, int per_block, i
 // Lets `Kernel` use `bytes` of dynamic shared memory on the context's device (needed above 48 KB): asked for once per
 // kernel and device.
 template <auto Kernel> inline prad_status allow_smem(prad_ctx* ctx, int bytes) {
-  if (bytes <= 32 * 1024) return PRAD_OK;     // (48 KB less what a kernel declares itself)
+  if (bytes <= 24 * 1024) return PRAD_OK;     // (48 KB less what a kernel declares itself)
   static std::atomic<uint64_t> done{0};
   const uint64_t bit = 1ull << (ctx->device & 63);
   if (!(done.load(std::memory_order_acquire) & bit)) {

@@ -6,6 +6,7 @@
 #include <memory>
 
 #include "common.cuh"
+#include "graph_plan.cuh"
 
 namespace prad {
 
@@ -43,10 +44,137 @@ struct prad_graph {
   std::vector<prad::GValue> values;
   std::vector<prad::GNode> nodes;
   std::vector<void*> owned;    // every device block the graph allocated
+  // Walks made into plans (graph_plan.cu).  A plan holds for the nodes it was made from; a backward also for its start values
+  // and their gradients, of which the last few sets are kept.
+  struct Walk {
+    bool tried = false;
+    size_t nodes = 0;
+    std::vector<int> starts;
+    std::vector<const void*> d_starts;
+    std::vector<void*> grads;         // what the walk leaves in the values
+    std::vector<int> consumers;
+    prad::GraphPlanPtr plan;          // null: one launch per operation is better
+  };
+  Walk forward_walk;
+  std::vector<Walk> backward_walks;
+  std::vector<prad::GraphPlanPtr> retired;
   uint32_t magic = 0x47524146u;
 };
 
 namespace prad {
+
+constexpr size_t KEPT_BACKWARD_WALKS = 4;
+
+// The operations of a walk: launched one by one, or written down (`rec`) for a plan.
+struct Ops {
+  prad_ctx* c;
+  prad_dtype dt;
+  std::vector<Prim>* rec;
+
+  Prim& add(PrimKind k, std::vector<const void*> in, std::vector<void*> out) const {
+    rec->emplace_back();
+    Prim& p = rec->back();
+    p.kind = k;
+    p.in = std::move(in);
+    p.out = std::move(out);
+    return p;
+  }
+  prad_status each(PrimKind k, std::vector<const void*> in, std::vector<void*> out, int64_t n, int act = 0, double s = 0) const {
+    Prim& p = add(k, std::move(in), std::move(out));
+    p.n = n;
+    p.act = act;
+    p.scalar = s;
+    return PRAD_OK;
+  }
+  prad_status rows_op(PrimKind k, std::vector<const void*> in, std::vector<void*> out, int64_t rows, int cols, int depth = 1) const {
+    Prim& p = add(k, std::move(in), std::move(out));
+    p.rows = rows;
+    p.cols = cols;
+    p.depth = depth;
+    return PRAD_OK;
+  }
+  prad_status product(bool tA, bool tB, int M, int N, int K, double alpha, const void* A, const void* B, void* C, int batch = 1,
+                      int64_t sA = 0, int64_t sB = 0, int64_t sC = 0) const {
+    if (rec) {
+      Prim& p = add(PRIM_PRODUCT, {A, B}, {C});
+      p.tA = tA; p.tB = tB; p.M = M; p.N = N; p.K = K; p.scalar = alpha;
+      p.batch = batch; p.sA = sA; p.sB = sB; p.sC = sC;
+      return PRAD_OK;
+    }
+    return prad_gemm(c, dt, tA, tB, M, N, K, alpha, A, tA ? M : K, B, tB ? K : N, 0.0, C, N, batch, sA, sB, sC);
+  }
+  prad_status product_backward(const void* A, const void* B, const void* dC, void* dA, void* dB, int M, int K, int N) const {
+    if (!rec) return prad_matmul_backward(c, dt, A, B, dC, dA, dB, M, K, N, 0, 1.0, PRAD_ACT_NONE, nullptr, 0.0);
+    product(false, true, M, K, N, 1.0, dC, B, dA);
+    return product(true, false, K, N, M, 1.0, A, dC, dB);
+  }
+  prad_status act_forward(prad_act a, const void* x, void* y, int64_t n, double s) const {
+    return rec ? each(PRIM_ACT_FORWARD, {x}, {y}, n, a, s) : prad_act_forward(c, dt, a, x, y, n, s);
+  }
+  prad_status act_backward(prad_act a, const void* saved, const void* dy, void* dx, int64_t n, double s) const {
+    return rec ? each(PRIM_ACT_BACKWARD, {saved, dy}, {dx}, n, a, s) : prad_act_backward(c, dt, a, saved, dy, dx, n, s);
+  }
+  prad_status add2(const void* a, const void* b, void* y, int64_t n) const {
+    return rec ? each(PRIM_ADD2, {a, b}, {y}, n) : prad_add_forward(c, dt, a, b, nullptr, y, n);
+  }
+  prad_status add3(const void* a, const void* b, const void* d, void* y, int64_t n) const {
+    return rec ? each(PRIM_ADD3, {a, b, d}, {y}, n) : prad_add_forward(c, dt, a, b, d, y, n);
+  }
+  prad_status add_row(const void* x, const void* row, void* y, int rows, int cols) const {
+    if (!rec) return prad_add_broadcast_forward(c, dt, x, row, y, rows, cols);
+    each(PRIM_ADD_ROW, {x, row}, {y}, (int64_t)rows * cols);
+    rec->back().cols = cols;
+    return PRAD_OK;
+  }
+  prad_status hadamard(const void* a, const void* b, void* y, int64_t n) const {
+    return rec ? each(PRIM_MUL2, {a, b}, {y}, n) : prad_hadamard_forward(c, dt, a, b, y, n);
+  }
+  prad_status hadamard_backward(const void* a, const void* b, const void* d, void* da, void* db, int64_t n) const {
+    return rec ? each(PRIM_MUL_BACKWARD, {a, b, d}, {da, db}, n) : prad_hadamard_backward(c, dt, a, b, d, da, db, n);
+  }
+  prad_status scale(const void* x, void* y, int64_t n, double s) const {
+    return rec ? each(PRIM_SCALE, {x}, {y}, n, 0, s) : prad_scale(c, dt, x, y, n, s);
+  }
+  prad_status accumulate(void* dst, const void* src, int64_t n) const {
+    return rec ? each(PRIM_ADD2, {dst, src}, {dst}, n) : prad_accumulate(c, dt, dst, src, n);
+  }
+  prad_status sum(const void* const* srcs, int count, void* out, int64_t n) const {
+    if (!rec) return prad_segmented_sum(c, dt, srcs, count, out, n);
+    // eight at a time, the running sum first, as prad_segmented_sum does
+    for (int done = 0; done < count;) {
+      std::vector<const void*> in;
+      if (done) in.push_back(out);
+      while (in.size() < 8 && done < count) in.push_back(srcs[done++]);
+      each(PRIM_SUM, std::move(in), {out}, n);
+    }
+    return PRAD_OK;
+  }
+  prad_status column_sum(const void* x, void* out, int rows, int cols) const {
+    return rec ? rows_op(PRIM_COLUMN_SUM, {x}, {out}, rows, cols) : prad_add_broadcast_backward(c, dt, x, out, rows, cols, 0);
+  }
+  prad_status transpose(const void* x, void* y, int rows, int cols, int depth) const {
+    return rec ? rows_op(PRIM_TRANSPOSE, {x}, {y}, rows, cols, depth) : prad_transpose(c, dt, x, y, rows, cols, depth);
+  }
+  prad_status softmax(const void* x, void* y, int64_t rows, int cols) const {
+    return rec ? rows_op(PRIM_SOFTMAX, {x}, {y}, rows, cols) : prad_softmax_forward(c, dt, x, y, rows, cols);
+  }
+  prad_status softmax_backward(const void* y, const void* dy, void* dx, int64_t rows, int cols) const {
+    return rec ? rows_op(PRIM_SOFTMAX_BACKWARD, {y, dy}, {dx}, rows, cols) : prad_softmax_backward(c, dt, y, dy, dx, rows, cols);
+  }
+  prad_status sine_softmax(const void* x, void* y, int64_t rows, int cols) const {
+    return rec ? rows_op(PRIM_SINE_SOFTMAX, {x}, {y}, rows, cols) : prad_sine_softmax_forward(c, dt, x, y, rows, cols);
+  }
+  prad_status sine_softmax_backward(const void* x, const void* dy, void* dx, int64_t rows, int cols) const {
+    return rec ? rows_op(PRIM_SINE_SOFTMAX_BACKWARD, {x, dy}, {dx}, rows, cols) : prad_sine_softmax_backward(c, dt, x, dy, dx, rows, cols);
+  }
+  prad_status layernorm(const void* x, void* y, void* mean, void* sigma, int64_t rows, int cols) const {
+    return rec ? rows_op(PRIM_LAYERNORM, {x}, {y, mean, sigma}, rows, cols) : prad_layernorm_forward(c, dt, x, y, mean, sigma, rows, cols);
+  }
+  prad_status layernorm_backward(const void* x, const void* mean, const void* sigma, const void* dy, void* dx, int64_t rows, int cols) const {
+    return rec ? rows_op(PRIM_LAYERNORM_BACKWARD, {x, mean, sigma, dy}, {dx}, rows, cols)
+               : prad_layernorm_backward(c, dt, x, mean, sigma, dy, dx, rows, cols);
+  }
+};
 
 static bool graph_ok(const prad_graph* g) { return g && g->magic == 0x47524146u && ctx_ok(g->ctx); }
 
@@ -133,6 +261,9 @@ prad_status prad_graph_set_gradient_destination(prad_graph* g, int value, void* 
   PRAD_REQUIRE(value >= 0 && value < (int)g->values.size() && grad_matrix, PRAD_ERR_INVALID,
                "prad_graph_set_gradient_destination: bad value id or null matrix");
   g->values[value].grad_dst = grad_matrix;
+  // plans have the old destination in them (a recorded launch sequence may still run one: those stay until the graph goes)
+  for (auto& w : g->backward_walks) g->retired.push_back(std::move(w.plan));
+  g->backward_walks.clear();
   return PRAD_OK;
 }
 
@@ -254,10 +385,8 @@ namespace prad {
     if (s_ != PRAD_OK) return s_;     \
   } while (0)
 
-static prad_status node_forward(prad_graph* g, GNode& n) {
+static prad_status node_forward(prad_graph* g, GNode& n, const Ops& ops) {
   auto& V = g->values;
-  prad_ctx* c = g->ctx;
-  const prad_dtype dt = g->dt;
   GValue& o = V[n.out];
   const GValue& a = V[n.in[0]];
   const int64_t cnt = o.count();
@@ -266,40 +395,38 @@ static prad_status node_forward(prad_graph* g, GNode& n) {
   switch (n.op) {
     case PRAD_OP_MATMUL: {
       const GValue& b = V[n.in[1]];
-      if (D == 1)
-        return prad_matmul_forward(c, dt, a.data, b.data, o.data, a.rows, a.cols, b.cols, nullptr, nullptr, PRAD_ACT_NONE, 0.0);
-      if (a.depth == D)    // (DeepMatrix, DeepMatrix) and (DeepMatrix, Matrix)
-        return prad_batch_matmul_forward(c, dt, a.data, b.data, o.data, D, a.rows, a.cols, b.cols, b.depth == 1);
-      // (Matrix, DeepMatrix): every slice is multiplied from the left by the same matrix
-      return prad_gemm(c, dt, 0, 0, a.rows, b.cols, a.cols, 1.0, a.data, a.cols, b.data, b.cols, 0.0, o.data, b.cols, D, 0,
-                       b.slice(), o.slice());
+      if (D == 1) return ops.product(false, false, a.rows, b.cols, a.cols, 1.0, a.data, b.data, o.data);
+      if (a.depth == D && b.depth == 1)    // (DeepMatrix, Matrix): one tall product
+        return ops.product(false, false, D * a.rows, b.cols, a.cols, 1.0, a.data, b.data, o.data);
+      // (DeepMatrix, DeepMatrix), or (Matrix, DeepMatrix): every slice is multiplied from the left by the same matrix
+      return ops.product(false, false, a.rows, b.cols, a.cols, 1.0, a.data, b.data, o.data, D, a.depth == D ? a.slice() : 0, b.slice(),
+                         o.slice());
     }
     case PRAD_OP_ADD:
       if (V[n.in[1]].depth != D)   // (DeepMatrix, Matrix): the matrix is a "row" added to each of the D slices
-        return prad_add_broadcast_forward(c, dt, a.data, V[n.in[1]].data, o.data, D, (int)a.slice());
-      return prad_add_forward(c, dt, a.data, V[n.in[1]].data, nullptr, o.data, cnt);
+        return ops.add_row(a.data, V[n.in[1]].data, o.data, D, (int)a.slice());
+      return ops.add2(a.data, V[n.in[1]].data, o.data, cnt);
     case PRAD_OP_ADD3:
       if (V[n.in[2]].depth != D) {   // (a + b) + bias, the bias shared by the slices
-        G_TRY(prad_add_forward(c, dt, a.data, V[n.in[1]].data, nullptr, o.data, cnt));
-        return prad_add_broadcast_forward(c, dt, o.data, V[n.in[2]].data, o.data, D, (int)a.slice());
+        G_TRY(ops.add2(a.data, V[n.in[1]].data, o.data, cnt));
+        return ops.add_row(o.data, V[n.in[2]].data, o.data, D, (int)a.slice());
       }
-      return prad_add_forward(c, dt, a.data, V[n.in[1]].data, V[n.in[2]].data, o.data, cnt);
-    case PRAD_OP_ADD_BROADCAST:
-      return prad_add_broadcast_forward(c, dt, a.data, V[n.in[1]].data, o.data, (int)rows_all, a.cols);
-    case PRAD_OP_HADAMARD: return prad_hadamard_forward(c, dt, a.data, V[n.in[1]].data, o.data, cnt);
+      return ops.add3(a.data, V[n.in[1]].data, V[n.in[2]].data, o.data, cnt);
+    case PRAD_OP_ADD_BROADCAST: return ops.add_row(a.data, V[n.in[1]].data, o.data, (int)rows_all, a.cols);
+    case PRAD_OP_HADAMARD: return ops.hadamard(a.data, V[n.in[1]].data, o.data, cnt);
     case PRAD_OP_LEAKY_RELU: case PRAD_OP_SIGMOID: case PRAD_OP_TANH: case PRAD_OP_GELU:
     case PRAD_OP_RELU: case PRAD_OP_AMPLIFIED_SIGMOID:
-      return prad_act_forward(c, dt, act_of(n.op), a.data, o.data, cnt, n.scalar);
-    case PRAD_OP_SOFTMAX: return prad_softmax_forward(c, dt, a.data, o.data, rows_all, a.cols);
-    case PRAD_OP_SINE_SOFTMAX: return prad_sine_softmax_forward(c, dt, a.data, o.data, rows_all, a.cols);
+      return ops.act_forward(act_of(n.op), a.data, o.data, cnt, n.scalar);
+    case PRAD_OP_SOFTMAX: return ops.softmax(a.data, o.data, rows_all, a.cols);
+    case PRAD_OP_SINE_SOFTMAX: return ops.sine_softmax(a.data, o.data, rows_all, a.cols);
     case PRAD_OP_LAYERNORM:
       if (!n.aux0) {
         G_TRY(g_alloc(g, (size_t)rows_all, &n.aux0));
         G_TRY(g_alloc(g, (size_t)rows_all, &n.aux1));
       }
-      return prad_layernorm_forward(c, dt, a.data, o.data, n.aux0, n.aux1, rows_all, a.cols);
-    case PRAD_OP_SCALE: return prad_scale(c, dt, a.data, o.data, cnt, n.scalar);
-    case PRAD_OP_TRANSPOSE: return prad_transpose(c, dt, a.data, o.data, a.rows, a.cols, D);
+      return ops.layernorm(a.data, o.data, n.aux0, n.aux1, rows_all, a.cols);
+    case PRAD_OP_SCALE: return ops.scale(a.data, o.data, cnt, n.scalar);
+    case PRAD_OP_TRANSPOSE: return ops.transpose(a.data, o.data, a.rows, a.cols, D);
   }
   return PRAD_ERR_INVALID;
 }
@@ -319,15 +446,13 @@ static prad_status in_grad_buf(prad_graph* g, GNode& n, int i, void** out) {
 // exactly as MatrixAddBroadcastingOperation.Backward returns dOutput itself.
 // mean over the D slices of `deep` (D x per elements) into `out` (per elements): the visitor's combined
 // gradient of a Matrix shared by the slices of a batch operation (sum of the slices times 1/D)
-static prad_status slice_mean(prad_graph* g, const void* deep, void* out, int D, int64_t per) {
-  G_TRY(prad_add_broadcast_backward(g->ctx, g->dt, deep, out, D, (int)per, 0));
-  return prad_scale(g->ctx, g->dt, out, out, per, 1.0 / (double)D);
+static prad_status slice_mean(const Ops& ops, const void* deep, void* out, int D, int64_t per) {
+  G_TRY(ops.column_sum(deep, out, D, (int)per));
+  return ops.scale(out, out, per, 1.0 / (double)D);
 }
 
-static prad_status node_backward(prad_graph* g, GNode& n, void* d) {
+static prad_status node_backward(prad_graph* g, GNode& n, void* d, const Ops& ops) {
   auto& V = g->values;
-  prad_ctx* c = g->ctx;
-  const prad_dtype dt = g->dt;
   const GValue& o = V[n.out];
   const GValue& a = V[n.in[0]];
   const int64_t cnt = o.count();
@@ -342,19 +467,21 @@ static prad_status node_backward(prad_graph* g, GNode& n, void* d) {
       G_TRY(in_grad_buf(g, n, 1, &gb));
       const int M = a.rows, K = a.cols, N = b.cols;
       if (D == 1) {
-        G_TRY(prad_matmul_backward(c, dt, a.data, b.data, d, ga, gb, M, K, N, 0, 1.0, PRAD_ACT_NONE, nullptr, 0.0));
+        G_TRY(ops.product_backward(a.data, b.data, d, ga, gb, M, K, N));
       } else if (a.depth == D && b.depth == D) {
-        G_TRY(prad_batch_matmul_backward(c, dt, a.data, b.data, d, ga, gb, nullptr, D, M, K, N, 0));
+        G_TRY(ops.product(false, true, M, K, N, 1.0, d, b.data, ga, D, o.slice(), b.slice(), a.slice()));
+        G_TRY(ops.product(true, false, K, N, M, 1.0, a.data, d, gb, D, a.slice(), o.slice(), b.slice()));
       } else if (a.depth == D) {   // shared second operand: its gradient is the mean of the slices' A_d^T dC_d
-        G_TRY(prad_batch_matmul_backward(c, dt, a.data, b.data, d, ga, nullptr, gb, D, M, K, N, 1));
+        G_TRY(ops.product(false, true, D * M, K, N, 1.0, d, b.data, ga));
+        G_TRY(ops.product(true, false, K, N, D * M, 1.0 / (double)D, a.data, d, gb));
       } else {                     // shared first operand W: dX_d = W^T dC_d ; dW = (1/D) sum_d dC_d X_d^T
-        G_TRY(prad_gemm(c, dt, 1, 0, K, N, M, 1.0, a.data, K, d, N, 0.0, gb, N, D, 0, o.slice(), b.slice()));
+        G_TRY(ops.product(true, false, K, N, M, 1.0, a.data, d, gb, D, 0, o.slice(), b.slice()));
         if (N == 1) {              // column vectors: the slices of dC and X are the rows of two matrices
-          G_TRY(prad_gemm(c, dt, 1, 0, M, K, D, 1.0 / (double)D, d, M, b.data, K, 0.0, ga, K, 1, 0, 0, 0));
+          G_TRY(ops.product(true, false, M, K, D, 1.0 / (double)D, d, b.data, ga));
         } else {
           if (!n.aux0) G_TRY(g_alloc(g, (size_t)D * M * K, &n.aux0));
-          G_TRY(prad_gemm(c, dt, 0, 1, M, K, N, 1.0, d, N, b.data, N, 0.0, n.aux0, K, D, o.slice(), b.slice(), (int64_t)M * K));
-          G_TRY(slice_mean(g, n.aux0, ga, D, (int64_t)M * K));
+          G_TRY(ops.product(false, true, M, K, N, 1.0, d, b.data, n.aux0, D, o.slice(), b.slice(), (int64_t)M * K));
+          G_TRY(slice_mean(ops, n.aux0, ga, D, (int64_t)M * K));
         }
       }
       V[n.in[0]].contrib.push_back(ga);
@@ -369,53 +496,53 @@ static prad_status node_backward(prad_graph* g, GNode& n, void* d) {
         } else {                   // the Matrix shared by the slices
           void* gs = nullptr;
           G_TRY(in_grad_buf(g, n, (int)i, &gs));
-          G_TRY(slice_mean(g, d, gs, D, iv.slice()));
+          G_TRY(slice_mean(ops, d, gs, D, iv.slice()));
           iv.contrib.push_back(gs);
         }
       }
       return PRAD_OK;
     case PRAD_OP_ADD_BROADCAST:
       G_TRY(in_grad_buf(g, n, 1, &gb));
-      G_TRY(prad_add_broadcast_backward(c, dt, d, gb, (int)rows_all, o.cols, 0));
-      if (D > 1) G_TRY(prad_scale(c, dt, gb, gb, o.cols, 1.0 / (double)D));   // mean of the slices' column sums
+      G_TRY(ops.column_sum(d, gb, (int)rows_all, o.cols));
+      if (D > 1) G_TRY(ops.scale(gb, gb, o.cols, 1.0 / (double)D));   // mean of the slices' column sums
       V[n.in[0]].contrib.push_back(d);
       V[n.in[1]].contrib.push_back(gb);
       return PRAD_OK;
     case PRAD_OP_HADAMARD:
       G_TRY(in_grad_buf(g, n, 0, &ga));
       G_TRY(in_grad_buf(g, n, 1, &gb));
-      G_TRY(prad_hadamard_backward(c, dt, a.data, V[n.in[1]].data, d, ga, gb, cnt));
+      G_TRY(ops.hadamard_backward(a.data, V[n.in[1]].data, d, ga, gb, cnt));
       V[n.in[0]].contrib.push_back(ga);
       V[n.in[1]].contrib.push_back(gb);
       return PRAD_OK;
     case PRAD_OP_LEAKY_RELU: case PRAD_OP_GELU: case PRAD_OP_RELU: case PRAD_OP_AMPLIFIED_SIGMOID:   // Backward reads the input
       G_TRY(in_grad_buf(g, n, 0, &ga));
-      G_TRY(prad_act_backward(c, dt, act_of(n.op), a.data, d, ga, cnt, n.scalar));
+      G_TRY(ops.act_backward(act_of(n.op), a.data, d, ga, cnt, n.scalar));
       break;
     case PRAD_OP_SIGMOID: case PRAD_OP_TANH:        // Backward reads the output
       G_TRY(in_grad_buf(g, n, 0, &ga));
-      G_TRY(prad_act_backward(c, dt, act_of(n.op), o.data, d, ga, cnt, n.scalar));
+      G_TRY(ops.act_backward(act_of(n.op), o.data, d, ga, cnt, n.scalar));
       break;
     case PRAD_OP_SOFTMAX:
       G_TRY(in_grad_buf(g, n, 0, &ga));
-      G_TRY(prad_softmax_backward(c, dt, o.data, d, ga, rows_all, o.cols));
+      G_TRY(ops.softmax_backward(o.data, d, ga, rows_all, o.cols));
       break;
     case PRAD_OP_SINE_SOFTMAX:                      // Backward reads the input
       G_TRY(in_grad_buf(g, n, 0, &ga));
-      G_TRY(prad_sine_softmax_backward(c, dt, a.data, d, ga, rows_all, o.cols));
+      G_TRY(ops.sine_softmax_backward(a.data, d, ga, rows_all, o.cols));
       break;
     case PRAD_OP_LAYERNORM:
       PRAD_REQUIRE(n.aux0, PRAD_ERR_INVALID, "prad_graph_backward: LayerNorm node has no forward state (run prad_graph_forward)");
       G_TRY(in_grad_buf(g, n, 0, &ga));
-      G_TRY(prad_layernorm_backward(c, dt, a.data, n.aux0, n.aux1, d, ga, rows_all, a.cols));
+      G_TRY(ops.layernorm_backward(a.data, n.aux0, n.aux1, d, ga, rows_all, a.cols));
       break;
     case PRAD_OP_SCALE:
       G_TRY(in_grad_buf(g, n, 0, &ga));
-      G_TRY(prad_scale(c, dt, d, ga, cnt, n.scalar));
+      G_TRY(ops.scale(d, ga, cnt, n.scalar));
       break;
     case PRAD_OP_TRANSPOSE:
       G_TRY(in_grad_buf(g, n, 0, &ga));
-      G_TRY(prad_transpose(c, dt, d, ga, o.rows, o.cols, D));
+      G_TRY(ops.transpose(d, ga, o.rows, o.cols, D));
       break;
   }
   V[n.in[0]].contrib.push_back(ga);
@@ -426,15 +553,39 @@ static prad_status node_backward(prad_graph* g, GNode& n, void* d) {
 
 extern "C" {
 
-prad_status prad_graph_forward(prad_graph* g) {
-  PRAD_CHECK_GRAPH(g);
+// A plan multiplies exactly; another choice of product kernel keeps the launches one by one.  A walk that is being recorded
+// into a launch sequence uses a plan that is there, but cannot make one.
+static bool may_plan(const prad_ctx* c) {
+  return c->graph_plan && (c->gemm_f32 == GemmF32::Auto || c->gemm_f32 == GemmF32::Simt) && (c->gemm_f64 == GemmF64::Auto || c->gemm_f64 == GemmF64::Simt);
+}
+
+static prad_status forward_walk(prad_graph* g, const Ops& ops) {
   for (GNode& n : g->nodes) {
     for (int i : n.in)
       PRAD_REQUIRE(g->values[i].data, PRAD_ERR_INVALID, "prad_graph_forward: value %d has no data and no producer before its use", i);
-    G_TRY(node_forward(g, n));
+    G_TRY(node_forward(g, n, ops));
   }
   return PRAD_OK;
 }
+
+prad_status prad_graph_forward(prad_graph* g) {
+  PRAD_CHECK_GRAPH(g);
+  PRAD_CHECK_CTX(g->ctx);
+  auto& w = g->forward_walk;
+  if (may_plan(g->ctx)) {
+    if ((!w.tried || w.nodes != g->nodes.size()) && !g->ctx->capturing) {
+      std::vector<Prim> ops;
+      G_TRY(forward_walk(g, Ops{g->ctx, g->dt, &ops}));
+      w.plan = graph_plan_build(g->ctx, g->dt, ops);
+      w.tried = true;
+      w.nodes = g->nodes.size();
+    }
+    if (w.plan && w.nodes == g->nodes.size()) return graph_plan_run(g->ctx, w.plan.get());
+  }
+  return forward_walk(g, Ops{g->ctx, g->dt, nullptr});
+}
+
+static prad_status backward_walk(prad_graph* g, const int* start_values, const void* const* d_starts, int count, const Ops& ops);
 
 prad_status prad_graph_backward_multi(prad_graph* g, const int* start_values, const void* const* d_starts, int count) {
   PRAD_CHECK_GRAPH(g);
@@ -447,6 +598,39 @@ prad_status prad_graph_backward_multi(prad_graph* g, const int* start_values, co
       PRAD_REQUIRE(start_values[j] != start_values[i], PRAD_ERR_INVALID, "prad_graph_backward: start value %d is listed twice",
                    start_values[i]);
   }
+  PRAD_CHECK_CTX(g->ctx);
+  if (!may_plan(g->ctx)) return backward_walk(g, start_values, d_starts, count, Ops{g->ctx, g->dt, nullptr});
+  prad_graph::Walk* w = nullptr;
+  bool hopeless = false;              // the same walk with other gradients was better launched one by one
+  for (auto& k : g->backward_walks)
+    if (k.nodes == g->nodes.size() && k.starts.size() == (size_t)count && std::equal(k.starts.begin(), k.starts.end(), start_values) && !k.plan)
+      hopeless = true;
+  for (auto& k : g->backward_walks)
+    if (k.nodes == g->nodes.size() && k.starts.size() == (size_t)count && std::equal(k.starts.begin(), k.starts.end(), start_values) &&
+        std::equal(k.d_starts.begin(), k.d_starts.end(), d_starts))
+      w = &k;
+  if (!w && !hopeless && !g->ctx->capturing) {
+    std::vector<Prim> ops;
+    G_TRY(backward_walk(g, start_values, d_starts, count, Ops{g->ctx, g->dt, &ops}));
+    if (g->backward_walks.size() >= KEPT_BACKWARD_WALKS) {
+      if (g->ctx->live_sequences > 0) g->retired.push_back(std::move(g->backward_walks.front().plan));
+      g->backward_walks.erase(g->backward_walks.begin());
+    }
+    g->backward_walks.emplace_back();
+    w = &g->backward_walks.back();
+    w->nodes = g->nodes.size();
+    w->starts.assign(start_values, start_values + count);
+    w->d_starts.assign(d_starts, d_starts + count);
+    for (const GValue& v : V) { w->grads.push_back(v.grad); w->consumers.push_back(v.consumers); }
+    w->plan = graph_plan_build(g->ctx, g->dt, ops);
+  }
+  if (!w || !w->plan) return backward_walk(g, start_values, d_starts, count, Ops{g->ctx, g->dt, nullptr});
+  for (size_t i = 0; i < w->grads.size(); ++i) { V[i].grad = w->grads[i]; V[i].consumers = w->consumers[i]; }
+  return graph_plan_run(g->ctx, w->plan.get());
+}
+
+static prad_status backward_walk(prad_graph* g, const int* start_values, const void* const* d_starts, int count, const Ops& ops) {
+  auto& V = g->values;
   // 1. which nodes lie on a path to a start value, and how many consumers each value has
   //    there (OperationGraphVisitor's dependency counts)
   std::vector<char> needed(V.size(), 0), is_start(V.size(), 0);
@@ -471,10 +655,10 @@ prad_status prad_graph_backward_multi(prad_graph* g, const int* start_values, co
       v.grad = v.contrib[0];
     } else {
       if (!v.sum_buf) G_TRY(g_alloc(g, (size_t)v.count(), &v.sum_buf));
-      G_TRY(prad_segmented_sum(g->ctx, g->dt, v.contrib.data(), (int)v.contrib.size(), v.sum_buf, v.count()));
+      G_TRY(ops.sum(v.contrib.data(), (int)v.contrib.size(), v.sum_buf, v.count()));
       v.grad = v.sum_buf;
     }
-    if (v.grad_dst) G_TRY(prad_accumulate(g->ctx, g->dt, v.grad_dst, v.grad, v.count()));
+    if (v.grad_dst) G_TRY(ops.accumulate(v.grad_dst, v.grad, v.count()));
     return PRAD_OK;
   };
   auto external_of = [&](int value) -> const void* {
@@ -489,7 +673,7 @@ prad_status prad_graph_backward_multi(prad_graph* g, const int* start_values, co
     GValue& o = V[n.out];
     G_TRY(finalize(o, external_of(n.out)));
     PRAD_REQUIRE(o.grad, PRAD_ERR_INVALID, "prad_graph_backward: node %d is on the path but received no gradient", k);
-    G_TRY(node_backward(g, n, o.grad));
+    G_TRY(node_backward(g, n, o.grad, ops));
   }
   // 3. leaves (inputs, weights): fan-in sum and `destination += gradient`
   for (size_t i = 0; i < V.size(); ++i)

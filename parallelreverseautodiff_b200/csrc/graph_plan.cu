@@ -1,0 +1,706 @@
+// Runs a graph's walk as ONE kernel.
+//
+// What bounded it: an unrolled network from a JSON architecture is hundreds of operations on a few hundred values each.  An
+// eight-step two-layer LSTM of 64 units is 1058 launches of 2 - 6 us per training step, 4.9 ms, for 25 MFLOP.
+//
+// Here the walk is recorded once as a list of primitive operations.  A level of the plan holds operations that depend on
+// earlier levels only; chains of elementwise operations on the same elements (a gate's sum and activation, a cell update, the
+// += of a shared weight's gradients over the time steps) share a level too, as a small program that keeps every value of one
+// element in shared memory from its load to its store.  One cluster of 16 CTAs runs the levels with the cluster's hardware
+// barrier between them (no waiting loops, no other CTA to wait for); the pieces of a level -- 256 elements or 256 outputs each
+// -- are dealt to the CTAs when the plan is made, and a CTA fetches the next piece's program while it runs this one.
+//
+// Values are those of the separate kernels bit for bit for elementwise operations and products (k ascending, product and sum
+// rounded separately); row reductions and column sums add in double or in the same lane order.  (Compiled with -fmad=false.)
+#include <algorithm>
+#include <cstring>
+#include <map>
+
+#include "act_math.cuh"
+#include "graph_plan.cuh"
+
+namespace prad {
+namespace gp {
+
+constexpr int NT = 256;
+constexpr int SLOTS = 64;                 // values of one element a program keeps
+constexpr int MAX_INS = 96;
+constexpr int PROG_BYTES = 32 + SLOTS * 16 + MAX_INS * 24 + SLOTS * 16;
+constexpr int MAX_ITEMS = 1024;           // pieces per CTA
+constexpr int STAGE_BYTES = 64 * 1024;    // operands of a product in shared memory
+
+// a piece of work of one CTA
+struct Item { uint32_t prog, bytes, chunk, barrier; };
+
+struct Head { int32_t kind, n_load, n_ins, n_store; int64_t n; int64_t pad; };
+struct Load { const void* p; uint32_t cols, slot; };        // cols: 0 = element i, else element i % cols
+struct Ins { uint8_t op, act, n_in, pad; uint8_t dst[2], pad2[2]; uint8_t src[8]; double scalar; };
+struct Store { void* p; uint32_t slot, pad; };
+static_assert(sizeof(Head) == 32 && sizeof(Load) == 16 && sizeof(Ins) == 24 && sizeof(Store) == 16, "program layout");
+struct ProductProg {
+  Head h;                                                    // kind = PRIM_PRODUCT
+  const void *A, *B;
+  void* C;
+  int64_t sA, sB, sC;
+  double alpha;
+  int32_t tA, tB, M, N, K, tm, tn, ks, tiles_n, tiles_mn;
+};
+struct RowProg { Head h; const void* in[4]; void* out[3]; int64_t rows; int32_t cols, depth; double scalar; };
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+template <int BYTES> __device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// ---- elementwise programs: 256 elements, one per thread; v[slot][thread]
+template <typename T>
+__device__ void run_elementwise(const Head* h, int chunk, T (*v)[NT]) {
+  const int tid = threadIdx.x;
+  const int64_t i = (int64_t)chunk * NT + tid;
+  if (i >= h->n) return;
+  const Load* ld = reinterpret_cast<const Load*>(h + 1);
+  const Ins* ins = reinterpret_cast<const Ins*>(ld + h->n_load);
+  const Store* st = reinterpret_cast<const Store*>(ins + h->n_ins);
+  for (int k = 0; k < h->n_load; ++k) {      // all on their way at once
+    const int64_t at = ld[k].cols ? i % ld[k].cols : i;
+    copy_async<sizeof(T)>(&v[ld[k].slot][tid], (const T*)ld[k].p + at);
+  }
+  copy_wait();
+  for (int k = 0; k < h->n_ins; ++k) {
+    const Ins c = ins[k];
+    const T a = v[c.src[0]][tid], s = (T)c.scalar;
+    T r;
+    switch (c.op) {
+      case PRIM_ACT_FORWARD: r = act_value<T>((prad_act)c.act, a, s); break;
+      case PRIM_ACT_BACKWARD: r = mul_rn(v[c.src[1]][tid], act_derivative<T>((prad_act)c.act, a, s)); break;
+      case PRIM_ADD2: case PRIM_ADD_ROW: r = add_rn(a, v[c.src[1]][tid]); break;
+      case PRIM_ADD3: r = add_rn(add_rn(a, v[c.src[1]][tid]), v[c.src[2]][tid]); break;
+      case PRIM_MUL2: r = mul_rn(a, v[c.src[1]][tid]); break;
+      case PRIM_MUL_BACKWARD: {              // a, b, dy -> dy b, dy a
+        const T b = v[c.src[1]][tid], d = v[c.src[2]][tid];
+        v[c.dst[1]][tid] = mul_rn(d, a);
+        r = mul_rn(d, b);
+        break;
+      }
+      case PRIM_SCALE: r = mul_rn(a, s); break;
+      default: {                             // PRIM_SUM: in list order, in double, cast once
+        double acc = (double)a;
+        for (int q = 1; q < c.n_in; ++q) acc += (double)v[c.src[q]][tid];
+        r = (T)acc;
+      }
+    }
+    v[c.dst[0]][tid] = r;
+  }
+  for (int k = 0; k < h->n_store; ++k) ((T*)st[k].p)[i] = v[st[k].slot][tid];
+}
+
+// ---- products: a tm x tn tile, one output per thread, both operands of ks values of k in shared memory
+template <typename T>
+__device__ void run_product(const ProductProg* p, int chunk, T* smem) {
+  const int tid = threadIdx.x, tm = p->tm, tn = p->tn, ks = p->ks, K = p->K, M = p->M, N = p->N;
+  const int bz = chunk / p->tiles_mn, t2 = chunk % p->tiles_mn;
+  const int m0 = t2 / p->tiles_n * tm, n0 = t2 % p->tiles_n * tn;
+  const T* A = (const T*)p->A + bz * p->sA;
+  const T* B = (const T*)p->B + bz * p->sB;
+  T* C = (T*)p->C + bz * p->sC;
+  const int pa = ks | 1;                     // odd pitch: the rows of a warp's threads in different banks
+  T* As = smem;                              // [tm][pa]
+  T* Bs = smem + tm * pa;                    // [tn][pa]
+  const int mi = tid / tn, ni = tid % tn;
+  const bool on = mi < tm;
+  T acc = (T)0;
+  for (int k0 = 0; k0 < K; k0 += ks) {
+    const int kc = K - k0 < ks ? K - k0 : ks;
+    if (k0) __syncthreads();
+    if (p->tA) {                             // memory is [k][m]
+      for (int e = tid; e < kc * tm; e += NT) {
+        const int k = e / tm, m = e % tm;
+        if (m0 + m < M) copy_async<sizeof(T)>(As + m * pa + k, A + (int64_t)(k0 + k) * M + m0 + m);
+      }
+    } else {
+      for (int e = tid; e < tm * kc; e += NT) {
+        const int m = e / kc, k = e % kc;
+        if (m0 + m < M) copy_async<sizeof(T)>(As + m * pa + k, A + (int64_t)(m0 + m) * K + k0 + k);
+      }
+    }
+    if (p->tB) {                             // memory is [n][k]
+      for (int e = tid; e < tn * kc; e += NT) {
+        const int n = e / kc, k = e % kc;
+        if (n0 + n < N) copy_async<sizeof(T)>(Bs + n * pa + k, B + (int64_t)(n0 + n) * K + k0 + k);
+      }
+    } else {
+      for (int e = tid; e < kc * tn; e += NT) {
+        const int k = e / tn, n = e % tn;
+        if (n0 + n < N) copy_async<sizeof(T)>(Bs + n * pa + k, B + (int64_t)(k0 + k) * N + n0 + n);
+      }
+    }
+    copy_wait();
+    __syncthreads();
+    if (on && kc > 0) {
+      const T* a = As + mi * pa;
+      const T* b = Bs + ni * pa;
+      // the operands of the next four k are read, and their products formed, ahead of the sums of these
+      int k = 0;
+      if (kc >= 4) {
+        T x[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] = mul_rn(a[q], b[q]);
+        for (k = 4; k + 4 <= kc; k += 4) {
+          T y[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) y[q] = mul_rn(a[k + q], b[k + q]);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) { acc = add_rn(acc, x[q]); x[q] = y[q]; }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc = add_rn(acc, x[q]);
+      }
+      for (; k < kc; ++k) acc = add_rn(acc, mul_rn(a[k], b[k]));
+    }
+  }
+  if (on && m0 + mi < M && n0 + ni < N) C[(int64_t)(m0 + mi) * N + n0 + ni] = mul_rn((T)p->alpha, acc);
+}
+
+template <typename A> __device__ __forceinline__ A warp_sum(A v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <typename T> __device__ __forceinline__ T sine_exp(T x) { return (T)exp((double)(T)sin((double)x)); }
+
+// ---- row-wise operations: one warp per row, eight rows per piece (the arithmetic of the kernels in rowops.cu); column sums
+// and transposes: 256 outputs per piece
+template <typename T>
+__device__ void run_rows(const RowProg* p, int chunk) {
+  const int lane = threadIdx.x & 31, cols = p->cols;
+  const T* x = (const T*)p->in[0];
+  const T* in1 = (const T*)p->in[1];
+  T* out = (T*)p->out[0];
+  if (p->h.kind == PRIM_COLUMN_SUM) {        // out[j] = scalar * sum of rows (scalar 1: as is)
+    const int64_t j = (int64_t)chunk * NT + threadIdx.x;
+    if (j >= cols) return;
+    double acc = 0.0;
+    int64_t r = 0;
+    for (; r + 4 <= p->rows; r += 4) {
+      T v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = x[(r + q) * cols + j];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc += (double)v[q];
+    }
+    for (; r < p->rows; ++r) acc += (double)x[r * cols + j];
+    out[j] = (T)acc;
+    return;
+  }
+  if (p->h.kind == PRIM_TRANSPOSE) {
+    const int64_t e = (int64_t)chunk * NT + threadIdx.x, per = p->rows * cols;
+    if (e >= per * p->depth) return;
+    const int64_t d = e / per, q = e % per, c = q / p->rows, r = q % p->rows;
+    out[e] = x[d * per + r * cols + c];
+    return;
+  }
+  const int64_t r = (int64_t)chunk * (NT / 32) + (threadIdx.x >> 5);
+  if (r >= p->rows) return;
+  const T* xr = x + r * cols;
+  T* yr = out + r * cols;
+  switch (p->h.kind) {
+    case PRIM_SOFTMAX: {
+      T mx = -INFINITY;
+      for (int j = lane; j < cols; j += 32) { const T v = xr[j]; mx = v > mx ? v : mx; }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) { const T u = __shfl_xor_sync(0xffffffffu, mx, o); mx = u > mx ? u : mx; }
+      T sum = 0;
+      for (int j = lane; j < cols; j += 32) sum += t_exp(sub_rn(xr[j], mx));
+      sum = warp_sum(sum);
+      for (int j = lane; j < cols; j += 32) yr[j] = div_rn(t_exp(sub_rn(xr[j], mx)), sum);
+      break;
+    }
+    case PRIM_SOFTMAX_BACKWARD: {            // in: y, dy
+      const T* dr = in1 + r * cols;
+      T dot = 0;
+      for (int j = lane; j < cols; j += 32) dot += mul_rn(dr[j], xr[j]);
+      dot = warp_sum(dot);
+      for (int j = lane; j < cols; j += 32) yr[j] = mul_rn(xr[j], sub_rn(dr[j], dot));
+      break;
+    }
+    case PRIM_SINE_SOFTMAX: case PRIM_SINE_SOFTMAX_BACKWARD: {
+      T m = 0;
+      for (int j = lane; j < cols; j += 32) m += sine_exp<T>(xr[j]);
+      m = warp_sum(m);
+      for (int j = lane; j < cols; j += 32) {
+        const T e = sine_exp<T>(xr[j]);
+        if (p->h.kind == PRIM_SINE_SOFTMAX) {
+          yr[j] = div_rn(e, add_rn(m, e));
+        } else {
+          const T num = mul_rn(mul_rn(m, e), (T)cos((double)xr[j])), s = add_rn(m, e);
+          yr[j] = mul_rn(in1[r * cols + j], div_rn(num, mul_rn(s, s)));
+        }
+      }
+      break;
+    }
+    case PRIM_LAYERNORM: {                   // out: y, mean, sigma
+      double s = 0.0;
+      for (int j = lane; j < cols; j += 32) s += (double)xr[j];
+      s = warp_sum(s);
+      const T mu = (T)(s / (double)cols);
+      double v = 0.0;
+      for (int j = lane; j < cols; j += 32) { const T d = sub_rn(xr[j], mu); v += (double)mul_rn(d, d); }
+      v = warp_sum(v);
+      const T sd = sqrt_rn(div_rn((T)v, (T)cols));
+      if (lane == 0) { ((T*)p->out[1])[r] = mu; ((T*)p->out[2])[r] = sd; }
+      const T den = add_rn(sd, sizeof(T) == 4 ? (T)1e-9f : (T)1e-9);
+      for (int j = lane; j < cols; j += 32) yr[j] = div_rn(sub_rn(xr[j], mu), den);
+      break;
+    }
+    case PRIM_LAYERNORM_BACKWARD: {          // in: x, mean, sigma, dy
+      const T mu = in1[r], se = add_rn(((const T*)p->in[2])[r], sizeof(T) == 4 ? (T)1e-9f : (T)1e-9);
+      const T* dr = (const T*)p->in[3] + r * cols;
+      const T exp1 = mul_rn(sub_rn((T)1, div_rn((T)1, (T)cols)), div_rn((T)1, se));
+      const T den = mul_rn((T)cols, mul_rn(mul_rn(se, se), se));
+      for (int j = lane; j < cols; j += 32) {
+        const T d = sub_rn(xr[j], mu);
+        yr[j] = mul_rn(dr[j], sub_rn(exp1, div_rn(mul_rn(d, d), den)));
+      }
+      break;
+    }
+  }
+}
+
+template <typename T> constexpr int smem_bytes() {
+  const int slots = SLOTS * NT * (int)sizeof(T);
+  return MAX_ITEMS * (int)sizeof(Item) + 2 * PROG_BYTES + (slots > STAGE_BYTES ? slots : STAGE_BYTES);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(NT)
+walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ items, const int* __restrict__ count) {
+  extern __shared__ __align__(16) unsigned char gp_smem[];
+  Item* mine = reinterpret_cast<Item*>(gp_smem);
+  unsigned char* prog = gp_smem + MAX_ITEMS * sizeof(Item);
+  unsigned char* work = prog + 2 * PROG_BYTES;
+  const int n = count[blockIdx.x];
+  for (int i = threadIdx.x; i < n; i += NT) mine[i] = items[(size_t)blockIdx.x * MAX_ITEMS + i];
+  __syncthreads();
+  auto fetch = [&](int i) {
+    if (i < n)
+      for (uint32_t b = threadIdx.x * 8; b < mine[i].bytes; b += NT * 8) copy_async<8>(prog + (i & 1) * PROG_BYTES + b, blob + mine[i].prog + b);
+  };
+  fetch(0);
+  for (int i = 0; i < n; ++i) {
+    copy_wait();
+    __syncthreads();                         // this piece's program is here, the last piece is done with the working memory
+    fetch(i + 1);
+    if (mine[i].bytes) {
+      const Head* h = reinterpret_cast<const Head*>(prog + (i & 1) * PROG_BYTES);
+      if (h->kind <= PRIM_LAST_ELEMENTWISE) run_elementwise<T>(h, (int)mine[i].chunk, reinterpret_cast<T(*)[NT]>(work));
+      else if (h->kind == PRIM_PRODUCT) run_product<T>(reinterpret_cast<const ProductProg*>(h), (int)mine[i].chunk, reinterpret_cast<T*>(work));
+      else run_rows<T>(reinterpret_cast<const RowProg*>(h), (int)mine[i].chunk);
+    }
+    if (mine[i].barrier) cluster_barrier();
+  }
+}
+
+}  // namespace gp
+
+struct GraphPlan {
+  int device = 0, ctas = 0;
+  prad_dtype dt = PRAD_F32;
+  void* mem = nullptr;                       // [items][count][blob]
+  const unsigned char* blob = nullptr;
+  const gp::Item* items = nullptr;
+  const int* count = nullptr;
+};
+
+void GraphPlanFree::operator()(GraphPlan* p) const {
+  if (!p) return;
+  if (p->mem) {
+    cudaSetDevice(p->device);
+    cudaFree(p->mem);                        // waits for a run that may still read it
+  }
+  delete p;
+}
+
+namespace gp {
+
+static bool elementwise(const Prim& p) { return p.kind <= PRIM_LAST_ELEMENTWISE; }
+
+// What an operation reads and writes.  `local`: value i of the operation touches element i of the buffer only.
+struct Access { uintptr_t lo, hi; bool write, local; };
+
+static void accesses(const Prim& p, size_t es, std::vector<Access>& out) {
+  out.clear();
+  auto add = [&](const void* q, int64_t elems, bool write, bool local) {
+    if (q && elems > 0) out.push_back({(uintptr_t)q, (uintptr_t)q + (size_t)elems * es, write, local});
+  };
+  if (elementwise(p)) {
+    for (size_t i = 0; i < p.in.size(); ++i)
+      if (p.kind == PRIM_ADD_ROW && i == 1) add(p.in[i], p.cols, false, false);
+      else add(p.in[i], p.n, false, true);
+    for (void* q : p.out) add(q, p.n, true, true);
+    return;
+  }
+  if (p.kind == PRIM_PRODUCT) {
+    add(p.in[0], (p.batch - 1) * p.sA + (int64_t)p.M * p.K, false, false);
+    add(p.in[1], (p.batch - 1) * p.sB + (int64_t)p.K * p.N, false, false);
+    add(p.out[0], (p.batch - 1) * p.sC + (int64_t)p.M * p.N, true, false);
+    return;
+  }
+  const int64_t all = p.rows * p.cols * p.depth;
+  switch (p.kind) {
+    case PRIM_COLUMN_SUM: add(p.in[0], all, false, false); add(p.out[0], p.cols, true, false); return;
+    case PRIM_LAYERNORM:
+      add(p.in[0], all, false, false);
+      add(p.out[0], all, true, false);
+      add(p.out[1], p.rows, true, false);
+      add(p.out[2], p.rows, true, false);
+      return;
+    case PRIM_LAYERNORM_BACKWARD:
+      add(p.in[0], all, false, false);
+      add(p.in[1], p.rows, false, false);
+      add(p.in[2], p.rows, false, false);
+      add(p.in[3], all, false, false);
+      add(p.out[0], all, true, false);
+      return;
+    default:
+      for (const void* q : p.in) add(q, all, false, false);
+      add(p.out[0], all, true, false);
+  }
+}
+
+// Memory as regions with their last writers and the readers since.  Accesses that overlap without being the same join their
+// regions (gradient destinations that are parts of one buffer, say, only ever meet themselves).
+struct Region {
+  uintptr_t lo, hi;
+  bool local;                                // every access so far was element-local to the same interval
+  std::vector<int> writers, readers;
+};
+
+// An elementwise program in the making.
+struct Group {
+  int64_t n = 0;
+  std::vector<int> ops;                      // ascending
+};
+
+// (buffer, columns of a row operand or 0): what has a place of its own in a program
+using Place = std::pair<const void*, int>;
+static Place place_of(const Prim& p, size_t k) { return {p.in[k], p.kind == PRIM_ADD_ROW && k == 1 ? p.cols : 0}; }
+static int places(const std::vector<Prim>& all, const std::vector<int>& ops) {
+  std::vector<Place> seen;
+  for (int o : ops) {
+    for (size_t k = 0; k < all[o].in.size(); ++k) seen.push_back(place_of(all[o], k));
+    for (void* q : all[o].out) seen.push_back({q, 0});
+  }
+  std::sort(seen.begin(), seen.end());
+  return (int)(std::unique(seen.begin(), seen.end()) - seen.begin());
+}
+
+struct Piece { uint32_t prog, bytes, chunk; double cost; };
+
+// Time of an operation's own launch on the whole device, for comparison (us).
+static double launch_cost(const Prim& p, int sms) {
+  const double base = 2.6;
+  if (p.kind == PRIM_PRODUCT) {
+    const double outs = (double)p.M * p.N * p.batch;
+    return base + p.K * 0.013 * std::max(1.0, outs / 256.0 / sms / 2.0);
+  }
+  const double n = elementwise(p) ? (double)p.n : (double)p.rows * p.cols * p.depth;
+  return base + n / 400e3;
+}
+
+template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& ops, int ctas, std::vector<unsigned char>& blob,
+                                        std::vector<std::vector<Item>>& lists, double* est_us, double* launch_us) {
+  const size_t es = sizeof(T);
+  const int N = (int)ops.size();
+  std::vector<int> level(N, 0), group_of(N, -1);
+  std::vector<Group> groups;
+  std::map<uintptr_t, Region> mem;
+  std::vector<Access> acc;
+  *launch_us = 0;
+  auto region_at = [&](const Access& a) -> Region& {
+    auto it = mem.upper_bound(a.lo);
+    if (it != mem.begin()) {
+      auto p = std::prev(it);
+      if (p->second.hi > a.lo) it = p;
+    }
+    if (it == mem.end() || it->first >= a.hi) return mem.emplace(a.lo, Region{a.lo, a.hi, true, {}, {}}).first->second;
+    if (it->first == a.lo && it->second.hi == a.hi) return it->second;
+    Region joined{a.lo, a.hi, false, {}, {}};      // overlaps: one region for all of them
+    while (it != mem.end() && it->first < a.hi) {
+      joined.lo = std::min(joined.lo, it->first);
+      joined.hi = std::max(joined.hi, it->second.hi);
+      joined.writers.insert(joined.writers.end(), it->second.writers.begin(), it->second.writers.end());
+      joined.readers.insert(joined.readers.end(), it->second.readers.begin(), it->second.readers.end());
+      it = mem.erase(it);
+    }
+    const uintptr_t lo = joined.lo;
+    return mem.emplace(lo, std::move(joined)).first->second;
+  };
+  for (int i = 0; i < N; ++i) {
+    *launch_us += launch_cost(ops[i], ctx->sm_count);
+    accesses(ops[i], es, acc);
+    int lv = 0;
+    std::vector<int> near;                   // operations this one may share a program with
+    for (const Access& a : acc) {
+      Region& r = region_at(a);
+      auto depend = [&](int d) {
+        if (d == i) return;
+        const bool local = a.local && r.local && elementwise(ops[i]) && elementwise(ops[d]) && ops[i].n == ops[d].n;
+        lv = std::max(lv, local ? level[d] : level[d] + 1);
+        if (local) near.push_back(d);
+      };
+      for (int d : r.writers) depend(d);
+      if (a.write)
+        for (int d : r.readers) depend(d);
+    }
+    if (elementwise(ops[i])) {
+      // join the programs of the local neighbours at this level, if one program can hold them all
+      Group merged;
+      merged.n = ops[i].n;
+      std::vector<int> join;
+      for (int d : near)
+        if (level[d] == lv && std::find(join.begin(), join.end(), group_of[d]) == join.end()) join.push_back(group_of[d]);
+      for (int g : join) merged.ops.insert(merged.ops.end(), groups[g].ops.begin(), groups[g].ops.end());
+      std::sort(merged.ops.begin(), merged.ops.end());
+      merged.ops.push_back(i);
+      if (!join.empty() && ((int)merged.ops.size() > MAX_INS || places(ops, merged.ops) > SLOTS)) {
+        ++lv;                                // a program of its own, behind a barrier
+        join.clear();
+        merged.ops.assign(1, i);
+      }
+      for (int g : join) groups[g].ops.clear();
+      const int id = (int)groups.size();
+      for (int o : merged.ops) group_of[o] = id;
+      groups.push_back(std::move(merged));
+    }
+    level[i] = lv;
+    for (const Access& a : acc) {
+      Region& r = region_at(a);
+      r.local = r.local && a.local;
+      if (!a.write) { r.readers.push_back(i); continue; }
+      if (r.lo == a.lo && r.hi == a.hi) { r.writers.clear(); r.readers.clear(); }
+      r.writers.push_back(i);
+    }
+  }
+
+  // programs, and the pieces of every level
+  const int levels = N ? *std::max_element(level.begin(), level.end()) + 1 : 0;
+  std::vector<std::vector<Piece>> pieces(levels);
+  auto put = [&](const void* p, size_t bytes) {
+    const size_t at = blob.size();
+    blob.resize(at + ((bytes + 15) & ~(size_t)15));
+    memcpy(blob.data() + at, p, bytes);
+    return (uint32_t)at;
+  };
+  for (int i = 0; i < N; ++i) {
+    const Prim& p = ops[i];
+    if (elementwise(p)) {
+      const Group& g = groups[group_of[i]];
+      if (g.ops.front() != i) continue;
+      std::vector<Load> loads;
+      std::vector<Ins> ins;
+      std::vector<Store> stores;
+      std::map<Place, int> slot;
+      int slots = 0;
+      for (int o : g.ops) {
+        const Prim& q = ops[o];
+        Ins c;
+        memset(&c, 0, sizeof(c));
+        c.op = (uint8_t)q.kind;
+        c.act = (uint8_t)q.act;
+        c.n_in = (uint8_t)q.in.size();
+        c.scalar = q.scalar;
+        for (size_t k = 0; k < q.in.size(); ++k) {
+          const Place at = place_of(q, k);
+          auto it = slot.find(at);
+          if (it == slot.end()) {
+            it = slot.emplace(at, slots++).first;
+            loads.push_back({at.first, (uint32_t)at.second, (uint32_t)it->second});
+          }
+          c.src[k] = (uint8_t)it->second;
+        }
+        for (size_t k = 0; k < q.out.size(); ++k) {
+          auto it = slot.find(Place{q.out[k], 0});
+          if (it == slot.end()) it = slot.emplace(Place{q.out[k], 0}, slots++).first;
+          c.dst[k] = (uint8_t)it->second;
+          bool stored = false;
+          for (const Store& s : stores) stored = stored || s.p == q.out[k];
+          if (!stored) stores.push_back({q.out[k], (uint32_t)it->second, 0});
+        }
+        ins.push_back(c);
+      }
+      Head h{};
+      h.kind = PRIM_ACT_FORWARD;
+      h.n_load = (int)loads.size();
+      h.n_ins = (int)ins.size();
+      h.n_store = (int)stores.size();
+      h.n = g.n;
+      std::vector<unsigned char> prog(sizeof(Head) + loads.size() * sizeof(Load) + ins.size() * sizeof(Ins) + stores.size() * sizeof(Store));
+      unsigned char* w = prog.data();
+      memcpy(w, &h, sizeof(h)); w += sizeof(h);
+      memcpy(w, loads.data(), loads.size() * sizeof(Load)); w += loads.size() * sizeof(Load);
+      memcpy(w, ins.data(), ins.size() * sizeof(Ins)); w += ins.size() * sizeof(Ins);
+      memcpy(w, stores.data(), stores.size() * sizeof(Store));
+      const uint32_t at = put(prog.data(), prog.size());
+      double cost = 0.9 + 0.02 * (double)loads.size() + 0.06 * (double)ins.size();
+      for (const Ins& c : ins) cost += c.op == PRIM_ACT_FORWARD || c.op == PRIM_ACT_BACKWARD ? 0.15 : 0;
+      for (int64_t c = 0; c < ceil_div(g.n, NT); ++c) pieces[level[i]].push_back({at, (uint32_t)((prog.size() + 7) & ~(size_t)7), (uint32_t)c, cost});
+      continue;
+    }
+    if (p.kind == PRIM_PRODUCT) {
+      ProductProg q{};
+      q.h.kind = PRIM_PRODUCT;
+      q.A = p.in[0]; q.B = p.in[1]; q.C = p.out[0];
+      q.sA = p.sA; q.sB = p.sB; q.sC = p.sC;
+      q.alpha = p.scalar;
+      q.tA = p.tA; q.tB = p.tB; q.M = p.M; q.N = p.N; q.K = p.K;
+      q.tn = p.N >= 16 ? 16 : p.N >= 8 ? 8 : p.N >= 4 ? 4 : p.N >= 2 ? 2 : 1;
+      q.tm = std::min(NT / q.tn, 64);
+      q.ks = std::min(p.K, STAGE_BYTES / (int)es / (q.tm + q.tn) - 1);     // (the pitch is ks or ks + 1)
+      q.tiles_n = (int)ceil_div(p.N, q.tn);
+      q.tiles_mn = (int)ceil_div(p.M, q.tm) * q.tiles_n;
+      const uint32_t at = put(&q, sizeof(q));
+      const double cost = 1.2 + p.K * (es == 8 ? 0.017 : 0.012) + 0.5 * (double)(ceil_div(p.K, q.ks) - 1);
+      for (int64_t c = 0; c < (int64_t)q.tiles_mn * p.batch; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 7) & ~(size_t)7), (uint32_t)c, cost});
+      continue;
+    }
+    RowProg q{};
+    q.h.kind = p.kind;
+    for (size_t k = 0; k < p.in.size(); ++k) q.in[k] = p.in[k];
+    for (size_t k = 0; k < p.out.size(); ++k) q.out[k] = p.out[k];
+    q.rows = p.rows; q.cols = p.cols; q.depth = p.depth;
+    q.scalar = p.scalar;
+    int64_t chunks;
+    double cost;
+    if (p.kind == PRIM_COLUMN_SUM) { chunks = ceil_div(p.cols, NT); cost = 0.8 + 0.15 * (double)p.rows; }
+    else if (p.kind == PRIM_TRANSPOSE) { chunks = ceil_div(p.rows * p.cols * p.depth, NT); cost = 0.9; }
+    else { q.rows = p.rows * p.depth; chunks = ceil_div(q.rows, NT / 32); cost = 2.0 + 0.1 * (double)p.cols; }
+    const uint32_t at = put(&q, sizeof(q));
+    for (int64_t c = 0; c < chunks; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 7) & ~(size_t)7), (uint32_t)c, cost});
+  }
+
+  // deal the pieces of a level to the CTAs, the longest first to whoever has least; a barrier behind every level
+  lists.assign(ctas, {});
+  *est_us = 4.0;
+  std::vector<double> busy(ctas);
+  for (int lv = 0; lv < levels; ++lv) {
+    std::stable_sort(pieces[lv].begin(), pieces[lv].end(), [](const Piece& a, const Piece& b) { return a.cost > b.cost; });
+    std::fill(busy.begin(), busy.end(), 0.0);
+    std::vector<size_t> before(ctas);
+    for (int c = 0; c < ctas; ++c) before[c] = lists[c].size();
+    for (const Piece& p : pieces[lv]) {
+      const int c = (int)(std::min_element(busy.begin(), busy.end()) - busy.begin());
+      busy[c] += p.cost;
+      lists[c].push_back({p.prog, p.bytes, p.chunk, 0});
+    }
+    for (int c = 0; c < ctas; ++c) {
+      if (lists[c].size() == before[c]) lists[c].push_back({0, 0, 0, 1});
+      else lists[c].back().barrier = 1;
+    }
+    *est_us += 0.4 + *std::max_element(busy.begin(), busy.end());
+  }
+}
+
+// 16 CTAs if the device runs such a cluster of this kernel, else 8, else none
+template <typename T> static int cluster_ctas(prad_ctx* ctx) {
+  static std::atomic<int> known[64];
+  std::atomic<int>& k = known[ctx->device & 63];
+  int n = k.load(std::memory_order_acquire);
+  if (n) return n - 1;
+  n = 0;
+  cudaError_t e = cudaFuncSetAttribute(walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<T>());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(walk_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  for (int cs : {16, 8}) {
+    if (e != cudaSuccess || n) break;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)cs);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem_bytes<T>();
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, walk_kernel<T>, &cfg) == cudaSuccess && fit > 0) n = cs;
+    else (void)cudaGetLastError();
+  }
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  k.store(n + 1, std::memory_order_release);
+  return n;
+}
+
+template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype dt, const std::vector<Prim>& ops) {
+  if (ops.size() < 3 || ops.size() > 20000) return nullptr;
+  const int ctas = cluster_ctas<T>(ctx);
+  if (!ctas) return nullptr;
+  // an operation that deserves the whole device makes the walk one for separate launches
+  for (const Prim& p : ops) {
+    if (p.kind == PRIM_PRODUCT && (p.K < 1 || (double)p.M * p.N * p.K * p.batch > 4e6)) return nullptr;
+    if (elementwise(p) ? p.n > 65536 : p.kind != PRIM_PRODUCT && (double)p.rows * p.cols * p.depth > 65536) return nullptr;
+    if (p.in.size() > 8) return nullptr;
+  }
+  std::vector<unsigned char> blob;
+  std::vector<std::vector<Item>> lists;
+  double est = 0, launches = 0;
+  build<T>(ctx, ops, ctas, blob, lists, &est, &launches);
+  size_t most = 0;
+  for (auto& l : lists) most = std::max(most, l.size());
+  if (est >= launches || most > MAX_ITEMS) return nullptr;
+  const size_t items_bytes = (size_t)ctas * MAX_ITEMS * sizeof(Item), count_bytes = 256;
+  std::vector<unsigned char> host(items_bytes + count_bytes + blob.size());
+  for (int c = 0; c < ctas; ++c) {
+    memcpy(host.data() + (size_t)c * MAX_ITEMS * sizeof(Item), lists[c].data(), lists[c].size() * sizeof(Item));
+    const int n = (int)lists[c].size();
+    memcpy(host.data() + items_bytes + c * sizeof(int), &n, sizeof(int));
+  }
+  memcpy(host.data() + items_bytes + count_bytes, blob.data(), blob.size());
+  GraphPlanPtr plan(new GraphPlan());
+  plan->device = ctx->device;
+  plan->ctas = ctas;
+  plan->dt = dt;
+  if (device_malloc(&plan->mem, host.size()) != cudaSuccess ||
+      cudaMemcpyAsync(plan->mem, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
+      cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  plan->items = (const Item*)plan->mem;
+  plan->count = (const int*)((const unsigned char*)plan->mem + items_bytes);
+  plan->blob = (const unsigned char*)plan->mem + items_bytes + count_bytes;
+  return plan;
+}
+
+}  // namespace gp
+
+GraphPlanPtr graph_plan_build(prad_ctx* ctx, prad_dtype dt, const std::vector<Prim>& ops) {
+  return dt == PRAD_F32 ? gp::build_plan<float>(ctx, dt, ops) : gp::build_plan<double>(ctx, dt, ops);
+}
+
+prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = plan->ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)plan->ctas);
+  cfg.blockDim = dim3(gp::NT);
+  cfg.stream = ctx->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (plan->dt == PRAD_F32) {
+    cfg.dynamicSmemBytes = gp::smem_bytes<float>();
+    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<float>, plan->blob, plan->items, plan->count));
+  } else {
+    cfg.dynamicSmemBytes = gp::smem_bytes<double>();
+    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<double>, plan->blob, plan->items, plan->count));
+  }
+  PRAD_LAUNCHED(ctx);
+  return PRAD_OK;
+}
+
+}  // namespace prad

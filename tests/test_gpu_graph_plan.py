@@ -1,0 +1,105 @@
+"""Graph walks as one kernel against one launch per operation: every operation type, shared and deep values, fan-in beyond
+eight, pieces at the edges of 256 elements and of the product tiles, gradient destinations in one buffer."""
+import numpy as np
+import pytest
+
+from parallelreverseautodiff_b200 import engine as E
+from parallelreverseautodiff_b200.graph import Graph
+from util import rng
+
+pytestmark = pytest.mark.gpu
+
+
+def _network(g, eng, dt, rows, cols, inner, r, store):
+    """A graph that uses every node type; `store` keeps (weight, gradient) matrices."""
+    up = lambda *s: eng.upload((r.standard_normal(s) * 0.5).astype(dt))  # noqa: E731
+
+    def weight(*s):
+        m, d = up(*s), eng.zeros(s, dt)
+        store.append(d)
+        return g.weight(m, d)
+
+    x = g.input(up(rows, inner))
+    h = g.node("MatrixMultiplyOperation", [x, weight(inner, cols)])
+    h = g.node("MatrixAddBroadcastingOperation", [h, weight(1, cols)])
+    parts = []
+    for op in ("LeakyReLUOperation", "SigmoidOperation", "TanhOperation", "GELUOperation", "ReLUOperation", "AmplifiedSigmoidOperation",
+               "SoftmaxOperation", "LayerNormalizationOperation", "SineSoftmaxOperation"):
+        parts.append(g.node(op, [h], scalar=0.01))
+    had = g.node("HadamardProductOperation", [parts[0], parts[1]])
+    s3 = g.node("MatrixAddThreeOperation", [had, parts[2], parts[3]])
+    s3 = g.node("MatrixAddOperation", [s3, parts[4]])
+    s3 = g.node("MatrixMultiplyScalarOperation", [s3], scalar=0.7)
+    for p in parts[5:]:
+        s3 = g.node("MatrixAddOperation", [s3, p])
+    t = g.node("MatrixTransposeOperation", [s3])
+    q = g.node("MatrixMultiplyOperation", [t, s3])               # cols x cols
+    w = weight(cols, cols)
+    outs = [g.node("MatrixMultiplyOperation", [q, w]), g.node("HadamardProductOperation", [q, w])]
+    return g.node("MatrixAddOperation", outs), outs[0]
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("rows,cols,inner", [(1, 1, 1), (3, 5, 2), (16, 16, 300), (17, 31, 9), (64, 8, 64), (65, 33, 40), (100, 1, 7)])
+def test_plan_equals_separate_launches(engine, dtype, rows, cols, inner):
+    results = []
+    for plan in ("1", "0"):
+        r = rng(rows * 10 + cols)
+        engine.set_option("graph_plan", plan)
+        try:
+            store = []
+            g = Graph(engine, dtype)
+            end, mid = _network(g, engine, dtype, rows, cols, inner, r, store)
+            d = engine.upload(r.standard_normal((cols, cols)).astype(dtype))
+            got, launches = [], []
+            for _ in range(2):                        # the second pass adds to the destinations
+                n0 = engine.launch_count()
+                g.forward()
+                g.backward(end, d)
+                launches.append(engine.launch_count() - n0)
+                got += [g.data(end).numpy(), g.gradient(mid).numpy()] + [s.numpy() for s in store]
+            assert g.consumers(mid) == 1
+            results.append((got, launches))
+            g.close()
+        finally:
+            engine.set_option("graph_plan", "1")
+    (a, la), (b, lb) = results
+    assert la == [2, 2] and lb[0] > 40
+    tol = dict(rtol=1e-12, atol=1e-12) if dtype == np.float64 else dict(rtol=1e-5, atol=1e-5)   # (row and column sums)
+    for x, y in zip(a, b):
+        np.testing.assert_allclose(x, y, **tol)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_products_sums_and_elementwise_chains_are_the_same_bits(engine, dtype):
+    """Shared weights over many uses (fan-in and += chains longer than eight), one flat gradient buffer, changing start gradients."""
+    n, uses = 37, 11
+    results = []
+    for plan in ("1", "0"):
+        r = rng(3)
+        engine.set_option("graph_plan", plan)
+        try:
+            flat = engine.zeros((2 * n * n,), dtype)
+            wm = engine.upload((r.standard_normal((n, n)) * 0.3).astype(dtype))
+            g = Graph(engine, dtype)
+            h = x = g.input(engine.upload(r.standard_normal((n, n)).astype(dtype)))
+            hs = []
+            for k in range(uses):
+                w = g.weight(wm, flat.view((n, n), (k % 2) * n * n))
+                h = g.node("TanhOperation", [g.node("MatrixMultiplyOperation", [w, h])])
+                hs.append(g.node("HadamardProductOperation", [h, x]))
+            total = hs[0]
+            for k in hs[1:]:
+                total = g.node("MatrixAddOperation", [total, k])
+            starts = [engine.upload(r.standard_normal((n, n)).astype(dtype)) for _ in range(6)]
+            got = []
+            for d in starts + starts[:2]:
+                g.forward()
+                g.backward(total, d)
+                got += [g.data(total).numpy(), g.gradient(x).numpy(), flat.numpy()]
+            results.append(got)
+            g.close()
+        finally:
+            engine.set_option("graph_plan", "1")
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
