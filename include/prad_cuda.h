@@ -615,6 +615,9 @@ prad_status prad_graph_add_value(prad_graph* g, int rows, int cols, void* data, 
 prad_status prad_graph_add_deep_value(prad_graph* g, int depth, int rows, int cols, void* data, int* out_value);
 /* Weight-style value: its gradient is ADDED into this caller-owned matrix on every backward. */
 prad_status prad_graph_set_gradient_destination(prad_graph* g, int value, void* grad_matrix);
+/* NeuralNetwork.AutomaticForwardPropagate's CopyResult: after every prad_graph_forward the value's data is copied to `matrix`
+ * (of the value's size), in the order of these calls. */
+prad_status prad_graph_set_result_copy(prad_graph* g, int value, void* matrix);
 /* Nodes must be added in forward (topological) order; `out_value` must be graph-owned. */
 prad_status prad_graph_add_node(prad_graph* g, prad_op op, const int* in_values, int n_in,
                                 int out_value, double scalar, int* out_node);

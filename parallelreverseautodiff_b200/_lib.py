@@ -125,6 +125,7 @@ SIGNATURES = {
     "prad_graph_add_value": [vp, i32, i32, vp, C.POINTER(C.c_int)],
     "prad_graph_add_deep_value": [vp, i32, i32, i32, vp, C.POINTER(C.c_int)],
     "prad_graph_set_gradient_destination": [vp, i32, vp],
+    "prad_graph_set_result_copy": [vp, i32, vp],
     "prad_graph_add_node": [vp, i32, C.POINTER(C.c_int), i32, i32, f64, C.POINTER(C.c_int)],
     "prad_graph_forward": [vp],
     "prad_graph_backward": [vp, i32, vp],

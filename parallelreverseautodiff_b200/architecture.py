@@ -100,7 +100,6 @@ class ArchitectureGraph:
         self.operations: Dict[str, OperationRef] = {}
         self.order: List[OperationRef] = []               # StartOperation, .Next, ...
         self._keep = []
-        self._copies = []                                 # (operation, destination matrix) of setResultTo
 
     def close(self) -> None:
         if self.h:
@@ -259,14 +258,13 @@ class ArchitectureGraph:
             dst = self._intermediates[key](li)
             if tuple(dst.shape) != tuple(out_shape):
                 raise ArchitectureError(f"setResultTo '{key}' of '{ref.Id}': shape {dst.shape} does not match {out_shape}")
-            self._copies.append((ref, dst))
+            check(self.eng.lib.prad_graph_set_result_copy(self.h, ref.value, C.c_void_p(dst.ptr)))
+            self._keep.append(dst)
 
     # ------------------------------------------------------------ execution
     def forward(self) -> None:
         """Every operation's Forward in list order, then the setResultTo copies."""
         check(self.eng.lib.prad_graph_forward(self.h))
-        for ref, dst in self._copies:
-            self.eng.copy(dst, self.output(ref.SpecificId))
 
     def backward(self, starts: Union[str, Sequence[str]], gradients: Union[E.DeviceMatrix, Sequence[E.DeviceMatrix]]) -> None:
         """Backward from one operation (``BackwardInput = dLoss`` + visitor traversal) or from several at

@@ -58,6 +58,7 @@ struct prad_graph {
   Walk forward_walk;
   std::vector<Walk> backward_walks;
   std::vector<prad::GraphPlanPtr> retired;
+  std::vector<std::pair<int, void*>> copies;    // (value, matrix its data is copied to after every forward)
   uint32_t magic = 0x47524146u;
 };
 
@@ -134,6 +135,9 @@ struct Ops {
   }
   prad_status scale(const void* x, void* y, int64_t n, double s) const {
     return rec ? each(PRIM_SCALE, {x}, {y}, n, 0, s) : prad_scale(c, dt, x, y, n, s);
+  }
+  prad_status copy(void* dst, const void* src, int64_t n) const {
+    return rec ? each(PRIM_COPY, {src}, {dst}, n) : prad_copy(c, dst, src, (size_t)n * dtype_size(dt));
   }
   prad_status accumulate(void* dst, const void* src, int64_t n) const {
     return rec ? each(PRIM_ADD2, {dst, src}, {dst}, n) : prad_accumulate(c, dt, dst, src, n);
@@ -264,6 +268,16 @@ prad_status prad_graph_set_gradient_destination(prad_graph* g, int value, void* 
   // plans have the old destination in them (a recorded launch sequence may still run one: those stay until the graph goes)
   for (auto& w : g->backward_walks) g->retired.push_back(std::move(w.plan));
   g->backward_walks.clear();
+  return PRAD_OK;
+}
+
+prad_status prad_graph_set_result_copy(prad_graph* g, int value, void* matrix) {
+  PRAD_CHECK_GRAPH(g);
+  PRAD_REQUIRE(value >= 0 && value < (int)g->values.size() && matrix, PRAD_ERR_INVALID,
+               "prad_graph_set_result_copy: bad value id or null matrix");
+  g->copies.emplace_back(value, matrix);
+  if (g->forward_walk.plan) g->retired.push_back(std::move(g->forward_walk.plan));
+  g->forward_walk.tried = false;
   return PRAD_OK;
 }
 
@@ -565,6 +579,7 @@ static prad_status forward_walk(prad_graph* g, const Ops& ops) {
       PRAD_REQUIRE(g->values[i].data, PRAD_ERR_INVALID, "prad_graph_forward: value %d has no data and no producer before its use", i);
     G_TRY(node_forward(g, n, ops));
   }
+  for (auto& k : g->copies) G_TRY(ops.copy(k.second, g->values[k.first].data, g->values[k.first].count()));
   return PRAD_OK;
 }
 

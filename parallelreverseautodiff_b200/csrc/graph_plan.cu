@@ -7,8 +7,10 @@
 // earlier levels only; chains of elementwise operations on the same elements (a gate's sum and activation, a cell update, the
 // += of a shared weight's gradients over the time steps) share a level too, as a small program that keeps every value of one
 // element in shared memory from its load to its store.  One cluster of 16 CTAs runs the levels with the cluster's hardware
-// barrier between them (no waiting loops, no other CTA to wait for); the pieces of a level -- 256 elements or 256 outputs each
-// -- are dealt to the CTAs when the plan is made, and a CTA fetches the next piece's program while it runs this one.
+// barrier between them (no waiting loops, no other CTA to wait for).  A level is latency: a barrier, a program, loads from L2,
+// a chain of 64 additions.  So the pieces of a level -- 64 or 256 elements, 256 or 1024 outputs -- are dealt to 64 workers when
+// the plan is made, four to an SM, and a worker fetches its next program while it runs this one. 
+// (One worker per SM took 240 us per walk of that LSTM, four take 150 us.)
 //
 // Values are those of the separate kernels bit for bit for elementwise operations and products (k ascending, product and sum
 // rounded separately); row reductions and column sums add in double or in the same lane order.  (Compiled with -fmad=false.)
@@ -22,19 +24,22 @@
 namespace prad {
 namespace gp {
 
-constexpr int NT = 256;
+constexpr int NT = 256;                   // threads of a worker
+constexpr int WORKERS = 4;                // workers of a CTA: a piece is mostly latency, so several share an SM
 constexpr int SLOTS = 64;                 // values of one element a program keeps
 constexpr int MAX_INS = 96;
 constexpr int PROG_BYTES = 32 + SLOTS * 16 + MAX_INS * 24 + SLOTS * 16;
-constexpr int MAX_ITEMS = 1024;           // pieces per CTA
-constexpr int STAGE_BYTES = 64 * 1024;    // operands of a product in shared memory
+constexpr int WORK_BYTES = 44 * 1024;     // a worker's shared memory: the slots of its elements, or the operands of a product
 
-// a piece of work of one CTA
+// a piece of one worker
 struct Item { uint32_t prog, bytes, chunk, barrier; };
 
-struct Head { int32_t kind, n_load, n_ins, n_store; int64_t n; int64_t pad; };
+// team: 4 where four threads share an element's instructions (a piece is 64 elements then), else 1
+struct Head { int32_t kind, n_load, n_ins, n_store; int64_t n; int64_t team; };
 struct Load { const void* p; uint32_t cols, slot; };        // cols: 0 = element i, else element i % cols
-struct Ins { uint8_t op, act, n_in, pad; uint8_t dst[2], pad2[2]; uint8_t src[8]; double scalar; };
+// phase: in the first instruction of a phase (instructions that do not touch one another's values), how many it has
+struct Ins { uint8_t op, act, n_in, phase; uint8_t dst[2], pad2[2]; uint8_t src[8]; double scalar; };
+constexpr uint8_t INS_FOLD = 64;          // ((src0 + src1) + src2) + ... in T: a run of dst += src
 struct Store { void* p; uint32_t slot, pad; };
 static_assert(sizeof(Head) == 32 && sizeof(Load) == 16 && sizeof(Ins) == 24 && sizeof(Store) == 16, "program layout");
 struct ProductProg {
@@ -43,7 +48,7 @@ struct ProductProg {
   void* C;
   int64_t sA, sB, sC;
   double alpha;
-  int32_t tA, tB, M, N, K, tm, tn, ks, tiles_n, tiles_mn;
+  int32_t tA, tB, M, N, K, tm, tn, ks, tiles_n, tiles_mn, r;   // r: r x r outputs per thread
 };
 struct RowProg { Head h; const void* in[4]; void* out[3]; int64_t rows; int32_t cols, depth; double scalar; };
 
@@ -56,113 +61,178 @@ template <int BYTES> __device__ __forceinline__ void copy_async(void* dst, const
 }
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// ---- elementwise programs: 256 elements, one per thread; v[slot][thread]
+// a worker's threads meet
+__device__ __forceinline__ void worker_sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)(threadIdx.x / NT)), "n"(NT) : "memory"); }
+
+// ---- elementwise programs
+// One instruction on one element; v[slot * stride] is the element's value in a slot.
 template <typename T>
-__device__ void run_elementwise(const Head* h, int chunk, T (*v)[NT]) {
-  const int tid = threadIdx.x;
-  const int64_t i = (int64_t)chunk * NT + tid;
-  if (i >= h->n) return;
+__device__ __forceinline__ void execute(const Ins& c, T* v, int stride) {
+  const T a = v[c.src[0] * stride], s = (T)c.scalar;
+  T r;
+  switch (c.op) {
+    case PRIM_ACT_FORWARD: r = act_value<T>((prad_act)c.act, a, s); break;
+    case PRIM_ACT_BACKWARD: r = mul_rn(v[c.src[1] * stride], act_derivative<T>((prad_act)c.act, a, s)); break;
+    case PRIM_ADD2: case PRIM_ADD_ROW: r = add_rn(a, v[c.src[1] * stride]); break;
+    case PRIM_ADD3: r = add_rn(add_rn(a, v[c.src[1] * stride]), v[c.src[2] * stride]); break;
+    case PRIM_MUL2: r = mul_rn(a, v[c.src[1] * stride]); break;
+    case PRIM_MUL_BACKWARD: {              // a, b, dy -> dy b, dy a
+      const T b = v[c.src[1] * stride], d = v[c.src[2] * stride];
+      v[c.dst[1] * stride] = mul_rn(d, a);
+      r = mul_rn(d, b);
+      break;
+    }
+    case PRIM_SCALE: r = mul_rn(a, s); break;
+    case PRIM_COPY: r = a; break;
+    case INS_FOLD: {
+      r = a;
+      for (int q = 1; q < c.n_in; ++q) r = add_rn(r, v[c.src[q] * stride]);
+      break;
+    }
+    default: {                             // PRIM_SUM: in list order, in double, cast once
+      double acc = (double)a;
+      for (int q = 1; q < c.n_in; ++q) acc += (double)v[c.src[q] * stride];
+      r = (T)acc;
+    }
+  }
+  v[c.dst[0] * stride] = r;
+}
+
+// A piece: 256 elements, one per thread, or 64 elements with four threads each, which take the loads, the instructions of a
+// phase and the stores in turn (four gates' exponentials side by side instead of one after another).
+template <typename T>
+__device__ void run_elementwise(const Head* h, int chunk, T* v) {
+  const int tid = threadIdx.x % NT, team = (int)h->team;
+  const int per = NT / team, e = tid % per, q0 = tid / per;
   const Load* ld = reinterpret_cast<const Load*>(h + 1);
   const Ins* ins = reinterpret_cast<const Ins*>(ld + h->n_load);
   const Store* st = reinterpret_cast<const Store*>(ins + h->n_ins);
-  for (int k = 0; k < h->n_load; ++k) {      // all on their way at once
-    const int64_t at = ld[k].cols ? i % ld[k].cols : i;
-    copy_async<sizeof(T)>(&v[ld[k].slot][tid], (const T*)ld[k].p + at);
-  }
+  const int64_t i = (int64_t)chunk * per + e;
+  const bool on = i < h->n;
+  v += e;
+  if (on)
+    for (int k = q0; k < h->n_load; k += team)      // all on their way at once
+      copy_async<sizeof(T)>(v + ld[k].slot * per, (const T*)ld[k].p + (ld[k].cols ? i % ld[k].cols : i));
   copy_wait();
-  for (int k = 0; k < h->n_ins; ++k) {
-    const Ins c = ins[k];
-    const T a = v[c.src[0]][tid], s = (T)c.scalar;
-    T r;
-    switch (c.op) {
-      case PRIM_ACT_FORWARD: r = act_value<T>((prad_act)c.act, a, s); break;
-      case PRIM_ACT_BACKWARD: r = mul_rn(v[c.src[1]][tid], act_derivative<T>((prad_act)c.act, a, s)); break;
-      case PRIM_ADD2: case PRIM_ADD_ROW: r = add_rn(a, v[c.src[1]][tid]); break;
-      case PRIM_ADD3: r = add_rn(add_rn(a, v[c.src[1]][tid]), v[c.src[2]][tid]); break;
-      case PRIM_MUL2: r = mul_rn(a, v[c.src[1]][tid]); break;
-      case PRIM_MUL_BACKWARD: {              // a, b, dy -> dy b, dy a
-        const T b = v[c.src[1]][tid], d = v[c.src[2]][tid];
-        v[c.dst[1]][tid] = mul_rn(d, a);
-        r = mul_rn(d, b);
-        break;
-      }
-      case PRIM_SCALE: r = mul_rn(a, s); break;
-      default: {                             // PRIM_SUM: in list order, in double, cast once
-        double acc = (double)a;
-        for (int q = 1; q < c.n_in; ++q) acc += (double)v[c.src[q]][tid];
-        r = (T)acc;
-      }
+  if (team > 1) {
+    worker_sync();
+    for (int k0 = 0; k0 < h->n_ins;) {
+      const int c = ins[k0].phase;
+      if (on)
+        for (int k = k0 + q0; k < k0 + c; k += team) execute<T>(ins[k], v, per);
+      worker_sync();
+      k0 += c;
     }
-    v[c.dst[0]][tid] = r;
+  } else if (on) {
+    for (int k = 0; k < h->n_ins; ++k) execute<T>(ins[k], v, per);
   }
-  for (int k = 0; k < h->n_store; ++k) ((T*)st[k].p)[i] = v[st[k].slot][tid];
+  if (on)
+    for (int k = q0; k < h->n_store; k += team) ((T*)st[k].p)[i] = v[st[k].slot * per];
 }
 
-// ---- products: a tm x tn tile, one output per thread, both operands of ks values of k in shared memory
-template <typename T>
+// ---- products: a tm x tn tile, R x R outputs per thread, both operands of ks values of k in shared memory
+// rows of 16-byte vectors plus one: the rows of neighbouring threads fall into different banks
+template <typename T> __host__ __device__ constexpr int product_pitch(int ks) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  return (ks + VEC - 1) / VEC * VEC + VEC;
+}
+// `rows` operand rows of kc values of k into s[row][pitch]; KC: memory is [row][k], otherwise [k][row] (rows a power of two)
+template <typename T, bool KC>
+__device__ __forceinline__ void copy_operand(T* s, int pitch, const T* g, int64_t ld, int row0, int X, int rows, int kc) {
+  const int tid = threadIdx.x % NT, lane = tid & 31, warp = tid >> 5;
+  if (KC) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    g += (int64_t)row0 * ld;
+    const bool vec = kc % VEC == 0 && ld % VEC == 0 && ((uintptr_t)g & 15) == 0;
+    for (int r = warp; r < rows && row0 + r < X; r += NT / 32)
+      if (vec) {
+        for (int k = lane * VEC; k < kc; k += 32 * VEC) {
+          const uint32_t d = (uint32_t)__cvta_generic_to_shared(s + r * pitch + k);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g + (int64_t)r * ld + k) : "memory");
+        }
+      } else {
+        for (int k = lane; k < kc; k += 32) copy_async<sizeof(T)>(s + r * pitch + k, g + (int64_t)r * ld + k);
+      }
+  } else {
+    const int sh = 31 - __clz(rows), r = tid & (rows - 1);
+    if (row0 + r < X)
+      for (int k = tid >> sh; k < kc; k += NT >> sh) copy_async<sizeof(T)>(s + r * pitch + k, g + (int64_t)k * ld + row0 + r);
+  }
+}
+
+template <typename T, int R>
 __device__ void run_product(const ProductProg* p, int chunk, T* smem) {
-  const int tid = threadIdx.x, tm = p->tm, tn = p->tn, ks = p->ks, K = p->K, M = p->M, N = p->N;
+  const int tid = threadIdx.x % NT, tm = p->tm, tn = p->tn, ks = p->ks, K = p->K, M = p->M, N = p->N;
   const int bz = chunk / p->tiles_mn, t2 = chunk % p->tiles_mn;
   const int m0 = t2 / p->tiles_n * tm, n0 = t2 % p->tiles_n * tn;
   const T* A = (const T*)p->A + bz * p->sA;
   const T* B = (const T*)p->B + bz * p->sB;
   T* C = (T*)p->C + bz * p->sC;
-  const int pa = ks | 1;                     // odd pitch: the rows of a warp's threads in different banks
+  const int pa = product_pitch<T>(ks);
   T* As = smem;                              // [tm][pa]
   T* Bs = smem + tm * pa;                    // [tn][pa]
-  const int mi = tid / tn, ni = tid % tn;
-  const bool on = mi < tm;
-  T acc = (T)0;
+  const int tx = tn / R, ty = tm / R, mi = tid / tx, ni = tid % tx;
+  const bool on = mi < ty;
+  T acc[R][R];
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < R; ++j) acc[i][j] = (T)0;
   for (int k0 = 0; k0 < K; k0 += ks) {
     const int kc = K - k0 < ks ? K - k0 : ks;
-    if (k0) __syncthreads();
-    if (p->tA) {                             // memory is [k][m]
-      for (int e = tid; e < kc * tm; e += NT) {
-        const int k = e / tm, m = e % tm;
-        if (m0 + m < M) copy_async<sizeof(T)>(As + m * pa + k, A + (int64_t)(k0 + k) * M + m0 + m);
-      }
-    } else {
-      for (int e = tid; e < tm * kc; e += NT) {
-        const int m = e / kc, k = e % kc;
-        if (m0 + m < M) copy_async<sizeof(T)>(As + m * pa + k, A + (int64_t)(m0 + m) * K + k0 + k);
-      }
-    }
-    if (p->tB) {                             // memory is [n][k]
-      for (int e = tid; e < tn * kc; e += NT) {
-        const int n = e / kc, k = e % kc;
-        if (n0 + n < N) copy_async<sizeof(T)>(Bs + n * pa + k, B + (int64_t)(n0 + n) * K + k0 + k);
-      }
-    } else {
-      for (int e = tid; e < kc * tn; e += NT) {
-        const int k = e / tn, n = e % tn;
-        if (n0 + n < N) copy_async<sizeof(T)>(Bs + n * pa + k, B + (int64_t)(k0 + k) * N + n0 + n);
-      }
-    }
+    if (k0) worker_sync();
+    if (p->tA) copy_operand<T, false>(As, pa, A + (int64_t)k0 * M, M, m0, M, tm, kc);
+    else copy_operand<T, true>(As, pa, A + k0, K, m0, M, tm, kc);
+    if (p->tB) copy_operand<T, true>(Bs, pa, B + k0, K, n0, N, tn, kc);
+    else copy_operand<T, false>(Bs, pa, B + (int64_t)k0 * N, N, n0, N, tn, kc);
     copy_wait();
-    __syncthreads();
-    if (on && kc > 0) {
+    worker_sync();
+    if (on) {
       const T* a = As + mi * pa;
       const T* b = Bs + ni * pa;
-      // the operands of the next four k are read, and their products formed, ahead of the sums of these
-      int k = 0;
-      if (kc >= 4) {
-        T x[4];
+      T x[R][R], y[R][R];
+      auto products = [&](T (&d)[R][R], int k) {
+        T av[R], bv[R];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) x[q] = mul_rn(a[q], b[q]);
-        for (k = 4; k + 4 <= kc; k += 4) {
-          T y[4];
+        for (int i = 0; i < R; ++i) { av[i] = a[i * ty * pa + k]; bv[i] = b[i * tx * pa + k]; }
 #pragma unroll
-          for (int q = 0; q < 4; ++q) y[q] = mul_rn(a[k + q], b[k + q]);
+        for (int i = 0; i < R; ++i)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) { acc = add_rn(acc, x[q]); x[q] = y[q]; }
-        }
+          for (int j = 0; j < R; ++j) d[i][j] = mul_rn(av[i], bv[j]);
+      };
+      auto sums = [&](const T (&d)[R][R]) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc = add_rn(acc, x[q]);
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int j = 0; j < R; ++j) acc[i][j] = add_rn(acc[i][j], d[i][j]);
+      };
+      // the products of the next k are formed ahead of the sums of this one
+      products(x, 0);
+      int k = 1;
+#pragma unroll 4
+      for (; k + 1 < kc; k += 2) {
+        products(y, k);
+        sums(x);
+        products(x, k + 1);
+        sums(y);
       }
-      for (; k < kc; ++k) acc = add_rn(acc, mul_rn(a[k], b[k]));
+      if (k < kc) {
+        products(y, k);
+        sums(x);
+        sums(y);
+      } else {
+        sums(x);
+      }
     }
   }
-  if (on && m0 + mi < M && n0 + ni < N) C[(int64_t)(m0 + mi) * N + n0 + ni] = mul_rn((T)p->alpha, acc);
+  if (on)
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int m = m0 + mi + i * ty, n = n0 + ni + j * tx;
+        if (m < M && n < N) C[(int64_t)m * N + n] = mul_rn((T)p->alpha, acc[i][j]);
+      }
 }
 
 template <typename A> __device__ __forceinline__ A warp_sum(A v) {
@@ -176,12 +246,12 @@ template <typename T> __device__ __forceinline__ T sine_exp(T x) { return (T)exp
 // and transposes: 256 outputs per piece
 template <typename T>
 __device__ void run_rows(const RowProg* p, int chunk) {
-  const int lane = threadIdx.x & 31, cols = p->cols;
+  const int tid = threadIdx.x % NT, lane = tid & 31, cols = p->cols;
   const T* x = (const T*)p->in[0];
   const T* in1 = (const T*)p->in[1];
   T* out = (T*)p->out[0];
   if (p->h.kind == PRIM_COLUMN_SUM) {        // out[j] = scalar * sum of rows (scalar 1: as is)
-    const int64_t j = (int64_t)chunk * NT + threadIdx.x;
+    const int64_t j = (int64_t)chunk * NT + tid;
     if (j >= cols) return;
     double acc = 0.0;
     int64_t r = 0;
@@ -197,13 +267,13 @@ __device__ void run_rows(const RowProg* p, int chunk) {
     return;
   }
   if (p->h.kind == PRIM_TRANSPOSE) {
-    const int64_t e = (int64_t)chunk * NT + threadIdx.x, per = p->rows * cols;
+    const int64_t e = (int64_t)chunk * NT + tid, per = p->rows * cols;
     if (e >= per * p->depth) return;
     const int64_t d = e / per, q = e % per, c = q / p->rows, r = q % p->rows;
     out[e] = x[d * per + r * cols + c];
     return;
   }
-  const int64_t r = (int64_t)chunk * (NT / 32) + (threadIdx.x >> 5);
+  const int64_t r = (int64_t)chunk * (NT / 32) + (tid >> 5);
   if (r >= p->rows) return;
   const T* xr = x + r * cols;
   T* yr = out + r * cols;
@@ -270,37 +340,40 @@ __device__ void run_rows(const RowProg* p, int chunk) {
   }
 }
 
-template <typename T> constexpr int smem_bytes() {
-  const int slots = SLOTS * NT * (int)sizeof(T);
-  return MAX_ITEMS * (int)sizeof(Item) + 2 * PROG_BYTES + (slots > STAGE_BYTES ? slots : STAGE_BYTES);
-}
+constexpr int SMEM_BYTES = WORKERS * (2 * PROG_BYTES + WORK_BYTES);
 
 template <typename T>
-__global__ void __launch_bounds__(NT)
-walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ items, const int* __restrict__ count) {
+__global__ void __launch_bounds__(WORKERS * NT)
+walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ items, const int* __restrict__ first) {
   extern __shared__ __align__(16) unsigned char gp_smem[];
-  Item* mine = reinterpret_cast<Item*>(gp_smem);
-  unsigned char* prog = gp_smem + MAX_ITEMS * sizeof(Item);
-  unsigned char* work = prog + 2 * PROG_BYTES;
-  const int n = count[blockIdx.x];
-  for (int i = threadIdx.x; i < n; i += NT) mine[i] = items[(size_t)blockIdx.x * MAX_ITEMS + i];
-  __syncthreads();
-  auto fetch = [&](int i) {
-    if (i < n)
-      for (uint32_t b = threadIdx.x * 8; b < mine[i].bytes; b += NT * 8) copy_async<8>(prog + (i & 1) * PROG_BYTES + b, blob + mine[i].prog + b);
+  const int tid = threadIdx.x % NT, worker = blockIdx.x * WORKERS + threadIdx.x / NT;
+  unsigned char* prog = gp_smem + (threadIdx.x / NT) * (2 * PROG_BYTES + WORK_BYTES);
+  T* work = reinterpret_cast<T*>(prog + 2 * PROG_BYTES);
+  items += first[worker];
+  const int n = first[worker + 1] - first[worker];
+  auto fetch = [&](const Item& it, int i) {
+    for (uint32_t b = tid * 8; b < it.bytes; b += NT * 8) copy_async<8>(prog + (i & 1) * PROG_BYTES + b, blob + it.prog + b);
   };
-  fetch(0);
+  Item cur{0, 0, 0, 0}, nxt{0, 0, 0, 0};
+  if (n > 0) { cur = items[0]; fetch(cur, 0); }
+  if (n > 1) nxt = items[1];
   for (int i = 0; i < n; ++i) {
     copy_wait();
-    __syncthreads();                         // this piece's program is here, the last piece is done with the working memory
-    fetch(i + 1);
-    if (mine[i].bytes) {
+    worker_sync();                           // this piece's program is here, the last piece is done with the working memory
+    if (i + 1 < n) fetch(nxt, i + 1);
+    Item later{0, 0, 0, 0};
+    if (i + 2 < n) later = items[i + 2];
+    if (cur.bytes) {
       const Head* h = reinterpret_cast<const Head*>(prog + (i & 1) * PROG_BYTES);
-      if (h->kind <= PRIM_LAST_ELEMENTWISE) run_elementwise<T>(h, (int)mine[i].chunk, reinterpret_cast<T(*)[NT]>(work));
-      else if (h->kind == PRIM_PRODUCT) run_product<T>(reinterpret_cast<const ProductProg*>(h), (int)mine[i].chunk, reinterpret_cast<T*>(work));
-      else run_rows<T>(reinterpret_cast<const RowProg*>(h), (int)mine[i].chunk);
+      const ProductProg* pp = reinterpret_cast<const ProductProg*>(h);
+      if (h->kind <= PRIM_LAST_ELEMENTWISE) run_elementwise<T>(h, (int)cur.chunk, work);
+      else if (h->kind == PRIM_PRODUCT && pp->r == 1) run_product<T, 1>(pp, (int)cur.chunk, work);
+      else if (h->kind == PRIM_PRODUCT) run_product<T, 2>(pp, (int)cur.chunk, work);
+      else run_rows<T>(reinterpret_cast<const RowProg*>(h), (int)cur.chunk);
     }
-    if (mine[i].barrier) cluster_barrier();
+    if (cur.barrier) cluster_barrier();
+    cur = nxt;
+    nxt = later;
   }
 }
 
@@ -309,10 +382,10 @@ walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ ite
 struct GraphPlan {
   int device = 0, ctas = 0;
   prad_dtype dt = PRAD_F32;
-  void* mem = nullptr;                       // [items][count][blob]
+  void* mem = nullptr;                       // [items][first item of each worker][blob]
   const unsigned char* blob = nullptr;
   const gp::Item* items = nullptr;
-  const int* count = nullptr;
+  const int* first = nullptr;
 };
 
 void GraphPlanFree::operator()(GraphPlan* p) const {
@@ -388,6 +461,10 @@ struct Group {
 // (buffer, columns of a row operand or 0): what has a place of its own in a program
 using Place = std::pair<const void*, int>;
 static Place place_of(const Prim& p, size_t k) { return {p.in[k], p.kind == PRIM_ADD_ROW && k == 1 ? p.cols : 0}; }
+constexpr int64_t TEAM_ELEMENTS = 2048;      // up to here four threads can share an element
+template <typename T> static int slot_limit(int64_t n) {
+  return n <= TEAM_ELEMENTS ? SLOTS : std::min(SLOTS, WORK_BYTES / (NT * (int)sizeof(T)));
+}
 static int places(const std::vector<Prim>& all, const std::vector<int>& ops) {
   std::vector<Place> seen;
   for (int o : ops) {
@@ -399,6 +476,60 @@ static int places(const std::vector<Prim>& all, const std::vector<int>& ops) {
 }
 
 struct Piece { uint32_t prog, bytes, chunk; double cost; };
+
+static int outputs(const Ins& c) { return c.op == PRIM_MUL_BACKWARD ? 2 : 1; }
+static bool writes(const Ins& c, int slot) { return c.dst[0] == slot || (outputs(c) == 2 && c.dst[1] == slot); }
+static bool reads(const Ins& c, int slot) {
+  for (int k = 0; k < c.n_in; ++k)
+    if (c.src[k] == slot) return true;
+  return false;
+}
+
+// Appends an instruction; dst += src that continues a run (nothing in between has to do with it) joins that run's fold.
+static void fold_into(std::vector<Ins>& ins, const Ins& c) {
+  if (c.op == PRIM_ADD2 && c.src[0] == c.dst[0] && c.src[1] != c.dst[0])
+    for (size_t y = ins.size(); y-- > 0;) {
+      Ins& p = ins[y];
+      if (p.dst[0] == c.dst[0] && (p.op == INS_FOLD || (p.op == PRIM_ADD2 && p.src[0] == p.dst[0] && p.src[1] != p.dst[0]))) {
+        bool free = p.n_in < 8;
+        for (size_t z = y + 1; z < ins.size() && free; ++z)
+          for (int k = 1; k < p.n_in; ++k) free = free && !writes(ins[z], p.src[k]);
+        if (!free) break;
+        Ins joined = p;
+        joined.op = INS_FOLD;
+        joined.src[joined.n_in++] = c.src[1];
+        ins.erase(ins.begin() + y);
+        ins.push_back(joined);
+        return;
+      }
+      if (writes(p, c.dst[0]) || reads(p, c.dst[0])) break;
+    }
+  ins.push_back(c);
+}
+
+// Sorts a program into phases: an instruction comes behind those whose values it reads or replaces.  Returns how many.
+static int order_by_phase(std::vector<Ins>& ins) {
+  std::vector<int> phase(ins.size(), 0);
+  int phases = 0;
+  for (size_t x = 0; x < ins.size(); ++x) {
+    for (size_t y = 0; y < x; ++y) {
+      bool after = false;
+      for (int k = 0; k < ins[x].n_in; ++k) after = after || writes(ins[y], ins[x].src[k]);
+      for (int k = 0; k < outputs(ins[x]); ++k) after = after || writes(ins[y], ins[x].dst[k]) || reads(ins[y], ins[x].dst[k]);
+      if (after) phase[x] = std::max(phase[x], phase[y] + 1);
+    }
+    phases = std::max(phases, phase[x] + 1);
+  }
+  std::vector<Ins> sorted;
+  for (int ph = 0; ph < phases; ++ph) {
+    const size_t first = sorted.size();
+    for (size_t x = 0; x < ins.size(); ++x)
+      if (phase[x] == ph) sorted.push_back(ins[x]);
+    sorted[first].phase = (uint8_t)(sorted.size() - first);
+  }
+  ins.swap(sorted);
+  return phases;
+}
 
 // Time of an operation's own launch on the whole device, for comparison (us).
 static double launch_cost(const Prim& p, int sms) {
@@ -466,7 +597,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       for (int g : join) merged.ops.insert(merged.ops.end(), groups[g].ops.begin(), groups[g].ops.end());
       std::sort(merged.ops.begin(), merged.ops.end());
       merged.ops.push_back(i);
-      if (!join.empty() && ((int)merged.ops.size() > MAX_INS || places(ops, merged.ops) > SLOTS)) {
+      if (!join.empty() && ((int)merged.ops.size() > MAX_INS || places(ops, merged.ops) > slot_limit<T>(merged.n))) {
         ++lv;                                // a program of its own, behind a barrier
         join.clear();
         merged.ops.assign(1, i);
@@ -530,14 +661,16 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
           for (const Store& s : stores) stored = stored || s.p == q.out[k];
           if (!stored) stores.push_back({q.out[k], (uint32_t)it->second, 0});
         }
-        ins.push_back(c);
+        fold_into(ins, c);
       }
+      const int phases = order_by_phase(ins);
       Head h{};
       h.kind = PRIM_ACT_FORWARD;
       h.n_load = (int)loads.size();
       h.n_ins = (int)ins.size();
       h.n_store = (int)stores.size();
       h.n = g.n;
+      h.team = g.n <= TEAM_ELEMENTS && (ins.size() >= 4 || slots > WORK_BYTES / (NT * (int)es)) ? 4 : 1;
       std::vector<unsigned char> prog(sizeof(Head) + loads.size() * sizeof(Load) + ins.size() * sizeof(Ins) + stores.size() * sizeof(Store));
       unsigned char* w = prog.data();
       memcpy(w, &h, sizeof(h)); w += sizeof(h);
@@ -545,9 +678,14 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       memcpy(w, ins.data(), ins.size() * sizeof(Ins)); w += ins.size() * sizeof(Ins);
       memcpy(w, stores.data(), stores.size() * sizeof(Store));
       const uint32_t at = put(prog.data(), prog.size());
-      double cost = 0.9 + 0.02 * (double)loads.size() + 0.06 * (double)ins.size();
-      for (const Ins& c : ins) cost += c.op == PRIM_ACT_FORWARD || c.op == PRIM_ACT_BACKWARD ? 0.15 : 0;
-      for (int64_t c = 0; c < ceil_div(g.n, NT); ++c) pieces[level[i]].push_back({at, (uint32_t)((prog.size() + 7) & ~(size_t)7), (uint32_t)c, cost});
+      double cost = 1.0 + 0.02 * (double)loads.size() / (double)h.team;
+      if (h.team > 1) {
+        cost += 0.35 * phases;
+      } else {
+        cost += 0.1 * (double)ins.size();
+        for (const Ins& c : ins) cost += c.op == PRIM_ACT_FORWARD || c.op == PRIM_ACT_BACKWARD ? 0.3 : 0;
+      }
+      for (int64_t c = 0; c < ceil_div(g.n, NT / h.team); ++c) pieces[level[i]].push_back({at, (uint32_t)((prog.size() + 7) & ~(size_t)7), (uint32_t)c, cost});
       continue;
     }
     if (p.kind == PRIM_PRODUCT) {
@@ -557,13 +695,20 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       q.sA = p.sA; q.sB = p.sB; q.sC = p.sC;
       q.alpha = p.scalar;
       q.tA = p.tA; q.tB = p.tB; q.M = p.M; q.N = p.N; q.K = p.K;
-      q.tn = p.N >= 16 ? 16 : p.N >= 8 ? 8 : p.N >= 4 ? 4 : p.N >= 2 ? 2 : 1;
-      q.tm = std::min(NT / q.tn, 64);
-      q.ks = std::min(p.K, STAGE_BYTES / (int)es / (q.tm + q.tn) - 1);     // (the pitch is ks or ks + 1)
+      // 32 x 32 outputs while that many are there and the chain is short (a weight gradient's outer products), else 256
+      q.r = p.K <= 32 && p.M > 16 && p.N > 16 ? 2 : 1;
+      if (q.r == 1) {
+        q.tn = p.N > 8 ? 16 : p.N > 4 ? 8 : p.N > 2 ? 4 : p.N > 1 ? 2 : 1;
+        q.tm = std::min(NT / q.tn, 64);
+      } else {
+        q.tm = q.tn = 32;
+      }
+      q.ks = p.K;
+      while ((q.tm + q.tn) * product_pitch<T>(q.ks) * (int)es > WORK_BYTES) q.ks = (q.ks + 1) / 2;
       q.tiles_n = (int)ceil_div(p.N, q.tn);
       q.tiles_mn = (int)ceil_div(p.M, q.tm) * q.tiles_n;
       const uint32_t at = put(&q, sizeof(q));
-      const double cost = 1.2 + p.K * (es == 8 ? 0.017 : 0.012) + 0.5 * (double)(ceil_div(p.K, q.ks) - 1);
+      const double cost = 1.2 + p.K * (es == 8 ? 0.017 : 0.012) * (q.r == 2 ? 2 : 1) + 0.6 * (double)(ceil_div(p.K, q.ks) - 1);
       for (int64_t c = 0; c < (int64_t)q.tiles_mn * p.batch; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 7) & ~(size_t)7), (uint32_t)c, cost});
       continue;
     }
@@ -582,25 +727,27 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     for (int64_t c = 0; c < chunks; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 7) & ~(size_t)7), (uint32_t)c, cost});
   }
 
-  // deal the pieces of a level to the CTAs, the longest first to whoever has least; a barrier behind every level
-  lists.assign(ctas, {});
+  // deal the pieces of a level to the workers, the longest first to whoever has least (and to another SM before the same one
+  // again); a barrier behind every level
+  const int workers = ctas * WORKERS;
+  lists.assign(workers, {});
   *est_us = 4.0;
-  std::vector<double> busy(ctas);
+  std::vector<double> busy(workers);         // worker k of the dealing order is number k / ctas of CTA k % ctas
   for (int lv = 0; lv < levels; ++lv) {
     std::stable_sort(pieces[lv].begin(), pieces[lv].end(), [](const Piece& a, const Piece& b) { return a.cost > b.cost; });
     std::fill(busy.begin(), busy.end(), 0.0);
-    std::vector<size_t> before(ctas);
-    for (int c = 0; c < ctas; ++c) before[c] = lists[c].size();
+    std::vector<size_t> before(workers);
+    for (int c = 0; c < workers; ++c) before[c] = lists[c].size();
     for (const Piece& p : pieces[lv]) {
-      const int c = (int)(std::min_element(busy.begin(), busy.end()) - busy.begin());
-      busy[c] += p.cost;
-      lists[c].push_back({p.prog, p.bytes, p.chunk, 0});
+      const int k = (int)(std::min_element(busy.begin(), busy.end()) - busy.begin());
+      busy[k] += p.cost;
+      lists[k % ctas * WORKERS + k / ctas].push_back({p.prog, p.bytes, p.chunk, 0});
     }
-    for (int c = 0; c < ctas; ++c) {
+    for (int c = 0; c < workers; ++c) {
       if (lists[c].size() == before[c]) lists[c].push_back({0, 0, 0, 1});
       else lists[c].back().barrier = 1;
     }
-    *est_us += 0.4 + *std::max_element(busy.begin(), busy.end());
+    *est_us += 0.8 + *std::max_element(busy.begin(), busy.end());
   }
 }
 
@@ -611,7 +758,7 @@ template <typename T> static int cluster_ctas(prad_ctx* ctx) {
   int n = k.load(std::memory_order_acquire);
   if (n) return n - 1;
   n = 0;
-  cudaError_t e = cudaFuncSetAttribute(walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<T>());
+  cudaError_t e = cudaFuncSetAttribute(walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(walk_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   for (int cs : {16, 8}) {
     if (e != cudaSuccess || n) break;
@@ -621,8 +768,8 @@ template <typename T> static int cluster_ctas(prad_ctx* ctx) {
     at[0].val.clusterDim.x = cs;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)cs);
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = smem_bytes<T>();
+    cfg.blockDim = dim3(WORKERS * NT);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int fit = 0;
@@ -648,17 +795,19 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
   std::vector<std::vector<Item>> lists;
   double est = 0, launches = 0;
   build<T>(ctx, ops, ctas, blob, lists, &est, &launches);
-  size_t most = 0;
-  for (auto& l : lists) most = std::max(most, l.size());
-  if (est >= launches || most > MAX_ITEMS) return nullptr;
-  const size_t items_bytes = (size_t)ctas * MAX_ITEMS * sizeof(Item), count_bytes = 256;
-  std::vector<unsigned char> host(items_bytes + count_bytes + blob.size());
-  for (int c = 0; c < ctas; ++c) {
-    memcpy(host.data() + (size_t)c * MAX_ITEMS * sizeof(Item), lists[c].data(), lists[c].size() * sizeof(Item));
-    const int n = (int)lists[c].size();
-    memcpy(host.data() + items_bytes + c * sizeof(int), &n, sizeof(int));
+  if (est >= launches) return nullptr;
+  std::vector<Item> items;
+  std::vector<int> first;
+  for (auto& l : lists) {
+    first.push_back((int)items.size());
+    items.insert(items.end(), l.begin(), l.end());
   }
-  memcpy(host.data() + items_bytes + count_bytes, blob.data(), blob.size());
+  first.push_back((int)items.size());
+  const size_t items_bytes = items.size() * sizeof(Item), first_bytes = (first.size() * sizeof(int) + 15) & ~(size_t)15;
+  std::vector<unsigned char> host(items_bytes + first_bytes + blob.size());
+  memcpy(host.data(), items.data(), items_bytes);
+  memcpy(host.data() + items_bytes, first.data(), first.size() * sizeof(int));
+  memcpy(host.data() + items_bytes + first_bytes, blob.data(), blob.size());
   GraphPlanPtr plan(new GraphPlan());
   plan->device = ctx->device;
   plan->ctas = ctas;
@@ -670,8 +819,8 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
     return nullptr;
   }
   plan->items = (const Item*)plan->mem;
-  plan->count = (const int*)((const unsigned char*)plan->mem + items_bytes);
-  plan->blob = (const unsigned char*)plan->mem + items_bytes + count_bytes;
+  plan->first = (const int*)((const unsigned char*)plan->mem + items_bytes);
+  plan->blob = (const unsigned char*)plan->mem + items_bytes + first_bytes;
   return plan;
 }
 
@@ -688,16 +837,16 @@ prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan) {
   at[0].val.clusterDim.x = plan->ctas;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3((unsigned)plan->ctas);
-  cfg.blockDim = dim3(gp::NT);
+  cfg.blockDim = dim3(gp::WORKERS * gp::NT);
   cfg.stream = ctx->stream;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   if (plan->dt == PRAD_F32) {
-    cfg.dynamicSmemBytes = gp::smem_bytes<float>();
-    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<float>, plan->blob, plan->items, plan->count));
+    cfg.dynamicSmemBytes = gp::SMEM_BYTES;
+    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<float>, plan->blob, plan->items, plan->first));
   } else {
-    cfg.dynamicSmemBytes = gp::smem_bytes<double>();
-    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<double>, plan->blob, plan->items, plan->count));
+    cfg.dynamicSmemBytes = gp::SMEM_BYTES;
+    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<double>, plan->blob, plan->items, plan->first));
   }
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;

@@ -10,7 +10,7 @@ namespace prad {
 
 enum PrimKind : int {
   // elementwise over n values
-  PRIM_ACT_FORWARD, PRIM_ACT_BACKWARD, PRIM_ADD2, PRIM_ADD3, PRIM_MUL2, PRIM_MUL_BACKWARD, PRIM_SCALE, PRIM_SUM, PRIM_ADD_ROW,
+  PRIM_ACT_FORWARD, PRIM_ACT_BACKWARD, PRIM_ADD2, PRIM_ADD3, PRIM_MUL2, PRIM_MUL_BACKWARD, PRIM_SCALE, PRIM_COPY, PRIM_SUM, PRIM_ADD_ROW,
   PRIM_LAST_ELEMENTWISE = PRIM_ADD_ROW,
   PRIM_PRODUCT, PRIM_COLUMN_SUM, PRIM_TRANSPOSE, PRIM_SOFTMAX, PRIM_SOFTMAX_BACKWARD, PRIM_SINE_SOFTMAX, PRIM_SINE_SOFTMAX_BACKWARD,
   PRIM_LAYERNORM, PRIM_LAYERNORM_BACKWARD
