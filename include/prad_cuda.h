@@ -331,6 +331,16 @@ prad_status prad_batch_matmul_backward(prad_ctx* ctx, prad_dtype dt, const void*
                                        void* dB_mean, int depth, int M, int K, int N,
                                        int b_shared);
 
+/* Windowed self-attention over a [windows * window x 3 * heads * head_dim] matrix whose columns are the heads of Q, of K and of
+ * V, float only, windows of at most 64 tokens, head_dim 16, 32 or 64 (otherwise PRAD_ERR_UNSUPPORTED):
+ *   forward   P = softmax(scale * Q K^T) ([window][head][token x token]) and out = P V ([tokens x heads * head_dim]);
+ *   backward  d_qkv (every column) from P and d_out.
+ * One launch each; the composition of BatchMatrixMultiplyOperation, MatrixMultiplyScalarOperation and SoftmaxOperation, whose
+ * scores and score gradients are not stored. */
+prad_status prad_window_attention_forward(prad_ctx* ctx, prad_dtype dt, const void* qkv, void* P, void* out, int windows,
+                                          int window, int heads, int head_dim, double scale);
+prad_status prad_window_attention_backward(prad_ctx* ctx, prad_dtype dt, const void* qkv, const void* P, const void* d_out,
+                                           void* d_qkv, int windows, int window, int heads, int head_dim, double scale);
 /* (Gpu)MatrixMultiplyAndSumOperation (src/RMAD/GpuMatrixMultiplyAndSumOperation.cs:114-154,
  * src/RMAD/MatrixMultiplyAndSumOperation.cs:50-89): out[q] = sum_ij (A*B_q)_ij ; backward
  * dB_q = A^T*dOut[q], dA = sum_q B_q^T*dOut[q] (scalar products, not GEMMs).

@@ -67,6 +67,8 @@ SIGNATURES = {
     "prad_hadamard_forward": [vp, i32, vp, vp, vp, i64],
     "prad_hadamard_backward": [vp, i32, vp, vp, vp, vp, vp, i64],
     "prad_lstm_cell_backward": [vp, i32, i64, vp, vp, f64, pvp, i32, vp, pvp, vp, vp, pvp, vp],
+    "prad_window_attention_forward": [vp, i32, vp, vp, vp, i32, i32, i32, i32, f64],
+    "prad_window_attention_backward": [vp, i32, vp, vp, vp, vp, i32, i32, i32, i32, f64],
     "prad_lstm_forward": [vp, i32, i32, i32, i32, vp, pvp, vp, pvp, vp, vp, vp, vp, vp, vp],
     "prad_lstm_backward": [vp, i32, i32, i32, i32, vp, vp, vp, f64, pvp, vp, vp, vp, vp],
     "prad_add_forward": [vp, i32, vp, vp, vp, vp, i64],

@@ -602,7 +602,7 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
   // (Columns: the warp's 128 or, at the right edge, a multiple of 16, so that each store instruction is all or nothing.)
   const int ncols = N - col0 < 128 ? N - col0 : 128;
   if (ncols <= 0 || row0 >= M) return;
-  if (vecC && epi.beta == 0.f && !epi.bias && !epi.row_exp && row0 + 32 <= M && (ncols & 15) == 0) {
+  if (vecC && epi.beta == 0.f && ((uintptr_t)epi.bias & 15) == 0 && !epi.row_exp && row0 + 32 <= M && (ncols & 15) == 0) {
     float* rp[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) rp[s] = C + (int64_t)(qrow + s) * ldc + col0 + 4 * i;
@@ -612,6 +612,16 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
       for (int g = 0; g < 4; ++g)
 #pragma unroll
         for (int j = 0; j < 32; ++j) sum[g][j] = alpha * sum[g][j];
+    }
+    if (epi.bias) {      // a lane still holds whole row parts here: the same four columns for all lanes, one load for the warp
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          if (32 * g + j < ncols) {
+            const float4 b = *reinterpret_cast<const float4*>(epi.bias + col0 + 32 * g + j);
+            sum[g][j] += b.x; sum[g][j + 1] += b.y; sum[g][j + 2] += b.z; sum[g][j + 3] += b.w;
+          }
     }
 #pragma unroll
     for (int g = 0; g < 4; ++g) {

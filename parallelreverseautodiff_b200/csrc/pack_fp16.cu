@@ -397,6 +397,80 @@ pack_tile_kernel(PackSource src, bool vec, int R, int C, PackedForm fr, PackedFo
   }
 }
 
+// ---------------------------------------------------------------- small plain matrices, one form
+// A weight matrix of a narrow layer (96 x 384) is three 128 x 128 tiles: on three CTAs of the kernel above, one round trip to
+// memory after another, it took 15 us.  Here a CTA takes one 128-k block of 8 operand rows (by rows: a warp per row) or of
+// 32 operand rows (by columns: its lanes are the rows, its warps share the k), every load in flight at once: 4 us.
+__global__ void __launch_bounds__(256)
+pack_small_rows_kernel(const float* __restrict__ x, int64_t ld, PackedForm f) {
+  const int lane = threadIdx.x & 31;
+  const int64_t r = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
+  const int c0 = blockIdx.x * 128 + lane * 4;
+  if (r >= f.rows) return;
+  float v[4];
+  uint32_t m = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    v[q] = c0 + q < f.k ? x[r * ld + c0 + q] : 0.f;
+    m = max(m, absbits(v[q]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const int sh = shift_of(m);
+  const float scale = pow2f(sh);
+  if (lane == 0) f.blk[(int64_t)blockIdx.x * f.rows_ld + r] = pow2f(-sh);
+  if (c0 >= f.kp) return;
+  __half2 p0[2], p1[2];
+  pieces2(v[0] * scale, v[1] * scale, p0[0], p1[0]);
+  pieces2(v[2] * scale, v[3] * scale, p0[1], p1[1]);
+  __half* d = f.h + r * f.pitch + (int64_t)(c0 >> 5) * 64 + (c0 & 31);
+  *reinterpret_cast<uint2*>(d) = *reinterpret_cast<const uint2*>(p0);
+  *reinterpret_cast<uint2*>(d + 32) = *reinterpret_cast<const uint2*>(p1);
+}
+__global__ void __launch_bounds__(256)
+pack_small_cols_kernel(const float* __restrict__ x, int64_t ld, PackedForm f) {
+  __shared__ uint32_t part[8][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t r = (int64_t)blockIdx.y * 32 + lane;        // operand row = matrix column
+  const int64_t k0 = (int64_t)blockIdx.x * 128 + w * 16;
+  float v[16];
+  uint32_t m = 0;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    v[q] = r < f.rows && k0 + q < f.k ? x[(k0 + q) * ld + r] : 0.f;
+    m = max(m, absbits(v[q]));
+  }
+  part[w][lane] = m;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) m = max(m, part[q][lane]);
+  if (r >= f.rows) return;
+  const int sh = shift_of(m);
+  const float scale = pow2f(sh);
+  if (w == 0) f.blk[(int64_t)blockIdx.x * f.rows_ld + r] = pow2f(-sh);
+  if (k0 >= f.kp) return;                                   // kp is a multiple of 32
+  __half2 p0[8], p1[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) pieces2(v[2 * q] * scale, v[2 * q + 1] * scale, p0[q], p1[q]);
+  __half* d = f.h + r * f.pitch + (k0 >> 5) * 64 + (k0 & 31);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    reinterpret_cast<uint4*>(d)[q] = reinterpret_cast<const uint4*>(p0)[q];
+    reinterpret_cast<uint4*>(d + 32)[q] = reinterpret_cast<const uint4*>(p1)[q];
+  }
+}
+static prad_status launch_small(prad_ctx* ctx, const PackSource& src, const PackedForm* by_rows, const PackedForm* by_cols) {
+  if (by_rows) {
+    pack_small_rows_kernel<<<dim3((unsigned)by_rows->nchunk, (unsigned)ceil_div(by_rows->rows, 8)), 256, 0, ctx->stream>>>(src.x, src.ld, *by_rows);
+    PRAD_LAUNCHED(ctx);
+  }
+  if (by_cols) {
+    pack_small_cols_kernel<<<dim3((unsigned)by_cols->nchunk, (unsigned)ceil_div(by_cols->rows, 32)), 256, 0, ctx->stream>>>(src.x, src.ld, *by_cols);
+    PRAD_LAUNCHED(ctx);
+  }
+  return PRAD_OK;
+}
+
 template <int TR, int TC>
 static prad_status launch_pack(prad_ctx* ctx, const PackSource& src, bool vec, int R, int C, const PackedForm& fr,
                                const PackedForm& fc, int fast_tiles_r = 0, int fast_tiles_c = 0) {
@@ -442,6 +516,9 @@ prad_status pack_fp16(prad_ctx* ctx, const PackSource& src, int R, int C, const 
                  "operand packing: the by-columns form does not fit a %d x %d matrix", R, C);
   }
   const int tc = by_rows ? by_rows->chunk : 128, tr = by_cols ? by_cols->chunk : 128;
+  // fewer 128 x 128 tiles than a quarter of the SMs: small CTAs, even at the price of reading the matrix once per form
+  if (src.kind == 0 && !src.out && tr == 128 && tc == 128 && ceil_div(R, 128) * ceil_div(C, 128) * 4 <= ctx->sm_count)
+    return pk::launch_small(ctx, src, by_rows, by_cols);
   if (tr == 256 && tc == 256) {
     // a 256 x 256 tile does not fit in shared memory: one pass per form (the FP32 copy is written by the first)
     prad_status s = pk::launch_pack<128, 256>(ctx, src, vec, R, C, *by_rows, none);

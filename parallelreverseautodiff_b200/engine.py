@@ -494,6 +494,15 @@ class Engine:
                                                loss_scale, contrib, len(dh_contrib), self._p(dc_next), gates, tanh_c.ptr,
                                                self._p(c_prev), dpre, self._p(dc_prev)))
 
+    def window_attention_forward(self, qkv, P, out, windows, window, heads, head_dim, scale):
+        """P = softmax(scale Q K^T) and out = P V per window and head (prad_window_attention_forward)."""
+        check(self.lib.prad_window_attention_forward(self.ctx, dtype_code(qkv.dtype), qkv.ptr, P.ptr, out.ptr, windows, window,
+                                                     heads, head_dim, scale))
+
+    def window_attention_backward(self, qkv, P, d_out, d_qkv, windows, window, heads, head_dim, scale):
+        check(self.lib.prad_window_attention_backward(self.ctx, dtype_code(qkv.dtype), qkv.ptr, P.ptr, d_out.ptr, d_qkv.ptr, windows,
+                                                      window, heads, head_dim, scale))
+
     def lstm_forward(self, steps, batch, U, bias_ifgo, pre, gates_ifgo, C_, tanh_c, H, H_prev, FC, IG):
         """The recurrent part of an LSTM layer's Forward, all time steps (prad_lstm_forward)."""
         check(self.lib.prad_lstm_forward(self.ctx, dtype_code(H.dtype), steps, batch, H.shape[1], U.ptr, self._ptr_list(bias_ifgo),

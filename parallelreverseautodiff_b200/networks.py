@@ -672,6 +672,8 @@ class SwinBlock:
                   "W1": z(d, h), "b1": z(1, h), "W2": z(h, d), "b2": z(1, d)}
         self.g = {k: z(*v.shape) for k, v in self.p.items()}
         self.scale = 1.0 / float(np.sqrt(self.hd))
+        # the shapes prad_window_attention_* is made for; others are composed from strided-batched products
+        self.fused_attention = self.dtype == np.float32 and window <= 64 and self.hd in (16, 32, 64)
         self._cache = {}
 
     def _buf(self, name, shape):
@@ -693,13 +695,13 @@ class SwinBlock:
                alpha=alpha, beta=beta, M=M, N=N, K=K, lda=lda, ldb=ldb, ldc=ldc, batch=batch, strideA=sA,
                strideB=sB, strideC=sC)
 
-    def forward(self, x: E.DeviceMatrix):
-        e, d, ws, H, hd = self.eng, self.dim, self.ws, self.heads, self.hd
-        T = x.shape[0]
-        nw = T // ws
-        self.x, self.nw = x, nw
-        self.ln1, self.mu1, self.sd1 = e.layernorm_forward(x)
-        self.qkv = e.matmul_forward(self.ln1, self.p["Wqkv"], bias=self.p["bqkv"])
+    def _attention_forward(self, T):
+        e, d, ws, H, hd, nw = self.eng, self.dim, self.ws, self.heads, self.hd, self.nw
+        if self.fused_attention:
+            self.P = e.empty((nw * H * ws, ws), self.dtype)       # [window][head][ws x ws]
+            self.attn = e.empty((T, d), self.dtype)
+            e.window_attention_forward(self.qkv, self.P, self.attn, nw, ws, H, hd, self.scale)
+            return
         self.S = e.empty((nw * H * ws, ws), self.dtype)           # [window][head][ws x ws]
         for h in range(H):                                        # S = (Q K^T) * scale
             self._attn_gemm(self.qkv, h * hd, 3 * d, ws * 3 * d, self.qkv, d + h * hd, 3 * d, ws * 3 * d,
@@ -709,6 +711,36 @@ class SwinBlock:
         for h in range(H):                                        # O_h = P V, written at column h*hd
             self._attn_gemm(self.P, h * ws * ws, ws, H * ws * ws, self.qkv, 2 * d + h * hd, 3 * d, ws * 3 * d,
                             self.attn, h * hd, d, ws * d, ws, hd, ws, batch=nw)
+
+    def _attention_backward(self, d_attn, d_qkv):
+        e, d, ws, H, hd, nw = self.eng, self.dim, self.ws, self.heads, self.hd, self.nw
+        if self.fused_attention:
+            e.window_attention_backward(self.qkv, self.P, d_attn, d_qkv, nw, ws, H, hd, self.scale)
+            return
+        B_ = self._buf
+        dP = B_("dP", self.P.shape)
+        for h in range(H):
+            # O_h = P_h V_h :  dP_h = dO_h V_h^T ,  dV_h = P_h^T dO_h
+            self._attn_gemm(d_attn, h * hd, d, ws * d, self.qkv, 2 * d + h * hd, 3 * d, ws * 3 * d,
+                            dP, h * ws * ws, ws, H * ws * ws, ws, ws, hd, transB=True, batch=nw)
+            self._attn_gemm(self.P, h * ws * ws, ws, H * ws * ws, d_attn, h * hd, d, ws * d,
+                            d_qkv, 2 * d + h * hd, 3 * d, ws * 3 * d, ws, hd, ws, transA=True, batch=nw)
+        dS = e.softmax_backward(self.P, dP, out=B_("dS", self.P.shape))
+        for h in range(H):
+            # S_h = scale * Q_h K_h^T :  dQ_h = scale * dS_h K_h ,  dK_h = scale * dS_h^T Q_h
+            self._attn_gemm(dS, h * ws * ws, ws, H * ws * ws, self.qkv, d + h * hd, 3 * d, ws * 3 * d,
+                            d_qkv, h * hd, 3 * d, ws * 3 * d, ws, hd, ws, alpha=self.scale, batch=nw)
+            self._attn_gemm(dS, h * ws * ws, ws, H * ws * ws, self.qkv, h * hd, 3 * d, ws * 3 * d,
+                            d_qkv, d + h * hd, 3 * d, ws * 3 * d, ws, hd, ws, transA=True, alpha=self.scale, batch=nw)
+
+    def forward(self, x: E.DeviceMatrix):
+        e, d, ws, H, hd = self.eng, self.dim, self.ws, self.heads, self.hd
+        T = x.shape[0]
+        nw = T // ws
+        self.x, self.nw = x, nw
+        self.ln1, self.mu1, self.sd1 = e.layernorm_forward(x)
+        self.qkv = e.matmul_forward(self.ln1, self.p["Wqkv"], bias=self.p["bqkv"])
+        self._attention_forward(T)
         self.proj = e.matmul_forward(self.attn, self.p["Wproj"], bias=self.p["bproj"])
         self.r1 = e.add_forward(x, self.proj)
         self.ln2, self.mu2, self.sd2 = e.layernorm_forward(self.r1)
@@ -735,23 +767,10 @@ class SwinBlock:
         e.add_broadcast_backward(d_r1, dbias=g["bproj"])
         d_attn, _ = e.matmul_backward(self.attn, p["Wproj"], d_r1, dA=B_("d_attn", (T, d)), dB=g["Wproj"])
         d_qkv = B_("d_qkv", (T, 3 * d))     # every element is written by the three per-head products below
-        dP = B_("dP", self.P.shape)
-        for h in range(H):
-            # O_h = P_h V_h :  dP_h = dO_h V_h^T ,  dV_h = P_h^T dO_h
-            self._attn_gemm(d_attn, h * hd, d, ws * d, self.qkv, 2 * d + h * hd, 3 * d, ws * 3 * d,
-                            dP, h * ws * ws, ws, H * ws * ws, ws, ws, hd, transB=True, batch=nw)
-            self._attn_gemm(self.P, h * ws * ws, ws, H * ws * ws, d_attn, h * hd, d, ws * d,
-                            d_qkv, 2 * d + h * hd, 3 * d, ws * 3 * d, ws, hd, ws, transA=True, batch=nw)
-        dS = e.softmax_backward(self.P, dP, out=B_("dS", self.P.shape))
-        for h in range(H):
-            # S_h = scale * Q_h K_h^T :  dQ_h = scale * dS_h K_h ,  dK_h = scale * dS_h^T Q_h
-            self._attn_gemm(dS, h * ws * ws, ws, H * ws * ws, self.qkv, d + h * hd, 3 * d, ws * 3 * d,
-                            d_qkv, h * hd, 3 * d, ws * 3 * d, ws, hd, ws, alpha=self.scale, batch=nw)
-            self._attn_gemm(dS, h * ws * ws, ws, H * ws * ws, self.qkv, h * hd, 3 * d, ws * 3 * d,
-                            d_qkv, d + h * hd, 3 * d, ws * 3 * d, ws, hd, ws, transA=True, alpha=self.scale, batch=nw)
+        self._attention_backward(d_attn, d_qkv)
         e.add_broadcast_backward(d_qkv, dbias=g["bqkv"])
         d_ln1, _ = e.matmul_backward(self.ln1, p["Wqkv"], d_qkv, dA=B_("d_ln1", (T, d)), dB=g["Wqkv"])
         d_x_b = e.layernorm_backward(self.x, self.mu1, self.sd1, d_ln1, out=B_("d_x_b", (T, d)))
         self.d_x = e.segmented_sum([d_r1, d_x_b], out=B_("d_x", (T, d)))  # fan-in at x: residual + LN1 branch
-        self.d_qkv, self.dS, self.dP, self.d_attn = d_qkv, dS, dP, d_attn
+        self.d_qkv, self.d_attn = d_qkv, d_attn
         return self.d_x
