@@ -279,6 +279,15 @@ prad_status prad_act_backward_pack(prad_packed* p, prad_act act, const void* sav
  * activation's Backward in one pass, the loss gradient never stored. */
 prad_status prad_mse_act_backward_pack(prad_packed* p, prad_act act, const void* saved, const void* output, const void* target,
                                        int64_t rows_total, void* dx, double act_alpha);
+/* Every later packing of p also leaves the column sums of the packed values (a bias gradient: MatrixAddBroadcastingOperation
+ * .Backward) in out, one value per column of the matrix; NULL ends it.  Needs the by-columns form. */
+prad_status prad_packed_column_sums(prad_packed* p, void* out);
+/* LayerNormalizationOperation of x, or of sum = x + residual (both or neither given), packed in both forms; mean and stdv are
+ * the operation's state.  And its Backward plus the residual path's gradient: dx = residual + Backward(dy), stored and packed.
+ * Rows of at most 128 columns, a multiple of four, 16-byte aligned (otherwise PRAD_ERR_UNSUPPORTED). */
+prad_status prad_layernorm_pack(prad_packed* p, const void* x, const void* residual, void* sum, void* mean, void* stdv);
+prad_status prad_layernorm_backward_pack(prad_packed* p, const void* x, const void* mean, const void* stdv, const void* dy,
+                                         const void* residual, void* dx);
 prad_status prad_gemm_packed(prad_ctx* ctx, const prad_packed* A, int form_a, const prad_packed* B, int form_b,
                              double alpha, double beta, void* C, int64_t ldc, const void* bias);
 
@@ -467,6 +476,9 @@ prad_status prad_layernorm_forward(prad_ctx* ctx, prad_dtype dt, const void* x, 
 prad_status prad_layernorm_backward(prad_ctx* ctx, prad_dtype dt, const void* x,
                                     const void* mean, const void* stdv, const void* dy, void* dx,
                                     int64_t rows, int cols);
+/* dx = residual + prad_layernorm_backward(...): the fan-in at a residual connection */
+prad_status prad_layernorm_backward_add(prad_ctx* ctx, prad_dtype dt, const void* x, const void* mean, const void* stdv,
+                                        const void* dy, const void* residual, void* dx, int64_t rows, int cols);
 /* MatrixSumOperation.cs:38-68 and MatrixAverageOperation.cs:38-67 (average != 0): y[i] = LINQ Sum /
  * Average of row i (`rows` values); backward: dx[i][j] = dy[i] (or dy[i] / cols). */
 prad_status prad_row_sum_forward(prad_ctx* ctx, prad_dtype dt, const void* x, void* y, int64_t rows, int cols,

@@ -15,6 +15,7 @@
 //   words: no bank conflicts) and writes one whole 128-byte line of pieces.
 // TR is the by-columns block length, TC the by-rows block length.
 #include <atomic>
+#include <type_traits>
 
 #include "act_math.cuh"
 #include "pack_fp16.cuh"
@@ -90,7 +91,8 @@ __device__ __forceinline__ void fetch4(const PackSource& s, bool vec, int64_t r,
 // 128-long blocks: no bounds tests, the operation fixed at compile time, conversions two values at a
 // time (cvt.rn.f16x2.f32).  OP: 0 plain; 1 / 2 / 3 forward GELU / LeakyReLU / any activation;
 // 4 / 5 / 6 backward likewise; 7 / 8 mean-squared-error gradient times the GELU / any derivative;
-// 9 / 10 / 11 are 1 / 4 / 7 (the GELU cases) in short arithmetic, chosen when no FP32 copy is written.
+// 9 / 10 / 11 are 1 / 4 / 7 (the GELU cases) in short arithmetic, chosen when no FP32 copy is written;
+// 12 / 13 LayerNormalization of x / of x + dy, 14 its Backward plus the residual path's gradient (a warp has the whole row).
 //
 // Short arithmetic: the copy-less result exists only as pieces of 22 significant bits, so the GELU terms
 // are contracted into fused multiply-adds and tanh is 1 - 2 / (1 + 2^(2 log2(e) u)) with the hardware's
@@ -141,18 +143,44 @@ __device__ __forceinline__ float apply_op(const PackSource& s, float a, float d,
 // slots is conflict-free); in pass 2 a lane reads four consecutive k of one column and the eight lanes that
 // share a column quad read eight different slot positions: 32 different banks.
 //
-// EDGE: the one column tile that the matrix fills only in part (C is a multiple of four, so whole float4 lie inside or
-// outside): columns from C on read as zeros, pieces are written up to the padded k of the by-rows form and for the
-// existing operand rows of the by-columns form only.
+// EDGE: tiles that the matrix fills only in part (C is a multiple of four, so whole float4 lie inside or outside): columns
+// from C and rows from R on read as zeros, pieces are written up to the padded k of either form and for existing operand rows
+// only.
+//
+// Column sums (a bias gradient) cost the second pass sixteen additions per lane and quad: the values are in shared memory anyway,
+// and a pass of their own over a 200704 x 384 gradient takes 72 us.
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// LayerNormalizationOperation.cs:56-85 on the row whose four values at column c each lane holds
+__device__ __forceinline__ void layernorm_row(float (&v)[4], bool inside, int C, float* mean, float* sigma, bool write) {
+  double s = 0.0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) s += (double)v[q];
+  s = lane_sum(inside ? s : 0.0);
+  const float mu = (float)(s / (double)C);
+  double t = 0.0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { v[q] = sub_rn(v[q], mu); t += (double)mul_rn(v[q], v[q]); }
+  t = lane_sum(inside ? t : 0.0);
+  const float sd = sqrt_rn(div_rn((float)t, (float)C));
+  if (write) { *mean = mu; *sigma = sd; }
+  const float den = add_rn(sd, 1e-9f);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = div_rn(v[q], den);
+}
 template <int OP, bool ROWS, bool COLS, int NT, bool EDGE>
 __global__ void __launch_bounds__(NT, NT == 512 ? 2 : (OP == 0 ? 5 : 3))
-pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_c0, int C) {
-  constexpr int T = 128, U = 2, NW = NT / 32, NB = T / NW / U;      // NW warps, each takes every NW-th tile row
-  constexpr bool HAS_DY = OP >= 4 && OP != 9, HAS_TG = OP == 7 || OP == 8 || OP == 11;
+pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_r0, int tile_c0, int R, int C) {
+  constexpr int T = 128, U = OP == 13 || OP == 14 ? 1 : 2, NW = NT / 32, NB = T / NW / U;      // NW warps, each takes every NW-th tile row
+  constexpr bool HAS_DY = OP >= 4 && OP != 9 && OP != 12, HAS_TG = OP == 7 || OP == 8 || OP == 11 || OP == 14;
   extern __shared__ float stash[];       // [T][T] when COLS
   __shared__ unsigned colmax[T];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t r0 = (int64_t)blockIdx.y * T;
+  const int rtile = tile_r0 + blockIdx.y;
+  const int64_t r0 = (int64_t)rtile * T;
   const int ctile = tile_c0 + blockIdx.x;
   const int c0 = ctile * T, c = c0 + lane * 4;
   const bool inside = !EDGE || c < C;                  // this lane's four columns exist
@@ -163,8 +191,8 @@ pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_c0, int 
   auto load = [&](int buf, int b) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int64_t off = (r0 + warp + NW * (b * U + u)) * src.ld + c;
-      if (EDGE && !inside) {
+      const int64_t r = r0 + warp + NW * (b * U + u), off = r * src.ld + c;
+      if (EDGE && (!inside || r >= R)) {
         a[buf][u] = d[buf][u] = tg[buf][u] = make_float4(0.f, 0.f, 0.f, 0.f);
         continue;
       }
@@ -182,13 +210,36 @@ pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_c0, int 
     for (int u = 0; u < U; ++u) {
       const int tr = warp + NW * (b * U + u);
       const int64_t r = r0 + tr;
+      const bool row = !EDGE || r < R;
       float v[4];
-      v[0] = apply_op<OP>(src, a[cur][u].x, HAS_DY ? d[cur][u].x : 0.f, HAS_TG ? tg[cur][u].x : 0.f);
-      v[1] = apply_op<OP>(src, a[cur][u].y, HAS_DY ? d[cur][u].y : 0.f, HAS_TG ? tg[cur][u].y : 0.f);
-      v[2] = apply_op<OP>(src, a[cur][u].z, HAS_DY ? d[cur][u].z : 0.f, HAS_TG ? tg[cur][u].z : 0.f);
-      v[3] = apply_op<OP>(src, a[cur][u].w, HAS_DY ? d[cur][u].w : 0.f, HAS_TG ? tg[cur][u].w : 0.f);
-      if (EDGE && !inside) v[0] = v[1] = v[2] = v[3] = 0.f;      // an activation of zero need not be zero
-      if (OP >= 1 && OP <= 8 && src.out && inside)
+      if constexpr (OP == 12 || OP == 13) {
+        v[0] = a[cur][u].x; v[1] = a[cur][u].y; v[2] = a[cur][u].z; v[3] = a[cur][u].w;
+        if constexpr (OP == 13) {
+          v[0] = add_rn(v[0], d[cur][u].x); v[1] = add_rn(v[1], d[cur][u].y);
+          v[2] = add_rn(v[2], d[cur][u].z); v[3] = add_rn(v[3], d[cur][u].w);
+          if (inside && row) __stcs(reinterpret_cast<float4*>(src.out + r * src.ld + c), make_float4(v[0], v[1], v[2], v[3]));
+        }
+        layernorm_row(v, inside, C, src.mean + r, src.sigma + r, lane == 0 && row);
+      } else if constexpr (OP == 14) {
+        // LayerNormalizationOperation.cs:88-112, then the sum of the two paths
+        const float mu = row ? src.mean[r] : 0.f, se = add_rn(row ? src.sigma[r] : 1.f, 1e-9f);
+        const float exp1 = mul_rn(sub_rn(1.f, div_rn(1.f, (float)C)), div_rn(1.f, se));
+        const float rden = div_rn(1.f, mul_rn((float)C, mul_rn(mul_rn(se, se), se)));      // (as layernorm_backward_flat)
+        const float x4[4] = {a[cur][u].x, a[cur][u].y, a[cur][u].z, a[cur][u].w}, d4[4] = {d[cur][u].x, d[cur][u].y, d[cur][u].z, d[cur][u].w};
+        const float g4[4] = {tg[cur][u].x, tg[cur][u].y, tg[cur][u].z, tg[cur][u].w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float t = sub_rn(x4[q], mu);
+          v[q] = add_rn(g4[q], mul_rn(d4[q], sub_rn(exp1, mul_rn(mul_rn(t, t), rden))));
+        }
+      } else {
+        v[0] = apply_op<OP>(src, a[cur][u].x, HAS_DY ? d[cur][u].x : 0.f, HAS_TG ? tg[cur][u].x : 0.f);
+        v[1] = apply_op<OP>(src, a[cur][u].y, HAS_DY ? d[cur][u].y : 0.f, HAS_TG ? tg[cur][u].y : 0.f);
+        v[2] = apply_op<OP>(src, a[cur][u].z, HAS_DY ? d[cur][u].z : 0.f, HAS_TG ? tg[cur][u].z : 0.f);
+        v[3] = apply_op<OP>(src, a[cur][u].w, HAS_DY ? d[cur][u].w : 0.f, HAS_TG ? tg[cur][u].w : 0.f);
+      }
+      if (EDGE && !(inside && row)) v[0] = v[1] = v[2] = v[3] = 0.f;      // an activation of zero need not be zero
+      if (((OP >= 1 && OP <= 8) || OP == 14) && src.out && inside && row)
         __stcs(reinterpret_cast<float4*>(src.out + r * src.ld + c), make_float4(v[0], v[1], v[2], v[3]));
       uint32_t m = 0;
 #pragma unroll
@@ -204,12 +255,12 @@ pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_c0, int 
         for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
         const int sh = shift_of(m);
         const float scale = pow2f(sh);
-        if (lane == 0) fr.blk[(int64_t)ctile * fr.rows_ld + r] = pow2f(-sh);
+        if (lane == 0 && row) fr.blk[(int64_t)ctile * fr.rows_ld + r] = pow2f(-sh);
         __half2 p0[2], p1[2];
         pieces2(v[0] * scale, v[1] * scale, p0[0], p1[0]);
         pieces2(v[2] * scale, v[3] * scale, p0[1], p1[1]);
         __half* dst = fr.h + r * fr.pitch + (int64_t)(c >> 5) * 64 + (c & 31);
-        if (!EDGE || c < fr.kp) {                          // the row is padded with zeros up to kp and ends there
+        if (!EDGE || (row && c < fr.kp)) {                 // the row is padded with zeros up to kp and ends there
           *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(p0);
           *reinterpret_cast<uint2*>(dst + 32) = *reinterpret_cast<const uint2*>(p1);
         }
@@ -232,23 +283,58 @@ pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_c0, int 
     if (EDGE && c0 + quad * 4 >= C) break;           // no operand rows from here on (whole quads: C is a multiple of 4)
     const int sh = shift_of(colmax[tc]);
     const float scale = pow2f(sh);
-    if (g == 0) fc.blk[(int64_t)blockIdx.y * fc.rows_ld + c0 + tc] = pow2f(-sh);
+    if (g == 0) fc.blk[(int64_t)rtile * fc.rows_ld + c0 + tc] = pow2f(-sh);
     const float* sp = stash + (4 * g) * T + (((quad ^ g) << 2) | cc);      // (k >> 2) & 7 == g for k = 32 kg + 4g + i
     __half* dst = fc.h + (int64_t)(c0 + tc) * fc.pitch + (r0 >> 5) * 64 + 4 * g;
+    double sum = 0.0;
 #pragma unroll
     for (int kg = 0; kg < 4; ++kg) {
+      const float x0 = sp[(kg * 32) * T], x1 = sp[(kg * 32 + 1) * T], x2 = sp[(kg * 32 + 2) * T], x3 = sp[(kg * 32 + 3) * T];
+      if (src.colsum) sum += ((double)x0 + (double)x1) + ((double)x2 + (double)x3);
+      if (EDGE && r0 + kg * 32 >= fc.kp) continue;
       __half2 p0[2], p1[2];
-      pieces2(sp[(kg * 32) * T] * scale, sp[(kg * 32 + 1) * T] * scale, p0[0], p1[0]);
-      pieces2(sp[(kg * 32 + 2) * T] * scale, sp[(kg * 32 + 3) * T] * scale, p0[1], p1[1]);
+      pieces2(x0 * scale, x1 * scale, p0[0], p1[0]);
+      pieces2(x2 * scale, x3 * scale, p0[1], p1[1]);
       *reinterpret_cast<uint2*>(dst + kg * 64) = *reinterpret_cast<const uint2*>(p0);
       *reinterpret_cast<uint2*>(dst + kg * 64 + 32) = *reinterpret_cast<const uint2*>(p1);
+    }
+    if (src.colsum) {
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (g == 0) src.colsum[(int64_t)rtile * C + c0 + tc] = sum;
     }
   }
 }
 
+// out[c] = sum of the partial column sums, in a fixed order: 32 warps share the rows of 32 columns
+__global__ void __launch_bounds__(1024)
+column_sum_kernel(const double* __restrict__ part, float* __restrict__ out, int rows, int C) {
+  __shared__ double sm[32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  double acc = 0.0;
+  if (c < C)
+    for (int r0 = w; r0 < rows; r0 += 128) {
+      double v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = r0 + 32 * u < rows ? part[(int64_t)(r0 + 32 * u) * C + c] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc += v[u];
+    }
+  sm[w][lane] = acc;
+  __syncthreads();
+  if (w == 0 && c < C) {
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) t += sm[k][lane];
+    out[c] = (float)t;
+  }
+}
+
+// R x C matrix: whole tiles, then the last column of tiles, then the last row of tiles
 template <int OP, bool ROWS, bool COLS>
-static prad_status launch_fast(prad_ctx* ctx, const PackSource& src, int tiles_r, int tiles_c, const PackedForm& fr,
-                               const PackedForm& fc, int C, bool edge) {
+static prad_status launch_fast(prad_ctx* ctx, const PackSource& src, const PackedForm& fr, const PackedForm& fc, int R, int C) {
+  const unsigned tr = (unsigned)(R / 128), tc = (unsigned)(C / 128), er = R % 128 != 0, ec = C % 128 != 0;
+  PRAD_REQUIRE(tr + er <= 65535, PRAD_ERR_UNSUPPORTED, "operand packing: too many row tiles (%u)", tr + er);
   // with a stash (64 KB per tile) two CTAs of 16 warps hide the loads better than three of 8
   constexpr int NT = COLS ? 512 : 256;
   const int smem = COLS ? 128 * 128 * (int)sizeof(float) : 0;
@@ -267,26 +353,28 @@ static prad_status launch_fast(prad_ctx* ctx, const PackSource& src, int tiles_r
       done.fetch_or(bit, std::memory_order_release);
     }
   }
-  if (tiles_c > 0) {
-    pack_fast_kernel<OP, ROWS, COLS, NT, false><<<dim3((unsigned)tiles_c, (unsigned)tiles_r), NT, smem, ctx->stream>>>(src, fr, fc, 0, C);
+  auto launch = [&](auto edge, unsigned x, unsigned y, unsigned r0, unsigned c0) -> prad_status {
+    if (x == 0 || y == 0) return PRAD_OK;
+    pack_fast_kernel<OP, ROWS, COLS, NT, decltype(edge)::value><<<dim3(x, y), NT, smem, ctx->stream>>>(src, fr, fc, (int)r0, (int)c0, R, C);
     PRAD_LAUNCHED(ctx);
-  }
-  if (edge) {
-    pack_fast_kernel<OP, ROWS, COLS, NT, true><<<dim3(1u, (unsigned)tiles_r), NT, smem, ctx->stream>>>(src, fr, fc, tiles_c, C);
-    PRAD_LAUNCHED(ctx);
-  }
-  return PRAD_OK;
+    return PRAD_OK;
+  };
+  prad_status s = launch(std::false_type(), tc, tr, 0, 0);
+  if (!s) s = launch(std::true_type(), ec, tr, 0, tc);
+  if (!s) s = launch(std::true_type(), tc + ec, er, tr, 0);
+  return s;
 }
 template <int OP>
-static prad_status launch_fast_forms(prad_ctx* ctx, const PackSource& src, int tiles_r, int tiles_c, const PackedForm& fr,
-                                     const PackedForm& fc, int C, bool edge) {
-  if (fr.h && fc.h) return launch_fast<OP, true, true>(ctx, src, tiles_r, tiles_c, fr, fc, C, edge);
-  if (fr.h) return launch_fast<OP, true, false>(ctx, src, tiles_r, tiles_c, fr, fc, C, edge);
-  return launch_fast<OP, false, true>(ctx, src, tiles_r, tiles_c, fr, fc, C, edge);
+static prad_status launch_fast_forms(prad_ctx* ctx, const PackSource& src, const PackedForm& fr, const PackedForm& fc, int R, int C) {
+  if (fr.h && fc.h) return launch_fast<OP, true, true>(ctx, src, fr, fc, R, C);
+  if (fr.h) return launch_fast<OP, true, false>(ctx, src, fr, fc, R, C);
+  return launch_fast<OP, false, true>(ctx, src, fr, fc, R, C);
 }
 // which compile-time operation serves this source
 static int fast_op_of(const PackSource& s) {
   if (s.kind == 0) return 0;
+  if (s.kind == 4) return s.dy ? 13 : 12;
+  if (s.kind == 5) return 14;
   const bool gelu = s.act == PRAD_ACT_GELU, leaky = s.act == PRAD_ACT_LEAKY_RELU;
   if (gelu && !s.out) return s.kind == 1 ? 9 : (s.kind == 2 ? 10 : 11);
   if (s.kind == 1) return gelu ? 1 : (leaky ? 2 : 3);
@@ -296,9 +384,7 @@ static int fast_op_of(const PackSource& s) {
 
 template <int TR, int TC>
 __global__ void __launch_bounds__(256)
-pack_tile_kernel(PackSource src, bool vec, int R, int C, PackedForm fr, PackedForm fc, int fast_tiles_r, int fast_tiles_c) {
-  // tiles inside the first fast_tiles_r x fast_tiles_c are written by pack_fast_kernel
-  if ((int)blockIdx.y < fast_tiles_r && (int)blockIdx.x < fast_tiles_c) return;
+pack_tile_kernel(PackSource src, bool vec, int R, int C, PackedForm fr, PackedForm fc) {
   constexpr int W = TC / 128;            // float4 per lane and tile row
   constexpr int STRIDE = TC + 4;         // stash pitch in floats (16-byte multiple; see pass 2)
   constexpr int U = 4;                   // tile rows a warp loads before it starts converting
@@ -375,6 +461,11 @@ pack_tile_kernel(PackSource src, bool vec, int R, int C, PackedForm fr, PackedFo
     for (int q = 0; q < 4; ++q)
       if (cm[w][q] != 0) atomicMax(&colmax[lane * 4 + 128 * w + q], cm[w][q]);
   __syncthreads();
+  if (src.colsum && threadIdx.x < TC && c0 + (int)threadIdx.x < C) {
+    double t = 0.0;
+    for (int r = 0; r < TR; ++r) t += (double)stash[r * STRIDE + threadIdx.x];
+    src.colsum[(int64_t)blockIdx.y * C + c0 + threadIdx.x] = t;
+  }
   constexpr int CG = TC / 32, KG = TR / 32;
   for (int item = warp; item < CG * KG; item += 8) {
     const int cg = item % CG, kg = item / CG;
@@ -473,7 +564,7 @@ static prad_status launch_small(prad_ctx* ctx, const PackSource& src, const Pack
 
 template <int TR, int TC>
 static prad_status launch_pack(prad_ctx* ctx, const PackSource& src, bool vec, int R, int C, const PackedForm& fr,
-                               const PackedForm& fc, int fast_tiles_r = 0, int fast_tiles_c = 0) {
+                               const PackedForm& fc) {
   const int smem = fc.h ? TR * (TC + 4) * (int)sizeof(float) : 0;
   if (smem > 48 * 1024) {
     static std::atomic<uint64_t> done{0};
@@ -493,8 +584,7 @@ static prad_status launch_pack(prad_ctx* ctx, const PackSource& src, bool vec, i
   const int64_t cols_cover = fr.h ? (fr.kp > C ? fr.kp : C) : C;
   dim3 grid((unsigned)ceil_div(cols_cover, TC), (unsigned)ceil_div(rows_cover, TR));
   PRAD_REQUIRE(grid.y <= 65535, PRAD_ERR_UNSUPPORTED, "operand packing: too many row tiles (%u)", grid.y);
-  if ((int)grid.y <= fast_tiles_r && (int)grid.x <= fast_tiles_c) return PRAD_OK;    // nothing left for this kernel
-  pack_tile_kernel<TR, TC><<<grid, 256, smem, ctx->stream>>>(src, vec, R, C, fr, fc, fast_tiles_r, fast_tiles_c);
+  pack_tile_kernel<TR, TC><<<grid, 256, smem, ctx->stream>>>(src, vec, R, C, fr, fc);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
@@ -517,46 +607,45 @@ prad_status pack_fp16(prad_ctx* ctx, const PackSource& src, int R, int C, const 
   }
   const int tc = by_rows ? by_rows->chunk : 128, tr = by_cols ? by_cols->chunk : 128;
   // fewer 128 x 128 tiles than a quarter of the SMs: small CTAs, even at the price of reading the matrix once per form
-  if (src.kind == 0 && !src.out && tr == 128 && tc == 128 && ceil_div(R, 128) * ceil_div(C, 128) * 4 <= ctx->sm_count)
+  if (src.kind == 0 && !src.out && !src.colsum && tr == 128 && tc == 128 && ceil_div(R, 128) * ceil_div(C, 128) * 4 <= ctx->sm_count)
     return pk::launch_small(ctx, src, by_rows, by_cols);
+  PRAD_REQUIRE(src.kind < 4 || (tr == 128 && tc == 128), PRAD_ERR_UNSUPPORTED, "operand packing: LayerNormalization needs 128-long blocks");
   if (tr == 256 && tc == 256) {
     // a 256 x 256 tile does not fit in shared memory: one pass per form (the FP32 copy is written by the first)
-    prad_status s = pk::launch_pack<128, 256>(ctx, src, vec, R, C, *by_rows, none);
-    if (s) return s;
     PackSource again = src;
-    if (src.out) { again = PackSource(); again.kind = 0; again.x = src.out; again.ld = src.ld; }
+    if (src.out) { again = PackSource(); again.kind = 0; again.x = src.out; again.ld = src.ld; again.colsum = src.colsum; }
+    PackSource first = src;
+    first.colsum = nullptr;
+    prad_status s = pk::launch_pack<128, 256>(ctx, first, vec, R, C, *by_rows, none);
+    if (s) return s;
     return pk::launch_pack<256, 128>(ctx, again, vec, R, C, none, *by_cols);
   }
   const PackedForm& fr = by_rows ? *by_rows : none;
   const PackedForm& fc = by_cols ? *by_cols : none;
   if (tr == 256) return pk::launch_pack<256, 128>(ctx, src, vec, R, C, fr, fc);
   if (tc == 256) return pk::launch_pack<128, 256>(ctx, src, vec, R, C, fr, fc);
-  // 128-long blocks: interior tiles through the specialised kernel, the ragged edges through the general one
-  int fr_t = 0, fc_t = 0;
-  if (vec && R >= 128 && (C >= 128 || C % 4 == 0)) {
-    fr_t = R / 128;
-    fc_t = C / 128;
-    // the last, partly filled column tile takes the same kernel when whole float4 lie inside or outside the matrix
-    const bool edge = C % 128 != 0 && C % 4 == 0;
-    prad_status s = PRAD_OK;
+  // 128-long blocks of a matrix in whole float4: the specialised kernel
+  if (vec && C % 4 == 0) {
     switch (pk::fast_op_of(src)) {
-      case 0: s = pk::launch_fast_forms<0>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 1: s = pk::launch_fast_forms<1>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 2: s = pk::launch_fast_forms<2>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 3: s = pk::launch_fast_forms<3>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 4: s = pk::launch_fast_forms<4>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 5: s = pk::launch_fast_forms<5>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 6: s = pk::launch_fast_forms<6>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 7: s = pk::launch_fast_forms<7>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 8: s = pk::launch_fast_forms<8>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 9: s = pk::launch_fast_forms<9>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      case 10: s = pk::launch_fast_forms<10>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
-      default: s = pk::launch_fast_forms<11>(ctx, src, fr_t, fc_t, fr, fc, C, edge); break;
+      case 0: return pk::launch_fast_forms<0>(ctx, src, fr, fc, R, C);
+      case 1: return pk::launch_fast_forms<1>(ctx, src, fr, fc, R, C);
+      case 2: return pk::launch_fast_forms<2>(ctx, src, fr, fc, R, C);
+      case 3: return pk::launch_fast_forms<3>(ctx, src, fr, fc, R, C);
+      case 4: return pk::launch_fast_forms<4>(ctx, src, fr, fc, R, C);
+      case 5: return pk::launch_fast_forms<5>(ctx, src, fr, fc, R, C);
+      case 6: return pk::launch_fast_forms<6>(ctx, src, fr, fc, R, C);
+      case 7: return pk::launch_fast_forms<7>(ctx, src, fr, fc, R, C);
+      case 8: return pk::launch_fast_forms<8>(ctx, src, fr, fc, R, C);
+      case 9: return pk::launch_fast_forms<9>(ctx, src, fr, fc, R, C);
+      case 10: return pk::launch_fast_forms<10>(ctx, src, fr, fc, R, C);
+      case 12: return pk::launch_fast<12, true, true>(ctx, src, fr, fc, R, C);
+      case 13: return pk::launch_fast<13, true, true>(ctx, src, fr, fc, R, C);
+      case 14: return pk::launch_fast<14, true, true>(ctx, src, fr, fc, R, C);
+      default: return pk::launch_fast_forms<11>(ctx, src, fr, fc, R, C);
     }
-    if (s) return s;
-    if (edge) ++fc_t;
   }
-  return pk::launch_pack<128, 128>(ctx, src, vec, R, C, fr, fc, fr_t, fc_t);
+  PRAD_REQUIRE(src.kind < 4, PRAD_ERR_UNSUPPORTED, "operand packing: LayerNormalization needs rows of whole, aligned float4 and 128-long blocks");
+  return pk::launch_pack<128, 128>(ctx, src, vec, R, C, fr, fc);
 }
 
 }  // namespace prad
@@ -567,6 +656,7 @@ struct prad_packed {
   int rows = 0, cols = 0;
   prad::PackedForm by_rows, by_cols;   // h == nullptr when the form was not requested
   bool filled = false;
+  float* column_sums = nullptr;        // where the column sums of what is packed go
   uint32_t magic = 0x50414b44u;        // "PAKD"
 };
 
@@ -648,10 +738,64 @@ prad_status prad_packed_destroy(prad_packed* p) {
 }
 
 static prad_status pack_into(prad_packed* p, PackSource src) {
+  const int part_rows = p->column_sums ? (int)ceil_div(p->rows, p->by_cols.chunk) : 0;
+  if (part_rows) {
+    prad_status w = ensure_workspace(p->ctx, (size_t)part_rows * p->cols * sizeof(double));
+    if (w) return w;
+    src.colsum = (double*)p->ctx->ws;
+  }
   prad_status s = pack_fp16(p->ctx, src, p->rows, p->cols, p->by_rows.h ? &p->by_rows : nullptr,
                             p->by_cols.h ? &p->by_cols : nullptr);
-  if (s == PRAD_OK) p->filled = true;
-  return s;
+  if (s) return s;
+  p->filled = true;
+  if (part_rows) {
+    pk::column_sum_kernel<<<(unsigned)ceil_div(p->cols, 32), 1024, 0, p->ctx->stream>>>(src.colsum, p->column_sums, part_rows, p->cols);
+    PRAD_LAUNCHED(p->ctx);
+  }
+  return PRAD_OK;
+}
+
+prad_status prad_packed_column_sums(prad_packed* p, void* out) {
+  PRAD_CHECK_PACKED(p, "prad_packed_column_sums");
+  PRAD_REQUIRE(!out || p->by_cols.h, PRAD_ERR_INVALID, "prad_packed_column_sums: the object has no by-columns form");
+  p->column_sums = (float*)out;
+  return PRAD_OK;
+}
+
+prad_status prad_layernorm_pack(prad_packed* p, const void* x, const void* residual, void* sum, void* mean, void* stdv) {
+  PRAD_CHECK_PACKED(p, "prad_layernorm_pack");
+  PRAD_CHECK_CTX(p->ctx);
+  PRAD_REQUIRE(x && mean && stdv && (residual != nullptr) == (sum != nullptr), PRAD_ERR_INVALID, "prad_layernorm_pack: null pointer");
+  PRAD_REQUIRE(p->cols <= 128 && p->by_rows.h && p->by_cols.h, PRAD_ERR_UNSUPPORTED,
+               "prad_layernorm_pack: rows of at most 128 columns, both forms");
+  PackSource src;
+  src.kind = 4;
+  src.x = (const float*)x;
+  src.dy = (const float*)residual;
+  src.out = (float*)sum;
+  src.mean = (float*)mean;
+  src.sigma = (float*)stdv;
+  src.ld = p->cols;
+  return pack_into(p, src);
+}
+
+prad_status prad_layernorm_backward_pack(prad_packed* p, const void* x, const void* mean, const void* stdv, const void* dy,
+                                         const void* residual, void* dx) {
+  PRAD_CHECK_PACKED(p, "prad_layernorm_backward_pack");
+  PRAD_CHECK_CTX(p->ctx);
+  PRAD_REQUIRE(x && mean && stdv && dy && residual && dx, PRAD_ERR_INVALID, "prad_layernorm_backward_pack: null pointer");
+  PRAD_REQUIRE(p->cols <= 128 && p->by_rows.h && p->by_cols.h, PRAD_ERR_UNSUPPORTED,
+               "prad_layernorm_backward_pack: rows of at most 128 columns, both forms");
+  PackSource src;
+  src.kind = 5;
+  src.x = (const float*)x;
+  src.dy = (const float*)dy;
+  src.target = (const float*)residual;
+  src.out = (float*)dx;
+  src.mean = const_cast<float*>((const float*)mean);
+  src.sigma = const_cast<float*>((const float*)stdv);
+  src.ld = p->cols;
+  return pack_into(p, src);
 }
 
 prad_status prad_pack(prad_packed* p, const void* x, int64_t ld) {

@@ -451,17 +451,19 @@ template <typename T> struct RowVec;
 template <> struct RowVec<float> { using type = float4; static constexpr int N = 4; };
 template <> struct RowVec<double> { using type = double2; static constexpr int N = 2; };
 
-template <typename T>
+// RES: plus the gradient of the path around the operation (residual), added last.
+template <typename T, bool RES>
 __global__ void __launch_bounds__(256)
 layernorm_backward_flat(const T* __restrict__ x, const T* __restrict__ mean, const T* __restrict__ stdv,
-                        const T* __restrict__ dy, T* __restrict__ dx, int64_t nvec, int vec_per_row, int cols) {
+                        const T* __restrict__ dy, const T* __restrict__ res, T* __restrict__ dx, int64_t nvec, int vec_per_row,
+                        int cols) {
   constexpr int VEC = RowVec<T>::N;
   using V = typename RowVec<T>::type;
   constexpr int U = 4;   // vectors in flight per thread
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const T one_minus = sub_rn((T)1, div_rn((T)1, (T)cols));
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; base < nvec; base += stride * U) {
-    V xv[U], dv[U];
+    V xv[U], dv[U], rv[RES ? U : 1];
     T mu[U], sg[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -469,6 +471,7 @@ layernorm_backward_flat(const T* __restrict__ x, const T* __restrict__ mean, con
       if (i < nvec) {
         xv[u] = __ldcs(reinterpret_cast<const V*>(x) + i);
         dv[u] = __ldcs(reinterpret_cast<const V*>(dy) + i);
+        if (RES) rv[u] = __ldcs(reinterpret_cast<const V*>(res) + i);
         const int64_t r = i / vec_per_row;
         mu[u] = mean[r];
         sg[u] = stdv[r];
@@ -490,6 +493,7 @@ layernorm_backward_flat(const T* __restrict__ x, const T* __restrict__ mean, con
           T d = sub_rn(reinterpret_cast<const T*>(&xv[u])[q], mu[u]);
           reinterpret_cast<T*>(&o)[q] =
               mul_rn(reinterpret_cast<const T*>(&dv[u])[q], sub_rn(exp1, mul_rn(mul_rn(d, d), rden)));
+          if (RES) reinterpret_cast<T*>(&o)[q] = add_rn(reinterpret_cast<const T*>(&rv[u])[q], reinterpret_cast<T*>(&o)[q]);
         }
         __stcs(reinterpret_cast<V*>(dx) + i, o);
       }
@@ -602,8 +606,8 @@ prad_status prad_layernorm_backward(prad_ctx* ctx, prad_dtype dt, const void* x,
   if (cols % vecn == 0 && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) & 15) == 0) {
     const int64_t nvec = rows * (cols / vecn);
     const int grid = stream_grid(ctx, ceil_div(nvec, 4), 256, 8);
-    if (dt == PRAD_F32) layernorm_backward_flat<float><<<grid, 256, 0, ctx->stream>>>((const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, (float*)dx, nvec, cols / vecn, cols);
-    else layernorm_backward_flat<double><<<grid, 256, 0, ctx->stream>>>((const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, (double*)dx, nvec, cols / vecn, cols);
+    if (dt == PRAD_F32) layernorm_backward_flat<float, false><<<grid, 256, 0, ctx->stream>>>((const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, nullptr, (float*)dx, nvec, cols / vecn, cols);
+    else layernorm_backward_flat<double, false><<<grid, 256, 0, ctx->stream>>>((const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, nullptr, (double*)dx, nvec, cols / vecn, cols);
   } else if (short_e(cols)) {
     if (dt == PRAD_F32) PRAD_SHORT_ROWS(layernorm_backward_short, float, (const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, (float*)dx, rows, cols);
     else PRAD_SHORT_ROWS(layernorm_backward_short, double, (const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, (double*)dx, rows, cols);
@@ -611,6 +615,26 @@ prad_status prad_layernorm_backward(prad_ctx* ctx, prad_dtype dt, const void* x,
   else layernorm_backward_kernel<double><<<row_grid(ctx, rows), ROW_WARPS * 32, 0, ctx->stream>>>((const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, (double*)dx, rows, cols);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
+}
+
+prad_status prad_layernorm_backward_add(prad_ctx* ctx, prad_dtype dt, const void* x, const void* mean, const void* stdv,
+                                        const void* dy, const void* residual, void* dx, int64_t rows, int cols) {
+  PRAD_CHECK_CTX(ctx);
+  PRAD_REQUIRE(dtype_ok(dt) && rows >= 0 && cols >= 0, PRAD_ERR_INVALID, "prad_layernorm_backward_add: bad argument");
+  if (rows == 0 || cols == 0) return PRAD_OK;
+  PRAD_REQUIRE(x && mean && stdv && dy && residual && dx && dx != residual, PRAD_ERR_INVALID,
+               "prad_layernorm_backward_add: null pointer, or the result over the residual gradient");
+  const int vecn = dt == PRAD_F32 ? 4 : 2;
+  if (cols % vecn == 0 && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx | (uintptr_t)residual) & 15) == 0) {
+    const int64_t nvec = rows * (cols / vecn);
+    const int grid = stream_grid(ctx, ceil_div(nvec, 4), 256, 8);
+    if (dt == PRAD_F32) layernorm_backward_flat<float, true><<<grid, 256, 0, ctx->stream>>>((const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, (const float*)residual, (float*)dx, nvec, cols / vecn, cols);
+    else layernorm_backward_flat<double, true><<<grid, 256, 0, ctx->stream>>>((const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, (const double*)residual, (double*)dx, nvec, cols / vecn, cols);
+    PRAD_LAUNCHED(ctx);
+    return PRAD_OK;
+  }
+  prad_status s = prad_layernorm_backward(ctx, dt, x, mean, stdv, dy, dx, rows, cols);
+  return s ? s : prad_add_forward(ctx, dt, residual, dx, nullptr, dx, rows * cols);
 }
 
 #define PRAD_ROW_LAUNCH(KERNEL, ...)                                                                     \

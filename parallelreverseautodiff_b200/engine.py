@@ -131,6 +131,22 @@ class PackedOperand:
                                                          dx.ptr if dx is not None else None, alpha))
         return self
 
+    def column_sums(self, out: Optional["DeviceMatrix"]) -> "PackedOperand":
+        """Later packings also leave the column sums of the packed values in `out` (prad_packed_column_sums)."""
+        check(self.engine.lib.prad_packed_column_sums(self.handle, out.ptr if out is not None else None))
+        return self
+
+    def layernorm(self, x, mean, std, residual=None, sum_out=None):
+        """LayerNormalization of x (or of sum_out = x + residual), packed (prad_layernorm_pack)."""
+        check(self.engine.lib.prad_layernorm_pack(self.handle, x.ptr, residual.ptr if residual is not None else None,
+                                                  sum_out.ptr if sum_out is not None else None, mean.ptr, std.ptr))
+        return self
+
+    def layernorm_backward(self, x, mean, std, dy, residual, dx):
+        """dx = residual + LayerNormalization.Backward(dy), stored and packed (prad_layernorm_backward_pack)."""
+        check(self.engine.lib.prad_layernorm_backward_pack(self.handle, x.ptr, mean.ptr, std.ptr, dy.ptr, residual.ptr, dx.ptr))
+        return self
+
     def free(self) -> None:
         if self.handle and self.engine is not None and self.engine.ctx:
             self.engine.lib.prad_packed_destroy(self.handle)
@@ -588,6 +604,13 @@ class Engine:
         check(self.lib.prad_layernorm_backward(self.ctx, dtype_code(x.dtype), x.ptr, mean.ptr,
                                                std.ptr, dy.ptr, out.ptr, x.size // x.shape[-1],
                                                x.shape[-1]))
+        return out
+
+    def layernorm_backward_add(self, x, mean, std, dy, residual, out=None):
+        """residual + layernorm_backward(...): the fan-in at a residual connection."""
+        out = out or self.empty(x.shape, x.dtype)
+        check(self.lib.prad_layernorm_backward_add(self.ctx, dtype_code(x.dtype), x.ptr, mean.ptr, std.ptr, dy.ptr, residual.ptr,
+                                                   out.ptr, x.size // x.shape[-1], x.shape[-1]))
         return out
 
     def swish_forward(self, x, beta, out=None):
