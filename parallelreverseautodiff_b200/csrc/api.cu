@@ -49,6 +49,9 @@ prad_status ensure_host_workspace(prad_ctx* ctx, size_t bytes) {
 prad_status ensure_stage(prad_ctx* ctx, size_t bytes) {
   return grow(ctx, &ctx->stage, &ctx->stage_bytes, bytes, false, "growth of the staging scratch");
 }
+prad_status ensure_parts(prad_ctx* ctx, size_t bytes) {
+  return grow(ctx, &ctx->parts, &ctx->parts_bytes, bytes, false, "growth of the scratch for partial products");
+}
 
 prad_status dp_destroy(prad_ctx* ctx);  // dp.cu
 void runtime_destroy(prad_ctx* ctx);    // runtime.cu
@@ -118,6 +121,7 @@ prad_status prad_shutdown(prad_ctx* ctx) {
   if (ctx->host_flag) cudaFreeHost(ctx->host_flag);
   for (void* r : ctx->retired) cudaFree(r);
   if (ctx->stage) cudaFree(ctx->stage);
+  if (ctx->parts) cudaFree(ctx->parts);
   if (ctx->host_ws) cudaFreeHost(ctx->host_ws);
   if (ctx->copy_stream) { cudaStreamSynchronize(ctx->copy_stream); cudaStreamDestroy(ctx->copy_stream); }
   if (ctx->copy_done) cudaEventDestroy(ctx->copy_done);

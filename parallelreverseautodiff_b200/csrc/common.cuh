@@ -43,6 +43,9 @@ struct prad_ctx {
   // host-buffer entry points keep their device staging here
   void* stage = nullptr;
   size_t stage_bytes = 0;
+  // partial products of contractions cut into k slices (never the staging block: a host entry point's operands are there)
+  void* parts = nullptr;
+  size_t parts_bytes = 0;
   prad::DpState* dp = nullptr;
   prad::DevicePool* pool = nullptr;
   size_t total_mem = 0;               // device memory in bytes
@@ -144,6 +147,7 @@ prad_status ensure_workspace(prad_ctx* ctx, size_t bytes);
 // grows the pinned host scratch
 prad_status ensure_host_workspace(prad_ctx* ctx, size_t bytes);
 prad_status ensure_stage(prad_ctx* ctx, size_t bytes);
+prad_status ensure_parts(prad_ctx* ctx, size_t bytes);
 
 // device memory with a bounded cache of freed blocks (pool.cu)
 prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out);

@@ -245,9 +245,9 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
     S = (int)ceil_div(K, k_slice);
     if (S >= 2) {
       const int64_t mn = (int64_t)M * N;
-      st = ensure_stage(ctx, (size_t)batch * S * mn * sizeof(double));
+      st = ensure_parts(ctx, (size_t)batch * S * mn * sizeof(double));
       if (st) return st;
-      double* part = (double*)ctx->stage;
+      double* part = (double*)ctx->parts;
       pr.slices = S;
       pr.k_slice = k_slice;
       pr.p.alpha = 1.0;

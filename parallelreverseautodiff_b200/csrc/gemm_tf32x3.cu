@@ -1747,9 +1747,9 @@ static prad_status launch_tf32x3(prad_ctx* ctx, const SplitOperand& a, const Spl
     PRAD_LAUNCHED(ctx);
   } else {
     const int64_t mn = (int64_t)M * N;
-    prad_status st = ensure_stage(ctx, (size_t)splits * mn * sizeof(float));
+    prad_status st = ensure_parts(ctx, (size_t)splits * mn * sizeof(float));
     if (st) return st;
-    float* part = (float*)ctx->stage;
+    float* part = (float*)ctx->parts;
     Epi raw = epi;
     raw.alpha = 1.f;
     raw.beta = 0.f;
@@ -1855,9 +1855,9 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
     PRAD_LAUNCHED(ctx);
   } else {
     const int64_t mn = (int64_t)M * N;
-    prad_status st = ensure_stage(ctx, (size_t)splits * mn * sizeof(float));
+    prad_status st = ensure_parts(ctx, (size_t)splits * mn * sizeof(float));
     if (st) return st;
-    float* part = (float*)ctx->stage;
+    float* part = (float*)ctx->parts;
     Epi raw = epi;
     raw.alpha = 1.f;
     raw.beta = 0.f;
