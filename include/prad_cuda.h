@@ -195,6 +195,9 @@ prad_status prad_download(prad_ctx* ctx, void* dst_host, const void* src, size_t
  * still running on the compute stream (use a second buffer). */
 prad_status prad_upload_prefetch(prad_ctx* ctx, void* dst, const void* src_host, size_t bytes);
 prad_status prad_upload_join(prad_ctx* ctx);
+/* Prefetches issued from here on start after everything the compute stream was given before this call: a destination which that
+ * work still reads may then be written.  (From pageable memory a prefetch returns once it has consumed src_host.) */
+prad_status prad_upload_fence(prad_ctx* ctx);
 /* jagged form: `rows` host row pointers of row_bytes each <-> one dense device matrix */
 prad_status prad_upload_rows(prad_ctx* ctx, void* dst, const void* const* src_rows, int rows,
                              size_t row_bytes);
@@ -231,7 +234,8 @@ prad_status prad_free_host(prad_ctx* ctx, void* hptr);
 
 /* ---------------------------------------------------------------- GEMM
  * General row-major product C = alpha*op(A)*op(B) + beta*C over `batch` slices
- * (stride 0 = operand shared by all slices).  op(A) is MxK, op(B) is KxN.
+ * (stride 0 = operand shared by all slices).  op(A) is MxK, op(B) is KxN.  strideC = 0 with more than one slice: C receives
+ * alpha * (P_0 + P_1 + ...) + beta * C, the slices' products added in order (the fan-in of an input used by several gates).
  * Replaces the ILGPU tiled kernel (src/RMAD/GpuMatrixMultiplyOperation.cs:39-91)
  * and the cuBLAS Gemm call (src/RMAD/CudaBlas.cs:245,293). */
 prad_status prad_gemm(prad_ctx* ctx, prad_dtype dt, int transA, int transB, int M, int N, int K,
@@ -429,6 +433,10 @@ prad_status prad_add_broadcast_forward(prad_ctx* ctx, prad_dtype dt, const void*
                                        const void* bias, void* y, int rows, int cols);
 prad_status prad_add_broadcast_backward(prad_ctx* ctx, prad_dtype dt, const void* dy,
                                         void* dbias, int rows, int cols, int accumulate);
+/* The same sums for `batch` matrices of rows x cols, `stride` elements apart, each multiplied by scale: row q of out
+ * (out_stride elements apart) = scale * column sums of matrix q.  The bias gradients of an LSTM's gates in one call. */
+prad_status prad_column_sums(prad_ctx* ctx, prad_dtype dt, const void* x, int rows, int cols, int batch, int64_t stride,
+                             double scale, void* out, int64_t out_stride);
 /* Allocation-free form of prad_add_broadcast_backward.  It has no counterpart in the
  * reference.  It exists for callers that must not allocate device memory at the moment they
  * need the bias gradient: a plug-in running inside a host application that has handed out

@@ -52,6 +52,8 @@ SIGNATURES = {
     "prad_act_forward_pack": [vp, i32, vp, vp, f64],
     "prad_act_backward_pack": [vp, i32, vp, vp, vp, f64],
     "prad_mse_act_backward_pack": [vp, i32, vp, vp, vp, i64, vp, f64],
+    "prad_column_sums": [vp, i32, vp, i32, i32, i32, i64, f64, vp, i64],
+    "prad_upload_fence": [vp],
     "prad_packed_column_sums": [vp, vp],
     "prad_layernorm_pack": [vp, vp, vp, vp, vp, vp],
     "prad_layernorm_backward_pack": [vp, vp, vp, vp, vp, vp, vp],

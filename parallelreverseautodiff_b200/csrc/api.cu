@@ -337,15 +337,30 @@ prad_status prad_download(prad_ctx* ctx, void* dst_host, const void* src, size_t
   return gemm_tf32x3_check(ctx);
 }
 
+static prad_status ensure_copy_stream(prad_ctx* ctx) {
+  if (ctx->copy_stream) return PRAD_OK;
+  PRAD_CUDA(cudaEventCreateWithFlags(&ctx->copy_done, cudaEventDisableTiming));
+  PRAD_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+  return PRAD_OK;
+}
+
+prad_status prad_upload_fence(prad_ctx* ctx) {
+  PRAD_CHECK_CTX(ctx);
+  PRAD_NOT_CAPTURING(ctx, "prad_upload_fence");
+  prad_status s = ensure_copy_stream(ctx);
+  if (s) return s;
+  PRAD_CUDA(cudaEventRecord(ctx->copy_done, ctx->stream));
+  PRAD_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_done, 0));
+  return PRAD_OK;
+}
+
 prad_status prad_upload_prefetch(prad_ctx* ctx, void* dst, const void* src_host, size_t bytes) {
   PRAD_CHECK_CTX(ctx);
   PRAD_NOT_CAPTURING(ctx, "prad_upload_prefetch");
   PRAD_REQUIRE((dst && src_host) || bytes == 0, PRAD_ERR_INVALID, "prad_upload_prefetch: null pointer");
   if (bytes == 0) return PRAD_OK;
-  if (!ctx->copy_stream) {
-    PRAD_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
-    PRAD_CUDA(cudaEventCreateWithFlags(&ctx->copy_done, cudaEventDisableTiming));
-  }
+  prad_status s = ensure_copy_stream(ctx);
+  if (s) return s;
   PRAD_CUDA(cudaMemcpyAsync(dst, src_host, bytes, cudaMemcpyHostToDevice, ctx->copy_stream));
   ctx->copy_pending = true;
   return PRAD_OK;

@@ -155,10 +155,21 @@ __global__ void add_broadcast_kernel(const T* x, const T* __restrict__ bias, T* 
 // Two deterministic stages: each CTA sums a band of rows for a 32-column strip into
 // partial[band][col] (coalesced 128-byte row segments), then one pass adds the bands in
 // band order.  Accumulation is in double for float data (LINQ Sum accumulates in double).
+// blockIdx.z: matrix of a batch, x_stride elements apart in, out_stride apart out; every result is multiplied by `scale` (one
+// rounding, as a scaling of its own).
+template <typename T>
+__device__ __forceinline__ void put_colsum(T* out, double s, T scale, int accumulate) {
+  T v = (T)s;
+  if (scale != (T)1) v = mul_rn(v, scale);
+  *out = accumulate ? add_rn(*out, v) : v;
+}
 template <typename T>
 __global__ void __launch_bounds__(256)
 colsum_partial_kernel(const T* __restrict__ x, double* __restrict__ partial, int64_t rows,
-                      int cols, int rows_per_band, T* __restrict__ direct_out, int accumulate) {
+                      int cols, int rows_per_band, T* __restrict__ direct_out, int accumulate, int64_t x_stride = 0,
+                      int64_t out_stride = 0, T scale = (T)1) {
+  x += blockIdx.z * x_stride;
+  if (!direct_out) partial += (int64_t)blockIdx.z * gridDim.y * cols;
   // direct_out: there is one band only (a short matrix) and the sums go straight to the result: one launch
   __shared__ double sm[8][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -168,6 +179,7 @@ colsum_partial_kernel(const T* __restrict__ x, double* __restrict__ partial, int
   if (r1 > rows) r1 = rows;
   double acc = 0.0;
   if (col < cols)
+#pragma unroll 4
     for (int64_t r = r0 + w; r < r1; r += 8) acc += (double)x[r * cols + col];
   sm[w][lane] = acc;
   __syncthreads();
@@ -177,8 +189,7 @@ colsum_partial_kernel(const T* __restrict__ x, double* __restrict__ partial, int
     for (int k = 0; k < 8; ++k) s += sm[k][lane];
     if (col < cols) {
       if (direct_out) {
-        const T v = (T)s;
-        direct_out[col] = accumulate ? add_rn(direct_out[col], v) : v;
+        put_colsum(direct_out + blockIdx.z * out_stride + col, s, scale, accumulate);
       } else {
         partial[(int64_t)blockIdx.y * cols + col] = s;
       }
@@ -189,7 +200,9 @@ colsum_partial_kernel(const T* __restrict__ x, double* __restrict__ partial, int
 // (8 warps with one row each took 6.9 us for 256 x 512, this 4.7 us).
 template <typename T>
 __global__ void __launch_bounds__(1024)
-colsum_short_kernel(const T* __restrict__ x, T* __restrict__ out, int rows, int cols, int accumulate) {
+colsum_short_kernel(const T* __restrict__ x, T* __restrict__ out, int rows, int cols, int accumulate, int64_t x_stride,
+                    int64_t out_stride, T scale) {
+  x += blockIdx.z * x_stride;
   __shared__ double sm[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
@@ -208,19 +221,19 @@ colsum_short_kernel(const T* __restrict__ x, T* __restrict__ out, int rows, int 
     double s = 0.0;
 #pragma unroll
     for (int k = 0; k < 32; ++k) s += sm[k][lane];
-    const T v = (T)s;
-    out[col] = accumulate ? add_rn(out[col], v) : v;
+    put_colsum(out + blockIdx.z * out_stride + col, s, scale, accumulate);
   }
 }
 template <typename T>
 __global__ void colsum_final_kernel(const double* __restrict__ partial, T* __restrict__ out,
-                                    int cols, int bands, int accumulate) {
+                                    int cols, int bands, int accumulate, int64_t out_stride = 0, T scale = (T)1) {
   int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= cols) return;
+  partial += (int64_t)blockIdx.z * bands * cols;
   double s = 0.0;
+#pragma unroll 8
   for (int b = 0; b < bands; ++b) s += partial[(int64_t)b * cols + col];
-  T v = (T)s;
-  out[col] = accumulate ? add_rn(out[col], v) : v;
+  put_colsum(out + blockIdx.z * out_stride + col, s, scale, accumulate);
 }
 
 // Streaming form of the same column sums for matrices whose rows are a whole number of
@@ -312,11 +325,12 @@ colsum_flat_final_kernel(const double* __restrict__ partial, T* __restrict__ out
   }
 }
 
+// The column sums of `batch` matrices, `stride` elements apart, each multiplied by scale, in rows of out `out_stride` apart
 template <typename T>
-static prad_status add_broadcast_backward_t(prad_ctx* ctx, const void* dy, void* dbias,
-                                            int64_t rows, int cols, int accumulate) {
+static prad_status add_broadcast_backward_t(prad_ctx* ctx, const void* dy, void* dbias, int64_t rows, int cols, int accumulate,
+                                            int batch = 1, int64_t stride = 0, int64_t out_stride = 0, T scale = (T)1) {
   constexpr int VEC = Vec16<T>::N;
-  if (cols % VEC == 0 && ((uintptr_t)dy & 15) == 0 && rows * (int64_t)cols >= (1 << 20)) {
+  if (batch == 1 && scale == (T)1 && cols % VEC == 0 && ((uintptr_t)dy & 15) == 0 && rows * (int64_t)cols >= (1 << 20)) {
     const int vec_per_row = cols / VEC;
     int64_t threads = (int64_t)ctx->sm_count * 8 * 256;
     const int64_t nvec = rows * vec_per_row;
@@ -342,31 +356,32 @@ static prad_status add_broadcast_backward_t(prad_ctx* ctx, const void* dy, void*
     }
   }
   int strips = (int)ceil_div(cols, 32);
-  int64_t want_bands = ceil_div((int64_t)ctx->sm_count * 8, strips);
+  int64_t want_bands = ceil_div((int64_t)ctx->sm_count * 8, (int64_t)strips * batch);
   int64_t max_bands = ceil_div(rows, 64);
   int bands = (int)(want_bands < max_bands ? want_bands : max_bands);
   if (bands < 1) bands = 1;
   if (bands > 65535) bands = 65535;
   if (rows <= 512) {
-    colsum_short_kernel<T><<<(unsigned)strips, 1024, 0, ctx->stream>>>((const T*)dy, (T*)dbias, (int)rows, cols, accumulate);
+    colsum_short_kernel<T><<<dim3(strips, 1, batch), 1024, 0, ctx->stream>>>((const T*)dy, (T*)dbias, (int)rows, cols, accumulate,
+                                                                            stride, out_stride, scale);
     PRAD_LAUNCHED(ctx);
     return PRAD_OK;
   }
   int rows_per_band = (int)ceil_div(rows, bands);
   bands = (int)ceil_div(rows, rows_per_band);
   if (bands == 1) {
-    colsum_partial_kernel<T><<<dim3(strips, 1), 256, 0, ctx->stream>>>((const T*)dy, nullptr, rows, cols, rows_per_band,
-                                                                      (T*)dbias, accumulate);
+    colsum_partial_kernel<T><<<dim3(strips, 1, batch), 256, 0, ctx->stream>>>((const T*)dy, nullptr, rows, cols, rows_per_band,
+                                                                             (T*)dbias, accumulate, stride, out_stride, scale);
     PRAD_LAUNCHED(ctx);
     return PRAD_OK;
   }
-  prad_status s = ensure_workspace(ctx, (size_t)bands * cols * sizeof(double));
+  prad_status s = ensure_workspace(ctx, (size_t)batch * bands * cols * sizeof(double));
   if (s) return s;
-  colsum_partial_kernel<T><<<dim3(strips, bands), 256, 0, ctx->stream>>>(
-      (const T*)dy, (double*)ctx->ws, rows, cols, rows_per_band, nullptr, 0);
+  colsum_partial_kernel<T><<<dim3(strips, bands, batch), 256, 0, ctx->stream>>>(
+      (const T*)dy, (double*)ctx->ws, rows, cols, rows_per_band, nullptr, 0, stride);
   PRAD_LAUNCHED(ctx);
-  colsum_final_kernel<T><<<(unsigned)ceil_div(cols, 128), 128, 0, ctx->stream>>>(
-      (const double*)ctx->ws, (T*)dbias, cols, bands, accumulate);
+  colsum_final_kernel<T><<<dim3((unsigned)ceil_div(cols, 32), 1, batch), 32, 0, ctx->stream>>>(
+      (const double*)ctx->ws, (T*)dbias, cols, bands, accumulate, out_stride, scale);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
@@ -592,6 +607,17 @@ prad_status prad_add_broadcast_backward(prad_ctx* ctx, prad_dtype dt, const void
   }
   return DISPATCH_DT(dt, add_broadcast_backward_t<float>(ctx, dy, dbias, rows, cols, accumulate),
                      add_broadcast_backward_t<double>(ctx, dy, dbias, rows, cols, accumulate));
+}
+
+prad_status prad_column_sums(prad_ctx* ctx, prad_dtype dt, const void* x, int rows, int cols, int batch, int64_t stride, double scale,
+                             void* out, int64_t out_stride) {
+  PRAD_CHECK_CTX(ctx);
+  PRAD_REQUIRE(dtype_ok(dt) && rows >= 1 && cols >= 0 && batch >= 0 && batch <= 65535 && out_stride >= cols && stride >= 0,
+               PRAD_ERR_INVALID, "prad_column_sums: bad argument");
+  if (cols == 0 || batch == 0) return PRAD_OK;
+  PRAD_REQUIRE(x && out, PRAD_ERR_INVALID, "prad_column_sums: null pointer");
+  return DISPATCH_DT(dt, add_broadcast_backward_t<float>(ctx, x, out, rows, cols, 0, batch, stride, out_stride, (float)scale),
+                     add_broadcast_backward_t<double>(ctx, x, out, rows, cols, 0, batch, stride, out_stride, scale));
 }
 
 prad_status prad_scale(prad_ctx* ctx, prad_dtype dt, const void* x, void* y, int64_t n,

@@ -238,12 +238,15 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
   // four are 32 tiles): k is cut into slices of at least 256 that run as further tiles into scratch, enough of them for two
   // CTAs on every SM, and an ordered pass adds them.
   const bool plain = !e.bias && !e.z_out && e.act == PRAD_ACT_NONE && e.dact == PRAD_ACT_NONE;
-  if (plain && tiles * 2 <= ctx->sm_count && K >= 512) {
+  // The sum over a batch (sC = 0) is that with the batch entries as further slices.
+  const bool sum = batch > 1 && sC == 0;
+  if (plain && (sum || (tiles * 2 <= ctx->sm_count && K >= 512))) {
     int S = (int)(2 * ctx->sm_count / tiles);
     if (S > K / 256) S = K / 256;
+    if (S < 1) S = 1;
     const int k_slice = (int)(ceil_div(ceil_div(K, S), dm::BK) * dm::BK);
     S = (int)ceil_div(K, k_slice);
-    if (S >= 2) {
+    if (S >= 2 || sum) {
       const int64_t mn = (int64_t)M * N;
       st = ensure_parts(ctx, (size_t)batch * S * mn * sizeof(double));
       if (st) return st;
@@ -258,7 +261,8 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
       pr.p.vecC = N % 2 == 0 && mn % 2 == 0;
       if ((st = dm::launch(ctx, tA, tB, pr, tiles * S))) return st;
       const int cg = stream_grid(ctx, mn, 256, 8);
-      dm::combine_kernel<<<dim3((unsigned)cg, (unsigned)batch), 256, 0, ctx->stream>>>(part, S, mn, N, (double*)C, ldc, sC, alpha, beta);
+      dm::combine_kernel<<<dim3((unsigned)cg, sum ? 1u : (unsigned)batch), 256, 0, ctx->stream>>>(
+          part, sum ? S * batch : S, mn, N, (double*)C, ldc, sC, alpha, beta);
       PRAD_LAUNCHED(ctx);
       return PRAD_OK;
     }

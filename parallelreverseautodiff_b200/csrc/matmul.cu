@@ -47,6 +47,26 @@ prad_status gemm_dispatch(prad_ctx* ctx, prad_dtype dt, bool tA, bool tB, int M,
                           int64_t sC, const GemmEpilogue& epi) {
   if (M == 0 || N == 0 || batch == 0) return PRAD_OK;
   const bool tc = wants_tensor_cores(ctx, dt, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi);
+  // One result for the whole batch: the sum over its products.  On the FP64 tensor cores they are k slices (gemm_f64_dmma);
+  // otherwise one launch writes them side by side and another adds them, or, where C has a pitch or an old value to keep, each
+  // is added by the next product.
+  if (batch > 1 && sC == 0 && !(tc && dt == PRAD_F64)) {
+    const size_t es = dtype_size(dt);
+    const int64_t mn = (int64_t)M * N;
+    prad_status s;
+    if (!tc && ldc == N && beta == 0.0 && batch <= 8 && mn <= (1 << 20)) {
+      if ((s = ensure_parts(ctx, (size_t)batch * mn * es))) return s;
+      const void* parts[8];
+      for (int b = 0; b < batch; ++b) parts[b] = (char*)ctx->parts + b * mn * es;
+      if ((s = gemm_dispatch(ctx, dt, tA, tB, M, N, K, alpha, A, lda, B, ldb, 0.0, ctx->parts, N, batch, sA, sB, mn, epi))) return s;
+      return prad_segmented_sum(ctx, dt, parts, batch, C, mn);
+    }
+    for (int b = 0; b < batch; ++b)
+      if ((s = gemm_dispatch(ctx, dt, tA, tB, M, N, K, alpha, (const char*)A + b * sA * es, lda, (const char*)B + b * sB * es, ldb,
+                             b ? 1.0 : beta, C, ldc, 1, 0, 0, 0, epi)))
+        return s;
+    return PRAD_OK;
+  }
   if (dt == PRAD_F32)
     return tc ? gemm_tf32x3(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, false)
               : gemm_simt<float>(ctx, ctx->gemm_f32 != GemmF32::SimtFma, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,

@@ -334,6 +334,10 @@ class Engine:
         assert a.flags.c_contiguous and out.nbytes == a.nbytes
         check(self.lib.prad_upload_prefetch(self.ctx, out.ptr, a.ctypes.data, a.nbytes))
 
+    def upload_fence(self) -> None:
+        """Later prefetches start after the work given to the compute stream so far."""
+        check(self.lib.prad_upload_fence(self.ctx))
+
     def upload_join(self) -> None:
         check(self.lib.prad_upload_join(self.ctx))
 
@@ -540,6 +544,11 @@ class Engine:
         check(self.lib.prad_add_broadcast_forward(self.ctx, dtype_code(x.dtype), x.ptr, bias.ptr,
                                                   out.ptr, x.shape[0], x.shape[1]))
         return out
+
+    def column_sums(self, x, out, rows, batch, scale=1.0):
+        """out[q] = scale * column sums of matrix q of the `batch` stacked rows x cols matrices in x."""
+        cols = out.shape[-1]
+        check(self.lib.prad_column_sums(self.ctx, dtype_code(x.dtype), x.ptr, rows, cols, batch, rows * cols, scale, out.ptr, cols))
 
     def add_broadcast_backward(self, dy, dbias=None, accumulate=False):
         dbias = dbias or self.empty((1, dy.shape[1]), dy.dtype)

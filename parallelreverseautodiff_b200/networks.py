@@ -530,7 +530,7 @@ class LstmNetwork:
         self.b = {g: z(1, n_hidden) for g in self.GATES}
         self._dW_all, self.dW = stacked(n_hidden, n_in)
         self._dU_all, self.dU = stacked(n_hidden, n_hidden)
-        self.db = {g: z(1, n_hidden) for g in self.GATES}
+        self._db_all, self.db = stacked(1, n_hidden)
         self.X = z(TB, n_in)
         self.Y = z(TB, n_hidden)                                  # targets
         self._pre_all, self.pre = stacked(TB, n_hidden)           # gate pre-activations
@@ -562,7 +562,7 @@ class LstmNetwork:
         """x_host [T, B, in], y_host [T, B, hidden]."""
         e, T, B = self.eng, self.T, self.B
         e.upload(np.ascontiguousarray(x_host, self.dtype).reshape(T * B, -1), out=self.X)
-        e.upload(np.ascontiguousarray(y_host, self.dtype).reshape(T * B, -1), out=self.Y)
+        e.upload_fence()
         nh, n_in, TB, G = self.n_h, self.n_in, T * B, len(self.GATES)
         first = self.GATES[0]
         # input contribution of all steps and gates: X_all * W_g^T, one strided-batched product
@@ -571,6 +571,9 @@ class LstmNetwork:
         # per step + h_{t-1} * U_g^T + b_g (MatrixAddThree: (Wx + Uh) + b), the gates and the cell
         e.lstm_forward(T, B, self._U_all, [self.b[g] for g in self.GATES], self._pre_all, [self.gate[g] for g in self.GATES],
                        self.C, self.tanhC, self.H, self.Hprev, self.FC, self.IG)
+        # the targets, which only Backward needs, travel beside these kernels
+        e.upload_prefetch(np.ascontiguousarray(y_host, self.dtype).reshape(T * B, -1), self.Y)
+        e.upload_join()
         return self.H
 
     def backward(self):
@@ -585,22 +588,15 @@ class LstmNetwork:
             e.lstm_backward(T, B, self._U_all, self.H, self.Y, 2.0 / nh, [self.gate[g] for g in self.GATES], self.tanhC, self.C,
                             self._dpre_all, self._seq_scratch)
         inv_b = 1.0 / B
-        first = True
         g0, G, TB = self.GATES[0], len(self.GATES), T * B
         # dW_g = (1/B) * dZ_all^T X_all ; dU_g = (1/B) * dZ_all^T Hprev_all : the four gates per launch
         e.gemm(self.dpre[g0], self.X, self.dW[g0], transA=True, alpha=inv_b, batch=G, strideA=TB * nh, strideB=0,
                strideC=nh * self.n_in)
         e.gemm(self.dpre[g0], self.Hprev, self.dU[g0], transA=True, alpha=inv_b, batch=G, strideA=TB * nh,
                strideB=0, strideC=nh * nh)
-        for g in self.GATES:
-            # db_g = (1/B) colsum
-            e.add_broadcast_backward(self.dpre[g], dbias=self.db[g])
-            e.scale(self.db[g], inv_b, out=self.db[g])
-            # dX_all = sum over gates of dZ_g W_g (left fold in gate order)
-            e.gemm(self.dpre[g], self.W[g], self.dX, beta=0.0 if first else 1.0)
-            first = False
-
-
+        e.column_sums(self._dpre_all, self._db_all, TB, G, inv_b)          # db_g = (1/B) colsum
+        # dX_all = sum over gates of dZ_g W_g (left fold in gate order)
+        e.gemm(self.dpre[g0], self.W[g0], self.dX, batch=G, strideA=TB * nh, strideB=nh * self.n_in, strideC=0)
 
     def _backward_steps_by_operation(self):
         """The time loop of the backward with one library call per managed operation."""
