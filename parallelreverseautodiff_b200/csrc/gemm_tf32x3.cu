@@ -211,9 +211,9 @@ __host__ __device__ constexpr uint32_t idesc_tf32() {
 __host__ __device__ constexpr uint32_t idesc_bf16() {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
-// Instruction descriptor: D = F32, A = B = FP16, both K-major, M = 128, N = 256 (kind::f16).
-__host__ __device__ constexpr uint32_t idesc_fp16() {
-  return (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+// Instruction descriptor: D = F32, A = B = FP16, both K-major, M = 128, N = bn (kind::f16).
+__host__ __device__ constexpr uint32_t idesc_fp16(int bn) {
+  return (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -592,7 +592,8 @@ __device__ __forceinline__ void epilogue_quad(float o0, float o1, float o2, floa
 
 // sum[g][j] = column col0 + 32 g + j of row row0 + lane (modified in place)
 __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lane, int row0, int col0, int M, int N,
-                                                    float* __restrict__ C, int64_t ldc, bool vecC, const Epi& epi) {
+                                                    float* __restrict__ C, int64_t ldc, bool vecC, const Epi& epi,
+                                                    const float4* bias = nullptr) {     // epi.bias from col0 on
   const int qrow = row0 + 4 * (lane >> 2), i = lane & 3;
   // A tile inside the matrix with a plain epilogue (nearly every store of a large product): no bounds tests, no
   // per-quad address arithmetic -- four row pointers and immediate offsets.  This is about instruction fetch, not about
@@ -602,7 +603,7 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
   // (Columns: the warp's 128 or, at the right edge, a multiple of 16, so that each store instruction is all or nothing.)
   const int ncols = N - col0 < 128 ? N - col0 : 128;
   if (ncols <= 0 || row0 >= M) return;
-  if (vecC && epi.beta == 0.f && ((uintptr_t)epi.bias & 15) == 0 && !epi.row_exp && row0 + 32 <= M && (ncols & 15) == 0) {
+  if (vecC && epi.beta == 0.f && (bias || ((uintptr_t)epi.bias & 15) == 0) && !epi.row_exp && row0 + 32 <= M && (ncols & 15) == 0) {
     float* rp[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) rp[s] = C + (int64_t)(qrow + s) * ldc + col0 + 4 * i;
@@ -619,7 +620,7 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
           if (32 * g + j < ncols) {
-            const float4 b = *reinterpret_cast<const float4*>(epi.bias + col0 + 32 * g + j);
+            const float4 b = bias ? bias[8 * g + j / 4] : *reinterpret_cast<const float4*>(epi.bias + col0 + 32 * g + j);
             sum[g][j] += b.x; sum[g][j + 1] += b.y; sum[g][j + 2] += b.z; sum[g][j + 3] += b.w;
           }
     }
@@ -684,8 +685,12 @@ constexpr int UNITS = 4;
 constexpr int UNIT_BYTES = 48 * 1024;
 constexpr int CHUNK_KB = CHUNK_K / BK;
 constexpr int SCALE_BYTES = EPI_WARPS * 128 * 4;   // PMODE 3: each epilogue warp's copy of its 128 column scales of a block
-constexpr int SMEM_BYTES = UNITS * UNIT_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + SCALE_BYTES;
+constexpr int SMEM_BYTES = UNITS * UNIT_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + 2 * SCALE_BYTES /*scales, bias*/;
 static_assert(SMEM_BYTES <= 227 * 1024, "unit ring does not fit in shared memory");
+// PMODE 3: columns of an output tile.  256, or where a matrix of that many tiles leaves a good part of them empty, the width
+// that shares its columns evenly (a multiple of 32: half a tile per epilogue warp, 16 columns per store instruction): with
+// 256-wide tiles the 96 columns of a 200704 x 96 product were a third of what the tensor core and the epilogue worked on.
+inline int tile_width(int N) { return (int)ceil_div(ceil_div(N, ceil_div(N, BN)), 32) * 32; }
 }  // namespace p1
 
 struct TileSched {
@@ -695,6 +700,7 @@ struct TileSched {
   int panel_n;                    // column tiles per panel of the tile walk
   int64_t split_stride;           // elements between the partial products of consecutive slices
   int prefetch_kb;                // PMODE 3: k-blocks by which an L2 prefetch of the row operand runs ahead of its load (0 = none)
+  int bn = BN;                    // columns of a tile (PMODE 3; BN otherwise)
 };
 
 template <int PMODE>
@@ -771,7 +777,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
     const int r = t2 - p * ts.tiles_m * ts.panel_n;
     const int w = min(ts.panel_n, ts.tiles_n - p * ts.panel_n);
     m0 = (r / w) * BM;
-    n0 = (p * ts.panel_n + r % w) * BN;
+    n0 = (p * ts.panel_n + r % w) * ts.bn;
     kb0 = z * ts.kb_per_split;
     num_kb = min(ts.total_kb - kb0, ts.kb_per_split);
   };
@@ -799,8 +805,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
             const uint32_t slot = g & (UNITS - 1), round = g / UNITS;
             if (round > 0 && !mbar_wait(empty_bar(slot), (round - 1) & 1, err_flag, 1)) { ok = false; break; }
             const uint32_t st = base + slot * UNIT_BYTES;
-            mbar_expect_tx(full_bar(slot), UNIT_BYTES);
-            if (PMODE == 3) {  // one unit: A rows (h0 | h1) 16 KB, B rows (h0 | h1) 32 KB; x counts halves
+            mbar_expect_tx(full_bar(slot), PMODE == 3 ? 16 * 1024 + ts.bn * 128 : UNIT_BYTES);
+            if (PMODE == 3) {  // one unit: A rows (h0 | h1) 16 KB, B rows (h0 | h1) 128 bytes each; x counts halves
               tma_load_2d(st, &map_a_xb, full_bar(slot), 2 * x, m0);
               tma_load_2d(st + 16 * 1024, &map_b_xb, full_bar(slot), 2 * x, n0);
               // the row operand streams from DRAM: its tile of a later k-block is requested into L2 now
@@ -852,7 +858,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
           const int kb_end = min(num_kb, (ch + 1) * ts.chunk_kb);
           for (int kb = ch * ts.chunk_kb; kb < kb_end && ok; ++kb) {
             if (PMODE == 3) {   // one unit: A (h0 | h1 per row), B likewise; three FP16 products, smallest first
-              constexpr uint32_t idesc_q = idesc_fp16();
+              const uint32_t idesc_q = idesc_fp16(ts.bn);
               const uint32_t slot = g & (UNITS - 1);
               PROBE_WAIT(w_full, ok = mbar_wait(full_bar(slot), (g / UNITS) & 1, err_flag, 2));
               if (!ok) break;
@@ -917,7 +923,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int sub = warp & 3;                 // TMEM sub-partition this warp may read
-    const int half = (warp - 2) >> 2;         // which 128 columns of the tile
+    const int half = (warp - 2) >> 2;         // which half of the tile's columns
+    const int hw = ts.bn >> 1;
     uint32_t gc = 0, qi = 0;
     bool ok = true;
 #ifdef PRAD_GEMM_STALL_PROBE
@@ -946,9 +953,21 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       float4* const sb_slot = reinterpret_cast<float4*>(generic_base + UNITS * UNIT_BYTES + 256) + (warp - 2) * 32;
       auto fetch_scales = [&](int ch) {
         sa_next = __ldg(epi.blk_a + (int64_t)(chunk0 + ch) * epi.blk_lda + row_blk);
-        sb_next = __ldg(reinterpret_cast<const float4*>(epi.blk_b + (int64_t)(chunk0 + ch) * epi.blk_ldb + n0 + half * 128) + lane);
+        sb_next = __ldg(reinterpret_cast<const float4*>(epi.blk_b + (int64_t)(chunk0 + ch) * epi.blk_ldb + n0 + half * hw) + lane);
       };
       if (PMODE == 3) fetch_scales(0);
+      // the bias of the warp's columns waits in shared memory for the store: read from there when the product is done, it kept
+      // every tile waiting (200704 x 384 over k = 96: 136 us with it, 101 us without)
+      float4* const bias_slot = sb_slot + EPI_WARPS * 32;
+      if (PMODE == 3 && epi.bias) {
+        const int c = n0 + half * hw + 4 * lane;
+        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c < N) b.x = __ldg(epi.bias + c);
+        if (c + 1 < N) b.y = __ldg(epi.bias + c + 1);
+        if (c + 2 < N) b.z = __ldg(epi.bias + c + 2);
+        if (c + 3 < N) b.w = __ldg(epi.bias + c + 3);
+        bias_slot[lane] = b;            // (the last tile's readers passed the __syncwarp before its accumulator was released)
+      }
       for (int ch = 0; ch < num_chunks; ++ch, ++gc) {
         const uint32_t buf = gc & 1;
         float sa = 0.f;
@@ -968,7 +987,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
         const long long c2_ = clock64();
         e_wait += c2_ - c1_;
 #endif
-        const uint32_t taddr = tmem_base + ((uint32_t)(sub * 32) << 16) + buf * (uint32_t)BN + (uint32_t)(half * 128);
+        const uint32_t taddr = tmem_base + ((uint32_t)(sub * 32) << 16) + buf * (uint32_t)BN + (uint32_t)(half * hw);
         if (PMODE == 3) {
           // eight columns per load, the next load in flight while the current eight are added: the live
           // registers stay at 128 running sums + two loads
@@ -977,9 +996,10 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
           tmem_ld8(taddr, v[0]);
 #pragma unroll
           for (int g = 0; g < 16; ++g) {
+            if (g * 8 >= hw) break;
             uint32_t (&cur)[8] = v[g & 1];
             tmem_ld_wait8(cur);
-            if (g + 1 < 16) tmem_ld8(taddr + (uint32_t)((g + 1) * 8), v[(g + 1) & 1]);
+            if (g + 1 < 16 && (g + 1) * 8 < hw) tmem_ld8(taddr + (uint32_t)((g + 1) * 8), v[(g + 1) & 1]);
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
               const float4 t = sb_slot[g * 2 + q];
@@ -1017,7 +1037,9 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       // has another CTA given up?  Asked before the stores and looked at after them: the answer takes a trip to L2
       const int gave_up = *((volatile int*)err_flag);
       float* Ct = C + (int64_t)z * ts.split_stride;
-      epilogue_store_warp(sum, lane, m0 + sub * 32, n0 + half * 128, M, N, Ct, ldc, vecC, epi);
+      const int c0 = n0 + half * hw;
+      epilogue_store_warp(sum, lane, m0 + sub * 32, c0, M, min(N, c0 + hw), Ct, ldc, vecC, epi, PMODE == 3 ? bias_slot : nullptr);
+      __syncwarp();
       if (gave_up != 0) { ok = false; break; }
 #ifdef PRAD_GEMM_STALL_PROBE
       e_store += clock64() - st0_;
@@ -1591,11 +1613,48 @@ splitk_combine_kernel(const float* __restrict__ part, int splits, int64_t mn, in
   }
 }
 
+// The same for many slices of a small output (96 x 96 over k = 200704 is 143 slices): eight warps share the slices of 128
+// elements -- warp w adds slices w, w + 8, ... in order -- and the first adds the eight sums.
+__global__ void __launch_bounds__(256)
+splitk_combine_many_kernel(const float* __restrict__ part, int splits, int64_t mn, int N, float* __restrict__ C, int64_t ldc, float alpha, float beta) {
+  __shared__ float4 sm[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i = ((int64_t)blockIdx.x * 32 + lane) * 4;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [&](const float4& t) { acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w; };
+  if (i < mn) {
+    constexpr int U = 8;
+    for (int s0 = w; s0 < splits; s0 += 8 * U) {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        v[u] = s0 + 8 * u < splits ? *reinterpret_cast<const float4*>(part + (int64_t)(s0 + 8 * u) * mn + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < U; ++u) add(v[u]);
+    }
+  }
+  sm[w][lane] = acc;
+  __syncthreads();
+  if (w != 0 || i >= mn) return;
+  acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) add(sm[k][lane]);
+  float* c = C + (i / N) * ldc + (i % N);
+  float4 o = make_float4(alpha * acc.x, alpha * acc.y, alpha * acc.z, alpha * acc.w);
+  if (beta != 0.f) {
+    const float4 old = *reinterpret_cast<const float4*>(c);
+    o.x = fmaf(beta, old.x, o.x); o.y = fmaf(beta, old.y, o.y); o.z = fmaf(beta, old.z, o.z); o.w = fmaf(beta, old.w, o.w);
+  }
+  *reinterpret_cast<float4*>(c) = o;
+}
+
 // ---- host side --------------------------------------------------------------------------
 static void launch_splitk_combine(prad_ctx* ctx, const float* part, int splits, int64_t mn, int M, int N, float* C,
                                   int64_t ldc, float alpha, float beta) {
   const bool vec = N % 4 == 0 && ldc % 4 == 0 && (((uintptr_t)C | (uintptr_t)part) & 15) == 0;
-  if (vec) {
+  if (vec && splits >= 16 && mn <= (1 << 18)) {
+    splitk_combine_many_kernel<<<(unsigned)ceil_div(mn, 128), 256, 0, ctx->stream>>>(part, splits, mn, N, C, ldc, alpha, beta);
+  } else if (vec) {
     const int cg = stream_grid(ctx, mn / 4, 256, 8);
     splitk_combine_kernel<4><<<cg, 256, 0, ctx->stream>>>(part, splits, mn, M, N, C, ldc, alpha, beta);
   } else {
@@ -1790,9 +1849,10 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
                "gemm (tensor core): packed operands disagree in k (%lld, %lld) or block length (%d, %d)",
                (long long)a.kp, (long long)b.kp, a.chunk, b.chunk);
   CUtensorMap ma, mb;
+  const int bn = p1::tile_width(N);
   // interleaved pieces: a row is 2 kp halves, a k-group of 32 is one 128-byte box row (h0 | h1)
   const bool ok = make_map(&ma, a.h, M, (int)(2 * kp), a.pitch, BM, 2 * p1::BK, 2, true) &&
-                  make_map(&mb, b.h, N, (int)(2 * kp), b.pitch, BN, 2 * p1::BK, 2, true);
+                  make_map(&mb, b.h, N, (int)(2 * kp), b.pitch, bn, 2 * p1::BK, 2, true);
   PRAD_REQUIRE(ok, PRAD_ERR_CUDA, "gemm (tensor core): cuTensorMapEncodeTiled failed (M %d N %d K %lld)", M, N, (long long)kp);
   static std::atomic<uint64_t> p_done{0};
   const cudaError_t p_err = reserve_smem(gemm_persistent_kernel<3>, p1::SMEM_BYTES, ctx->device, p_done);
@@ -1807,7 +1867,8 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
   // which long k loops and wide outputs feel, while its tile transitions cost more -- 200704 x 96 outputs over k = 96 ..
   // 384 take 52 .. 90 us on single CTAs and 61 .. 105 us on pairs; 65536 x 4096 over k = 512 takes 733 and 721 us,
   // 65536 x 1024 over k = 512 about 200 us either way)
-  const bool pair = ctx->tc_pair != 0 && M > BM && (kp >= 1024 || N >= 1024 || ctx->tc_pair == 2) &&
+  // (nor where a pair's 256 columns would be a quarter empty: the single CTAs' tiles are as narrow as the matrix)
+  const bool pair = ctx->tc_pair != 0 && M > BM && (((kp >= 1024 || N >= 1024) && (int64_t)tiles_n * BN * 3 <= (int64_t)N * 4) || ctx->tc_pair == 2) &&
                     ctx->sm_count - ctx->tc_reserve_sms >= 2;
   CUtensorMap mb_half;
   if (pair) {
@@ -1826,7 +1887,7 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
       return (double)ctas / (double)(ceil_div(ctas, ctx->sm_count) * ctx->sm_count);
     };
     double best = eff(1) * 1.08;   // a split must pay for its extra pass
-    for (int sp = 2; sp <= 64; ++sp)
+    for (int sp = 2; sp <= 160; ++sp)
       if (kp / sp >= 1024 && eff(sp) > best * 1.02) { best = eff(sp); splits = sp; }
   }
   const bool vecC = (((uintptr_t)C & 15) == 0) && (ldc % 4 == 0);
@@ -1844,7 +1905,7 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
       gemm_pair_kernel<<<ctas, THREADS, p2::SMEM_BYTES, ctx->stream>>>(ma, mb_half, M, N, out, ldo, vec_out, ep, ctx->tc_err, ts);
       return;
     }
-    TileSched ts{tiles_m, tiles_n, nsplit, kbps, total_kb, chunk_kb, panel_n, stride, ctx->tc_prefetch};
+    TileSched ts{tiles_m, tiles_n, nsplit, kbps, total_kb, chunk_kb, panel_n, stride, ctx->tc_prefetch, bn};
     const int64_t total = tiles * nsplit;
     const unsigned ctas = (unsigned)(total < sms ? total : sms);
     gemm_persistent_kernel<3><<<ctas, THREADS, p1::SMEM_BYTES, ctx->stream>>>(ma, ma, ma, mb, mb, mb, M, N, out, ldo, vec_out,
