@@ -186,6 +186,15 @@ __device__ __forceinline__ void tmem_ld_wait8(uint32_t (&v)[8]) {
                :: "memory");
 }
 
+__device__ __forceinline__ void tmem_ld_wait32(uint32_t (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+                 "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
+                 "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+               :: "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major tile stored as rows of SW bytes (SW = 128, 64
 // or 32) with the SW-byte swizzle, i.e. what TMA writes with CU_TENSOR_MAP_SWIZZLE_{SW}B:
 // 8-row groups are 8*SW bytes apart (stride byte offset), the leading byte offset is unused
@@ -660,6 +669,71 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
   }
 }
 
+// The epilogue of a tile whose k is a single block: nothing to sum up in registers, so 32 columns at a time go from the
+// accumulator through the scales to memory in a rolled loop of some three hundred instructions.  The unrolled code above for 128
+// columns is fetched anew for every tile and the warps wait for it: 200704 x 384 outputs over k = 96 took 4.6 us per tile.
+// Whole rows of the tile exist, ncols is a multiple of 16 (or there are none); one block's scales start at block `blk`.
+__device__ __forceinline__ bool epilogue_one_block(int lane, int row0, int col0, int ncols, float* __restrict__ C, int64_t ldc, int64_t blk,
+                                                   const Epi& epi, float4* sb_slot, uint32_t taddr, uint32_t full, uint32_t parity,
+                                                   uint32_t empty, int* err_flag) {
+  const float sa = __ldg(epi.blk_a + blk * epi.blk_lda + row0 + lane);
+  float4* const bias_slot = sb_slot + EPI_WARPS * 32;
+  if (4 * lane < ncols) {
+    sb_slot[lane] = __ldg(reinterpret_cast<const float4*>(epi.blk_b + blk * epi.blk_ldb + col0) + lane);
+    if (epi.bias) {
+      const float* b = epi.bias + col0 + 4 * lane;
+      bias_slot[lane] = make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3));
+    }
+  }
+  __syncwarp();
+  float* rp = C + (int64_t)(row0 + 4 * (lane >> 2)) * ldc + col0 + 4 * (lane & 3);
+  const int gave_up = *((volatile int*)err_flag);
+  if (!__all_sync(0xffffffffu, mbar_wait(full, parity, err_flag, 3))) return false;
+  tc_fence_after();
+  uint32_t v[32];
+  const float2 sa2 = make_float2(sa, sa), zero = make_float2(0.f, 0.f);
+  if (ncols > 0) tmem_ld32(taddr, v);
+#pragma unroll 1
+  for (int c = 0; c < ncols; c += 32) {
+    float x[32];
+    tmem_ld_wait32(v);
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+      const float4 t = sb_slot[(c + j) >> 2];
+      const float2 p01 = __fmul2_rn(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), sa2);
+      const float2 p23 = __fmul2_rn(make_float2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), sa2);
+      const float2 r01 = __ffma2_rn(p01, make_float2(t.x, t.y), zero), r23 = __ffma2_rn(p23, make_float2(t.z, t.w), zero);
+      x[j] = r01.x; x[j + 1] = r01.y; x[j + 2] = r23.x; x[j + 3] = r23.y;
+    }
+    if (c + 32 < ncols) tmem_ld32(taddr + (uint32_t)(c + 32), v);
+    if (epi.alpha != 1.f) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = epi.alpha * x[j];
+    }
+    if (epi.bias) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        const float4 b = bias_slot[(c + j) >> 2];
+        x[j] += b.x; x[j + 1] += b.y; x[j + 2] += b.z; x[j + 3] += b.w;
+      }
+    }
+    quad_transpose(x, lane);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (c + 16 * h >= ncols) break;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int j = 4 * (s + 4 * h);
+        __stcs(reinterpret_cast<float4*>(rp + s * ldc + c + 16 * h), make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]));
+      }
+    }
+  }
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive_relaxed(empty);
+  return gave_up == 0;
+}
+
 // ---- persistent variant of MODE 1 (TF32 product + two BF16 corrections) -----------------
 // Same arithmetic and tile as gemm_tf32x3_kernel<Cfg<32,2,1>>, organised differently:
 //   * one CTA per SM walks output tiles (n-tile fastest, then m-tile, then k-slice): its
@@ -937,6 +1011,15 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       int m0, n0, z, kb0, num_kb;
       tile_of(t, m0, n0, z, kb0, num_kb);
       const int num_chunks = (num_kb + ts.chunk_kb - 1) / ts.chunk_kb;
+      if (PMODE == 3 && num_chunks == 1 && vecC && epi.beta == 0.f && m0 + BM <= M && ((N - n0) & 15) == 0) {
+        ok = epilogue_one_block(lane, m0 + sub * 32, n0 + half * hw, min(N - n0 - half * hw, hw), C + (int64_t)z * ts.split_stride, ldc,
+                                (int64_t)(kb0 / ts.chunk_kb), epi,
+                                reinterpret_cast<float4*>(generic_base + UNITS * UNIT_BYTES + 256) + (warp - 2) * 32,
+                                tmem_base + ((uint32_t)(sub * 32) << 16) + (gc & 1) * (uint32_t)BN + (uint32_t)(half * hw),
+                                acc_full(gc & 1), (gc >> 1) & 1, acc_empty(gc & 1), err_flag);
+        ++gc;
+        continue;
+      }
       float sum[4][32];
 #pragma unroll
       for (int g = 0; g < 4; ++g)

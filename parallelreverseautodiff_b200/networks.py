@@ -763,29 +763,32 @@ class SwinBlock:
         self.qkv = e.gemm_packed(ln1, rows, self._weight("Wqkv", True), cols, self._buf("qkv", (T, 3 * d)), bias=p["bqkv"])
         self._attention_forward(T)
         attn = self._packed("attn", T, d).pack(self.attn)
-        proj = e.gemm_packed(attn, rows, self._weight("Wproj", True), cols, self._buf("proj", (T, d)), bias=p["bproj"])
+        proj = e.gemm_packed(attn, rows, self._weight("Wproj", True), cols, self._buf("branch", (T, d)), bias=p["bproj"])
         self.r1 = self._buf("r1", (T, d))
-        ln2 = self._packed("ln2", T, d).layernorm(x, self.mu2, self.sd2, residual=proj, sum_out=self.r1)
+        ln2 = self._packed("ln2", T, d).column_sums(None).layernorm(x, self.mu2, self.sd2, residual=proj, sum_out=self.r1)
         self.z1 = e.gemm_packed(ln2, rows, self._weight("W1", True), cols, self._buf("z1", (T, h)), bias=p["b1"])
-        a1 = self._packed("a1", T, h).act_forward(E.ACT_GELU, self.z1)
-        m2 = e.gemm_packed(a1, rows, self._weight("W2", True), cols, self._buf("m2", (T, d)), bias=p["b2"])
+        a1 = self._packed("a1", T, h).column_sums(None).act_forward(E.ACT_GELU, self.z1)
+        m2 = e.gemm_packed(a1, rows, self._weight("W2", True), cols, self._buf("branch", (T, d)), bias=p["b2"])
         self.out = e.add_forward(self.r1, m2, out=new(T, d))
         return self.out
 
     def _backward_packed(self, d_out):
-        """The gradients likewise, with the bias gradients (column sums) out of the same passes."""
+        """The gradients likewise, with the bias gradients (column sums) out of the same passes.  A gradient takes the place of
+        the activation of its shape that has just been read for the last time."""
         e, d, h, g = self.eng, self.dim, self.hidden, self.g
         T = d_out.shape[0]
         rows, cols, B_ = E.PACK_ROWS, E.PACK_COLS, self._buf
         op = lambda name, w: self._packed(name, T, w)  # noqa: E731
-        narrow, wide, qkv = op("d narrow", d), op("d wide", h), op("d qkv", 3 * d)
+        narrow, qkv = op("d narrow", d), op("d qkv", 3 * d)
         narrow.column_sums(g["b2"]).pack(d_out)                       # out = r1 + m2 : both receive d_out
         e.gemm_packed(op("a1", h), cols, narrow, cols, g["W2"])
         d_a1 = e.gemm_packed(narrow, rows, self._weight("W2", False), rows, B_("d_a1", (T, h)))
+        wide = op("a1", h)
         wide.column_sums(g["b1"]).act_backward(E.ACT_GELU, self.z1, d_a1)
         e.gemm_packed(op("ln2", d), cols, wide, cols, g["W1"])
-        d_ln2 = e.gemm_packed(wide, rows, self._weight("W1", False), rows, B_("d_ln2", (T, d)))
+        d_ln2 = e.gemm_packed(wide, rows, self._weight("W1", False), rows, B_("branch", (T, d)))
         d_r1 = B_("d_r1", (T, d))                                     # fan-in at r1: residual + LN2 branch
+        narrow = op("ln2", d)
         narrow.column_sums(g["bproj"]).layernorm_backward(self.r1, self.mu2, self.sd2, d_ln2, d_out, d_r1)
         e.gemm_packed(op("attn", d), cols, narrow, cols, g["Wproj"])
         self.d_attn = e.gemm_packed(narrow, rows, self._weight("Wproj", False), rows, B_("d_attn", (T, d)))
@@ -793,7 +796,7 @@ class SwinBlock:
         self._attention_backward(self.d_attn, self.d_qkv)
         qkv.column_sums(g["bqkv"]).pack(self.d_qkv)
         e.gemm_packed(op("ln1", d), cols, qkv, cols, g["Wqkv"])
-        d_ln1 = e.gemm_packed(qkv, rows, self._weight("Wqkv", False), rows, B_("d_ln1", (T, d)))
+        d_ln1 = e.gemm_packed(qkv, rows, self._weight("Wqkv", False), rows, B_("branch", (T, d)))
         self.d_x = e.layernorm_backward_add(self.x, self.mu1, self.sd1, d_ln1, d_r1, out=B_("d_x", (T, d)))
         return self.d_x
 
