@@ -757,9 +757,12 @@ namespace p1 {
 constexpr int BK = 32;
 constexpr int UNITS = 4;
 constexpr int UNIT_BYTES = 48 * 1024;
+constexpr int RING_BYTES = UNITS * UNIT_BYTES;
+constexpr int MAX_UNITS = 8;          // PMODE 3: a narrow tile's units are smaller, and more of them are in flight
 constexpr int CHUNK_KB = CHUNK_K / BK;
 constexpr int SCALE_BYTES = EPI_WARPS * 128 * 4;   // PMODE 3: each epilogue warp's copy of its 128 column scales of a block
-constexpr int SMEM_BYTES = UNITS * UNIT_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + 2 * SCALE_BYTES /*scales, bias*/;
+constexpr int SMEM_BYTES = RING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + 2 * SCALE_BYTES /*scales, bias*/;
+static_assert(8 * (2 * MAX_UNITS + 5 + 2 * 4) + 4 * 4 <= 256, "barriers and the tile queue");
 static_assert(SMEM_BYTES <= 227 * 1024, "unit ring does not fit in shared memory");
 // PMODE 3: columns of an output tile.  256, or where a matrix of that many tiles leaves a good part of them empty, the width
 // that shares its columns evenly (a multiple of 32: half a tile per epilogue warp, 16 columns per store instruction): with
@@ -787,20 +790,22 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
   using namespace p1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bars = base + UNITS * UNIT_BYTES;
+  const uint32_t bars = base + RING_BYTES;
+  const uint32_t unit_bytes = PMODE == 3 ? 16 * 1024 + ts.bn * 128 : UNIT_BYTES;
+  const uint32_t units = PMODE == 3 ? min((uint32_t)MAX_UNITS, RING_BYTES / unit_bytes) : (uint32_t)UNITS;
   auto full_bar = [&](uint32_t s) { return bars + 8u * s; };
-  auto empty_bar = [&](uint32_t s) { return bars + 8u * (UNITS + s); };
-  auto acc_full = [&](uint32_t b) { return bars + 8u * (2 * UNITS + b); };
-  auto acc_empty = [&](uint32_t b) { return bars + 8u * (2 * UNITS + 2 + b); };
-  const uint32_t tmem_slot = bars + 8u * (2 * UNITS + 4);
+  auto empty_bar = [&](uint32_t s) { return bars + 8u * (MAX_UNITS + s); };
+  auto acc_full = [&](uint32_t b) { return bars + 8u * (2 * MAX_UNITS + b); };
+  auto acc_empty = [&](uint32_t b) { return bars + 8u * (2 * MAX_UNITS + 2 + b); };
+  const uint32_t tmem_slot = bars + 8u * (2 * MAX_UNITS + 4);
   constexpr int TQ = 4;                       // depth of the tile-index queue
-  auto tile_full = [&](uint32_t i) { return bars + 8u * (2 * UNITS + 5 + i); };
-  auto tile_empty = [&](uint32_t i) { return bars + 8u * (2 * UNITS + 5 + TQ + i); };
+  auto tile_full = [&](uint32_t i) { return bars + 8u * (2 * MAX_UNITS + 5 + i); };
+  auto tile_empty = [&](uint32_t i) { return bars + 8u * (2 * MAX_UNITS + 5 + TQ + i); };
   uint8_t* generic_base = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr =
-      reinterpret_cast<volatile uint32_t*>(generic_base + UNITS * UNIT_BYTES + 8 * (2 * UNITS + 4));
+      reinterpret_cast<volatile uint32_t*>(generic_base + RING_BYTES + 8 * (2 * MAX_UNITS + 4));
   volatile int* tile_q =
-      reinterpret_cast<volatile int*>(generic_base + UNITS * UNIT_BYTES + 8 * (2 * UNITS + 5 + 2 * TQ));
+      reinterpret_cast<volatile int*>(generic_base + RING_BYTES + 8 * (2 * MAX_UNITS + 5 + 2 * TQ));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total_tiles = ts.tiles_m * ts.tiles_n * ts.splits;
@@ -813,7 +818,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
   if (s_abort != 0) return;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < UNITS; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    for (int s = 0; s < MAX_UNITS; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), EPI_WARPS); }
     for (int i = 0; i < TQ; ++i) { mbar_init(tile_full(i), 1); mbar_init(tile_empty(i), 1 + EPI_WARPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -859,7 +864,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      uint32_t g = 0;    // units issued so far, over all tiles of this CTA
+      uint32_t slot = 0, round = 0;    // unit to be filled next and how often the ring has been round, over all tiles of this CTA
       uint32_t qi = 0;   // tile indices published so far
       bool ok = true;
       int t = blockIdx.x;
@@ -875,11 +880,10 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
         for (int kb = 0; kb < num_kb && ok; ++kb) {
           const int x = (kb0 + kb) * BK;
 #pragma unroll
-          for (int half = 0; half < (PMODE == 1 ? 2 : 1); ++half, ++g) {
-            const uint32_t slot = g & (UNITS - 1), round = g / UNITS;
+          for (int half = 0; half < (PMODE == 1 ? 2 : 1); ++half) {
             if (round > 0 && !mbar_wait(empty_bar(slot), (round - 1) & 1, err_flag, 1)) { ok = false; break; }
-            const uint32_t st = base + slot * UNIT_BYTES;
-            mbar_expect_tx(full_bar(slot), PMODE == 3 ? 16 * 1024 + ts.bn * 128 : UNIT_BYTES);
+            const uint32_t st = base + slot * unit_bytes;
+            mbar_expect_tx(full_bar(slot), unit_bytes);
             if (PMODE == 3) {  // one unit: A rows (h0 | h1) 16 KB, B rows (h0 | h1) 128 bytes each; x counts halves
               tma_load_2d(st, &map_a_xb, full_bar(slot), 2 * x, m0);
               tma_load_2d(st + 16 * 1024, &map_b_xb, full_bar(slot), 2 * x, n0);
@@ -894,6 +898,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
               tma_load_2d(st, &map_a_hi, full_bar(slot), x, m0);
               tma_load_2d(st + 16 * 1024, &map_b_hi, full_bar(slot), x, n0);
             }
+            if (++slot == units) { slot = 0; ++round; }
           }
         }
         t = (int)gridDim.x + atomicAdd(tile_counter, 1);
@@ -903,7 +908,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       constexpr uint32_t idesc = idesc_tf32(), idesc_h = idesc_bf16();
-      uint32_t g = 0, gc = 0, qi = 0;   // units consumed, chunks started, tiles taken
+      uint32_t slot = 0, phase = 0, gc = 0, qi = 0;   // unit to be consumed next and its parity, chunks started, tiles taken
+      auto next_unit = [&] { if (++slot == units) { slot = 0; phase ^= 1; } };
       bool ok = true;
       // -DPRAD_GEMM_STALL_PROBE: cycle counts of what this thread and one epilogue warp wait for, printed by
       // CTA 0 at the end of every launch (a diagnostic build; the numbers quoted in the design notes come from it)
@@ -933,11 +939,10 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
           for (int kb = ch * ts.chunk_kb; kb < kb_end && ok; ++kb) {
             if (PMODE == 3) {   // one unit: A (h0 | h1 per row), B likewise; three FP16 products, smallest first
               const uint32_t idesc_q = idesc_fp16(ts.bn);
-              const uint32_t slot = g & (UNITS - 1);
-              PROBE_WAIT(w_full, ok = mbar_wait(full_bar(slot), (g / UNITS) & 1, err_flag, 2));
+              PROBE_WAIT(w_full, ok = mbar_wait(full_bar(slot), phase, err_flag, 2));
               if (!ok) break;
               tc_fence_after();
-              const uint32_t st = base + slot * UNIT_BYTES;
+              const uint32_t st = base + slot * unit_bytes;
               // rows of 128 bytes (128-byte swizzle): h0 at byte 0, h1 at byte 64, 16-k slices 32 bytes apart
               const uint64_t a_0 = kmajor_desc<128>(st), a_1 = a_0 + 4;
               const uint64_t b_0 = kmajor_desc<128>(st + 16 * 1024), b_1 = b_0 + 4;
@@ -949,15 +954,14 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
                 umma_f16(d_tmem, a_0 + adv, b_0 + adv, idesc_q, 1);
               }
               umma_commit(empty_bar(slot));
-              ++g;
+              next_unit();
               continue;
             }
             {   // unit H: the two BF16 correction products, two 16-wide k-slices
-              const uint32_t slot = g & (UNITS - 1);
-              ok = mbar_wait(full_bar(slot), (g / UNITS) & 1, err_flag, 2);
+              ok = mbar_wait(full_bar(slot), phase, err_flag, 2);
               if (!ok) break;
               tc_fence_after();
-              const uint32_t st = base + slot * UNIT_BYTES;
+              const uint32_t st = base + slot * unit_bytes;
               const uint64_t a_hb = kmajor_desc<64>(st), a_lb = kmajor_desc<64>(st + 8 * 1024);
               const uint64_t b_hb = kmajor_desc<64>(st + 16 * 1024), b_lb = kmajor_desc<64>(st + 32 * 1024);
 #pragma unroll
@@ -967,14 +971,13 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
                 umma_f16(d_tmem, a_hb + adv, b_lb + adv, idesc_h, 1);
               }
               umma_commit(empty_bar(slot));
-              ++g;
+              next_unit();
             }
             {   // unit F: the TF32 product, four 8-wide k-slices
-              const uint32_t slot = g & (UNITS - 1);
-              ok = mbar_wait(full_bar(slot), (g / UNITS) & 1, err_flag, 2);
+              ok = mbar_wait(full_bar(slot), phase, err_flag, 2);
               if (!ok) break;
               tc_fence_after();
-              const uint32_t st = base + slot * UNIT_BYTES;
+              const uint32_t st = base + slot * unit_bytes;
               const uint64_t a_hi = kmajor_desc<128>(st), b_hi = kmajor_desc<128>(st + 16 * 1024);
 #pragma unroll
               for (int k = 0; k < BK / UMMA_K; ++k) {
@@ -982,7 +985,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
                 umma_tf32(d_tmem, a_hi + adv, b_hi + adv, idesc, 1);
               }
               umma_commit(empty_bar(slot));
-              ++g;
+              next_unit();
             }
           }
           umma_commit(acc_full(buf));    // chunk complete (arrives even after a give-up)
@@ -990,8 +993,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       }
 #ifdef PRAD_GEMM_STALL_PROBE
       if (blockIdx.x == 0)
-        printf("mma issuer: total %lld cycles, waited for operands %lld, for the accumulator %lld, for tiles %lld (units %u)\n",
-               clock64() - t_begin, w_full, w_acc, w_tile, g);
+        printf("mma issuer: total %lld cycles, waited for operands %lld, for the accumulator %lld, for tiles %lld\n",
+               clock64() - t_begin, w_full, w_acc, w_tile);
 #endif
     }
   } else {
@@ -1014,7 +1017,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       if (PMODE == 3 && num_chunks == 1 && vecC && epi.beta == 0.f && m0 + BM <= M && ((N - n0) & 15) == 0) {
         ok = epilogue_one_block(lane, m0 + sub * 32, n0 + half * hw, min(N - n0 - half * hw, hw), C + (int64_t)z * ts.split_stride, ldc,
                                 (int64_t)(kb0 / ts.chunk_kb), epi,
-                                reinterpret_cast<float4*>(generic_base + UNITS * UNIT_BYTES + 256) + (warp - 2) * 32,
+                                reinterpret_cast<float4*>(generic_base + RING_BYTES + 256) + (warp - 2) * 32,
                                 tmem_base + ((uint32_t)(sub * 32) << 16) + (gc & 1) * (uint32_t)BN + (uint32_t)(half * hw),
                                 acc_full(gc & 1), (gc >> 1) & 1, acc_empty(gc & 1), err_flag);
         ++gc;
@@ -1033,7 +1036,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       // put theirs into the warp's slot of shared memory, from where every lane reads all of them (broadcast)
       float sa_next = 0.f;
       float4 sb_next = make_float4(0.f, 0.f, 0.f, 0.f);
-      float4* const sb_slot = reinterpret_cast<float4*>(generic_base + UNITS * UNIT_BYTES + 256) + (warp - 2) * 32;
+      float4* const sb_slot = reinterpret_cast<float4*>(generic_base + RING_BYTES + 256) + (warp - 2) * 32;
       auto fetch_scales = [&](int ch) {
         sa_next = __ldg(epi.blk_a + (int64_t)(chunk0 + ch) * epi.blk_lda + row_blk);
         sb_next = __ldg(reinterpret_cast<const float4*>(epi.blk_b + (int64_t)(chunk0 + ch) * epi.blk_ldb + n0 + half * hw) + lane);

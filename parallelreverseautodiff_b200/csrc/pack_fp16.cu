@@ -149,32 +149,49 @@ __device__ __forceinline__ float apply_op(const PackSource& s, float a, float d,
 //
 // Column sums (a bias gradient) cost the second pass sixteen additions per lane and quad: the values are in shared memory anyway,
 // and a pass of their own over a 200704 x 384 gradient takes 72 us.
-__device__ __forceinline__ double lane_sum(double v) {
+// The sums over the lanes of U values at once: with two, the halves of the warp take one each after the first exchange, which is
+// seven exchanges instead of ten, and two rows' chains run side by side (a LayerNorm pass waits for little else).
+template <int U> __device__ __forceinline__ void lane_sums(double (&v)[U]) {
+  if constexpr (U == 1) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+    for (int o = 16; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  } else {
+    const bool high = (threadIdx.x & 16) != 0;
+    double t = (high ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, high ? v[0] : v[1], 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    v[0] = __shfl_sync(0xffffffffu, t, 0);
+    v[1] = __shfl_sync(0xffffffffu, t, 16);
+  }
 }
-// LayerNormalizationOperation.cs:56-85 on the row whose four values at column c each lane holds
-__device__ __forceinline__ void layernorm_row(float (&v)[4], bool inside, int C, float* mean, float* sigma, bool write) {
-  double s = 0.0;
+// LayerNormalizationOperation.cs:56-85 on U rows whose four values at a column each lane holds
+template <int U>
+__device__ __forceinline__ void layernorm_rows(float (&v)[U][4], bool inside, int C, float (&mu)[U], float (&sd)[U]) {
+  double s[U], t[U];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) s += (double)v[q];
-  s = lane_sum(inside ? s : 0.0);
-  const float mu = (float)(s / (double)C);
-  double t = 0.0;
+  for (int u = 0; u < U; ++u) s[u] = inside ? ((double)v[u][0] + (double)v[u][1]) + ((double)v[u][2] + (double)v[u][3]) : 0.0;
+  lane_sums<U>(s);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) { v[q] = sub_rn(v[q], mu); t += (double)mul_rn(v[q], v[q]); }
-  t = lane_sum(inside ? t : 0.0);
-  const float sd = sqrt_rn(div_rn((float)t, (float)C));
-  if (write) { *mean = mu; *sigma = sd; }
-  const float den = add_rn(sd, 1e-9f);
+  for (int u = 0; u < U; ++u) {
+    mu[u] = (float)(s[u] / (double)C);
+    t[u] = 0.0;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) v[q] = div_rn(v[q], den);
+    for (int q = 0; q < 4; ++q) { v[u][q] = sub_rn(v[u][q], mu[u]); t[u] += (double)mul_rn(v[u][q], v[u][q]); }
+    if (!inside) t[u] = 0.0;
+  }
+  lane_sums<U>(t);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    sd[u] = sqrt_rn(div_rn((float)t[u], (float)C));
+    const float den = add_rn(sd[u], 1e-9f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[u][q] = div_rn(v[u][q], den);
+  }
 }
 template <int OP, bool ROWS, bool COLS, int NT, bool EDGE>
 __global__ void __launch_bounds__(NT, NT == 512 ? 2 : (OP == 0 ? 5 : 3))
 pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_r0, int tile_c0, int R, int C) {
-  constexpr int T = 128, U = OP == 13 || OP == 14 ? 1 : 2, NW = NT / 32, NB = T / NW / U;      // NW warps, each takes every NW-th tile row
+  constexpr int T = 128, U = OP == 14 ? 1 : 2, NW = NT / 32, NB = T / NW / U;      // NW warps, each takes every NW-th tile row
   constexpr bool HAS_DY = OP >= 4 && OP != 9 && OP != 12, HAS_TG = OP == 7 || OP == 8 || OP == 11 || OP == 14;
   extern __shared__ float stash[];       // [T][T] when COLS
   __shared__ unsigned colmax[T];
@@ -206,20 +223,34 @@ pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_r0, int 
   for (int b = 0; b < NB; ++b) {
     const int cur = b & 1;
     if (b + 1 < NB) load(cur ^ 1, b + 1);
+    float v_of[U][4];
+    if constexpr (OP == 12 || OP == 13) {
+      float mu[U], sd[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t r = r0 + warp + NW * (b * U + u);
+        float (&v)[4] = v_of[u];
+        v[0] = a[cur][u].x; v[1] = a[cur][u].y; v[2] = a[cur][u].z; v[3] = a[cur][u].w;
+        if constexpr (OP == 13) {
+          v[0] = add_rn(v[0], d[cur][u].x); v[1] = add_rn(v[1], d[cur][u].y);
+          v[2] = add_rn(v[2], d[cur][u].z); v[3] = add_rn(v[3], d[cur][u].w);
+          if (inside && (!EDGE || r < R)) __stcs(reinterpret_cast<float4*>(src.out + r * src.ld + c), make_float4(v[0], v[1], v[2], v[3]));
+        }
+      }
+      layernorm_rows<U>(v_of, inside, C, mu, sd);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t r = r0 + warp + NW * (b * U + u);
+        if (lane == 0 && (!EDGE || r < R)) { src.mean[r] = mu[u]; src.sigma[r] = sd[u]; }
+      }
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int tr = warp + NW * (b * U + u);
       const int64_t r = r0 + tr;
       const bool row = !EDGE || r < R;
-      float v[4];
+      float (&v)[4] = v_of[u];
       if constexpr (OP == 12 || OP == 13) {
-        v[0] = a[cur][u].x; v[1] = a[cur][u].y; v[2] = a[cur][u].z; v[3] = a[cur][u].w;
-        if constexpr (OP == 13) {
-          v[0] = add_rn(v[0], d[cur][u].x); v[1] = add_rn(v[1], d[cur][u].y);
-          v[2] = add_rn(v[2], d[cur][u].z); v[3] = add_rn(v[3], d[cur][u].w);
-          if (inside && row) __stcs(reinterpret_cast<float4*>(src.out + r * src.ld + c), make_float4(v[0], v[1], v[2], v[3]));
-        }
-        layernorm_row(v, inside, C, src.mean + r, src.sigma + r, lane == 0 && row);
       } else if constexpr (OP == 14) {
         // LayerNormalizationOperation.cs:88-112, then the sum of the two paths
         const float mu = row ? src.mean[r] : 0.f, se = add_rn(row ? src.sigma[r] : 1.f, 1e-9f);
@@ -310,15 +341,16 @@ pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_r0, int 
 __global__ void __launch_bounds__(1024)
 column_sum_kernel(const double* __restrict__ part, float* __restrict__ out, int rows, int C) {
   __shared__ double sm[32][33];
+  constexpr int U = 12;                 // loads in flight per thread: 1568 partial rows are four trips
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   double acc = 0.0;
   if (c < C)
-    for (int r0 = w; r0 < rows; r0 += 128) {
-      double v[4];
+    for (int r0 = w; r0 < rows; r0 += 32 * U) {
+      double v[U];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = r0 + 32 * u < rows ? part[(int64_t)(r0 + 32 * u) * C + c] : 0.0;
+      for (int u = 0; u < U; ++u) v[u] = r0 + 32 * u < rows ? part[(int64_t)(r0 + 32 * u) * C + c] : 0.0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) acc += v[u];
+      for (int u = 0; u < U; ++u) acc += v[u];
     }
   sm[w][lane] = acc;
   __syncthreads();
