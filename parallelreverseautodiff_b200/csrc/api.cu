@@ -122,6 +122,10 @@ prad_status prad_shutdown(prad_ctx* ctx) {
   for (void* r : ctx->retired) cudaFree(r);
   if (ctx->stage) cudaFree(ctx->stage);
   if (ctx->parts) cudaFree(ctx->parts);
+  if (ctx->flag_read) cudaEventDestroy(ctx->flag_read);
+  if (ctx->branch_stream) cudaStreamDestroy(ctx->branch_stream);
+  for (cudaEvent_t e : ctx->branch_event)
+    if (e) cudaEventDestroy(e);
   if (ctx->host_ws) cudaFreeHost(ctx->host_ws);
   if (ctx->copy_stream) { cudaStreamSynchronize(ctx->copy_stream); cudaStreamDestroy(ctx->copy_stream); }
   if (ctx->copy_done) cudaEventDestroy(ctx->copy_done);
@@ -330,7 +334,12 @@ prad_status prad_download(prad_ctx* ctx, void* dst_host, const void* src, size_t
   PRAD_CHECK_CTX(ctx);
   PRAD_NOT_CAPTURING(ctx, "prad_download");
   PRAD_REQUIRE((dst_host && src) || bytes == 0, PRAD_ERR_INVALID, "prad_download: null pointer");
-  if (bytes) {
+  if (bytes > 0 && bytes <= 32) {         // a loss: by way of page-locked memory, which the driver need not stage
+    void* pinned = (char*)ctx->host_flag + 32;
+    PRAD_CUDA(cudaMemcpyAsync(pinned, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
+    memcpy(dst_host, pinned, bytes);
+  } else if (bytes) {
     PRAD_CUDA(cudaMemcpyAsync(dst_host, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
   }

@@ -50,6 +50,9 @@ struct prad_ctx {
   prad::DevicePool* pool = nullptr;
   size_t total_mem = 0;               // device memory in bytes
   int* host_flag = nullptr;   // page-locked int that kernels write and the host reads after a wait
+  cudaStream_t branch_stream = nullptr;   // second branch of a recording
+  cudaEvent_t branch_event[2] = {nullptr, nullptr};
+  cudaEvent_t flag_read = nullptr;    // recorded behind the kernel that writes host_flag where others follow it
   // give-up flag of the tensor-core GEMMs (device int, sticky until the host reads it)
   int* tc_err = nullptr;
   bool tc_pending_check = false;

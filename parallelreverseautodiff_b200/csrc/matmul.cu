@@ -136,7 +136,10 @@ static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void
   const bool tc_A = both && wants_tensor_cores(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA);
   const bool tc_B = both && wants_tensor_cores(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0,
                                                0, 0, e_dB);
-  if (both && !tc_A && !tc_B)
+  // Neither on the tensor cores: both products in one launch, or, in a recording, as two branches that run side by side, each
+  // in the tile shape that suits it.
+  const bool branches = both && !tc_A && !tc_B && ctx->capturing;
+  if (both && !tc_A && !tc_B && !branches)
     return dt == PRAD_F32 ? gemm_simt_backward<float>(ctx, ctx->gemm_f32 != GemmF32::SimtFma, A, B, dC, dA, dB, M, K, N,
                                                       accumulate_dB != 0, dB_scale, e_dA)
                           : gemm_simt_backward<double>(ctx, ctx->gemm_f64 != GemmF64::SimtFma, A, B, dC, dA, dB, M, K, N,
@@ -145,13 +148,27 @@ static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void
   if (both && tc_A && tc_B && dt == PRAD_F64 &&
       (ceil_div(M, 64) * ceil_div(K, 64) * 2 > ctx->sm_count || N < 512) && (ceil_div(K, 64) * ceil_div(N, 64) * 2 > ctx->sm_count || M < 512))
     return gemm_f64_dmma_backward(ctx, A, B, dC, dA, dB, M, K, N, accumulate_dB != 0, dB_scale, e_dA);
+  cudaStream_t main = ctx->stream;
+  if (branches) {
+    if (!ctx->branch_stream) PRAD_CUDA(cudaStreamCreateWithFlags(&ctx->branch_stream, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : ctx->branch_event)
+      if (!e) PRAD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    PRAD_CUDA(cudaEventRecord(ctx->branch_event[0], main));
+    PRAD_CUDA(cudaStreamWaitEvent(ctx->branch_stream, ctx->branch_event[0], 0));
+  }
   if (dA) {
     s = gemm_dispatch(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA);
     if (s) return s;
   }
   if (dB) {
+    if (branches) ctx->stream = ctx->branch_stream;
     s = gemm_dispatch(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0, 0, 0, e_dB);
+    ctx->stream = main;
     if (s) return s;
+  }
+  if (branches) {
+    PRAD_CUDA(cudaEventRecord(ctx->branch_event[1], ctx->branch_stream));
+    PRAD_CUDA(cudaStreamWaitEvent(main, ctx->branch_event[1], 0));
   }
   return PRAD_OK;
 }

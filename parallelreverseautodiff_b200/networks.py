@@ -122,6 +122,7 @@ class FeedForwardNetwork:
         self.dZ = [None, None]
         self.dX = None
         self.loss_dev = eng.zeros((1, 1), dtype)
+        self._host_key = self._host_sequence = self._host_dX = None      # see _forward_loss_backward
 
     # ---------------------------------------------------------------- set-up
     def set_weights(self, weights: Sequence[np.ndarray], biases: Optional[Sequence[np.ndarray]] = None):
@@ -455,11 +456,45 @@ class FeedForwardNetwork:
         self._ensure_buffers(x_host.shape[0])
         e.upload(x_host, out=self.A[0])
         e.upload(t_host, out=self.target)
-        self.forward()
-        loss = self.loss_value()
-        self.backward(rows_total=rows_total)
+        self._forward_loss_backward(rows_total)
         self.clip_and_optimize()
-        return float(loss.numpy()[0, 0])
+        return float(self.loss_dev.numpy()[0, 0])
+
+    def _forward_loss_backward(self, rows_total) -> None:
+        """forward, loss_value and backward of the uploaded batch.  A small network's launches take the host longer than
+        the GPU, so from the second step on that would launch the same again they go as one recorded sequence (the update
+        stays a call of its own: its hyperparameters change from step to step)."""
+        def run():
+            self.forward()
+            self.loss_value()
+            self.backward(rows_total=rows_total)
+
+        if self.world > 1 or self.packed:
+            return run()
+        # everything the launches depend on: buffers, sizes, the activation slope, library options
+        mats = self.W + self.b + self.dW + self.db + self.A + self.Z + sorted(self.dZ, key=lambda m: m.ptr) + [self.target, self.probs, self.loss_dev]
+        key = (self.rows, rows_total, self.loss, self.softmax_output, tuple(self.acts), self.Parameters.LeakyReLUAlpha,
+               tuple(self.eng.options.items()), tuple(m.ptr if m is not None else 0 for m in mats))
+        if key != self._host_key:
+            self._drop_host_sequence()
+            self._host_key = key
+            return run()                     # (the library's scratch gets its size here)
+        if self._host_sequence is None:
+            self._host_sequence = self.eng.record(run)
+            self._host_dX = self.dX
+        self._host_sequence.launch()
+        self.dX = self._host_dX
+
+    def _drop_host_sequence(self) -> None:
+        seq, self._host_sequence, self._host_key = self._host_sequence, None, None
+        if seq is not None and self.eng.ctx:
+            seq.close()
+
+    def __del__(self):
+        try:
+            self._drop_host_sequence()
+        except Exception:
+            pass
 
     def train_steps_host(self, batches, rows_total=None):
         """Same as train_step_host over a sequence of (x_host, t_host) page-locked batches, with

@@ -19,3 +19,35 @@ def test_host_backward_equals_device_backward(engine, dtype, m, k, n):
     np.testing.assert_array_equal(hP, dP.numpy())
     np.testing.assert_array_equal(hA, dA.numpy())
     np.testing.assert_array_equal(hB, dB.numpy())
+
+
+def test_host_steps_repeat_and_follow_changes(engine):
+    """train_step_host replays its launches from the second equal step on: changed slopes, batch sizes, learning rates and
+    options take effect, and every step equals the separate calls bit for bit."""
+    from parallelreverseautodiff_b200.networks import FeedForwardNetwork
+    r = rng(5)
+    sizes, nets = [12, 20, 9], []
+    for _ in range(2):
+        net = FeedForwardNetwork(engine, np.float64, sizes)
+        net.set_weights([rng(1).standard_normal((12, 20)), rng(2).standard_normal((20, 9))], [np.zeros((1, 20)), np.zeros((1, 9))])
+        nets.append(net)
+    a, b = nets
+    for step in range(12):
+        rows = 7 if step in (5, 6) else 16
+        if step == 8:
+            a.Parameters.LeakyReLUAlpha = b.Parameters.LeakyReLUAlpha = 0.3
+        a.Parameters.AdamIteration = b.Parameters.AdamIteration = step + 1
+        a.Parameters.LearningRate = b.Parameters.LearningRate = 1e-3 / (step + 1)
+        x, t = r.standard_normal((rows, 12)), r.standard_normal((rows, 9))
+        la = a.train_step_host(x, t)
+        b._ensure_buffers(rows)
+        engine.upload(x, out=b.A[0])
+        engine.upload(t, out=b.target)
+        b.forward()
+        lb = float(b.loss_value().numpy()[0, 0])
+        b.backward()
+        b.clip_and_optimize()
+        assert la == lb, step
+        np.testing.assert_array_equal(a.dX.numpy(), b.dX.numpy())
+        for p, q in zip(a.params, b.params):
+            np.testing.assert_array_equal(p.numpy(), q.numpy())
