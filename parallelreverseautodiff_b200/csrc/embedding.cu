@@ -51,13 +51,14 @@ embedding_gather_kernel(const T* __restrict__ index_col, const T* __restrict__ W
 // (With every CTA scanning the whole index column for its rows instead, a pass over 16384 indices of a 50000 x 512 table took
 // 560 us, most of it for scanning; now 64 us of kernels, the table's 102 MB being a third of it.)
 // Rows of many hits are the commonest words of a text: the commonest of 16384 appears a thousand times, and its additions are
-// a chain, so 64 vectors of such a row have a CTA to themselves whose four teams of threads copy rows of dOut into a ring in
-// shared memory, 64 rows ahead of the team that adds them (with 16 rows in flight in registers that one row took 150 us).
+// a chain, so 32 vectors of such a row have a CTA to themselves whose eight teams of threads copy rows of dOut into a ring in
+// shared memory, 48 rows ahead of the team that adds them (with 16 rows in flight in registers that one row took 150 us).  The
+// ring is 32 KB because the CTAs of the other rows, which make up most of the pass, have room for it too.
 constexpr int EMB_FEW = 32;                       // hits a warp orders by itself
 constexpr int EMB_WINDOW = 65536;                 // positions of one bitmap
 constexpr int EMB_LIST = 2048;                    // ordered positions handed to the summing loop at a time
 constexpr int EMB_ROWS = 8;                       // table rows a warp takes at once
-constexpr int EMB_GROUP = 64;                     // vectors of a row of many hits that a CTA takes
+constexpr int EMB_GROUP = 32;                     // vectors of a row of many hits that a CTA takes
 constexpr int EMB_CHUNK = 16, EMB_CHUNKS = 4;     // rows per step of the ring, steps in the ring
 
 struct EmbPlan {
@@ -96,6 +97,60 @@ emb_fill_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab) {
   for (int i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += gridDim.x * EMB_THREADS) {
     const int idx = (int)index_col[i];
     if (idx >= 0 && idx < vocab) p.list[p.offset[idx] + p.slot[i]] = i;
+  }
+}
+
+// Counting, places and filling of a small call in one cluster of eight CTAs, a cluster barrier between the passes: as a memset
+// and three launches the grouping of 16384 positions took 15 us, most of it launches.
+constexpr int EMB_PLAN_MOST = 1 << 17;            // positions and rows together
+__device__ __forceinline__ void emb_plan_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+template <typename T>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(1024)
+emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab, int* bad) {
+  constexpr int THREADS = 8 * 1024;
+  const int t = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31;
+  if (t < 2) p.cursor[t] = 0;
+#pragma unroll 8
+  for (int v = t; v < vocab; v += THREADS) p.count[v] = 0;
+  emb_plan_barrier();
+#pragma unroll 4
+  for (int i = t; i < n; i += THREADS) {
+    const int idx = (int)index_col[i];
+    if (idx < 0 || idx >= vocab) *(volatile int*)bad = i + 1;
+    else p.slot[i] = atomicAdd(p.count + idx, 1);
+  }
+  emb_plan_barrier();
+  constexpr int K = 8;                            // rows per thread and trip: one atomic round trip for 65536 rows
+  for (int v0 = t; v0 - lane < vocab; v0 += K * THREADS) {
+    int c[K], total = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) c[k] = v0 + k * THREADS < vocab ? __ldcg(p.count + v0 + k * THREADS) : 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) total += c[k];
+    int incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    int at = 0;
+    if (lane == 31 && incl) at = atomicAdd(p.cursor, incl);
+    at = __shfl_sync(0xffffffffu, at, 31) + incl - total;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int v = v0 + k * THREADS;
+      if (v < vocab) p.offset[v] = at;
+      at += c[k];
+      if (c[k] > EMB_FEW) p.hot[atomicAdd(p.cursor + 1, 1)] = v;
+    }
+  }
+  emb_plan_barrier();
+#pragma unroll 4
+  for (int i = t; i < n; i += THREADS) {
+    const int idx = (int)index_col[i];
+    if (idx >= 0 && idx < vocab) p.list[__ldcg(p.offset + idx) + p.slot[i]] = i;
   }
 }
 
@@ -243,7 +298,8 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
 }
 
 template <typename T>
-static prad_status scatter_t(prad_ctx* ctx, const void* index_col, const void* dOut, void* dW, int n, int vocab, int dim, int* bad) {
+static prad_status scatter_t(prad_ctx* ctx, const void* index_col, const void* dOut, void* dW, int n, int vocab, int dim, int* bad,
+                             cudaEvent_t checked = nullptr) {
   const size_t words = 3 * (size_t)vocab + 2 * (size_t)n + 64;
   prad_status s = ensure_stage(ctx, words * sizeof(int));
   if (s) return s;
@@ -254,18 +310,24 @@ static prad_status scatter_t(prad_ctx* ctx, const void* index_col, const void* d
   p.hot = p.offset + vocab;
   p.slot = p.hot + vocab;
   p.list = p.slot + n;
-  PRAD_CUDA(cudaMemsetAsync(p.cursor, 0, (64 + (size_t)vocab) * sizeof(int), ctx->stream));
   const T* idx = (const T*)index_col;
-  if (n > 0) {
+  const bool small = (int64_t)n + vocab <= EMB_PLAN_MOST && n > 0;
+  if (!small) PRAD_CUDA(cudaMemsetAsync(p.cursor, 0, (64 + (size_t)vocab) * sizeof(int), ctx->stream));
+  if (small) {
+    emb_plan_kernel<T><<<8, 1024, 0, ctx->stream>>>(idx, p, n, vocab, bad);
+    PRAD_LAUNCHED(ctx);
+    if (checked) PRAD_CUDA(cudaEventRecord(checked, ctx->stream));       // `bad` is known
+  } else if (n > 0) {
     const int g = stream_grid(ctx, n, EMB_THREADS, 8);
     emb_count_kernel<T><<<g, EMB_THREADS, 0, ctx->stream>>>(idx, p, n, vocab, bad);
     PRAD_LAUNCHED(ctx);
+    if (checked) PRAD_CUDA(cudaEventRecord(checked, ctx->stream));       // `bad` is known
     emb_place_kernel<<<(unsigned)ceil_div(vocab, EMB_THREADS), EMB_THREADS, 0, ctx->stream>>>(p, vocab);
     PRAD_LAUNCHED(ctx);
     emb_fill_kernel<T><<<g, EMB_THREADS, 0, ctx->stream>>>(idx, p, n, vocab);
     PRAD_LAUNCHED(ctx);
   }
-  const int hot = n > EMB_FEW ? ctx->sm_count : 0;
+  const int hot = n > EMB_FEW ? 2 * ctx->sm_count : 0;
   const unsigned grid = (unsigned)(hot + ceil_div(vocab, EMB_WARPS * EMB_ROWS));
   // shared memory for the ring only where a row can have many hits
   if (dim % EmbVec<T>::N == 0 && (((uintptr_t)dOut | (uintptr_t)dW) & 15) == 0) {
@@ -292,8 +354,9 @@ prad_status embedding_scatter_ordered(prad_ctx* ctx, prad_dtype dt, const void* 
 }
 
 // The offending position of a call arrives in page-locked host memory, so the check costs the wait alone.
-static prad_status check_bad_index(prad_ctx* ctx, const char* who) {
-  PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
+static prad_status check_bad_index(prad_ctx* ctx, const char* who, cudaEvent_t checked = nullptr) {
+  if (checked) PRAD_CUDA(cudaEventSynchronize(checked));
+  else PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
   const int h = *(volatile int*)ctx->host_flag;
   PRAD_REQUIRE(h == 0, PRAD_ERR_INVALID, "%s: index at input row %d is outside [0, vocab)", who, h - 1);
   return PRAD_OK;
@@ -339,8 +402,11 @@ prad_status prad_embedding_backward(prad_ctx* ctx, prad_dtype dt, const void* in
                "prad_embedding_backward: null pointer");
   PRAD_NOT_CAPTURING(ctx, "prad_embedding_backward");
   *(volatile int*)ctx->host_flag = 0;
-  prad_status s = embedding_scatter_ordered(ctx, dt, index_col, dOut, dW, n, vocab, dim, ctx->host_flag);
-  return s ? s : check_bad_index(ctx, "prad_embedding_backward");
+  // the indices have been looked at once the first kernel is done: the caller need not wait for the sums
+  if (!ctx->flag_read) PRAD_CUDA(cudaEventCreateWithFlags(&ctx->flag_read, cudaEventDisableTiming));
+  prad_status s = dt == PRAD_F32 ? scatter_t<float>(ctx, index_col, dOut, dW, n, vocab, dim, ctx->host_flag, ctx->flag_read)
+                                 : scatter_t<double>(ctx, index_col, dOut, dW, n, vocab, dim, ctx->host_flag, ctx->flag_read);
+  return s || n == 0 ? s : check_bad_index(ctx, "prad_embedding_backward", ctx->flag_read);
 }
 
 }  // extern "C"

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("n,vocab,dim,hot", [(1, 1, 1, 0), (31, 3, 5, 0), (32, 1, 8, 0), (33, 1, 8, 0), (1000, 17, 12, 500), (3000, 700, 33, 1500),
-                                             (5000, 9, 1030, 0), (70000, 50, 4, 40000), (140000, 3, 6, 0), (2000, 20000, 64, 100)])
+                                             (5000, 9, 1030, 0), (70000, 50, 4, 40000), (140000, 3, 6, 0), (2000, 20000, 64, 100), (100, 131000, 4, 0), (72, 131000, 4, 0)])
 def test_scatter_in_input_order(engine, dtype, n, vocab, dim, hot):
     r = rng(n + vocab)
     idx = r.integers(0, vocab, n)
