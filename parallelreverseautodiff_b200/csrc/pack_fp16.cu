@@ -699,19 +699,20 @@ static bool packed_ok(const prad_packed* p) { return p && p->magic == 0x50414b44
 #define PRAD_CHECK_PACKED(p, who)                                                                  \
   PRAD_REQUIRE(prad::packed_ok(p), PRAD_ERR_INVALID, who ": the packed operand is null or destroyed")
 
-static prad_status alloc_form(PackedForm& f) {
-  cudaError_t e = device_malloc((void**)&f.h, f.h_bytes() ? f.h_bytes() : 16);
-  if (e == cudaSuccess) e = device_malloc((void**)&f.blk, f.blk_bytes() ? f.blk_bytes() : 16);
-  if (e == cudaSuccess) e = cudaMemset(f.blk, 0, f.blk_bytes());     // rows beyond the matrix keep exponent 0
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    if (f.h) cudaFree(f.h);
-    if (f.blk) cudaFree(f.blk);
-    f.h = nullptr;
-    f.blk = nullptr;
-    set_error("prad_packed_create: %zu bytes could not be allocated: %s", f.h_bytes() + f.blk_bytes(), cudaGetErrorString(e));
-    return PRAD_ERR_OOM;
+static void free_form(prad_ctx* ctx, PackedForm& f) {
+  if (f.h) pool_free(ctx, f.h);
+  if (f.blk) pool_free(ctx, f.blk);
+  f.h = nullptr;
+  f.blk = nullptr;
+}
+static prad_status alloc_form(prad_ctx* ctx, PackedForm& f) {
+  prad_status s = pool_alloc(ctx, f.h_bytes() ? f.h_bytes() : 16, (void**)&f.h);
+  if (!s) s = pool_alloc(ctx, f.blk_bytes() ? f.blk_bytes() : 16, (void**)&f.blk);
+  if (s) {
+    free_form(ctx, f);
+    return s;
   }
+  PRAD_CUDA(cudaMemsetAsync(f.blk, 0, f.blk_bytes(), ctx->stream));     // rows beyond the matrix keep exponent 0
   return PRAD_OK;
 }
 // block length of a packed object unless the caller names one: 128 (one pass writes both forms from a
@@ -742,14 +743,15 @@ prad_status prad_packed_create(prad_ctx* ctx, int rows, int cols, int forms, int
   if (forms & PRAD_PACK_ROWS) {
     const int b = block_rows_form ? block_rows_form : chunk;
     p->by_rows = packed_form_shape(rows, cols, b);
-    s = alloc_form(p->by_rows);
+    s = alloc_form(ctx, p->by_rows);
   }
   if (!s && (forms & PRAD_PACK_COLS)) {
     p->by_cols = packed_form_shape(cols, rows, block_cols_form ? block_cols_form : chunk);
-    s = alloc_form(p->by_cols);
+    s = alloc_form(ctx, p->by_cols);
   }
   if (s) {
-    if (p->by_rows.h) { cudaFree(p->by_rows.h); cudaFree(p->by_rows.blk); }
+    free_form(ctx, p->by_rows);
+    free_form(ctx, p->by_cols);
     delete p;
     return s;
   }
@@ -759,11 +761,8 @@ prad_status prad_packed_create(prad_ctx* ctx, int rows, int cols, int forms, int
 
 prad_status prad_packed_destroy(prad_packed* p) {
   PRAD_CHECK_PACKED(p, "prad_packed_destroy");
-  cudaStreamSynchronize(p->ctx->stream);
-  for (PackedForm* f : {&p->by_rows, &p->by_cols}) {
-    if (f->h) cudaFree(f->h);
-    if (f->blk) cudaFree(f->blk);
-  }
+  free_form(p->ctx, p->by_rows);
+  free_form(p->ctx, p->by_cols);
   p->magic = 0;
   delete p;
   return PRAD_OK;
