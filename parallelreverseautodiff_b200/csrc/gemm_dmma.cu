@@ -192,6 +192,28 @@ combine_kernel(const double* __restrict__ part, int splits, int64_t mn, int N, d
   }
 }
 
+// Slices of a k: two CTAs on every SM, slices of at least 128 (256 beyond sixteen, which the ordered pass would feel).
+static int slices_of(const prad_ctx* ctx, int64_t tiles, int K) {
+  if (tiles * 2 > ctx->sm_count || K < 512) return 1;
+  const int most = K / 128 < 16 ? K / 128 : (K / 256 > 16 ? K / 256 : 16);
+  const int64_t S = 2 * ctx->sm_count / tiles;
+  return (int)(S < most ? S : most);
+}
+// One launch for both products of a Backward: where the longest tile (and a short one on the same SM, when there are more tiles
+// than SMs), or all of them spread over the SMs, takes less than the two products one after the other with their slices.  In
+// units of k per SM; a launch's ramp is about 64, the ordered pass 96.  512 x 512 over 512: 41 -> 27 us; 1024 x 512 over 256,
+// where one tile of k = 1024 would outlast everything, stays at 37 us in two launches (57 in one).
+static bool one_launch(const prad_ctx* ctx, int M, int K, int N) {
+  const int64_t tA = ceil_div(M, BM) * ceil_div(K, BN), tB = ceil_div(K, BM) * ceil_div(N, BN);
+  const int64_t both = (tA * N + tB * M) / ctx->sm_count, lo = N < M ? N : M, hi = N < M ? M : N;
+  const int64_t chain = hi + (tA + tB > ctx->sm_count ? lo : 0);
+  auto alone = [&](int64_t tiles, int k) {
+    const int S = slices_of(ctx, tiles, k);
+    return ceil_div(k, S) * ceil_div(tiles * S, ctx->sm_count) + (S > 1 ? 96 : 0);
+  };
+  return (both > chain ? both : chain) <= alone(tA, N) + alone(tB, M) + 64;
+}
+
 static prad_status set_problem(Problem& pr, const Product<double>& p, int batch, int64_t* tiles) {
   pr.p = p;
   pr.slices = 1;
@@ -235,18 +257,14 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
   prad_status st = dm::set_problem(pr, make_product<double>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC, e), batch, &tiles);
   if (st) return st;
   // Few output tiles and a long k (the time-batched weight gradients of an LSTM: 256 x 128 outputs over k = 2048 in a batch of
-  // four are 32 tiles): k is cut into slices of at least 256 that run as further tiles into scratch, enough of them for two
-  // CTAs on every SM, and an ordered pass adds them.
+  // four are 32 tiles): k is cut into slices that run as further tiles into scratch, and an ordered pass adds them.
   const bool plain = !e.bias && !e.z_out && e.act == PRAD_ACT_NONE && e.dact == PRAD_ACT_NONE;
   // The sum over a batch (sC = 0) is that with the batch entries as further slices.
   const bool sum = batch > 1 && sC == 0;
-  if (plain && (sum || (tiles * 2 <= ctx->sm_count && K >= 512))) {
-    int S = (int)(2 * ctx->sm_count / tiles);
-    if (S > K / 256) S = K / 256;
-    if (S < 1) S = 1;
+  if (int S = plain ? dm::slices_of(ctx, tiles, K) : 1; S > 1 || (plain && sum)) {
     const int k_slice = (int)(ceil_div(ceil_div(K, S), dm::BK) * dm::BK);
     S = (int)ceil_div(K, k_slice);
-    if (S >= 2 || sum) {
+    if (S > 1 || sum) {
       const int64_t mn = (int64_t)M * N;
       st = ensure_parts(ctx, (size_t)batch * S * mn * sizeof(double));
       if (st) return st;
@@ -269,6 +287,8 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
   }
   return dm::launch(ctx, tA, tB, pr, tiles);
 }
+
+bool gemm_f64_dmma_one_launch(prad_ctx* ctx, int M, int K, int N) { return dm::one_launch(ctx, M, K, N); }
 
 // dA (M x K) = dC (M x N) * B^T (.) act'(saved)  and  dB (K x N) = scale * A^T * dC [+ dB] of a product both of whose
 // gradients belong on the tensor cores, in one launch

@@ -38,6 +38,7 @@ static bool wants_tensor_cores(prad_ctx* ctx, prad_dtype dt, bool tA, bool tB, i
          gemm_f64_dmma(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, true) == PRAD_OK;
 }
 
+bool gemm_f64_dmma_one_launch(prad_ctx* ctx, int M, int K, int N);
 prad_status gemm_f64_dmma_backward(prad_ctx* ctx, const void* A, const void* B, const void* dC, void* dA, void* dB, int M, int K, int N,
                                    bool accumulate_dB, double dB_scale, const GemmEpilogue& e_dA);
 
@@ -144,9 +145,7 @@ static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void
                                                       accumulate_dB != 0, dB_scale, e_dA)
                           : gemm_simt_backward<double>(ctx, ctx->gemm_f64 != GemmF64::SimtFma, A, B, dC, dA, dB, M, K, N,
                                                        accumulate_dB != 0, dB_scale, e_dA);
-  // one launch where neither would be cut into k slices
-  if (both && tc_A && tc_B && dt == PRAD_F64 &&
-      (ceil_div(M, 64) * ceil_div(K, 64) * 2 > ctx->sm_count || N < 512) && (ceil_div(K, 64) * ceil_div(N, 64) * 2 > ctx->sm_count || M < 512))
+  if (both && tc_A && tc_B && dt == PRAD_F64 && gemm_f64_dmma_one_launch(ctx, M, K, N))
     return gemm_f64_dmma_backward(ctx, A, B, dC, dA, dB, M, K, N, accumulate_dB != 0, dB_scale, e_dA);
   cudaStream_t main = ctx->stream;
   if (branches) {

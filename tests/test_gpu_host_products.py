@@ -8,7 +8,8 @@ from util import rng
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dtype,m,k,n", [(np.float64, 4096, 256, 128), (np.float32, 8192, 128, 128)])
+@pytest.mark.parametrize("dtype,m,k,n", [(np.float64, 4096, 256, 128), (np.float32, 8192, 128, 128),
+                                           (np.float64, 512, 512, 512), (np.float64, 70, 4000, 520), (np.float64, 1024, 512, 256)])
 def test_host_backward_equals_device_backward(engine, dtype, m, k, n):
     r = rng(m)
     A, B = r.standard_normal((m, k)).astype(dtype), r.standard_normal((k, n)).astype(dtype)
@@ -19,6 +20,9 @@ def test_host_backward_equals_device_backward(engine, dtype, m, k, n):
     np.testing.assert_array_equal(hP, dP.numpy())
     np.testing.assert_array_equal(hA, dA.numpy())
     np.testing.assert_array_equal(hB, dB.numpy())
+    tol = 1e-13 if dtype == np.float64 else 2e-5
+    for got, want in ((hA, hP.astype(np.float64) @ B.T), (hB, A.astype(np.float64).T @ hP)):
+        np.testing.assert_allclose(got, want, rtol=0, atol=tol * np.abs(want).max())
 
 
 def test_host_steps_repeat_and_follow_changes(engine):
