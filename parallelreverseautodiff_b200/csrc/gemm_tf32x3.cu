@@ -2152,6 +2152,52 @@ prad_status gemm_tf32x3(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, do
   }
 }
 
+// Both products of a large float Backward from packed operands: dA (M x K) = dC B^T (.) act'(saved) and dB (K x N) =
+// dB_scale A^T dC [+ dB].  dC (M x N) feeds both and is packed in both orientations by one pass -- the one that computes it,
+// where it is dOut (.) act'(saved_out) (act != none; dC receives it).  8192 x 2048 x 1536: 65 us for the activation's Backward and
+// two packing passes, 47 us in one.  PRAD_ERR_UNSUPPORTED: not the FP16 scheme with its 128-long blocks.
+prad_status gemm_fp16x3_backward(prad_ctx* ctx, const void* A, const void* B, const void* dOut, prad_act act, const void* saved,
+                                 double act_alpha, void* dC, void* dA, void* dB, int M, int K, int N, bool accumulate_dB,
+                                 double dB_scale, const GemmEpilogue& e_dA) {
+  const bool scheme = ctx->gemm_f32 == GemmF32::Fp16x3 || (ctx->gemm_f32 == GemmF32::Auto && ctx->tc_auto_mode == 3);
+  if (!scheme || (ctx->tc_chunk_k_set && ctx->tc_chunk_k >= 256)) return PRAD_ERR_UNSUPPORTED;
+  PackedForm cr = packed_form_shape(M, N, 128), cc = packed_form_shape(N, M, 128), b = packed_form_shape(K, N, 128),
+             a = packed_form_shape(K, M, 128);
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  size_t scales = 0, pieces = 0;
+  for (PackedForm* f : {&cr, &cc, &b, &a}) { scales += al(f->blk_bytes()); pieces += al(f->h_bytes()); }
+  if (scales + pieces > ctx->total_mem / 16) return PRAD_ERR_UNSUPPORTED;      // (one product at a time needs half of it)
+  prad_status s = ensure_workspace(ctx, scales + pieces);
+  if (s) return s;
+  char* w = (char*)ctx->ws;
+  for (PackedForm* f : {&cr, &cc, &b, &a}) { f->blk = (float*)w; w += al(f->blk_bytes()); }
+  for (PackedForm* f : {&cr, &cc, &b, &a}) { f->h = (__half*)w; w += al(f->h_bytes()); }
+  PRAD_CUDA(cudaMemsetAsync(ctx->ws, 0, scales, ctx->stream));       // rows beyond the matrices
+  PackSource src;
+  src.ld = N;
+  if (act == PRAD_ACT_NONE) {
+    src.x = (const float*)dC;
+  } else {
+    src.kind = 2;
+    src.x = (const float*)saved;
+    src.dy = (const float*)dOut;
+    src.out = (float*)dC;
+    src.act = (int)act;
+    src.act_alpha = (float)act_alpha;
+  }
+  if ((s = pack_fp16(ctx, src, M, N, &cr, &cc))) return s;
+  PackSource sb, sa;
+  sb.x = (const float*)B; sb.ld = N;
+  sa.x = (const float*)A; sa.ld = K;
+  if ((s = pack_fp16(ctx, sb, K, N, &b, nullptr))) return s;
+  if ((s = tc::launch_fp16x3(ctx, cr, b, (float*)dA, K, 1.f, 0.f, nullptr))) return s;
+  if (e_dA.dact != PRAD_ACT_NONE &&
+      (s = prad_act_backward(ctx, PRAD_F32, e_dA.dact, e_dA.saved, dA, dA, (int64_t)M * K, e_dA.act_alpha)))
+    return s;
+  if ((s = pack_fp16(ctx, sa, M, K, nullptr, &a))) return s;
+  return tc::launch_fp16x3(ctx, a, cc, (float*)dB, N, (float)dB_scale, accumulate_dB ? 1.f : 0.f, nullptr);
+}
+
 // ---- self-test of the give-up path ----------------------------------------------------------
 // One CTA initialises an mbarrier that nothing will ever arrive on and waits for it with the same
 // polling loop as the GEMM kernels, but with a caller-chosen limit of a few polls: the wait runs out,

@@ -122,11 +122,17 @@ mas_backward_dA_kernel(const T* __restrict__ B, const T* __restrict__ dOut, T* _
   }
 }
 
+prad_status gemm_fp16x3_backward(prad_ctx* ctx, const void* A, const void* B, const void* dOut, prad_act act, const void* saved,
+                                 double act_alpha, void* dC, void* dA, void* dB, int M, int K, int N, bool accumulate_dB,
+                                 double dB_scale, const GemmEpilogue& e_dA);
+
+// dOut given: dC is not there yet, it is to receive dOut (.) act'(saved)
 static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void* A,
                                         const void* B, const void* dC, void* dA, void* dB, int M,
                                         int K, int N, int accumulate_dB, double dB_scale,
                                         prad_act act_below, const void* saved_below,
-                                        double act_alpha) {
+                                        double act_alpha, const void* dOut = nullptr, prad_act act = PRAD_ACT_NONE,
+                                        const void* saved = nullptr) {
   prad_status s;
   GemmEpilogue e_dA, e_dB;
   e_dA.dact = act_below;
@@ -137,6 +143,14 @@ static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void
   const bool tc_A = both && wants_tensor_cores(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA);
   const bool tc_B = both && wants_tensor_cores(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0,
                                                0, 0, e_dB);
+  if (both && tc_A && tc_B && dt == PRAD_F32) {
+    s = gemm_fp16x3_backward(ctx, A, B, dOut, act, saved, act_alpha, const_cast<void*>(dC), dA, dB, M, K, N, accumulate_dB != 0, dB_scale, e_dA);
+    if (s != PRAD_ERR_UNSUPPORTED) return s;
+  }
+  if (dOut) {
+    s = prad_act_backward(ctx, dt, act, saved ? saved : dOut, dOut, const_cast<void*>(dC), (int64_t)M * N, act_alpha);
+    if (s) return s;
+  }
   // Neither on the tensor cores: both products in one launch, or, in a recording, as two branches that run side by side, each
   // in the tile shape that suits it.
   const bool branches = both && !tc_A && !tc_B && ctx->capturing;
@@ -238,9 +252,14 @@ prad_status prad_matmul_act_backward(prad_ctx* ctx, prad_dtype dt, const void* A
   CHECK_DIMS("prad_matmul_act_backward", M, K, N);
   PRAD_REQUIRE(dPre && dOut && (saved || act == PRAD_ACT_NONE), PRAD_ERR_INVALID,
                "prad_matmul_act_backward: null pointer");
-  prad_status s = prad_act_backward(ctx, dt, act, saved ? saved : dOut, dOut, dPre, (int64_t)M * N, act_alpha);
-  if (s) return s;
-  return matmul_backward_impl(ctx, dt, A, B, dPre, dA, dB, M, K, N, 0, 1.0, PRAD_ACT_NONE, nullptr, 0.0);
+  // (in place, or without an activation, dPre is computed first)
+  const bool apart = dPre != dOut && dPre != saved && act != PRAD_ACT_NONE;
+  if (!apart) {
+    prad_status s = prad_act_backward(ctx, dt, act, saved ? saved : dOut, dOut, dPre, (int64_t)M * N, act_alpha);
+    if (s) return s;
+  }
+  return matmul_backward_impl(ctx, dt, A, B, dPre, dA, dB, M, K, N, 0, 1.0, PRAD_ACT_NONE, nullptr, act_alpha, apart ? dOut : nullptr,
+                              apart ? act : PRAD_ACT_NONE, saved);
 }
 
 prad_status prad_matmul_act_backward_host(prad_ctx* ctx, prad_dtype dt, const void* A_host,

@@ -44,3 +44,24 @@ def test_many_slices(engine, m, n, beta):
     engine.gemm_packed(PX, E.PACK_COLS, PY, E.PACK_COLS, out, alpha=0.25, beta=beta)
     want = 0.25 * (X.astype(np.float64).T @ Y) + beta * C0
     np.testing.assert_allclose(out.numpy(), want, rtol=0, atol=2e-6 * np.sqrt(k))
+
+
+@pytest.mark.parametrize("m,k,n", [(1000, 520, 300), (4097, 130, 258), (640, 511, 515)])
+@pytest.mark.parametrize("act", [E.ACT_NONE, E.ACT_GELU, E.ACT_LEAKY_RELU, E.ACT_TANH])
+def test_backward_of_a_large_float_product(engine, m, k, n, act):
+    """Both gradients from one packing of dC: the bits of one product at a time, in one call with the activation or after it."""
+    r = rng(m + n)
+    A, B, dOut, saved = (engine.upload(r.standard_normal(s).astype(f)) for s in ((m, k), (k, n), (m, n), (m, n)))
+    dC = engine.act_backward(act, saved, dOut, 0.1) if act != E.ACT_NONE else dOut
+    dA1, _ = engine.matmul_backward(None, B, dC, need_dB=False)
+    _, dB1 = engine.matmul_backward(A, None, dC, need_dA=False)
+    dA2, dB2 = engine.matmul_backward(A, B, dC)
+    dP3, dA3, dB3 = engine.matmul_act_backward(A, B, dOut, act, saved, 0.1)
+    np.testing.assert_array_equal(dP3.numpy(), dC.numpy())
+    for got, want in ((dA2, dA1), (dB2, dB1), (dA3, dA1), (dB3, dB1)):
+        np.testing.assert_array_equal(got.numpy(), want.numpy())
+    acc = engine.upload(np.ones((k, n), f))
+    dA4 = engine.matmul_backward(A, B, dC, dB=acc, accumulate_dB=True, dB_scale=0.5, act_below=E.ACT_LEAKY_RELU,
+                                 saved_below=A, act_alpha=0.1)[0]
+    np.testing.assert_array_equal(dA4.numpy(), engine.act_backward(E.ACT_LEAKY_RELU, A, dA1, 0.1).numpy())
+    np.testing.assert_allclose(acc.numpy(), 1 + 0.5 * dB1.numpy(), rtol=0, atol=1e-5 * np.abs(dB1.numpy()).max())
