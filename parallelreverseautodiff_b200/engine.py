@@ -397,7 +397,8 @@ class Engine:
             raise _lib.PradError(_lib.ERR_SHAPE, "Input 1 columns do not match Input 2 rows")
         Y = Y or self.empty((M, N), A.dtype)
         check(self.lib.prad_matmul_forward(self.ctx, dtype_code(A.dtype), A.ptr, B.ptr, Y.ptr, M, K,
-                                           N, self._p(bias), self._p(Z_out), act, act_alpha))
+                                           N, None if bias is None else bias.ptr, None if Z_out is None else Z_out.ptr, act,
+                                           act_alpha))
         return Y
 
     def matmul_backward(self, A, B, dC, dA=None, dB=None, need_dA=True, need_dB=True,
@@ -410,9 +411,9 @@ class Engine:
         if need_dB and dB is None:
             dB = self.empty((K, N), dC.dtype)
         check(self.lib.prad_matmul_backward(
-            self.ctx, dtype_code(dC.dtype), self._p(A), self._p(B), dC.ptr,
-            self._p(dA if need_dA else None), self._p(dB if need_dB else None), M, K, N,
-            int(accumulate_dB), dB_scale, act_below, self._p(saved_below), act_alpha))
+            self.ctx, dtype_code(dC.dtype), None if A is None else A.ptr, None if B is None else B.ptr, dC.ptr,
+            dA.ptr if need_dA else None, dB.ptr if need_dB else None, M, K, N,
+            int(accumulate_dB), dB_scale, act_below, None if saved_below is None else saved_below.ptr, act_alpha))
         return dA, dB
 
     def matmul_act_backward(self, A, B, dOut, act, saved, act_alpha=0.0):
