@@ -600,6 +600,8 @@ __device__ __forceinline__ void epilogue_quad(float o0, float o1, float o2, floa
 }
 
 // sum[g][j] = column col0 + 32 g + j of row row0 + lane (modified in place)
+// BIAS is a template parameter of the kernels above it: the code that adds it, never run, cost the 65536 x 4096 products 1 %.
+template <bool BIAS>
 __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lane, int row0, int col0, int M, int N,
                                                     float* __restrict__ C, int64_t ldc, bool vecC, const Epi& epi,
                                                     const float4* bias = nullptr) {     // epi.bias from col0 on
@@ -612,7 +614,7 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
   // (Columns: the warp's 128 or, at the right edge, a multiple of 16, so that each store instruction is all or nothing.)
   const int ncols = N - col0 < 128 ? N - col0 : 128;
   if (ncols <= 0 || row0 >= M) return;
-  if (vecC && epi.beta == 0.f && (bias || ((uintptr_t)epi.bias & 15) == 0) && !epi.row_exp && row0 + 32 <= M && (ncols & 15) == 0) {
+  if (vecC && epi.beta == 0.f && (BIAS ? bias || ((uintptr_t)epi.bias & 15) == 0 : !epi.bias) && !epi.row_exp && row0 + 32 <= M && (ncols & 15) == 0) {
     float* rp[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) rp[s] = C + (int64_t)(qrow + s) * ldc + col0 + 4 * i;
@@ -623,7 +625,7 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
 #pragma unroll
         for (int j = 0; j < 32; ++j) sum[g][j] = alpha * sum[g][j];
     }
-    if (epi.bias) {      // a lane still holds whole row parts here: the same four columns for all lanes, one load for the warp
+    if (BIAS && epi.bias) {      // a lane still holds whole row parts here: the same four columns for all lanes, one load for the warp
 #pragma unroll
       for (int g = 0; g < 4; ++g)
 #pragma unroll
@@ -673,6 +675,7 @@ __device__ __forceinline__ void epilogue_store_warp(float (&sum)[4][32], int lan
 // accumulator through the scales to memory in a rolled loop of some three hundred instructions.  The unrolled code above for 128
 // columns is fetched anew for every tile and the warps wait for it: 200704 x 384 outputs over k = 96 took 4.6 us per tile.
 // Whole rows of the tile exist, ncols is a multiple of 16 (or there are none); one block's scales start at block `blk`.
+template <bool BIAS>
 __device__ __forceinline__ bool epilogue_one_block(int lane, int row0, int col0, int ncols, float* __restrict__ C, int64_t ldc, int64_t blk,
                                                    const Epi& epi, float4* sb_slot, uint32_t taddr, uint32_t full, uint32_t parity,
                                                    uint32_t empty, int* err_flag) {
@@ -680,7 +683,7 @@ __device__ __forceinline__ bool epilogue_one_block(int lane, int row0, int col0,
   float4* const bias_slot = sb_slot + EPI_WARPS * 32;
   if (4 * lane < ncols) {
     sb_slot[lane] = __ldg(reinterpret_cast<const float4*>(epi.blk_b + blk * epi.blk_ldb + col0) + lane);
-    if (epi.bias) {
+    if (BIAS && epi.bias) {
       const float* b = epi.bias + col0 + 4 * lane;
       bias_slot[lane] = make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3));
     }
@@ -710,7 +713,7 @@ __device__ __forceinline__ bool epilogue_one_block(int lane, int row0, int col0,
 #pragma unroll
       for (int j = 0; j < 32; ++j) x[j] = epi.alpha * x[j];
     }
-    if (epi.bias) {
+    if (BIAS && epi.bias) {
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
         const float4 b = bias_slot[(c + j) >> 2];
@@ -780,7 +783,7 @@ struct TileSched {
   int bn = BN;                    // columns of a tile (PMODE 3; BN otherwise)
 };
 
-template <int PMODE>
+template <int PMODE, bool BIAS>
 __global__ void __launch_bounds__(THREADS, 1)   // 10 warps, at most 3 per scheduler: 3 x 32 x 168 registers fit its 16 K file
 gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_constant__ CUtensorMap map_a_xb,
                                const __grid_constant__ CUtensorMap map_a_lb, const __grid_constant__ CUtensorMap map_b_hi,
@@ -1015,7 +1018,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       tile_of(t, m0, n0, z, kb0, num_kb);
       const int num_chunks = (num_kb + ts.chunk_kb - 1) / ts.chunk_kb;
       if (PMODE == 3 && num_chunks == 1 && vecC && epi.beta == 0.f && m0 + BM <= M && ((N - n0) & 15) == 0) {
-        ok = epilogue_one_block(lane, m0 + sub * 32, n0 + half * hw, min(N - n0 - half * hw, hw), C + (int64_t)z * ts.split_stride, ldc,
+        ok = epilogue_one_block<BIAS>(lane, m0 + sub * 32, n0 + half * hw, min(N - n0 - half * hw, hw), C + (int64_t)z * ts.split_stride, ldc,
                                 (int64_t)(kb0 / ts.chunk_kb), epi,
                                 reinterpret_cast<float4*>(generic_base + RING_BYTES + 256) + (warp - 2) * 32,
                                 tmem_base + ((uint32_t)(sub * 32) << 16) + (gc & 1) * (uint32_t)BN + (uint32_t)(half * hw),
@@ -1045,7 +1048,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       // the bias of the warp's columns waits in shared memory for the store: read from there when the product is done, it kept
       // every tile waiting (200704 x 384 over k = 96: 136 us with it, 101 us without)
       float4* const bias_slot = sb_slot + EPI_WARPS * 32;
-      if (PMODE == 3 && epi.bias) {
+      if (PMODE == 3 && BIAS && epi.bias) {
         const int c = n0 + half * hw + 4 * lane;
         float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c < N) b.x = __ldg(epi.bias + c);
@@ -1124,7 +1127,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __gri
       const int gave_up = *((volatile int*)err_flag);
       float* Ct = C + (int64_t)z * ts.split_stride;
       const int c0 = n0 + half * hw;
-      epilogue_store_warp(sum, lane, m0 + sub * 32, c0, M, min(N, c0 + hw), Ct, ldc, vecC, epi, PMODE == 3 ? bias_slot : nullptr);
+      epilogue_store_warp<BIAS>(sum, lane, m0 + sub * 32, c0, M, min(N, c0 + hw), Ct, ldc, vecC, epi, PMODE == 3 ? bias_slot : nullptr);
       __syncwarp();
       if (gave_up != 0) { ok = false; break; }
 #ifdef PRAD_GEMM_STALL_PROBE
@@ -1268,6 +1271,7 @@ __host__ __device__ constexpr uint32_t idesc_fp16_pair() {
   return (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(p2::BM2 >> 4) << 24);
 }
 
+template <bool BIAS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  int M, int N, float* __restrict__ C, int64_t ldc, bool vecC, Epi epi,
@@ -1513,7 +1517,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       // has another CTA given up?  Asked before the stores and looked at after them: the answer takes a trip to L2
       const int gave_up = *((volatile int*)err_flag);
       float* Ct = C + (int64_t)z * ts.split_stride;
-      epilogue_store_warp(sum, lane, m0 + sub * 32, n0 + half * 128, M, N, Ct, ldc, vecC, epi);
+      epilogue_store_warp<BIAS>(sum, lane, m0 + sub * 32, n0 + half * 128, M, N, Ct, ldc, vecC, epi);
       if (gave_up != 0) { ok = false; break; }
     }
   }
@@ -1863,7 +1867,7 @@ static prad_status launch_tf32x3(prad_ctx* ctx, const SplitOperand& a, const Spl
   const bool persistent = CFG::MODE == 1 && CFG::BK == p1::BK && ctx->tc_persistent;
   if (persistent) {
     static std::atomic<uint64_t> p_done{0};
-    const cudaError_t p_err = reserve_smem(gemm_persistent_kernel<PMODE>, p1::SMEM_BYTES, ctx->device, p_done);
+    const cudaError_t p_err = reserve_smem(gemm_persistent_kernel<PMODE, true>, p1::SMEM_BYTES, ctx->device, p_done);
     PRAD_REQUIRE(p_err == cudaSuccess, PRAD_ERR_CUDA, "gemm (persistent): cannot reserve %d bytes of shared memory: %s",
                  p1::SMEM_BYTES, cudaGetErrorString(p_err));
   }
@@ -1878,7 +1882,7 @@ static prad_status launch_tf32x3(prad_ctx* ctx, const SplitOperand& a, const Spl
       const int64_t total = tiles * nsplit;
       const int64_t sms = ctx->sm_count - ctx->tc_reserve_sms;
       const unsigned ctas = (unsigned)(total < sms ? total : sms);
-      gemm_persistent_kernel<PMODE><<<ctas, THREADS, p1::SMEM_BYTES, ctx->stream>>>(
+      gemm_persistent_kernel<PMODE, true><<<ctas, THREADS, p1::SMEM_BYTES, ctx->stream>>>(
           ma_hi, ma_x, ma_lo, mb_hi, mb_x, mb_lo, M, N, out, ldo, vec_out, ep, ctx->tc_err, ts);
     } else {
       dim3 g3 = grid;
@@ -1940,8 +1944,8 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
   const bool ok = make_map(&ma, a.h, M, (int)(2 * kp), a.pitch, BM, 2 * p1::BK, 2, true) &&
                   make_map(&mb, b.h, N, (int)(2 * kp), b.pitch, bn, 2 * p1::BK, 2, true);
   PRAD_REQUIRE(ok, PRAD_ERR_CUDA, "gemm (tensor core): cuTensorMapEncodeTiled failed (M %d N %d K %lld)", M, N, (long long)kp);
-  static std::atomic<uint64_t> p_done{0};
-  const cudaError_t p_err = reserve_smem(gemm_persistent_kernel<3>, p1::SMEM_BYTES, ctx->device, p_done);
+  static std::atomic<uint64_t> p_done[2];
+  const cudaError_t p_err = reserve_smem(bias ? gemm_persistent_kernel<3, true> : gemm_persistent_kernel<3, false>, p1::SMEM_BYTES, ctx->device, p_done[bias != nullptr]);
   PRAD_REQUIRE(p_err == cudaSuccess, PRAD_ERR_CUDA, "gemm (persistent): cannot reserve %d bytes of shared memory: %s",
                p1::SMEM_BYTES, cudaGetErrorString(p_err));
   const int tiles_m = (int)ceil_div(M, BM), tiles_n = (int)ceil_div(N, BN);
@@ -1960,8 +1964,8 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
   if (pair) {
     PRAD_REQUIRE(make_map(&mb_half, b.h, N, (int)(2 * kp), b.pitch, BN / 2, 2 * p1::BK, 2, true), PRAD_ERR_CUDA,
                  "gemm (tensor core): cuTensorMapEncodeTiled failed for the half column tile (N %d K %lld)", N, (long long)kp);
-    static std::atomic<uint64_t> pair_done{0};
-    const cudaError_t q_err = reserve_smem(gemm_pair_kernel, p2::SMEM_BYTES, ctx->device, pair_done);
+    static std::atomic<uint64_t> pair_done[2];
+    const cudaError_t q_err = reserve_smem(bias ? gemm_pair_kernel<true> : gemm_pair_kernel<false>, p2::SMEM_BYTES, ctx->device, pair_done[bias != nullptr]);
     PRAD_REQUIRE(q_err == cudaSuccess, PRAD_ERR_CUDA, "gemm (CTA pairs): cannot reserve %d bytes of shared memory: %s",
                  p2::SMEM_BYTES, cudaGetErrorString(q_err));
   }
@@ -1988,14 +1992,14 @@ static prad_status launch_fp16x3(prad_ctx* ctx, const PackedForm& a, const Packe
       const int64_t total = (int64_t)tiles_m2 * tiles_n * nsplit;
       const int64_t pairs = sms / 2;
       const unsigned ctas = 2u * (unsigned)(total < pairs ? total : pairs);
-      gemm_pair_kernel<<<ctas, THREADS, p2::SMEM_BYTES, ctx->stream>>>(ma, mb_half, M, N, out, ldo, vec_out, ep, ctx->tc_err, ts);
+      (ep.bias ? gemm_pair_kernel<true> : gemm_pair_kernel<false>)<<<ctas, THREADS, p2::SMEM_BYTES, ctx->stream>>>(ma, mb_half, M, N, out, ldo, vec_out, ep, ctx->tc_err, ts);
       return;
     }
     TileSched ts{tiles_m, tiles_n, nsplit, kbps, total_kb, chunk_kb, panel_n, stride, ctx->tc_prefetch, bn};
     const int64_t total = tiles * nsplit;
     const unsigned ctas = (unsigned)(total < sms ? total : sms);
-    gemm_persistent_kernel<3><<<ctas, THREADS, p1::SMEM_BYTES, ctx->stream>>>(ma, ma, ma, mb, mb, mb, M, N, out, ldo, vec_out,
-                                                                              ep, ctx->tc_err, ts);
+    (ep.bias ? gemm_persistent_kernel<3, true> : gemm_persistent_kernel<3, false>)<<<ctas, THREADS, p1::SMEM_BYTES, ctx->stream>>>(
+        ma, ma, ma, mb, mb, mb, M, N, out, ldo, vec_out, ep, ctx->tc_err, ts);
   };
   if (splits == 1) {
     launch(1, total_kb, 0, C, ldc, vecC, epi);
