@@ -20,6 +20,7 @@ template <int N> struct PtrsOut { void* p[N > 0 ? N : 1]; };
 template <typename T, int NIN, int NOUT, typename F, int UNROLL>
 __global__ void __launch_bounds__(256)
 map_kernel(PtrsIn<NIN> in, PtrsOut<NOUT> out, int64_t n, bool vec, F f) {
+  chain_begin();
   constexpr int VEC = Vec16<T>::N;
   using V = typename Vec16<T>::type;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -88,7 +89,7 @@ static prad_status launch_map(prad_ctx* ctx, const void* const (&in)[NIN], void*
   constexpr int UNROLL = 4;
   constexpr int VEC = Vec16<T>::N;
   int grid = stream_grid(ctx, ceil_div(n, VEC * UNROLL), 256, 8);
-  map_kernel<T, NIN, NOUT, F, UNROLL><<<grid, 256, 0, ctx->stream>>>(pi, po, n, vec, f);
+  launch_chained(map_kernel<T, NIN, NOUT, F, UNROLL>, grid, 256, 0, ctx->stream, pi, po, n, vec, f);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
@@ -202,6 +203,7 @@ template <typename T>
 __global__ void __launch_bounds__(1024)
 colsum_short_kernel(const T* __restrict__ x, T* __restrict__ out, int rows, int cols, int accumulate, int64_t x_stride,
                     int64_t out_stride, T scale) {
+  chain_begin();
   x += blockIdx.z * x_stride;
   __shared__ double sm[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -362,7 +364,7 @@ static prad_status add_broadcast_backward_t(prad_ctx* ctx, const void* dy, void*
   if (bands < 1) bands = 1;
   if (bands > 65535) bands = 65535;
   if (rows <= 512) {
-    colsum_short_kernel<T><<<dim3(strips, 1, batch), 1024, 0, ctx->stream>>>((const T*)dy, (T*)dbias, (int)rows, cols, accumulate,
+    launch_chained(colsum_short_kernel<T>, dim3(strips, 1, batch), 1024, 0, ctx->stream, (const T*)dy, (T*)dbias, (int)rows, cols, accumulate,
                                                                             stride, out_stride, scale);
     PRAD_LAUNCHED(ctx);
     return PRAD_OK;

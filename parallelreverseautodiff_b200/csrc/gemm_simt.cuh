@@ -336,6 +336,7 @@ __device__ __forceinline__ void product_tile(const Product<T>& p, int tile, T* s
 template <typename T, typename S, bool TA, bool TB, bool EXACT>
 __global__ void __launch_bounds__(S::THREADS)
 gemm_simt_kernel(const __grid_constant__ Product<T> p) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char simt_smem[];
   product_tile<T, S, TA, TB, EXACT>(p, blockIdx.x, reinterpret_cast<T*>(simt_smem));
 }
@@ -528,6 +529,7 @@ template <> struct SimtShapes<double> {
 template <typename T, typename S, bool EXACT>
 __global__ void __launch_bounds__(S::THREADS)
 gemm_simt_backward_kernel(const __grid_constant__ Product<T> nt, const __grid_constant__ Product<T> tn, int tn_first, int first_tiles) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char simt_smem[];
   T* smem = reinterpret_cast<T*>(simt_smem);
   const int tile = blockIdx.x;
@@ -556,7 +558,7 @@ static prad_status launch_shape(prad_ctx* ctx, bool exact, bool tA, bool tB, int
   do {                                                                                             \
     prad_status st_ = allow_smem<gemm_simt_kernel<T, S, TA_, TB_, EX_>>(ctx, S::SMEM);             \
     if (st_) return st_;                                                                           \
-    gemm_simt_kernel<T, S, TA_, TB_, EX_><<<(unsigned)all, S::THREADS, S::SMEM, ctx->stream>>>(p);      \
+    launch_chained(gemm_simt_kernel<T, S, TA_, TB_, EX_>, (unsigned)all, S::THREADS, S::SMEM, ctx->stream, p);      \
   } while (0)
 #define PRAD_GEMM_FORM(TA_, TB_)                       \
   do {                                                 \
@@ -584,10 +586,10 @@ static prad_status launch_backward(prad_ctx* ctx, bool exact, Product<T> nt, Pro
   const int first = (int)(tn_first ? n_tn : n_nt);
   if (exact) {
     if ((st = allow_smem<gemm_simt_backward_kernel<T, S, true>>(ctx, S::SMEM))) return st;
-    gemm_simt_backward_kernel<T, S, true><<<grid, S::THREADS, S::SMEM, ctx->stream>>>(nt, tn, tn_first, first);
+    launch_chained(gemm_simt_backward_kernel<T, S, true>, grid, S::THREADS, S::SMEM, ctx->stream, nt, tn, tn_first, first);
   } else {
     if ((st = allow_smem<gemm_simt_backward_kernel<T, S, false>>(ctx, S::SMEM))) return st;
-    gemm_simt_backward_kernel<T, S, false><<<grid, S::THREADS, S::SMEM, ctx->stream>>>(nt, tn, tn_first, first);
+    launch_chained(gemm_simt_backward_kernel<T, S, false>, grid, S::THREADS, S::SMEM, ctx->stream, nt, tn, tn_first, first);
   }
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;

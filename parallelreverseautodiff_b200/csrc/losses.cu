@@ -38,6 +38,7 @@ constexpr int LOSS_SMALL_THREADS = 1024, LOSS_SMALL = 16 * LOSS_SMALL_THREADS;
 template <typename T>
 __global__ void __launch_bounds__(LOSS_SMALL_THREADS)
 loss_small_kernel(const T* __restrict__ o, const T* __restrict__ t, T* loss, int n, int kind, T divisor) {
+  chain_begin();
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += LOSS_SMALL_THREADS) acc += (double)loss_term<T>(o[i], t[i], kind);
   const double s = block_sum_d<LOSS_SMALL_THREADS>(acc);
@@ -58,6 +59,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 mse_backward_kernel(const T* __restrict__ o, const T* __restrict__ t, T* __restrict__ g, int64_t n,
                     T scale) {
+  chain_begin();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
     g[i] = mul_rn(scale, sub_rn(o[i], t[i]));
@@ -67,6 +69,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 cce_backward_kernel(const T* __restrict__ o, const T* __restrict__ t, T* __restrict__ g, int64_t n,
                     T scale) {
+  chain_begin();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
     g[i] = div_rn(mul_rn(-scale, t[i]), add_rn(o[i], Eps15<T>::v()));
@@ -78,7 +81,7 @@ static prad_status loss_forward_t(prad_ctx* ctx, const void* o, const void* t, v
   int64_t n = rows * cols;
   const T divisor = kind == 0 ? (T)(rows * cols) : (T)rows;
   if (n <= LOSS_SMALL) {
-    loss_small_kernel<T><<<1, LOSS_SMALL_THREADS, 0, ctx->stream>>>((const T*)o, (const T*)t, (T*)loss, (int)n, kind, divisor);
+    launch_chained(loss_small_kernel<T>, 1, LOSS_SMALL_THREADS, 0, ctx->stream, (const T*)o, (const T*)t, (T*)loss, (int)n, kind, divisor);
     PRAD_LAUNCHED(ctx);
     return PRAD_OK;
   }
@@ -305,9 +308,9 @@ prad_status prad_mse_backward(prad_ctx* ctx, prad_dtype dt, const void* out, con
   PRAD_REQUIRE(out && target && grad, PRAD_ERR_INVALID, "prad_mse_backward: null pointer");
   int grid = stream_grid(ctx, n, 256 * 4, 8);
   if (dt == PRAD_F32)
-    mse_backward_kernel<float><<<grid, 256, 0, ctx->stream>>>((const float*)out, (const float*)target, (float*)grad, n, 2.0f / (float)(rows_total * cols));
+    launch_chained(mse_backward_kernel<float>, grid, 256, 0, ctx->stream, (const float*)out, (const float*)target, (float*)grad, n, 2.0f / (float)(rows_total * cols));
   else
-    mse_backward_kernel<double><<<grid, 256, 0, ctx->stream>>>((const double*)out, (const double*)target, (double*)grad, n, 2.0 / (double)(rows_total * cols));
+    launch_chained(mse_backward_kernel<double>, grid, 256, 0, ctx->stream, (const double*)out, (const double*)target, (double*)grad, n, 2.0 / (double)(rows_total * cols));
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
@@ -322,9 +325,9 @@ prad_status prad_cce_backward(prad_ctx* ctx, prad_dtype dt, const void* out, con
   PRAD_REQUIRE(out && target && grad, PRAD_ERR_INVALID, "prad_cce_backward: null pointer");
   int grid = stream_grid(ctx, n, 256 * 4, 8);
   if (dt == PRAD_F32)
-    cce_backward_kernel<float><<<grid, 256, 0, ctx->stream>>>((const float*)out, (const float*)target, (float*)grad, n, 1.0f / (float)rows_total);
+    launch_chained(cce_backward_kernel<float>, grid, 256, 0, ctx->stream, (const float*)out, (const float*)target, (float*)grad, n, 1.0f / (float)rows_total);
   else
-    cce_backward_kernel<double><<<grid, 256, 0, ctx->stream>>>((const double*)out, (const double*)target, (double*)grad, n, 1.0 / (double)rows_total);
+    launch_chained(cce_backward_kernel<double>, grid, 256, 0, ctx->stream, (const double*)out, (const double*)target, (double*)grad, n, 1.0 / (double)rows_total);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }

@@ -65,6 +65,7 @@ __device__ __forceinline__ int part_at(const MultiTensor& t, int kind) { return 
 template <typename T>
 __global__ void __launch_bounds__(MT_THREADS)
 mt_partial_kernel(MultiTensor t, double* __restrict__ stats, int kind) {
+  chain_begin();
   const int ti = find_tensor(t, blockIdx.x);
   const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
   int64_t end = start + t.chunk;
@@ -169,6 +170,7 @@ template <typename T>
 __global__ void __launch_bounds__(MT_THREADS)
 mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, T clip, T minv,
                 double max_norm, int do_adam, AdamScalars<T> a, int zero_grad, const int* __restrict__ gemm_gave_up) {
+  chain_begin();
   // A tensor-core product on this context ran out of a bounded wait: the gradients on the stream are
   // not valid, so weights, moments and gradients are left exactly as they are (one load per CTA; the
   // host learns of it at its next prad_sync / prad_download, which returns PRAD_ERR_TIMEOUT).
@@ -317,7 +319,7 @@ static prad_status clip_adam_t(prad_ctx* ctx, void* const* w, void* const* g, vo
     for (int first = 0; first < count; first += MT_MAX) {
       int cnt = count - first < MT_MAX ? count - first : MT_MAX;
       int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
-      mt_partial_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, 2);
+      launch_chained(mt_partial_kernel<T>, nb, MT_THREADS, 0, ctx->stream, t, stats, 2);
       PRAD_LAUNCHED(ctx);
       mt_finalize_ss_kernel<<<1, MT_THREADS, 0, ctx->stream>>>(nb, stats, first > 0);
       PRAD_LAUNCHED(ctx);
@@ -328,14 +330,14 @@ static prad_status clip_adam_t(prad_ctx* ctx, void* const* w, void* const* g, vo
     int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
     if (clip_mode == 1) {
       for (int kind = 0; kind < 2; ++kind) {
-        mt_partial_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, kind);
+        launch_chained(mt_partial_kernel<T>, nb, MT_THREADS, 0, ctx->stream, t, stats, kind);
         PRAD_LAUNCHED(ctx);
         if (t.fold) continue;
         mt_finalize_kernel<T><<<cnt, MT_THREADS, 0, ctx->stream>>>(t, stats, kind);
         PRAD_LAUNCHED(ctx);
       }
     }
-    mt_apply_kernel<T><<<nb, MT_THREADS, 0, ctx->stream>>>(t, stats, clip_mode, (T)clip_value,
+    launch_chained(mt_apply_kernel<T>, nb, MT_THREADS, 0, ctx->stream, t, stats, clip_mode, (T)clip_value,
                                                            (T)min_value, clip_value, do_adam, a,
                                                            zero_grad, ctx->tc_err);
     PRAD_LAUNCHED(ctx);

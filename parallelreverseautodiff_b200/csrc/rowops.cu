@@ -282,6 +282,7 @@ constexpr int SR = 4;   // rows per warp pass
 template <typename T, int E>
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 softmax_forward_short(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int cols) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * ROW_WARPS;
@@ -327,6 +328,7 @@ template <typename T, int E>
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 softmax_backward_short(const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx,
                        int64_t rows, int cols) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * ROW_WARPS;
@@ -363,6 +365,7 @@ template <typename T, int E>
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 layernorm_forward_short(const T* __restrict__ x, T* __restrict__ y, T* __restrict__ mean,
                         T* __restrict__ stdv, int64_t rows, int cols) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * ROW_WARPS;
@@ -408,6 +411,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32)
 layernorm_backward_short(const T* __restrict__ x, const T* __restrict__ mean,
                          const T* __restrict__ stdv, const T* __restrict__ dy, T* __restrict__ dx,
                          int64_t rows, int cols) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * ROW_WARPS;
@@ -510,10 +514,10 @@ static inline int short_grid(const prad_ctx* ctx, int64_t rows) {
   do {                                                                                           \
     const int g_ = short_grid(ctx, rows);                                                        \
     switch (short_e(cols)) {                                                                     \
-      case 1: KERNEL<T, 1><<<g_, ROW_WARPS * 32, 0, ctx->stream>>>(__VA_ARGS__); break;          \
-      case 2: KERNEL<T, 2><<<g_, ROW_WARPS * 32, 0, ctx->stream>>>(__VA_ARGS__); break;          \
-      case 4: KERNEL<T, 4><<<g_, ROW_WARPS * 32, 0, ctx->stream>>>(__VA_ARGS__); break;          \
-      default: KERNEL<T, 8><<<g_, ROW_WARPS * 32, 0, ctx->stream>>>(__VA_ARGS__); break;         \
+      case 1: launch_chained(KERNEL<T, 1>, g_, ROW_WARPS * 32, 0, ctx->stream, __VA_ARGS__); break;          \
+      case 2: launch_chained(KERNEL<T, 2>, g_, ROW_WARPS * 32, 0, ctx->stream, __VA_ARGS__); break;          \
+      case 4: launch_chained(KERNEL<T, 4>, g_, ROW_WARPS * 32, 0, ctx->stream, __VA_ARGS__); break;          \
+      default: launch_chained(KERNEL<T, 8>, g_, ROW_WARPS * 32, 0, ctx->stream, __VA_ARGS__); break;         \
     }                                                                                            \
   } while (0)
 
