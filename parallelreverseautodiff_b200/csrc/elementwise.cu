@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(256)
 colsum_partial_kernel(const T* __restrict__ x, double* __restrict__ partial, int64_t rows,
                       int cols, int rows_per_band, T* __restrict__ direct_out, int accumulate, int64_t x_stride = 0,
                       int64_t out_stride = 0, T scale = (T)1) {
+  chain_begin();
   x += blockIdx.z * x_stride;
   if (!direct_out) partial += (int64_t)blockIdx.z * gridDim.y * cols;
   // direct_out: there is one band only (a short matrix) and the sums go straight to the result: one launch
@@ -229,6 +230,7 @@ colsum_short_kernel(const T* __restrict__ x, T* __restrict__ out, int rows, int 
 template <typename T>
 __global__ void colsum_final_kernel(const double* __restrict__ partial, T* __restrict__ out,
                                     int cols, int bands, int accumulate, int64_t out_stride = 0, T scale = (T)1) {
+  chain_begin();
   int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= cols) return;
   partial += (int64_t)blockIdx.z * bands * cols;
@@ -250,6 +252,7 @@ template <typename T, bool CTA_SUM>
 __global__ void __launch_bounds__(256)
 colsum_flat_partial_kernel(const T* __restrict__ x, double* __restrict__ partial, int64_t nvec,
                            int64_t stride_threads, int vec_per_row) {
+  chain_begin();
   constexpr int VEC = Vec16<T>::N;
   using V = typename Vec16<T>::type;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -301,6 +304,7 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 colsum_flat_final_kernel(const double* __restrict__ partial, T* __restrict__ out, int vec_per_row,
                          int64_t stride_threads, int accumulate) {
+  chain_begin();
   constexpr int VEC = Vec16<T>::N;
   __shared__ double sm[4][VEC];
   const int group = blockIdx.x;            // column group = VEC consecutive columns
@@ -343,15 +347,15 @@ static prad_status add_broadcast_backward_t(prad_ctx* ctx, const void* dy, void*
       if (s) return s;
       const int64_t ctas = ceil_div(threads, 256);
       if (vec_per_row <= 256)
-        colsum_flat_partial_kernel<T, true><<<(unsigned)ctas, 256, 0, ctx->stream>>>((const T*)dy, (double*)ctx->ws, nvec,
+        launch_chained(colsum_flat_partial_kernel<T, true>, (unsigned)ctas, 256, 0, ctx->stream, (const T*)dy, (double*)ctx->ws, nvec,
                                                                                    threads, vec_per_row);
       else
-        colsum_flat_partial_kernel<T, false><<<(unsigned)ctas, 256, 0, ctx->stream>>>((const T*)dy, (double*)ctx->ws, nvec,
+        launch_chained(colsum_flat_partial_kernel<T, false>, (unsigned)ctas, 256, 0, ctx->stream, (const T*)dy, (double*)ctx->ws, nvec,
                                                                                     threads, vec_per_row);
       PRAD_LAUNCHED(ctx);
       // entries the final pass adds per column group: one per CTA, or one per thread for very wide rows
       const int64_t entries = vec_per_row <= 256 ? ctas * vec_per_row : threads;
-      colsum_flat_final_kernel<T><<<vec_per_row, 128, 0, ctx->stream>>>((const double*)ctx->ws, (T*)dbias,
+      launch_chained(colsum_flat_final_kernel<T>, vec_per_row, 128, 0, ctx->stream, (const double*)ctx->ws, (T*)dbias,
                                                                       vec_per_row, entries, accumulate);
       PRAD_LAUNCHED(ctx);
       return PRAD_OK;
@@ -372,18 +376,17 @@ static prad_status add_broadcast_backward_t(prad_ctx* ctx, const void* dy, void*
   int rows_per_band = (int)ceil_div(rows, bands);
   bands = (int)ceil_div(rows, rows_per_band);
   if (bands == 1) {
-    colsum_partial_kernel<T><<<dim3(strips, 1, batch), 256, 0, ctx->stream>>>((const T*)dy, nullptr, rows, cols, rows_per_band,
+    launch_chained(colsum_partial_kernel<T>, dim3(strips, 1, batch), 256, 0, ctx->stream, (const T*)dy, nullptr, rows, cols, rows_per_band,
                                                                              (T*)dbias, accumulate, stride, out_stride, scale);
     PRAD_LAUNCHED(ctx);
     return PRAD_OK;
   }
   prad_status s = ensure_workspace(ctx, (size_t)batch * bands * cols * sizeof(double));
   if (s) return s;
-  colsum_partial_kernel<T><<<dim3(strips, bands, batch), 256, 0, ctx->stream>>>(
-      (const T*)dy, (double*)ctx->ws, rows, cols, rows_per_band, nullptr, 0, stride);
+  launch_chained(colsum_partial_kernel<T>, dim3(strips, bands, batch), 256, 0, ctx->stream, (const T*)dy, (double*)ctx->ws, rows, cols, rows_per_band, nullptr, 0, stride,
+                 (int64_t)0, (T)1);
   PRAD_LAUNCHED(ctx);
-  colsum_final_kernel<T><<<dim3((unsigned)ceil_div(cols, 32), 1, batch), 32, 0, ctx->stream>>>(
-      (const double*)ctx->ws, (T*)dbias, cols, bands, accumulate, out_stride, scale);
+  launch_chained(colsum_final_kernel<T>, dim3((unsigned)ceil_div(cols, 32), 1, batch), 32, 0, ctx->stream, (const double*)ctx->ws, (T*)dbias, cols, bands, accumulate, out_stride, scale);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
@@ -433,6 +436,7 @@ __device__ __forceinline__ T nary_combine(const T (&v)[PRAD_MAX_SRCS], int count
 template <typename T, int U, int S>
 __global__ void __launch_bounds__(256)
 nary_sum_kernel(SrcTable t, T* out, int64_t n, int mode, T inv_count, bool vec) {
+  chain_begin();
   // `out` is not restrict-qualified: with more than PRAD_MAX_SRCS sources the running sum is read back
   // through the source table (every thread loads its element before it stores it).
   // U vectors per thread and trip and at most S sources (few sources: more trips' loads in flight).
@@ -503,9 +507,9 @@ static prad_status nary_t(prad_ctx* ctx, const void* const* srcs, int count, voi
     bool vec = ((uintptr_t)out & 15) == 0;
     for (int g = 0; g < t.count; ++g) vec = vec && (((uintptr_t)t.p[g] & 15) == 0);
     const T scale = (mode == 1 && last) ? inv : (T)1;
-    if (t.count <= 2) nary_sum_kernel<T, 4, 2><<<grid, 256, 0, ctx->stream>>>(t, (T*)out, n, m, scale, vec);
-    else if (t.count <= 4) nary_sum_kernel<T, 2, 4><<<grid, 256, 0, ctx->stream>>>(t, (T*)out, n, m, scale, vec);
-    else nary_sum_kernel<T, 1, PRAD_MAX_SRCS><<<grid, 256, 0, ctx->stream>>>(t, (T*)out, n, m, scale, vec);
+    if (t.count <= 2) launch_chained(nary_sum_kernel<T, 4, 2>, grid, 256, 0, ctx->stream, t, (T*)out, n, m, scale, vec);
+    else if (t.count <= 4) launch_chained(nary_sum_kernel<T, 2, 4>, grid, 256, 0, ctx->stream, t, (T*)out, n, m, scale, vec);
+    else launch_chained(nary_sum_kernel<T, 1, PRAD_MAX_SRCS>, grid, 256, 0, ctx->stream, t, (T*)out, n, m, scale, vec);
     PRAD_LAUNCHED(ctx);
     first = false;
   }

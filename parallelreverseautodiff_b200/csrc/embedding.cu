@@ -18,6 +18,7 @@ template <typename T, bool VECTORS>
 __global__ void __launch_bounds__(EMB_THREADS)
 embedding_gather_kernel(const T* __restrict__ index_col, const T* __restrict__ W, T* __restrict__ out, int n, int vocab, int dim,
                         int* bad) {
+  chain_begin();
   using V = typename std::conditional<VECTORS, typename EmbVec<T>::type, T>::type;
   const int lane = threadIdx.x & 31;
   const int vecs = VECTORS ? dim / EmbVec<T>::N : dim;
@@ -69,6 +70,7 @@ struct EmbPlan {
 template <typename T>
 __global__ void __launch_bounds__(EMB_THREADS)
 emb_count_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab, int* bad) {
+  chain_begin();
   for (int i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += gridDim.x * EMB_THREADS) {
     const int idx = (int)index_col[i];
     if (idx < 0 || idx >= vocab) *(volatile int*)bad = i + 1;
@@ -77,6 +79,7 @@ emb_count_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab, i
 }
 __global__ void __launch_bounds__(EMB_THREADS)
 emb_place_kernel(EmbPlan p, int vocab) {
+  chain_begin();
   const int v = blockIdx.x * EMB_THREADS + threadIdx.x, lane = threadIdx.x & 31;
   const int c = v < vocab ? p.count[v] : 0;
   int incl = c;
@@ -94,6 +97,7 @@ emb_place_kernel(EmbPlan p, int vocab) {
 template <typename T>
 __global__ void __launch_bounds__(EMB_THREADS)
 emb_fill_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab) {
+  chain_begin();
   for (int i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += gridDim.x * EMB_THREADS) {
     const int idx = (int)index_col[i];
     if (idx >= 0 && idx < vocab) p.list[p.offset[idx] + p.slot[i]] = i;
@@ -178,6 +182,7 @@ template <typename T, typename V> __device__ __forceinline__ V emb_zero() {
 template <typename T, bool VECTORS>
 __global__ void __launch_bounds__(EMB_THREADS)
 emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n, int vocab, int dim, int hot_ctas) {
+  chain_begin();
   using V = typename std::conditional<VECTORS, typename EmbVec<T>::type, T>::type;
   const int vecs = VECTORS ? dim / EmbVec<T>::N : dim;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -319,12 +324,12 @@ static prad_status scatter_t(prad_ctx* ctx, const void* index_col, const void* d
     if (checked) PRAD_CUDA(cudaEventRecord(checked, ctx->stream));       // `bad` is known
   } else if (n > 0) {
     const int g = stream_grid(ctx, n, EMB_THREADS, 8);
-    emb_count_kernel<T><<<g, EMB_THREADS, 0, ctx->stream>>>(idx, p, n, vocab, bad);
+    launch_chained(emb_count_kernel<T>, g, EMB_THREADS, 0, ctx->stream, idx, p, n, vocab, bad);
     PRAD_LAUNCHED(ctx);
     if (checked) PRAD_CUDA(cudaEventRecord(checked, ctx->stream));       // `bad` is known
-    emb_place_kernel<<<(unsigned)ceil_div(vocab, EMB_THREADS), EMB_THREADS, 0, ctx->stream>>>(p, vocab);
+    launch_chained(emb_place_kernel, (unsigned)ceil_div(vocab, EMB_THREADS), EMB_THREADS, 0, ctx->stream, p, vocab);
     PRAD_LAUNCHED(ctx);
-    emb_fill_kernel<T><<<g, EMB_THREADS, 0, ctx->stream>>>(idx, p, n, vocab);
+    launch_chained(emb_fill_kernel<T>, g, EMB_THREADS, 0, ctx->stream, idx, p, n, vocab);
     PRAD_LAUNCHED(ctx);
   }
   const int hot = n > EMB_FEW ? 2 * ctx->sm_count : 0;
@@ -334,12 +339,12 @@ static prad_status scatter_t(prad_ctx* ctx, const void* index_col, const void* d
     constexpr int ring = EMB_CHUNKS * EMB_CHUNK * EMB_GROUP * 16;
     s = allow_smem<emb_sum_kernel<T, true>>(ctx, ring);
     if (s) return s;
-    emb_sum_kernel<T, true><<<grid, EMB_THREADS, hot ? ring : 0, ctx->stream>>>((const T*)dOut, (T*)dW, p, n, vocab, dim, hot);
+    launch_chained(emb_sum_kernel<T, true>, grid, EMB_THREADS, hot ? ring : 0, ctx->stream, (const T*)dOut, (T*)dW, p, n, vocab, dim, hot);
   } else {
     constexpr int ring = EMB_CHUNKS * EMB_CHUNK * EMB_GROUP * (int)sizeof(T);
     s = allow_smem<emb_sum_kernel<T, false>>(ctx, ring);
     if (s) return s;
-    emb_sum_kernel<T, false><<<grid, EMB_THREADS, hot ? ring : 0, ctx->stream>>>((const T*)dOut, (T*)dW, p, n, vocab, dim, hot);
+    launch_chained(emb_sum_kernel<T, false>, grid, EMB_THREADS, hot ? ring : 0, ctx->stream, (const T*)dOut, (T*)dW, p, n, vocab, dim, hot);
   }
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
@@ -366,9 +371,9 @@ template <typename T>
 static prad_status gather_t(prad_ctx* ctx, const void* index_col, const void* W, void* out, int n, int vocab, int dim) {
   const int grid = stream_grid(ctx, n, EMB_WARPS, 8);
   if (dim % EmbVec<T>::N == 0 && (((uintptr_t)W | (uintptr_t)out) & 15) == 0)
-    embedding_gather_kernel<T, true><<<grid, EMB_THREADS, 0, ctx->stream>>>((const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag);
+    launch_chained(embedding_gather_kernel<T, true>, grid, EMB_THREADS, 0, ctx->stream, (const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag);
   else
-    embedding_gather_kernel<T, false><<<grid, EMB_THREADS, 0, ctx->stream>>>((const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag);
+    launch_chained(embedding_gather_kernel<T, false>, grid, EMB_THREADS, 0, ctx->stream, (const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }

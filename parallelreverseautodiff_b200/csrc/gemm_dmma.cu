@@ -161,6 +161,7 @@ __device__ __forceinline__ void tile_of(const Problem& pr, int tile, double* sme
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(THREADS, 2)
 gemm_kernel(const __grid_constant__ Problem p) {
+  chain_begin();
   extern __shared__ __align__(16) double dmma_smem[];
   tile_of<TA, TB>(p, blockIdx.x, dmma_smem);
 }
@@ -168,6 +169,7 @@ gemm_kernel(const __grid_constant__ Problem p) {
 // dA = dC*B^T and dB = A^T*dC of one Backward (see gemm_simt_backward_kernel)
 __global__ void __launch_bounds__(THREADS, 2)
 backward_kernel(const __grid_constant__ Problem nt, const __grid_constant__ Problem tn, int tn_first, int first_tiles) {
+  chain_begin();
   extern __shared__ __align__(16) double dmma_smem[];
   const bool first = (int)blockIdx.x < first_tiles;
   const int local = first ? blockIdx.x : blockIdx.x - first_tiles;
@@ -179,6 +181,7 @@ backward_kernel(const __grid_constant__ Problem nt, const __grid_constant__ Prob
 __global__ void __launch_bounds__(256)
 combine_kernel(const double* __restrict__ part, int splits, int64_t mn, int N, double* __restrict__ C, int64_t ldc, int64_t sC,
                double alpha, double beta) {
+  chain_begin();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   part += (int64_t)blockIdx.y * splits * mn;      // blockIdx.y = batch
   C += (int64_t)blockIdx.y * sC;
@@ -231,7 +234,7 @@ static prad_status launch(prad_ctx* ctx, bool tA, bool tB, const Problem& pr, in
 #define PRAD_DMMA(TA_, TB_)                                                                        \
   do {                                                                                             \
     if ((st = allow_smem<gemm_kernel<TA_, TB_>>(ctx, SMEM))) return st;                            \
-    gemm_kernel<TA_, TB_><<<(unsigned)tiles, THREADS, SMEM, ctx->stream>>>(pr);                    \
+    launch_chained(gemm_kernel<TA_, TB_>, (unsigned)tiles, THREADS, SMEM, ctx->stream, pr);                    \
   } while (0)
   if (!tA && !tB) PRAD_DMMA(false, false);
   else if (!tA && tB) PRAD_DMMA(false, true);
@@ -279,8 +282,7 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
       pr.p.vecC = N % 2 == 0 && mn % 2 == 0;
       if ((st = dm::launch(ctx, tA, tB, pr, tiles * S))) return st;
       const int cg = stream_grid(ctx, mn, 256, 8);
-      dm::combine_kernel<<<dim3((unsigned)cg, sum ? 1u : (unsigned)batch), 256, 0, ctx->stream>>>(
-          part, sum ? S * batch : S, mn, N, (double*)C, ldc, sC, alpha, beta);
+      launch_chained(dm::combine_kernel, dim3((unsigned)cg, sum ? 1u : (unsigned)batch), 256, 0, ctx->stream, part, sum ? S * batch : S, mn, N, (double*)C, ldc, sC, alpha, beta);
       PRAD_LAUNCHED(ctx);
       return PRAD_OK;
     }
@@ -303,7 +305,7 @@ prad_status gemm_f64_dmma_backward(prad_ctx* ctx, const void* A, const void* B, 
   if (!st) st = allow_smem<dm::backward_kernel>(ctx, dm::SMEM);
   if (st) return st;
   const int tn_first = tn.p.K >= nt.p.K;      // the longer tiles start first
-  dm::backward_kernel<<<(unsigned)(n_nt + n_tn), dm::THREADS, dm::SMEM, ctx->stream>>>(nt, tn, tn_first, (int)(tn_first ? n_tn : n_nt));
+  launch_chained(dm::backward_kernel, (unsigned)(n_nt + n_tn), dm::THREADS, dm::SMEM, ctx->stream, nt, tn, tn_first, (int)(tn_first ? n_tn : n_nt));
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }

@@ -1654,6 +1654,7 @@ template <int V>
 __global__ void __launch_bounds__(256)
 splitk_combine_kernel(const float* __restrict__ part, int splits, int64_t mn, int M, int N,
                       float* __restrict__ C, int64_t ldc, float alpha, float beta) {
+  chain_begin();
   constexpr int U = 8;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x * V;
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V; i < mn; i += stride) {
@@ -1707,6 +1708,7 @@ splitk_combine_kernel(const float* __restrict__ part, int splits, int64_t mn, in
 // elements -- warp w adds slices w, w + 8, ... in order -- and the first adds the eight sums.
 __global__ void __launch_bounds__(256)
 splitk_combine_many_kernel(const float* __restrict__ part, int splits, int64_t mn, int N, float* __restrict__ C, int64_t ldc, float alpha, float beta) {
+  chain_begin();
   __shared__ float4 sm[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t i = ((int64_t)blockIdx.x * 32 + lane) * 4;
@@ -1743,13 +1745,13 @@ static void launch_splitk_combine(prad_ctx* ctx, const float* part, int splits, 
                                   int64_t ldc, float alpha, float beta) {
   const bool vec = N % 4 == 0 && ldc % 4 == 0 && (((uintptr_t)C | (uintptr_t)part) & 15) == 0;
   if (vec && splits >= 16 && mn <= (1 << 18)) {
-    splitk_combine_many_kernel<<<(unsigned)ceil_div(mn, 128), 256, 0, ctx->stream>>>(part, splits, mn, N, C, ldc, alpha, beta);
+    launch_chained(splitk_combine_many_kernel, (unsigned)ceil_div(mn, 128), 256, 0, ctx->stream, part, splits, mn, N, C, ldc, alpha, beta);
   } else if (vec) {
     const int cg = stream_grid(ctx, mn / 4, 256, 8);
-    splitk_combine_kernel<4><<<cg, 256, 0, ctx->stream>>>(part, splits, mn, M, N, C, ldc, alpha, beta);
+    launch_chained(splitk_combine_kernel<4>, cg, 256, 0, ctx->stream, part, splits, mn, M, N, C, ldc, alpha, beta);
   } else {
     const int cg = stream_grid(ctx, mn, 256, 8);
-    splitk_combine_kernel<1><<<cg, 256, 0, ctx->stream>>>(part, splits, mn, M, N, C, ldc, alpha, beta);
+    launch_chained(splitk_combine_kernel<1>, cg, 256, 0, ctx->stream, part, splits, mn, M, N, C, ldc, alpha, beta);
   }
 }
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -191,6 +191,7 @@ __device__ __forceinline__ void layernorm_rows(float (&v)[U][4], bool inside, in
 template <int OP, bool ROWS, bool COLS, int NT, bool EDGE>
 __global__ void __launch_bounds__(NT, NT == 512 ? 2 : (OP == 0 ? 5 : 3))
 pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_r0, int tile_c0, int R, int C) {
+  chain_begin();
   constexpr int T = 128, U = OP == 14 ? 1 : 2, NW = NT / 32, NB = T / NW / U;      // NW warps, each takes every NW-th tile row
   constexpr bool HAS_DY = OP >= 4 && OP != 9 && OP != 12, HAS_TG = OP == 7 || OP == 8 || OP == 11 || OP == 14;
   extern __shared__ float stash[];       // [T][T] when COLS
@@ -340,6 +341,7 @@ pack_fast_kernel(PackSource src, PackedForm fr, PackedForm fc, int tile_r0, int 
 // out[c] = sum of the partial column sums, in a fixed order: 32 warps share the rows of 32 columns
 __global__ void __launch_bounds__(1024)
 column_sum_kernel(const double* __restrict__ part, float* __restrict__ out, int rows, int C) {
+  chain_begin();
   __shared__ double sm[32][33];
   constexpr int U = 12;                 // loads in flight per thread: 1568 partial rows are four trips
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
@@ -387,7 +389,7 @@ static prad_status launch_fast(prad_ctx* ctx, const PackSource& src, const Packe
   }
   auto launch = [&](auto edge, unsigned x, unsigned y, unsigned r0, unsigned c0) -> prad_status {
     if (x == 0 || y == 0) return PRAD_OK;
-    pack_fast_kernel<OP, ROWS, COLS, NT, decltype(edge)::value><<<dim3(x, y), NT, smem, ctx->stream>>>(src, fr, fc, (int)r0, (int)c0, R, C);
+    launch_chained(pack_fast_kernel<OP, ROWS, COLS, NT, decltype(edge)::value>, dim3(x, y), NT, smem, ctx->stream, src, fr, fc, (int)r0, (int)c0, R, C);
     PRAD_LAUNCHED(ctx);
     return PRAD_OK;
   };
@@ -417,6 +419,7 @@ static int fast_op_of(const PackSource& s) {
 template <int TR, int TC>
 __global__ void __launch_bounds__(256)
 pack_tile_kernel(PackSource src, bool vec, int R, int C, PackedForm fr, PackedForm fc) {
+  chain_begin();
   constexpr int W = TC / 128;            // float4 per lane and tile row
   constexpr int STRIDE = TC + 4;         // stash pitch in floats (16-byte multiple; see pass 2)
   constexpr int U = 4;                   // tile rows a warp loads before it starts converting
@@ -526,6 +529,7 @@ pack_tile_kernel(PackSource src, bool vec, int R, int C, PackedForm fr, PackedFo
 // 32 operand rows (by columns: its lanes are the rows, its warps share the k), every load in flight at once: 4 us.
 __global__ void __launch_bounds__(256)
 pack_small_rows_kernel(const float* __restrict__ x, int64_t ld, PackedForm f) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
   const int c0 = blockIdx.x * 128 + lane * 4;
@@ -552,6 +556,7 @@ pack_small_rows_kernel(const float* __restrict__ x, int64_t ld, PackedForm f) {
 }
 __global__ void __launch_bounds__(256)
 pack_small_cols_kernel(const float* __restrict__ x, int64_t ld, PackedForm f) {
+  chain_begin();
   __shared__ uint32_t part[8][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t r = (int64_t)blockIdx.y * 32 + lane;        // operand row = matrix column
@@ -584,11 +589,11 @@ pack_small_cols_kernel(const float* __restrict__ x, int64_t ld, PackedForm f) {
 }
 static prad_status launch_small(prad_ctx* ctx, const PackSource& src, const PackedForm* by_rows, const PackedForm* by_cols) {
   if (by_rows) {
-    pack_small_rows_kernel<<<dim3((unsigned)by_rows->nchunk, (unsigned)ceil_div(by_rows->rows, 8)), 256, 0, ctx->stream>>>(src.x, src.ld, *by_rows);
+    launch_chained(pack_small_rows_kernel, dim3((unsigned)by_rows->nchunk, (unsigned)ceil_div(by_rows->rows, 8)), 256, 0, ctx->stream, src.x, src.ld, *by_rows);
     PRAD_LAUNCHED(ctx);
   }
   if (by_cols) {
-    pack_small_cols_kernel<<<dim3((unsigned)by_cols->nchunk, (unsigned)ceil_div(by_cols->rows, 32)), 256, 0, ctx->stream>>>(src.x, src.ld, *by_cols);
+    launch_chained(pack_small_cols_kernel, dim3((unsigned)by_cols->nchunk, (unsigned)ceil_div(by_cols->rows, 32)), 256, 0, ctx->stream, src.x, src.ld, *by_cols);
     PRAD_LAUNCHED(ctx);
   }
   return PRAD_OK;
@@ -616,7 +621,7 @@ static prad_status launch_pack(prad_ctx* ctx, const PackSource& src, bool vec, i
   const int64_t cols_cover = fr.h ? (fr.kp > C ? fr.kp : C) : C;
   dim3 grid((unsigned)ceil_div(cols_cover, TC), (unsigned)ceil_div(rows_cover, TR));
   PRAD_REQUIRE(grid.y <= 65535, PRAD_ERR_UNSUPPORTED, "operand packing: too many row tiles (%u)", grid.y);
-  pack_tile_kernel<TR, TC><<<grid, 256, smem, ctx->stream>>>(src, vec, R, C, fr, fc);
+  launch_chained(pack_tile_kernel<TR, TC>, grid, 256, smem, ctx->stream, src, vec, R, C, fr, fc);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
@@ -780,7 +785,7 @@ static prad_status pack_into(prad_packed* p, PackSource src) {
   if (s) return s;
   p->filled = true;
   if (part_rows) {
-    pk::column_sum_kernel<<<(unsigned)ceil_div(p->cols, 32), 1024, 0, p->ctx->stream>>>(src.colsum, p->column_sums, part_rows, p->cols);
+    launch_chained(pk::column_sum_kernel, (unsigned)ceil_div(p->cols, 32), 1024, 0, p->ctx->stream, src.colsum, p->column_sums, part_rows, p->cols);
     PRAD_LAUNCHED(p->ctx);
   }
   return PRAD_OK;

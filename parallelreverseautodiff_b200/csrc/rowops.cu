@@ -461,6 +461,7 @@ __global__ void __launch_bounds__(256)
 layernorm_backward_flat(const T* __restrict__ x, const T* __restrict__ mean, const T* __restrict__ stdv,
                         const T* __restrict__ dy, const T* __restrict__ res, T* __restrict__ dx, int64_t nvec, int vec_per_row,
                         int cols) {
+  chain_begin();
   constexpr int VEC = RowVec<T>::N;
   using V = typename RowVec<T>::type;
   constexpr int U = 4;   // vectors in flight per thread
@@ -610,8 +611,8 @@ prad_status prad_layernorm_backward(prad_ctx* ctx, prad_dtype dt, const void* x,
   if (cols % vecn == 0 && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) & 15) == 0) {
     const int64_t nvec = rows * (cols / vecn);
     const int grid = stream_grid(ctx, ceil_div(nvec, 4), 256, 8);
-    if (dt == PRAD_F32) layernorm_backward_flat<float, false><<<grid, 256, 0, ctx->stream>>>((const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, nullptr, (float*)dx, nvec, cols / vecn, cols);
-    else layernorm_backward_flat<double, false><<<grid, 256, 0, ctx->stream>>>((const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, nullptr, (double*)dx, nvec, cols / vecn, cols);
+    if (dt == PRAD_F32) launch_chained(layernorm_backward_flat<float, false>, grid, 256, 0, ctx->stream, (const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, nullptr, (float*)dx, nvec, cols / vecn, cols);
+    else launch_chained(layernorm_backward_flat<double, false>, grid, 256, 0, ctx->stream, (const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, nullptr, (double*)dx, nvec, cols / vecn, cols);
   } else if (short_e(cols)) {
     if (dt == PRAD_F32) PRAD_SHORT_ROWS(layernorm_backward_short, float, (const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, (float*)dx, rows, cols);
     else PRAD_SHORT_ROWS(layernorm_backward_short, double, (const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, (double*)dx, rows, cols);
@@ -632,8 +633,8 @@ prad_status prad_layernorm_backward_add(prad_ctx* ctx, prad_dtype dt, const void
   if (cols % vecn == 0 && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx | (uintptr_t)residual) & 15) == 0) {
     const int64_t nvec = rows * (cols / vecn);
     const int grid = stream_grid(ctx, ceil_div(nvec, 4), 256, 8);
-    if (dt == PRAD_F32) layernorm_backward_flat<float, true><<<grid, 256, 0, ctx->stream>>>((const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, (const float*)residual, (float*)dx, nvec, cols / vecn, cols);
-    else layernorm_backward_flat<double, true><<<grid, 256, 0, ctx->stream>>>((const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, (const double*)residual, (double*)dx, nvec, cols / vecn, cols);
+    if (dt == PRAD_F32) launch_chained(layernorm_backward_flat<float, true>, grid, 256, 0, ctx->stream, (const float*)x, (const float*)mean, (const float*)stdv, (const float*)dy, (const float*)residual, (float*)dx, nvec, cols / vecn, cols);
+    else launch_chained(layernorm_backward_flat<double, true>, grid, 256, 0, ctx->stream, (const double*)x, (const double*)mean, (const double*)stdv, (const double*)dy, (const double*)residual, (double*)dx, nvec, cols / vecn, cols);
     PRAD_LAUNCHED(ctx);
     return PRAD_OK;
   }

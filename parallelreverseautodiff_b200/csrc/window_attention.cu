@@ -150,6 +150,7 @@ template <int R, int C> __device__ __forceinline__ void clear(float (&a)[R][C]) 
 template <int T, int HD>
 __global__ void __launch_bounds__(NT)
 forward_kernel(const float* __restrict__ qkv, float* __restrict__ P, float* __restrict__ out, int ws, int heads, float scale) {
+  chain_begin();
   using S = Shape<T, HD>;
   extern __shared__ __align__(16) float wa_smem[];
   const int dim = heads * HD, ps = score_pitch(ws), ty = threadIdx.x >> 3, tx = threadIdx.x & 7;
@@ -205,6 +206,7 @@ template <int T, int HD>
 __global__ void __launch_bounds__(NT)
 backward_kernel(const float* __restrict__ qkv, const float* __restrict__ P, const float* __restrict__ d_out, float* __restrict__ d_qkv,
                 int ws, int heads, float scale) {
+  chain_begin();
   using S = Shape<T, HD>;
   extern __shared__ __align__(16) float wa_smem[];
   const int dim = heads * HD, ps = score_pitch(ws), ty = threadIdx.x >> 3, tx = threadIdx.x & 7;
@@ -278,8 +280,8 @@ template <int T, int HD> static prad_status launch(prad_ctx* ctx, const Call& c)
   constexpr int most = 100 * 1024;
   prad_status st = c.backward ? allow_smem<backward_kernel<T, HD>>(ctx, most) : allow_smem<forward_kernel<T, HD>>(ctx, most);
   if (st) return st;
-  if (c.backward) backward_kernel<T, HD><<<grid, NT, smem, ctx->stream>>>(c.qkv, c.P_in, c.d_out, c.d_qkv, c.ws, c.heads, c.scale);
-  else forward_kernel<T, HD><<<grid, NT, smem, ctx->stream>>>(c.qkv, c.P, c.out, c.ws, c.heads, c.scale);
+  if (c.backward) launch_chained(backward_kernel<T, HD>, grid, NT, smem, ctx->stream, c.qkv, c.P_in, c.d_out, c.d_qkv, c.ws, c.heads, c.scale);
+  else launch_chained(forward_kernel<T, HD>, grid, NT, smem, ctx->stream, c.qkv, c.P, c.out, c.ws, c.heads, c.scale);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
