@@ -803,17 +803,23 @@ class SwinBlock:
         ln2 = self._packed("ln2", T, d).column_sums(None).layernorm(x, self.mu2, self.sd2, residual=proj, sum_out=self.r1)
         self.z1 = e.gemm_packed(ln2, rows, self._weight("W1", True), cols, self._buf("z1", (T, h)), bias=p["b1"])
         a1 = self._packed("a1", T, h).column_sums(None).act_forward(E.ACT_GELU, self.z1)
+        self._replaced = False           # whether a backward has put gradients where ln2 and a1 are
         m2 = e.gemm_packed(a1, rows, self._weight("W2", True), cols, self._buf("branch", (T, d)), bias=p["b2"])
         self.out = e.add_forward(self.r1, m2, out=new(T, d))
         return self.out
 
     def _backward_packed(self, d_out):
         """The gradients likewise, with the bias gradients (column sums) out of the same passes.  A gradient takes the place of
-        the activation of its shape that has just been read for the last time."""
+        the activation of its shape that has just been read for the last time; a further backward of the same forward packs
+        those activations again first."""
         e, d, h, g = self.eng, self.dim, self.hidden, self.g
         T = d_out.shape[0]
         rows, cols, B_ = E.PACK_ROWS, E.PACK_COLS, self._buf
         op = lambda name, w: self._packed(name, T, w)  # noqa: E731
+        if self._replaced:
+            op("ln2", d).column_sums(None).layernorm(self.r1, self.mu2, self.sd2)
+            op("a1", h).column_sums(None).act_forward(E.ACT_GELU, self.z1)
+        self._replaced = True
         narrow, qkv = op("d narrow", d), op("d qkv", 3 * d)
         narrow.column_sums(g["b2"]).pack(d_out)                       # out = r1 + m2 : both receive d_out
         e.gemm_packed(op("a1", h), cols, narrow, cols, g["W2"])
@@ -840,7 +846,8 @@ class SwinBlock:
         T = x.shape[0]
         nw = T // ws
         self.x, self.nw = x, nw
-        if self._wants_packed(T):
+        self._packed_state = self._wants_packed(T) and x.ptr % 16 == 0
+        if self._packed_state:
             return self._forward_packed(x)
         self.ln1, self.mu1, self.sd1 = e.layernorm_forward(x)
         self.qkv = e.matmul_forward(self.ln1, self.p["Wqkv"], bias=self.p["bqkv"])
@@ -858,8 +865,14 @@ class SwinBlock:
         e, d, ws, H, hd, nw = self.eng, self.dim, self.ws, self.heads, self.hd, self.nw
         g, p = self.g, self.p
         T = d_out.shape[0]
-        if self._wants_packed(T):
-            return self._backward_packed(d_out)
+        if self._packed_state:
+            if self._wants_packed(T) and d_out.ptr % 16 == 0:
+                return self._backward_packed(d_out)
+            # another choice of product kernels since the forward, or a gradient the packing passes cannot take
+            self.ln1, self.mu1, self.sd1 = e.layernorm_forward(self.x)
+            self.ln2, self.mu2, self.sd2 = e.layernorm_forward(self.r1)
+            self.a1 = e.act_forward(E.ACT_GELU, self.z1)
+            self._packed_state = False
         # out = r1 + m2 : both receive d_out (MatrixAddOperation.Backward)
         e.add_broadcast_backward(d_out, dbias=g["b2"])
         B_ = self._buf
