@@ -360,7 +360,9 @@ template <typename T> static Plan plan_of(int nh) {
   return best;
 }
 
-// Clusters of this kernel that fit the device at once; 0 if none does.  Asked once per kernel, cluster size and device.
+// Clusters of this kernel that fit the device at once; 0 if none does.  Asked once per kernel, cluster size and device.  (A kernel
+// serves several cluster sizes, and what it may use of shared memory is a property of the kernel: the most there is, for all.)
+constexpr int MOST_SMEM = 227 * 1024;
 template <auto Kernel> static int clusters_at_once(prad_ctx* ctx, int cs, int nt, size_t smem) {
   static std::atomic<int> known[64][5];
   int lg = 0;
@@ -369,7 +371,7 @@ template <auto Kernel> static int clusters_at_once(prad_ctx* ctx, int cs, int nt
   int n = k.load(std::memory_order_acquire);
   if (n) return n - 1;
   n = 0;
-  cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM);
   if (e == cudaSuccess && cs > 8) e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
@@ -433,7 +435,7 @@ static prad_status run_jp(prad_ctx* ctx, const Plan& pl, Args& a) {
   } while (0)
 #define PRAD_LSTM_WEIGH(BB_)                                                                                           \
   PRAD_LSTM_TILE(BB_, {                                                                                                \
-    const int fit = smem <= 227 * 1024 ? clusters_at_once<K>(ctx, pl.cs, L::NT, smem) : 0;                             \
+    const int fit = smem <= MOST_SMEM ? clusters_at_once<K>(ctx, pl.cs, L::NT, smem) : 0;                             \
     const int n = fit > 0 ? (int)ceil_div(tiles, fit) : 0;                                                             \
     if (n && (!turns || n < turns)) { turns = n; rows = BB_; }                                                         \
   })

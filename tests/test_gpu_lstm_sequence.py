@@ -1,5 +1,7 @@
 """prad_lstm_forward / prad_lstm_backward (all time steps in one launch) against the operations one by one, bit for bit:
 hidden sizes on both sides of every tile and cluster size, batches of one to several tiles and turns."""
+import multiprocessing
+
 import numpy as np
 import pytest
 
@@ -77,3 +79,39 @@ def test_sequence_equals_the_operations(engine, dtype, nh, B, T):
     _backward_by_step(b)
     for g in a.GATES:
         np.testing.assert_array_equal(a.dpre[g].numpy(), b.dpre[g].numpy(), err_msg="dpre " + g)
+
+
+def _take_turns(dtype, sizes):
+    """Steps of networks of these sizes one after another; a later step of a network repeats its first one."""
+    T, B, n_in = 3, 33, 5
+    with E.Engine(0) as engine:
+        nets, first = {}, {}
+        for nh in sizes:
+            r = rng(nh)
+            x, y = r.standard_normal((T, B, n_in)).astype(dtype), r.standard_normal((T, B, nh)).astype(dtype)
+            if nh not in nets:
+                nets[nh] = LstmNetwork(engine, dtype, n_in, nh, T, B)
+                nets[nh].set_parameters(*[{g: (r.standard_normal(s) * 0.2).astype(dtype) for g in LstmNetwork.GATES}
+                                          for s in ((nh, n_in), (nh, nh), (nh,))])
+            net = nets[nh]
+            n0 = engine.launch_count()
+            net.forward(x, y)
+            net.backward()
+            got = [net.H.numpy(), net.dX.numpy()] + [net.dU[g].numpy() for g in net.GATES]
+            launches = engine.launch_count() - n0
+            if nh in first:
+                assert launches == first[nh][1]
+                for a, b in zip(got, first[nh][0]):
+                    np.testing.assert_array_equal(a, b)
+            first.setdefault(nh, (got, launches))
+        del nets, net
+
+
+@pytest.mark.parametrize("dtype,sizes", [("float64", (128, 64, 128)), ("float32", (128, 64, 128)), ("float64", (192, 96, 192))])
+def test_networks_of_different_sizes_take_turns(dtype, sizes):
+    """One kernel serves several cluster sizes: a small network between two steps of a large one changes nothing.  In a process
+    of its own, whose first launches of these kernels are the ones here."""
+    p = multiprocessing.get_context("spawn").Process(target=_take_turns, args=(np.dtype(dtype), sizes))
+    p.start()
+    p.join(120)
+    assert p.exitcode == 0
