@@ -591,6 +591,7 @@ prad_status prad_graph_forward(prad_graph* g) {
     if ((!w.tried || w.nodes != g->nodes.size()) && !g->ctx->capturing) {
       std::vector<Prim> ops;
       G_TRY(forward_walk(g, Ops{g->ctx, g->dt, &ops}));
+      if (w.plan && g->ctx->live_sequences > 0) g->retired.push_back(std::move(w.plan));     // a recording may run it
       w.plan = graph_plan_build(g->ctx, g->dt, ops);
       w.tried = true;
       w.nodes = g->nodes.size();

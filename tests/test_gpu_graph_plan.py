@@ -103,3 +103,40 @@ def test_products_sums_and_elementwise_chains_are_the_same_bits(engine, dtype):
             engine.set_option("graph_plan", "1")
     for a, b in zip(*results):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_a_recorded_walk_survives_the_growth_of_its_graph(engine, dtype):
+    """A recording of the forward keeps running the plan it was made with after nodes were added and the graph planned anew."""
+    n, r = 24, rng(8)
+    x = engine.upload(r.standard_normal((n, n)).astype(dtype))
+    g = Graph(engine, dtype)
+    w, h = g.input(engine.upload((r.standard_normal((n, n)) * 0.3).astype(dtype))), g.input(x)
+
+    def layer(h):
+        m = g.node("MatrixMultiplyOperation", [w, h])
+        return g.node("MatrixAddOperation", [h, g.node("HadamardProductOperation", [g.node("TanhOperation", [m]), g.node("SigmoidOperation", [m])])])
+
+    for _ in range(6):
+        h = layer(h)
+    g.forward()
+    seq = engine.record(g.forward)
+    assert seq.launches == 1
+    end = h
+    for _ in range(4):
+        h = layer(h)
+        g.forward()
+    junk = [engine.zeros((n, n), dtype) for _ in range(64)]            # whatever was freed is in use again
+    want = []
+    for k in range(3):
+        engine.upload((rng(20 + k).standard_normal((n, n))).astype(dtype), out=x)
+        g.forward()
+        want.append((g.data(end).numpy(), g.data(h).numpy()))
+    for k in range(3):
+        engine.upload((rng(20 + k).standard_normal((n, n))).astype(dtype), out=x)
+        seq.launch()
+        np.testing.assert_array_equal(g.data(end).numpy(), want[k][0])
+        np.testing.assert_array_equal(g.data(h).numpy(), want[-1][1])  # the new nodes are not part of the recording
+    assert not any(m.numpy().any() for m in junk)
+    seq.close()
+    g.close()
