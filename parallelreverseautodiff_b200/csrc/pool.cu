@@ -135,6 +135,9 @@ prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out) {
 prad_status pool_free(prad_ctx* ctx, void* p) {
   std::lock_guard<std::mutex> lock(g_pool_mu);
   auto it = g_live.find(p);
+  if (it == g_live.end())
+    for (prad_ctx* c : g_pools)
+      PRAD_REQUIRE(!c->pool->cached.count(p), PRAD_ERR_CUDA, "prad_free: the block at %p was freed before", p);
   const size_t bytes = it == g_live.end() ? 0 : it->second.bytes;
   const bool own = it != g_live.end() && it->second.owner == ctx;
   if (it != g_live.end()) g_live.erase(it);

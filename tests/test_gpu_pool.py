@@ -56,3 +56,19 @@ def test_blocks_cross_contexts_and_recordings():
         np.testing.assert_array_equal(seq_out[0].numpy(), 3.0 * a)
         np.testing.assert_array_equal(junk[5].numpy(), 5.0 * a)
         seq.close()
+
+
+def test_a_block_is_freed_once():
+    a = np.arange(3000, dtype=np.float32)
+    with E.Engine(0) as e1, E.Engine(0) as e2:
+        m = e1.upload(a)
+        p = m.ptr
+        m.free()
+        for eng in (e1, e2):                                     # the owner again, and another context
+            with pytest.raises(E._lib.PradError, match="freed before"):
+                E.check(eng.lib.prad_free(eng.ctx, p))
+        n = e1.upload(a)                                         # the block is whole, and still given out once
+        assert n.ptr == p
+        k = e1.upload(a + 1)
+        assert k.ptr != p
+        np.testing.assert_array_equal(n.numpy(), a)
