@@ -192,7 +192,8 @@ prad_status prad_download(prad_ctx* ctx, void* dst_host, const void* src, size_t
  * kernels enqueued earlier (or later) on the compute stream execute; prad_upload_join makes
  * the compute stream wait for every prefetch issued so far.  src_host must be page-locked
  * (prad_alloc_host) and stay untouched until the join; dst must not be in use by work that is
- * still running on the compute stream (use a second buffer). */
+ * still running on the compute stream (use a second buffer).  A block that prad_alloc has just returned is not: the first
+ * prefetch into one that the context kept from an earlier prad_free waits for that one's work by itself. */
 prad_status prad_upload_prefetch(prad_ctx* ctx, void* dst, const void* src_host, size_t bytes);
 prad_status prad_upload_join(prad_ctx* ctx);
 /* Prefetches issued from here on start after everything the compute stream was given before this call: a destination which that

@@ -369,6 +369,7 @@ prad_status prad_upload_prefetch(prad_ctx* ctx, void* dst, const void* src_host,
   PRAD_REQUIRE((dst && src_host) || bytes == 0, PRAD_ERR_INVALID, "prad_upload_prefetch: null pointer");
   if (bytes == 0) return PRAD_OK;
   prad_status s = ensure_copy_stream(ctx);
+  if (!s) s = pool_before_prefetch(ctx, dst, bytes);
   if (s) return s;
   PRAD_CUDA(cudaMemcpyAsync(dst, src_host, bytes, cudaMemcpyHostToDevice, ctx->copy_stream));
   ctx->copy_pending = true;

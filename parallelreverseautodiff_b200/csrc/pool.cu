@@ -12,11 +12,14 @@
 //    waited for as well (an event per cached block), as the cudaFree before it did;
 //  - a block that another context frees, or that is freed while a prefetch copy is pending or on a
 //    context with data-parallel communication, takes the old path: wait and cudaFree;
+//  - a prefetch, which runs beside the context's stream, into a block that came out of the cache starts
+//    behind what that stream was given before (the first one does: later ones are ordered behind it);
 //  - nothing is taken from the cache while a launch sequence is recorded;
 //  - the cache of a context is bounded (1/16 of the device memory; the block that was freed first
 //    leaves first), and is given back when the context is shut down, when any allocation of this
 //    process' contexts fails for lack of memory, or by the option "pool_bytes" = "0".
 #include <deque>
+#include <map>
 #include <mutex>
 #include <unordered_map>
 
@@ -39,9 +42,10 @@ struct DevicePool {
 };
 
 namespace {
-struct Live { size_t bytes; prad_ctx* owner; };
+// recycled: came out of the cache, and no prefetch has been ordered behind its old work yet
+struct Live { size_t bytes; prad_ctx* owner; bool recycled; };
 std::mutex g_pool_mu;
-std::unordered_map<void*, Live> g_live;       // every block prad_alloc handed out
+std::map<void*, Live> g_live;                 // every block prad_alloc handed out
 std::vector<prad_ctx*> g_pools;               // contexts that have a cache
 
 size_t size_class(size_t bytes) {
@@ -117,7 +121,7 @@ prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out) {
     pool->held -= b.bytes;
     pool->cached.erase(b.p);
     pool->spare.push_back(b.freed);
-    g_live[b.p] = {want, ctx};
+    g_live[b.p] = {want, ctx, true};
     *out = b.p;
     return PRAD_OK;
   }
@@ -128,7 +132,7 @@ prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out) {
     set_error("prad_alloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? PRAD_ERR_OOM : PRAD_ERR_CUDA;
   }
-  g_live[*out] = {want, ctx};
+  g_live[*out] = {want, ctx, false};
   return PRAD_OK;
 }
 
@@ -172,6 +176,20 @@ prad_status pool_free(prad_ctx* ctx, void* p) {
   }
   PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
   PRAD_CUDA(cudaFree(p));
+  return PRAD_OK;
+}
+
+prad_status pool_before_prefetch(prad_ctx* ctx, void* dst, size_t bytes) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  auto it = g_live.upper_bound(dst);
+  if (it != g_live.begin()) --it;
+  for (; it != g_live.end() && (char*)it->first < (char*)dst + bytes; ++it) {
+    if (!it->second.recycled || (char*)it->first + it->second.bytes <= (char*)dst) continue;
+    it->second.recycled = false;
+    if (!it->second.owner) continue;          // its context is gone, and had waited for its work
+    PRAD_CUDA(cudaEventRecord(ctx->copy_done, it->second.owner->stream));
+    PRAD_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_done, 0));
+  }
   return PRAD_OK;
 }
 

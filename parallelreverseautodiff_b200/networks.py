@@ -512,6 +512,7 @@ class FeedForwardNetwork:
             self._in = [self.A[0], e.empty(self.A[0].shape, self.dtype)]
             self._tg = [self.target, e.empty(self.target.shape, self.dtype)]
             self._stage_rows = rows
+        e.upload_fence()                          # earlier steps may still read these buffers
         e.upload_prefetch(batches[0][0], self._in[0])
         e.upload_prefetch(batches[0][1], self._tg[0])
         for i in range(len(batches)):

@@ -72,3 +72,36 @@ def test_a_block_is_freed_once():
         k = e1.upload(a + 1)
         assert k.ptr != p
         np.testing.assert_array_equal(n.numpy(), a)
+
+
+def _long_work(eng, x, w, y):
+    """y = the sum of 40 products of x, some tens of milliseconds; x is read to the end."""
+    eng.zero_(y)
+    for _ in range(40):
+        eng.gemm(x, w, y, beta=1.0)
+
+
+@pytest.mark.parametrize("offset", [0, 4096])
+def test_a_prefetch_into_a_recycled_block_waits_for_its_old_work(offset):
+    n, r = 2048, np.random.default_rng(1)
+    with E.Engine(0) as eng:
+        a, w = r.standard_normal((n, n)), eng.upload(r.standard_normal((n, n)))
+        want, y = eng.empty((n, n), np.float64), eng.empty((n, n), np.float64)
+        x = eng.upload(a)
+        _long_work(eng, x, w, want)
+        want = want.numpy()
+        src = eng.pinned_empty((n * n - offset,), np.float64)
+        src[:] = r.standard_normal(src.size)
+        for _ in range(2):                        # the second time round the copy stream is there
+            _long_work(eng, x, w, y)
+            p = x.ptr
+            x.free()
+            new = eng.empty((n, n), np.float64)
+            assert new.ptr == p
+            part = new.view((n * n - offset,), offset)
+            eng.upload_prefetch(src, part)
+            eng.upload_join()
+            np.testing.assert_array_equal(y.numpy(), want)
+            np.testing.assert_array_equal(part.numpy(), src)
+            x = new
+            eng.upload(a, out=x)
