@@ -105,6 +105,7 @@ prad_status prad_init(int device, prad_ctx** out_ctx) {
     delete c;
     return PRAD_ERR_CUDA;
   }
+  pool_enter(c);
   *out_ctx = c;
   g_err[0] = 0;
   return PRAD_OK;
@@ -258,7 +259,7 @@ prad_status prad_use_stream(prad_ctx* ctx, void* stream) {
   PRAD_CHECK_CTX(ctx);
   PRAD_NOT_CAPTURING(ctx, "prad_use_stream");
   PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
-  ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;
+  pool_use_stream(ctx, stream ? (cudaStream_t)stream : ctx->own_stream);
   return PRAD_OK;
 }
 
@@ -431,7 +432,7 @@ prad_status prad_capture_begin(prad_ctx* ctx) {
   PRAD_CHECK_CTX(ctx);
   PRAD_REQUIRE(!ctx->capturing, PRAD_ERR_INVALID, "prad_capture_begin: a recording is already open");
   PRAD_REQUIRE(!ctx->copy_pending, PRAD_ERR_INVALID, "prad_capture_begin: join the pending prefetch first");
-  PRAD_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
+  PRAD_CUDA(pool_begin_capture(ctx));
   ctx->capturing = true;
   ctx->capture_launches0 = ctx->launches;
   return PRAD_OK;

@@ -182,7 +182,11 @@ prad_status pool_before_prefetch(prad_ctx* ctx, void* dst, size_t bytes);
 void pool_limit(prad_ctx* ctx, size_t cap);   // most bytes this context keeps
 // cudaMalloc; when memory is short every context's cached blocks go back to the device first
 cudaError_t device_malloc(void** out, size_t bytes);
+void pool_enter(prad_ctx* ctx);
 void pool_destroy(prad_ctx* ctx);
+// what the other contexts' frees look at changes under the cache's lock
+void pool_use_stream(prad_ctx* ctx, cudaStream_t stream);
+cudaError_t pool_begin_capture(prad_ctx* ctx);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -10,8 +10,11 @@
 //    back to the context that allocated them, whose stream orders their old work before their new work;
 //  - work on the legacy default stream and on blocking streams that was enqueued before the free is
 //    waited for as well (an event per cached block), as the cudaFree before it did;
-//  - a block that another context frees, or that is freed while a prefetch copy is pending or on a
-//    context with data-parallel communication, takes the old path: wait and cudaFree;
+//  - while a context shares its device with others of the process, blocks may be used by all of them: a
+//    free notes how far every one's stream is, and a block is handed out again when all of that is done
+//    (the host waits; the block that was freed first is taken), so that no context finds work pending on it;
+//  - a block that another context frees, or that is freed while a prefetch copy is pending, while another
+//    context records or on a context with data-parallel communication, takes the old path: wait and cudaFree;
 //  - a prefetch, which runs beside the context's stream, into a block that came out of the cache starts
 //    behind what that stream was given before (the first one does: later ones are ordered behind it);
 //  - nothing is taken from the cache while a launch sequence is recorded;
@@ -31,6 +34,7 @@ struct CachedBlock {
   void* p;
   size_t bytes;
   cudaEvent_t freed;   // on the legacy default stream
+  std::vector<cudaEvent_t> users;   // on the context's stream and those of the others on its device, if there were any
 };
 
 struct DevicePool {
@@ -42,11 +46,25 @@ struct DevicePool {
 };
 
 namespace {
-// recycled: came out of the cache, and no prefetch has been ordered behind its old work yet
+// recycled: came out of the cache with its old work ahead of it on the owner's stream, and no prefetch has been ordered behind its old work yet
 struct Live { size_t bytes; prad_ctx* owner; bool recycled; };
 std::mutex g_pool_mu;
 std::map<void*, Live> g_live;                 // every block prad_alloc handed out
+std::vector<prad_ctx*> g_contexts;            // every context
 std::vector<prad_ctx*> g_pools;               // contexts that have a cache
+
+std::vector<prad_ctx*> others_on_device(const prad_ctx* ctx) {
+  std::vector<prad_ctx*> out;
+  for (prad_ctx* c : g_contexts)
+    if (c != ctx && c->device == ctx->device) out.push_back(c);
+  return out;
+}
+bool recording(cudaStream_t stream) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return true;
+}
 
 size_t size_class(size_t bytes) {
   if (bytes <= 256) return 256;
@@ -70,6 +88,7 @@ void drop_block(DevicePool* pool, const CachedBlock& b) {
   pool->held -= b.bytes;
   pool->cached.erase(b.p);
   pool->spare.push_back(b.freed);
+  pool->spare.insert(pool->spare.end(), b.users.begin(), b.users.end());
   cudaFree(b.p);       // waits for the device: whatever still uses the block is done
 }
 
@@ -108,20 +127,29 @@ cudaError_t malloc_or_release(void** out, size_t bytes) {
 
 prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out) {
   const size_t want = size_class(bytes);
-  std::lock_guard<std::mutex> lock(g_pool_mu);
+  std::unique_lock<std::mutex> lock(g_pool_mu);
   DevicePool* pool = pool_of(ctx);
   auto it = pool->by_size.find(want);
   if (!ctx->capturing && it != pool->by_size.end() && !it->second.empty()) {
-    const CachedBlock b = it->second.back();      // the one freed last: likeliest in L2
-    it->second.pop_back();
-    if (cudaEventQuery(b.freed) != cudaSuccess) {
+    const bool alone = others_on_device(ctx).empty();
+    const size_t at = alone ? it->second.size() - 1 : 0;      // the one freed last: likeliest in L2
+    const CachedBlock b = it->second[at];
+    it->second.erase(it->second.begin() + at);
+    pool->held -= b.bytes;
+    pool->cached.erase(b.p);
+    const bool idle = !alone || !b.users.empty();
+    if (idle) {
+      lock.unlock();
+      PRAD_CUDA(cudaEventSynchronize(b.freed));
+      for (cudaEvent_t e : b.users) PRAD_CUDA(cudaEventSynchronize(e));
+      lock.lock();
+    } else if (cudaEventQuery(b.freed) != cudaSuccess) {
       (void)cudaGetLastError();
       PRAD_CUDA(cudaStreamWaitEvent(ctx->stream, b.freed, 0));
     }
-    pool->held -= b.bytes;
-    pool->cached.erase(b.p);
     pool->spare.push_back(b.freed);
-    g_live[b.p] = {want, ctx, true};
+    pool->spare.insert(pool->spare.end(), b.users.begin(), b.users.end());
+    g_live[b.p] = {want, ctx, !idle};
     *out = b.p;
     return PRAD_OK;
   }
@@ -146,16 +174,28 @@ prad_status pool_free(prad_ctx* ctx, void* p) {
   const bool own = it != g_live.end() && it->second.owner == ctx;
   if (it != g_live.end()) g_live.erase(it);
   DevicePool* pool = own ? pool_of(ctx) : nullptr;
-  if (own && bytes <= pool->cap / 4 && !ctx->copy_pending && !ctx->dp) {
-    CachedBlock b{p, bytes, nullptr};
-    cudaError_t e = cudaSuccess;
-    if (!pool->spare.empty()) {
-      b.freed = pool->spare.back();
-      pool->spare.pop_back();
-    } else {
-      e = cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming);
-    }
-    if (e == cudaSuccess) e = cudaEventRecord(b.freed, cudaStreamLegacy);
+  bool keep = own && bytes <= pool->cap / 4 && !ctx->copy_pending && !ctx->dp;
+  std::vector<cudaStream_t> streams;           // of everybody who may use the block, where that is not this context alone
+  for (const prad_ctx* c : others_on_device(ctx)) {
+    streams.push_back(c->stream);
+    keep = keep && !c->copy_pending && !c->dp && !recording(streams.back());
+  }
+  if (!streams.empty()) streams.push_back(ctx->stream);
+  if (keep) {
+    CachedBlock b{p, bytes, nullptr, {}};
+    auto mark = [&](cudaStream_t stream, cudaEvent_t* out) {
+      cudaError_t e = cudaSuccess;
+      if (!pool->spare.empty()) {
+        *out = pool->spare.back();
+        pool->spare.pop_back();
+      } else {
+        e = cudaEventCreateWithFlags(out, cudaEventDisableTiming);
+      }
+      return e == cudaSuccess ? cudaEventRecord(*out, stream) : e;
+    };
+    cudaError_t e = mark(cudaStreamLegacy, &b.freed);
+    b.users.assign(streams.size(), nullptr);
+    for (size_t i = 0; i < streams.size() && e == cudaSuccess; ++i) e = mark(streams[i], &b.users[i]);
     if (e == cudaSuccess) {
       pool->by_size[bytes].push_back(b);
       pool->order.push_back(p);
@@ -172,7 +212,9 @@ prad_status pool_free(prad_ctx* ctx, void* p) {
       return PRAD_OK;
     }
     (void)cudaGetLastError();
-    if (b.freed) pool->spare.push_back(b.freed);
+    b.users.push_back(b.freed);
+    for (cudaEvent_t u : b.users)
+      if (u) pool->spare.push_back(u);
   }
   PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
   PRAD_CUDA(cudaFree(p));
@@ -204,9 +246,32 @@ cudaError_t device_malloc(void** out, size_t bytes) {
   return malloc_or_release(out, bytes);
 }
 
+// called by prad_init.  What the others on the device freed so far was kept on the understanding that they use their blocks
+// alone: from here on none of those is handed out, and none they hold has old work pending.
+void pool_enter(prad_ctx* ctx) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  for (prad_ctx* c : others_on_device(ctx)) {
+    shrink(c, 0);
+    if (!recording(c->stream)) cudaStreamSynchronize(c->stream);
+    for (auto& kv : g_live)
+      if (kv.second.owner == c) kv.second.recycled = false;
+  }
+  g_contexts.push_back(ctx);
+}
+void pool_use_stream(prad_ctx* ctx, cudaStream_t stream) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ctx->stream = stream;
+}
+cudaError_t pool_begin_capture(prad_ctx* ctx) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  return cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed);
+}
+
 // called by prad_shutdown: cached blocks are freed, blocks still held by the caller stay valid
 void pool_destroy(prad_ctx* ctx) {
   std::lock_guard<std::mutex> lock(g_pool_mu);
+  for (size_t i = 0; i < g_contexts.size(); ++i)
+    if (g_contexts[i] == ctx) { g_contexts.erase(g_contexts.begin() + i); break; }
   for (auto& kv : g_live)
     if (kv.second.owner == ctx) kv.second.owner = nullptr;
   if (!ctx->pool) return;

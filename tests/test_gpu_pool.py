@@ -1,4 +1,6 @@
 """Reuse of freed device blocks (prad_alloc / prad_free): contents, size classes, recordings, limits."""
+import multiprocessing
+
 import numpy as np
 import pytest
 
@@ -81,8 +83,7 @@ def _long_work(eng, x, w, y):
         eng.gemm(x, w, y, beta=1.0)
 
 
-@pytest.mark.parametrize("offset", [0, 4096])
-def test_a_prefetch_into_a_recycled_block_waits_for_its_old_work(offset):
+def _prefetch_into_a_recycled_block(offset):
     n, r = 2048, np.random.default_rng(1)
     with E.Engine(0) as eng:
         a, w = r.standard_normal((n, n)), eng.upload(r.standard_normal((n, n)))
@@ -105,3 +106,61 @@ def test_a_prefetch_into_a_recycled_block_waits_for_its_old_work(offset):
             np.testing.assert_array_equal(part.numpy(), src)
             x = new
             eng.upload(a, out=x)
+        for m in (x, w, y):
+            m.free()
+
+
+@pytest.mark.parametrize("offset", [0, 4096])
+def test_a_prefetch_into_a_recycled_block_waits_for_its_old_work(offset):
+    """In a process of its own: with several contexts on the device a recycled block has no old work pending."""
+    p = multiprocessing.get_context("spawn").Process(target=_prefetch_into_a_recycled_block, args=(offset,))
+    p.start()
+    p.join(120)
+    assert p.exitcode == 0
+
+
+def test_a_block_that_another_context_still_reads_is_not_handed_out():
+    """The owner frees a matrix that another context's queued work reads, and goes on allocating."""
+    n, r = 2048, np.random.default_rng(2)
+    a, b = r.standard_normal((n, n)), r.standard_normal((n, n))
+    with E.Engine(0) as e1, E.Engine(0) as e2:
+        w, y = e2.upload(r.standard_normal((n, n))), e2.empty((n, n), np.float64)
+        m = e1.upload(a)
+        e1.sync()
+        theirs = E.DeviceMatrix(e2, m.ptr, m.shape, m.dtype, owned=False)
+        _long_work(e2, theirs, w, y)
+        want = y.numpy()
+        for _ in range(3):
+            _long_work(e2, theirs, w, y)
+            m.free()
+            m = e1.upload(b)                      # may be the same block
+            np.testing.assert_array_equal(y.numpy(), want)
+            np.testing.assert_array_equal(m.numpy(), b)
+            e1.upload(a, out=m)
+            e1.sync()
+            theirs.ptr = m.ptr
+
+
+def test_another_context_may_use_a_new_block_at_once():
+    """A block that its owner's queued work still writes is freed, allocated again and given to another context."""
+    n, r = 2048, np.random.default_rng(3)
+    b = r.standard_normal((n, n))
+    with E.Engine(0) as e1:
+        x, w = e1.upload(r.standard_normal((n, n))), e1.upload(r.standard_normal((n, n)))
+        early = e1.empty((n, n), np.float64)
+        _long_work(e1, x, w, early)
+        early.free()
+        early = e1.empty((n, n), np.float64)      # recycled while the context may be alone
+        with E.Engine(0) as e2:
+            for new in (early, None, None):
+                if new is None:
+                    y = e1.empty((n, n), np.float64)
+                    _long_work(e1, x, w, y)
+                    y.free()
+                    new = e1.empty((n, n), np.float64)
+                theirs = E.DeviceMatrix(e2, new.ptr, new.shape, new.dtype, owned=False)
+                e2.upload(b, out=theirs)
+                e2.sync()
+                e1.sync()
+                np.testing.assert_array_equal(theirs.numpy(), b)
+                new.free()
