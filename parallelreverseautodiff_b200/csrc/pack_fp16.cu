@@ -766,6 +766,8 @@ prad_status prad_packed_create(prad_ctx* ctx, int rows, int cols, int forms, int
 
 prad_status prad_packed_destroy(prad_packed* p) {
   PRAD_CHECK_PACKED(p, "prad_packed_destroy");
+  PRAD_CHECK_CTX(p->ctx);
+  PRAD_NOT_CAPTURING(p->ctx, "prad_packed_destroy");
   free_form(p->ctx, p->by_rows);
   free_form(p->ctx, p->by_cols);
   p->magic = 0;

@@ -149,7 +149,7 @@ class PackedOperand:
 
     def free(self) -> None:
         if self.handle and self.engine is not None and self.engine.ctx:
-            self.engine.lib.prad_packed_destroy(self.handle)
+            self.engine._destroy_packed(self.handle)
         self.handle = None
 
     def __del__(self):
@@ -224,7 +224,7 @@ class Engine:
         `fn()` once unrecorded first so that library scratch has its final size."""
         check(self.lib.prad_capture_begin(self.ctx))
         self._record_keep = keep = []
-        self._deferred_free = []
+        self._deferred_free, self._deferred_packed = [], []
         try:
             fn()
         except BaseException:
@@ -279,10 +279,19 @@ class Engine:
             return
         check(self.lib.prad_free(self.ctx, C.c_void_p(ptr)))
 
+    def _destroy_packed(self, handle) -> None:
+        if getattr(self, "_record_keep", None) is not None:    # likewise
+            self._deferred_packed.append(handle)
+            return
+        check(self.lib.prad_packed_destroy(handle))
+
     def _flush_deferred_free(self) -> None:
         pending, self._deferred_free = self._deferred_free, []
+        packed, self._deferred_packed = self._deferred_packed, []
         for ptr in pending:
             check(self.lib.prad_free(self.ctx, C.c_void_p(ptr)))
+        for handle in packed:
+            check(self.lib.prad_packed_destroy(handle))
 
     def upload(self, a: np.ndarray, out: Optional[DeviceMatrix] = None) -> DeviceMatrix:
         a = np.ascontiguousarray(a)

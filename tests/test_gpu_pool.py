@@ -164,3 +164,28 @@ def test_another_context_may_use_a_new_block_at_once():
                 e1.sync()
                 np.testing.assert_array_equal(theirs.numpy(), b)
                 new.free()
+
+
+def test_a_packed_operand_dropped_while_recording_is_destroyed_afterwards():
+    """As prad_free: its blocks go back to the cache when the recording is closed, and the library refuses to do it before."""
+    n, f = 256, np.float32
+    a = np.random.default_rng(4).standard_normal((n, n)).astype(f)
+    with E.Engine(0) as eng:
+        x, out = eng.upload(a), eng.empty((n, n), f)
+        ops = [eng.packed(n, n, E.PACK_ROWS | E.PACK_COLS).pack(x)]
+        eng.gemm_packed(ops[0], E.PACK_ROWS, ops[0], E.PACK_COLS, out)
+        want = out.numpy()
+
+        def step():
+            with pytest.raises(E._lib.PradError, match="cannot be recorded"):
+                E.check(eng.lib.prad_packed_destroy(ops[0].handle))
+            eng.gemm_packed(ops[0], E.PACK_ROWS, ops[0], E.PACK_COLS, out)
+            ops.pop().free()
+            assert len(eng._deferred_packed) == 1
+
+        eng.zero_(out)
+        seq = eng.record(step)
+        assert seq.launches >= 1 and not eng._deferred_packed
+        assert not out.numpy().any()
+        np.testing.assert_allclose(want, a @ a, atol=1e-5 * np.abs(a).max() ** 2 * n)
+        seq.close()
