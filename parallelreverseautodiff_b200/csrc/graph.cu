@@ -44,14 +44,14 @@ struct prad_graph {
   std::vector<prad::GValue> values;
   std::vector<prad::GNode> nodes;
   std::vector<void*> owned;    // every device block the graph allocated
-  // Walks made into plans (graph_plan.cu).  A plan holds for the nodes it was made from; a backward also for its start values
-  // and their gradients, of which the last few sets are kept.
+  // Walks made into plans (graph_plan.cu).  A plan holds for the nodes it was made from; a backward also for its start values,
+  // of which a number of sets are kept (further ones run one launch per operation).  Whose matrices the start gradients are is
+  // said at every run.
   struct Walk {
     bool tried = false;
     size_t nodes = 0;
     std::vector<int> starts;
-    std::vector<const void*> d_starts;
-    std::vector<void*> grads;         // what the walk leaves in the values
+    std::vector<void*> grads;         // what the walk leaves in the values (a start gradient by its stand-in)
     std::vector<int> consumers;
     prad::GraphPlanPtr plan;          // null: one launch per operation is better
   };
@@ -64,7 +64,7 @@ struct prad_graph {
 
 namespace prad {
 
-constexpr size_t KEPT_BACKWARD_WALKS = 4;
+constexpr size_t KEPT_BACKWARD_WALKS = 16;
 
 // The operations of a walk: launched one by one, or written down (`rec`) for a plan.
 struct Ops {
@@ -616,33 +616,40 @@ prad_status prad_graph_backward_multi(prad_graph* g, const int* start_values, co
   }
   PRAD_CHECK_CTX(g->ctx);
   if (!may_plan(g->ctx)) return backward_walk(g, start_values, d_starts, count, Ops{g->ctx, g->dt, nullptr});
+  auto& walks = g->backward_walks;
   prad_graph::Walk* w = nullptr;
-  bool hopeless = false;              // the same walk with other gradients was better launched one by one
-  for (auto& k : g->backward_walks)
-    if (k.nodes == g->nodes.size() && k.starts.size() == (size_t)count && std::equal(k.starts.begin(), k.starts.end(), start_values) && !k.plan)
-      hopeless = true;
-  for (auto& k : g->backward_walks)
-    if (k.nodes == g->nodes.size() && k.starts.size() == (size_t)count && std::equal(k.starts.begin(), k.starts.end(), start_values) &&
-        std::equal(k.d_starts.begin(), k.d_starts.end(), d_starts))
-      w = &k;
-  if (!w && !hopeless && !g->ctx->capturing) {
-    std::vector<Prim> ops;
-    G_TRY(backward_walk(g, start_values, d_starts, count, Ops{g->ctx, g->dt, &ops}));
-    if (g->backward_walks.size() >= KEPT_BACKWARD_WALKS) {
-      if (g->ctx->live_sequences > 0) g->retired.push_back(std::move(g->backward_walks.front().plan));
-      g->backward_walks.erase(g->backward_walks.begin());
+  for (auto& k : walks)
+    if (k.nodes == g->nodes.size() && k.starts.size() == (size_t)count && std::equal(k.starts.begin(), k.starts.end(), start_values)) w = &k;
+  if (!w && !g->ctx->capturing && count <= MOST_STARTS) {
+    for (size_t i = walks.size(); i-- > 0;)
+      if (walks[i].nodes != g->nodes.size()) {          // of a graph that has grown since
+        if (walks[i].plan && g->ctx->live_sequences > 0) g->retired.push_back(std::move(walks[i].plan));
+        walks.erase(walks.begin() + i);
+      }
+    if (walks.size() < KEPT_BACKWARD_WALKS) {
+      std::vector<const void*> stand_ins(count);
+      for (int i = 0; i < count; ++i) stand_ins[i] = start_stand_in(i);
+      std::vector<Prim> ops;
+      G_TRY(backward_walk(g, start_values, stand_ins.data(), count, Ops{g->ctx, g->dt, &ops}));
+      walks.emplace_back();
+      w = &walks.back();
+      w->nodes = g->nodes.size();
+      w->starts.assign(start_values, start_values + count);
+      for (const GValue& v : V) { w->grads.push_back(v.grad); w->consumers.push_back(v.consumers); }
+      w->plan = graph_plan_build(g->ctx, g->dt, ops);
     }
-    g->backward_walks.emplace_back();
-    w = &g->backward_walks.back();
-    w->nodes = g->nodes.size();
-    w->starts.assign(start_values, start_values + count);
-    w->d_starts.assign(d_starts, d_starts + count);
-    for (const GValue& v : V) { w->grads.push_back(v.grad); w->consumers.push_back(v.consumers); }
-    w->plan = graph_plan_build(g->ctx, g->dt, ops);
   }
-  if (!w || !w->plan) return backward_walk(g, start_values, d_starts, count, Ops{g->ctx, g->dt, nullptr});
-  for (size_t i = 0; i < w->grads.size(); ++i) { V[i].grad = w->grads[i]; V[i].consumers = w->consumers[i]; }
-  return graph_plan_run(g->ctx, w->plan.get());
+  // (a start gradient in memory that the walk writes is read when its turn comes: that needs the operations one by one)
+  bool planned = w && w->plan;
+  for (int i = 0; i < count && planned; ++i)
+    planned = !graph_plan_writes(w->plan.get(), d_starts[i], (size_t)V[start_values[i]].count() * dtype_size(g->dt));
+  if (!planned) return backward_walk(g, start_values, d_starts, count, Ops{g->ctx, g->dt, nullptr});
+  for (size_t i = 0; i < w->grads.size(); ++i) {
+    void* const grad = w->grads[i];
+    V[i].grad = is_stand_in(grad) ? const_cast<void*>(d_starts[stand_in_index(grad)]) : grad;
+    V[i].consumers = w->consumers[i];
+  }
+  return graph_plan_run(g->ctx, w->plan.get(), d_starts, count);
 }
 
 static prad_status backward_walk(prad_graph* g, const int* start_values, const void* const* d_starts, int count, const Ops& ops) {

@@ -64,6 +64,14 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" 
 // a worker's threads meet
 __device__ __forceinline__ void worker_sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)(threadIdx.x / NT)), "n"(NT) : "memory"); }
 
+// The start gradients of this run; most walks have few, and short arguments launch faster.
+template <int N> struct StartTable { const void* p[N]; };
+constexpr int FEW_STARTS = 64;
+template <typename T, int N> __device__ __forceinline__ const T* source(const void* p, const StartTable<N>& starts) {
+  const uint64_t a = (uint64_t)p;
+  return (const T*)((a >> 62) == 1 ? starts.p[(a >> 40) & 0x3fffff] : p);
+}
+
 // ---- elementwise programs
 // One instruction on one element; v[slot * stride] is the element's value in a slot.
 template <typename T>
@@ -100,8 +108,8 @@ __device__ __forceinline__ void execute(const Ins& c, T* v, int stride) {
 
 // A piece: 256 elements, one per thread, or 64 elements with four threads each, which take the loads, the instructions of a
 // phase and the stores in turn (four gates' exponentials side by side instead of one after another).
-template <typename T>
-__device__ void run_elementwise(const Head* h, int chunk, T* v) {
+template <typename T, int N>
+__device__ void run_elementwise(const Head* h, int chunk, T* v, const StartTable<N>& starts) {
   const int tid = threadIdx.x % NT, team = (int)h->team;
   const int per = NT / team, e = tid % per, q0 = tid / per;
   const Load* ld = reinterpret_cast<const Load*>(h + 1);
@@ -112,7 +120,7 @@ __device__ void run_elementwise(const Head* h, int chunk, T* v) {
   v += e;
   if (on)
     for (int k = q0; k < h->n_load; k += team)      // all on their way at once
-      copy_async<sizeof(T)>(v + ld[k].slot * per, (const T*)ld[k].p + (ld[k].cols ? i % ld[k].cols : i));
+      copy_async<sizeof(T)>(v + ld[k].slot * per, source<T>(ld[k].p, starts) + (ld[k].cols ? i % ld[k].cols : i));
   copy_wait();
   if (team > 1) {
     worker_sync();
@@ -160,13 +168,13 @@ __device__ __forceinline__ void copy_operand(T* s, int pitch, const T* g, int64_
   }
 }
 
-template <typename T, int R>
-__device__ void run_product(const ProductProg* p, int chunk, T* smem) {
+template <typename T, int R, int N_STARTS>
+__device__ void run_product(const ProductProg* p, int chunk, T* smem, const StartTable<N_STARTS>& starts) {
   const int tid = threadIdx.x % NT, tm = p->tm, tn = p->tn, ks = p->ks, K = p->K, M = p->M, N = p->N;
   const int bz = chunk / p->tiles_mn, t2 = chunk % p->tiles_mn;
   const int m0 = t2 / p->tiles_n * tm, n0 = t2 % p->tiles_n * tn;
-  const T* A = (const T*)p->A + bz * p->sA;
-  const T* B = (const T*)p->B + bz * p->sB;
+  const T* A = source<T>(p->A, starts) + bz * p->sA;
+  const T* B = source<T>(p->B, starts) + bz * p->sB;
   T* C = (T*)p->C + bz * p->sC;
   const int pa = product_pitch<T>(ks);
   T* As = smem;                              // [tm][pa]
@@ -244,11 +252,11 @@ template <typename T> __device__ __forceinline__ T sine_exp(T x) { return (T)exp
 
 // ---- row-wise operations: one warp per row, eight rows per piece (the arithmetic of the kernels in rowops.cu); column sums
 // and transposes: 256 outputs per piece
-template <typename T>
-__device__ void run_rows(const RowProg* p, int chunk) {
+template <typename T, int N>
+__device__ void run_rows(const RowProg* p, int chunk, const StartTable<N>& starts) {
   const int tid = threadIdx.x % NT, lane = tid & 31, cols = p->cols;
-  const T* x = (const T*)p->in[0];
-  const T* in1 = (const T*)p->in[1];
+  const T* x = source<T>(p->in[0], starts);
+  const T* in1 = source<T>(p->in[1], starts);
   T* out = (T*)p->out[0];
   if (p->h.kind == PRIM_COLUMN_SUM) {        // out[j] = scalar * sum of rows (scalar 1: as is)
     const int64_t j = (int64_t)chunk * NT + tid;
@@ -327,8 +335,8 @@ __device__ void run_rows(const RowProg* p, int chunk) {
       break;
     }
     case PRIM_LAYERNORM_BACKWARD: {          // in: x, mean, sigma, dy
-      const T mu = in1[r], se = add_rn(((const T*)p->in[2])[r], sizeof(T) == 4 ? (T)1e-9f : (T)1e-9);
-      const T* dr = (const T*)p->in[3] + r * cols;
+      const T mu = in1[r], se = add_rn(source<T>(p->in[2], starts)[r], sizeof(T) == 4 ? (T)1e-9f : (T)1e-9);
+      const T* dr = source<T>(p->in[3], starts) + r * cols;
       const T exp1 = mul_rn(sub_rn((T)1, div_rn((T)1, (T)cols)), div_rn((T)1, se));
       const T den = mul_rn((T)cols, mul_rn(mul_rn(se, se), se));
       for (int j = lane; j < cols; j += 32) {
@@ -342,9 +350,10 @@ __device__ void run_rows(const RowProg* p, int chunk) {
 
 constexpr int SMEM_BYTES = WORKERS * (2 * PROG_BYTES + WORK_BYTES);
 
-template <typename T>
+template <typename T, int N>
 __global__ void __launch_bounds__(WORKERS * NT)
-walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ items, const int* __restrict__ first) {
+walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ items, const int* __restrict__ first,
+            const __grid_constant__ StartTable<N> starts) {
   extern __shared__ __align__(16) unsigned char gp_smem[];
   const int tid = threadIdx.x % NT, worker = blockIdx.x * WORKERS + threadIdx.x / NT;
   unsigned char* prog = gp_smem + (threadIdx.x / NT) * (2 * PROG_BYTES + WORK_BYTES);
@@ -366,10 +375,10 @@ walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ ite
     if (cur.bytes) {
       const Head* h = reinterpret_cast<const Head*>(prog + (i & 1) * PROG_BYTES);
       const ProductProg* pp = reinterpret_cast<const ProductProg*>(h);
-      if (h->kind <= PRIM_LAST_ELEMENTWISE) run_elementwise<T>(h, (int)cur.chunk, work);
-      else if (h->kind == PRIM_PRODUCT && pp->r == 1) run_product<T, 1>(pp, (int)cur.chunk, work);
-      else if (h->kind == PRIM_PRODUCT) run_product<T, 2>(pp, (int)cur.chunk, work);
-      else run_rows<T>(reinterpret_cast<const RowProg*>(h), (int)cur.chunk);
+      if (h->kind <= PRIM_LAST_ELEMENTWISE) run_elementwise<T>(h, (int)cur.chunk, work, starts);
+      else if (h->kind == PRIM_PRODUCT && pp->r == 1) run_product<T, 1>(pp, (int)cur.chunk, work, starts);
+      else if (h->kind == PRIM_PRODUCT) run_product<T, 2>(pp, (int)cur.chunk, work, starts);
+      else run_rows<T>(reinterpret_cast<const RowProg*>(h), (int)cur.chunk, starts);
     }
     if (cur.barrier) cluster_barrier();
     cur = nxt;
@@ -386,6 +395,7 @@ struct GraphPlan {
   const unsigned char* blob = nullptr;
   const gp::Item* items = nullptr;
   const int* first = nullptr;
+  std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write, ascending, without overlaps
 };
 
 void GraphPlanFree::operator()(GraphPlan* p) const {
@@ -752,14 +762,23 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
 }
 
 // 16 CTAs if the device runs such a cluster of this kernel, else 8, else none
+template <typename T> static cudaError_t reserve(void) {
+  cudaError_t e = cudaSuccess;
+  auto one = [&](auto* kernel) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  };
+  one(walk_kernel<T, FEW_STARTS>);
+  one(walk_kernel<T, MOST_STARTS>);
+  return e;
+}
 template <typename T> static int cluster_ctas(prad_ctx* ctx) {
   static std::atomic<int> known[64];
   std::atomic<int>& k = known[ctx->device & 63];
   int n = k.load(std::memory_order_acquire);
   if (n) return n - 1;
   n = 0;
-  cudaError_t e = cudaFuncSetAttribute(walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(walk_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  const cudaError_t e = reserve<T>();
   for (int cs : {16, 8}) {
     if (e != cudaSuccess || n) break;
     cudaLaunchConfig_t cfg = {};
@@ -773,7 +792,7 @@ template <typename T> static int cluster_ctas(prad_ctx* ctx) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int fit = 0;
-    if (cudaOccupancyMaxActiveClusters(&fit, walk_kernel<T>, &cfg) == cudaSuccess && fit > 0) n = cs;
+    if (cudaOccupancyMaxActiveClusters(&fit, walk_kernel<T, FEW_STARTS>, &cfg) == cudaSuccess && fit > 0) n = cs;
     else (void)cudaGetLastError();
   }
   if (e != cudaSuccess) (void)cudaGetLastError();
@@ -818,6 +837,18 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
     (void)cudaGetLastError();
     return nullptr;
   }
+  std::vector<Access> acc;
+  for (const Prim& p : ops) {
+    accesses(p, sizeof(T), acc);
+    for (const Access& a : acc)
+      if (a.write) plan->written.emplace_back(a.lo, a.hi);
+  }
+  std::sort(plan->written.begin(), plan->written.end());
+  size_t kept = 0;
+  for (const auto& w : plan->written)
+    if (kept && w.first <= plan->written[kept - 1].second) plan->written[kept - 1].second = std::max(plan->written[kept - 1].second, w.second);
+    else plan->written[kept++] = w;
+  plan->written.resize(kept);
   plan->items = (const Item*)plan->mem;
   plan->first = (const int*)((const unsigned char*)plan->mem + items_bytes);
   plan->blob = (const unsigned char*)plan->mem + items_bytes + first_bytes;
@@ -830,7 +861,22 @@ GraphPlanPtr graph_plan_build(prad_ctx* ctx, prad_dtype dt, const std::vector<Pr
   return dt == PRAD_F32 ? gp::build_plan<float>(ctx, dt, ops) : gp::build_plan<double>(ctx, dt, ops);
 }
 
-prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan) {
+bool graph_plan_writes(const GraphPlan* plan, const void* p, size_t bytes) {
+  const uintptr_t lo = (uintptr_t)p, hi = lo + bytes;
+  auto it = std::upper_bound(plan->written.begin(), plan->written.end(), std::make_pair(lo, ~(uintptr_t)0));
+  return (it != plan->written.begin() && std::prev(it)->second > lo) || (it != plan->written.end() && it->first < hi);
+}
+
+template <typename T, int N>
+static prad_status run_walk(prad_ctx* ctx, const cudaLaunchConfig_t& cfg, const GraphPlan* plan, const void* const* starts, int count) {
+  gp::StartTable<N> table;
+  for (int i = 0; i < count; ++i) table.p[i] = starts[i];
+  PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<T, N>, plan->blob, plan->items, plan->first, table));
+  PRAD_LAUNCHED(ctx);
+  return PRAD_OK;
+}
+
+prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan, const void* const* starts, int count) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -838,18 +884,14 @@ prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3((unsigned)plan->ctas);
   cfg.blockDim = dim3(gp::WORKERS * gp::NT);
+  cfg.dynamicSmemBytes = gp::SMEM_BYTES;
   cfg.stream = ctx->stream;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (plan->dt == PRAD_F32) {
-    cfg.dynamicSmemBytes = gp::SMEM_BYTES;
-    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<float>, plan->blob, plan->items, plan->first));
-  } else {
-    cfg.dynamicSmemBytes = gp::SMEM_BYTES;
-    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<double>, plan->blob, plan->items, plan->first));
-  }
-  PRAD_LAUNCHED(ctx);
-  return PRAD_OK;
+  const bool few = count <= gp::FEW_STARTS;
+  if (plan->dt == PRAD_F32)
+    return few ? run_walk<float, gp::FEW_STARTS>(ctx, cfg, plan, starts, count) : run_walk<float, MOST_STARTS>(ctx, cfg, plan, starts, count);
+  return few ? run_walk<double, gp::FEW_STARTS>(ctx, cfg, plan, starts, count) : run_walk<double, MOST_STARTS>(ctx, cfg, plan, starts, count);
 }
 
 }  // namespace prad

@@ -32,6 +32,13 @@ struct Prim {
   int64_t sA = 0, sB = 0, sC = 0; // batch strides in elements (0: shared); leading dimensions are dense
 };
 
+// The start gradients of a Backward are another program's matrices every time.  Operations name the i-th one by this stand-in
+// (no device address has these high bits), and a run says which matrices they are.
+inline const void* start_stand_in(int i) { return (const void*)(((uint64_t)1 << 62) | ((uint64_t)i << 40)); }
+inline bool is_stand_in(const void* p) { return ((uint64_t)p >> 62) == 1; }
+inline int stand_in_index(const void* p) { return (int)(((uint64_t)p >> 40) & 0x3fffff); }
+constexpr int MOST_STARTS = 4000;            // what a kernel's arguments have room for
+
 struct GraphPlan;
 struct GraphPlanFree { void operator()(GraphPlan* p) const; };
 using GraphPlanPtr = std::unique_ptr<GraphPlan, GraphPlanFree>;
@@ -39,6 +46,8 @@ using GraphPlanPtr = std::unique_ptr<GraphPlan, GraphPlanFree>;
 // A plan for these operations, or null when one launch per operation is the better way to run them (few of them, large ones,
 // or a device that cannot run the cluster).
 GraphPlanPtr graph_plan_build(prad_ctx* ctx, prad_dtype dt, const std::vector<Prim>& ops);
-prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan);
+prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan, const void* const* starts = nullptr, int count = 0);
+// whether the plan's operations write anywhere in [p, p + bytes)
+bool graph_plan_writes(const GraphPlan* plan, const void* p, size_t bytes);
 
 }  // namespace prad

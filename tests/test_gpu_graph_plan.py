@@ -1,5 +1,7 @@
 """Graph walks as one kernel against one launch per operation: every operation type, shared and deep values, fan-in beyond
 eight, pieces at the edges of 256 elements and of the product tiles, gradient destinations in one buffer."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -139,4 +141,116 @@ def test_a_recorded_walk_survives_the_growth_of_its_graph(engine, dtype):
         np.testing.assert_array_equal(g.data(h).numpy(), want[-1][1])  # the new nodes are not part of the recording
     assert not any(m.numpy().any() for m in junk)
     seq.close()
+    g.close()
+
+
+def _backward_from(g, starts, gradients):
+    E.check(g.eng.lib.prad_graph_backward_multi(g.h, (C.c_int * len(starts))(*starts), E.Engine._ptr_list(gradients), len(starts)))
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_one_plan_serves_every_start_gradient(engine, dtype):
+    """A program gets new loss gradients from every pass: the plan of the first pass runs them too, and says whose gradient is whose."""
+    n, steps = 24, 5
+    r = rng(5)
+    up = lambda: engine.upload((r.standard_normal((n, n)) * 0.3).astype(dtype))  # noqa: E731
+    g = Graph(engine, dtype)
+    dw = engine.zeros((n, n), dtype)
+    w, h = g.weight(up(), dw), g.input(up())
+    starts = []
+    for _ in range(steps):
+        h = g.node("TanhOperation", [g.node("MatrixMultiplyOperation", [w, h])])
+        starts.append(g.node("MatrixAddOperation", [h, g.node("MatrixTransposeOperation", [h])]))
+    g.forward()
+    sets = [[up() for _ in starts] for _ in range(7)]
+    sets.append([sets[0][0]] * steps)                        # one gradient for all
+    flat = engine.upload(r.standard_normal((steps * n * n + 1,)).astype(dtype))
+    sets.append([flat.view((n, n), 1 + k * n * n) for k in range(steps)])      # off a 16-byte boundary
+    sets.append([flat.view((n, n), k * 3 * n) for k in range(steps)])         # overlapping
+    want = []
+    for d in sets:
+        engine.set_option("graph_plan", "0")
+        try:
+            engine.zero_(dw)
+            _backward_from(g, starts, d)
+            want.append([g.gradient(h).numpy(), g.gradient(starts[0]).numpy(), dw.numpy()])
+        finally:
+            engine.set_option("graph_plan", "1")
+    _backward_from(g, starts, sets[0])
+    for d, expected in zip(sets, want):
+        for recorded in (True, False):                       # a recording uses a plan that is there, but cannot make one
+            engine.zero_(dw)
+            if recorded:
+                seq = engine.record(lambda: _backward_from(g, starts, d))
+                assert seq.launches == 1
+                seq.launch()
+            else:
+                n0 = engine.launch_count()
+                _backward_from(g, starts, d)
+                assert engine.launch_count() - n0 == 1
+            for a, b in zip([g.gradient(h).numpy(), g.gradient(starts[0]).numpy(), dw.numpy()], expected):
+                np.testing.assert_array_equal(a, b)
+            assert g.gradient(starts[0]).ptr == d[0].ptr     # nothing else flows into it
+            if recorded:
+                seq.close()
+    g.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("starts", [3, 70])
+def test_start_gradients_that_the_walk_itself_writes(engine, dtype, starts):
+    """A start gradient in memory that Backward writes (a gradient destination, a gradient of the last pass) is read in turn; and
+    more start values than fit the kernel's short table."""
+    n = 8
+    results = []
+    for plan in ("1", "0"):
+        r = rng(11)
+        up = lambda: engine.upload((r.standard_normal((n, n)) * 0.3).astype(dtype))  # noqa: E731
+        engine.set_option("graph_plan", plan)
+        try:
+            g = Graph(engine, dtype)
+            dw = engine.zeros((n, n), dtype)
+            w, x = g.weight(up(), dw), g.input(up())
+            h, ends = x, []
+            for _ in range(starts):
+                h = g.node("SigmoidOperation", [g.node("MatrixMultiplyOperation", [w, h])])
+                ends.append(g.node("MatrixAddOperation", [g.node("MatrixMultiplyScalarOperation", [h], scalar=0.5), h]))
+            g.forward()
+            d = [up() for _ in ends]
+            got = []
+            n0 = engine.launch_count()
+            _backward_from(g, ends, d)
+            if plan == "1":
+                assert engine.launch_count() - n0 == 1
+            got += [dw.numpy(), g.gradient(x).numpy()]
+            for last in (dw, g.gradient(x), g.gradient(w), g.gradient(ends[0])):
+                _backward_from(g, ends, d[:-1] + [last])
+                got += [dw.numpy(), g.gradient(x).numpy()]
+            results.append(got)
+            g.close()
+        finally:
+            engine.set_option("graph_plan", "1")
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_plans_of_many_sets_of_start_values(engine):
+    """Sets of start values beyond those whose plans are kept run one launch per operation; the kept ones stay."""
+    n, r = 8, rng(12)
+    up = lambda: engine.upload((r.standard_normal((n, n)) * 0.3).astype(np.float32))  # noqa: E731
+    g = Graph(engine, np.float32)
+    w, h = g.input(up()), g.input(up())
+    for _ in range(6):
+        h = g.node("SigmoidOperation", [g.node("MatrixMultiplyOperation", [w, h])])
+    ends = [g.node("TanhOperation", [h]) for _ in range(20)]
+    g.forward()
+    d = up()
+    launches = []
+    for _ in range(3):
+        for end in ends:
+            n0 = engine.launch_count()
+            g.backward(end, d)
+            launches.append(engine.launch_count() - n0)
+    assert launches[:16] == [1] * 16 and min(launches[16:20]) > 6
+    assert launches[20:40] == launches[:20] == launches[40:]
     g.close()
