@@ -126,6 +126,10 @@ prad_status gemm_fp16x3_backward(prad_ctx* ctx, const void* A, const void* B, co
                                  double act_alpha, void* dC, void* dA, void* dB, int M, int K, int N, bool accumulate_dB,
                                  double dB_scale, const GemmEpilogue& e_dA);
 
+static bool overlap(const void* p, int64_t p_elems, const void* q, int64_t q_elems, size_t es) {
+  return p && q && (const char*)p < (const char*)q + q_elems * es && (const char*)q < (const char*)p + p_elems * es;
+}
+
 // dOut given: dC is not there yet, it is to receive dOut (.) act'(saved)
 static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void* A,
                                         const void* B, const void* dC, void* dA, void* dB, int M,
@@ -139,7 +143,13 @@ static prad_status matmul_backward_impl(prad_ctx* ctx, prad_dtype dt, const void
   e_dA.saved = saved_below;
   e_dA.act_alpha = act_alpha;
   // dA (MxK) = dC (MxN) * B^T  (B is KxN) ; dB (KxN) = A^T (A is MxK) * dC (MxN)
-  const bool both = dA && dB && M > 0 && K > 0 && N > 0;
+  // dA is there before dB is begun, except where the two products cannot tell: a result in the place of what the other one
+  // reads (dB over B, say) keeps that order
+  const size_t es = dtype_size(dt);
+  const int64_t mk = (int64_t)M * K, kn = (int64_t)K * N, mn = (int64_t)M * N;
+  const bool both = dA && dB && M > 0 && K > 0 && N > 0 && !overlap(dA, mk, A, mk, es) && !overlap(dA, mk, dC, mn, es) &&
+                    !overlap(dA, mk, dB, kn, es) && !overlap(dB, kn, B, kn, es) && !overlap(dB, kn, dC, mn, es) &&
+                    !overlap(dB, kn, saved_below, mk, es);
   const bool tc_A = both && wants_tensor_cores(ctx, dt, false, true, M, K, N, 1.0, dC, N, B, N, 0.0, dA, K, 1, 0, 0, 0, e_dA);
   const bool tc_B = both && wants_tensor_cores(ctx, dt, true, false, K, N, M, dB_scale, A, K, dC, N, accumulate_dB ? 1.0 : 0.0, dB, N, 1, 0,
                                                0, 0, e_dB);
