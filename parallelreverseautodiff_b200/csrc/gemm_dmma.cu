@@ -270,7 +270,7 @@ prad_status gemm_f64_dmma(prad_ctx* ctx, bool tA, bool tB, int M, int N, int K, 
     if (S > 1 || sum) {
       const int64_t mn = (int64_t)M * N;
       st = ensure_parts(ctx, (size_t)batch * S * mn * sizeof(double));
-      if (st) return st;
+      if (st) return sum ? PRAD_ERR_UNSUPPORTED : st;     // (a sum also goes product by product)
       double* part = (double*)ctx->parts;
       pr.slices = S;
       pr.k_slice = k_slice;

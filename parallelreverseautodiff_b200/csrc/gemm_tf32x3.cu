@@ -2172,9 +2172,10 @@ prad_status gemm_fp16x3_backward(prad_ctx* ctx, const void* A, const void* B, co
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
   size_t scales = 0, pieces = 0;
   for (PackedForm* f : {&cr, &cc, &b, &a}) { scales += al(f->blk_bytes()); pieces += al(f->h_bytes()); }
-  if (scales + pieces > ctx->total_mem / 16) return PRAD_ERR_UNSUPPORTED;      // (one product at a time needs half of it)
-  prad_status s = ensure_workspace(ctx, scales + pieces);
-  if (s) return s;
+  // one product at a time needs half of the scratch: that way where this is much of the memory, or where it cannot be had (a
+  // recording whose scratch was sized by single products, a device that is nearly full)
+  if (scales + pieces > ctx->total_mem / 16 || ensure_workspace(ctx, scales + pieces) != PRAD_OK) return PRAD_ERR_UNSUPPORTED;
+  prad_status s;
   char* w = (char*)ctx->ws;
   for (PackedForm* f : {&cr, &cc, &b, &a}) { f->blk = (float*)w; w += al(f->blk_bytes()); }
   for (PackedForm* f : {&cr, &cc, &b, &a}) { f->h = (__half*)w; w += al(f->h_bytes()); }

@@ -49,14 +49,17 @@ prad_status gemm_dispatch(prad_ctx* ctx, prad_dtype dt, bool tA, bool tB, int M,
   if (M == 0 || N == 0 || batch == 0) return PRAD_OK;
   const bool tc = wants_tensor_cores(ctx, dt, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi);
   // One result for the whole batch: the sum over its products.  On the FP64 tensor cores they are k slices (gemm_f64_dmma);
-  // otherwise one launch writes them side by side and another adds them, or, where C has a pitch or an old value to keep, each
-  // is added by the next product.
-  if (batch > 1 && sC == 0 && !(tc && dt == PRAD_F64)) {
+  // otherwise one launch writes them side by side and another adds them, or, where C has a pitch or an old value to keep or the
+  // scratch cannot be had, each is added by the next product.
+  if (batch > 1 && sC == 0) {
     const size_t es = dtype_size(dt);
     const int64_t mn = (int64_t)M * N;
     prad_status s;
-    if (!tc && ldc == N && beta == 0.0 && batch <= 8 && mn <= (1 << 20)) {
-      if ((s = ensure_parts(ctx, (size_t)batch * mn * es))) return s;
+    if (tc && dt == PRAD_F64) {
+      s = gemm_f64_dmma(ctx, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, batch, sA, sB, sC, epi, false);
+      if (s != PRAD_ERR_UNSUPPORTED) return s;
+    }
+    if (!tc && ldc == N && beta == 0.0 && batch <= 8 && mn <= (1 << 20) && ensure_parts(ctx, (size_t)batch * mn * es) == PRAD_OK) {
       const void* parts[8];
       for (int b = 0; b < batch; ++b) parts[b] = (char*)ctx->parts + b * mn * es;
       if ((s = gemm_dispatch(ctx, dt, tA, tB, M, N, K, alpha, A, lda, B, ldb, 0.0, ctx->parts, N, batch, sA, sB, mn, epi))) return s;

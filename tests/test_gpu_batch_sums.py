@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from parallelreverseautodiff_b200 import engine as E
 from util import rng
 
 pytestmark = pytest.mark.gpu
@@ -32,3 +33,38 @@ def test_column_sums_of_a_batch(engine, dtype, rows, cols, batch):
     out = engine.empty((batch, cols), dtype)
     engine.column_sums(engine.upload(x.reshape(-1, cols)), out, rows, batch, 0.125)
     np.testing.assert_allclose(out.numpy(), 0.125 * x.astype(np.float64).sum(1), rtol=1e-6 if dtype == np.float32 else 1e-12, atol=1e-9)
+
+
+@pytest.mark.parametrize("dtype,m,n,k", [(np.float32, 20, 30, 40), (np.float64, 20, 30, 40), (np.float64, 512, 256, 512)])
+def test_a_recorded_sum_without_scratch(dtype, m, n, k):
+    """A recording cannot grow scratch: the sum then goes product by product."""
+    batch, r = 4, rng(m)
+    A, B = r.standard_normal((batch, m, k)).astype(dtype), r.standard_normal((batch, k, n)).astype(dtype)
+    with E.Engine(0) as eng:
+        a, b, out = eng.upload(A.reshape(-1, k)), eng.upload(B.reshape(-1, n)), eng.zeros((m, n), dtype)
+        seq = eng.record(lambda: eng.gemm(a.view((m, k)), b.view((k, n)), out, batch=batch, strideA=m * k, strideB=k * n, strideC=0))
+        seq.launch()
+        want = np.einsum("bmk,bkn->mn", A.astype(np.float64), B.astype(np.float64))
+        np.testing.assert_allclose(out.numpy(), want, rtol=0, atol=(1e-5 if dtype == np.float32 else 1e-13) * batch * np.sqrt(k))
+        seq.close()
+        for x in (a, b, out):
+            x.free()
+
+
+def test_a_recorded_backward_with_the_scratch_of_single_products():
+    """Packing a float Backward's gradient once takes twice the scratch of one product: a recording that has only that much goes
+    product by product, with the same values."""
+    n, r = 512, rng(9)
+    up = [r.standard_normal((n, n)).astype(np.float32) for _ in range(3)]
+    with E.Engine(0) as eng:
+        A, B, dC = (eng.upload(x) for x in up)
+        want_a, _ = eng.matmul_backward(A, B, dC, need_dB=False)
+        _, want_b = eng.matmul_backward(A, B, dC, need_dA=False)
+        dA, dB = eng.zeros((n, n), np.float32), eng.zeros((n, n), np.float32)
+        seq = eng.record(lambda: eng.matmul_backward(A, B, dC, dA=dA, dB=dB))
+        seq.launch()
+        np.testing.assert_array_equal(dA.numpy(), want_a.numpy())
+        np.testing.assert_array_equal(dB.numpy(), want_b.numpy())
+        seq.close()
+        for x in (A, B, dC, want_a, want_b, dA, dB):
+            x.free()
