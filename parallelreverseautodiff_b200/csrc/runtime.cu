@@ -308,7 +308,7 @@ prad_status prad_device_info(prad_ctx* ctx, prad_device_info_t* out) {
   (void)cudaGetLastError();
   out->total_bytes = (uint64_t)total_b;
   out->free_bytes = (uint64_t)free_b;
-  out->scratch_bytes = (uint64_t)(ctx->ws_bytes + ctx->stage_bytes);
+  out->scratch_bytes = (uint64_t)(ctx->ws_bytes + ctx->stage_bytes + ctx->parts_bytes);
   strncpy(out->name, p.name, sizeof(out->name) - 1);
   return PRAD_OK;
 }

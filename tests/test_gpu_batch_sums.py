@@ -68,3 +68,15 @@ def test_a_recorded_backward_with_the_scratch_of_single_products():
         seq.close()
         for x in (A, B, dC, want_a, want_b, dA, dB):
             x.free()
+
+
+def test_partial_products_count_as_scratch():
+    """The products of a sum over a batch wait in scratch, which the device's facts include."""
+    n, batch = 100, 4
+    with E.Engine(0) as eng:
+        a, out = eng.zeros((batch * n, n), np.float32), eng.empty((n, n), np.float32)
+        before = eng.device_info()["scratch_bytes"]
+        eng.gemm(a.view((n, n)), a.view((n, n)), out, batch=batch, strideA=n * n, strideB=n * n, strideC=0)
+        assert eng.device_info()["scratch_bytes"] - before >= batch * n * n * 4
+        a.free()
+        out.free()
