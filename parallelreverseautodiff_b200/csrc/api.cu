@@ -361,6 +361,7 @@ prad_status prad_upload_fence(prad_ctx* ctx) {
   if (s) return s;
   PRAD_CUDA(cudaEventRecord(ctx->copy_done, ctx->stream));
   PRAD_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_done, 0));
+  pool_fenced(ctx);
   return PRAD_OK;
 }
 

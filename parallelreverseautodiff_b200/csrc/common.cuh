@@ -179,6 +179,7 @@ prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out);
 prad_status pool_free(prad_ctx* ctx, void* p);
 // orders ctx->copy_stream behind the old work of recycled blocks in [dst, dst + bytes)
 prad_status pool_before_prefetch(prad_ctx* ctx, void* dst, size_t bytes);
+void pool_fenced(prad_ctx* ctx);             // the copy stream was put behind everything on ctx->stream
 void pool_limit(prad_ctx* ctx, size_t cap);   // most bytes this context keeps
 // cudaMalloc; when memory is short every context's cached blocks go back to the device first
 cudaError_t device_malloc(void** out, size_t bytes);

@@ -16,13 +16,12 @@
 //  - a block that another context frees, or that is freed while a prefetch copy is pending, while another
 //    context records or on a context with data-parallel communication, takes the old path: wait and cudaFree;
 //  - a prefetch, which runs beside the context's stream, into a block that came out of the cache starts
-//    behind what that stream was given before (the first one does: later ones are ordered behind it);
+//    behind what that stream was given before, unless a fence or such a prefetch has seen to that already;
 //  - nothing is taken from the cache while a launch sequence is recorded;
 //  - the cache of a context is bounded (1/16 of the device memory; the block that was freed first
 //    leaves first), and is given back when the context is shut down, when any allocation of this
 //    process' contexts fails for lack of memory, or by the option "pool_bytes" = "0".
 #include <deque>
-#include <map>
 #include <mutex>
 #include <unordered_map>
 
@@ -43,13 +42,16 @@ struct DevicePool {
   std::unordered_map<void*, size_t> cached;   // block -> size, for `order`
   std::vector<cudaEvent_t> spare;
   size_t held = 0, cap = 0;
+  int64_t fences = 0;                 // how often the context's copy stream was put behind all of its stream's work
+  bool recycled = false;              // a block with old work pending was handed out since
 };
 
 namespace {
-// recycled: came out of the cache with its old work ahead of it on the owner's stream, and no prefetch has been ordered behind its old work yet
-struct Live { size_t bytes; prad_ctx* owner; bool recycled; };
+// recycled: what the owner's `fences` was when the block came out of the cache with old work ahead of it on the owner's stream,
+// -1 if there is none
+struct Live { size_t bytes; prad_ctx* owner; int64_t recycled; };
 std::mutex g_pool_mu;
-std::map<void*, Live> g_live;                 // every block prad_alloc handed out
+std::unordered_map<void*, Live> g_live;       // every block prad_alloc handed out
 std::vector<prad_ctx*> g_contexts;            // every context
 std::vector<prad_ctx*> g_pools;               // contexts that have a cache
 
@@ -133,7 +135,7 @@ prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out) {
   if (!ctx->capturing && it != pool->by_size.end() && !it->second.empty()) {
     const bool alone = others_on_device(ctx).empty();
     const size_t at = alone ? it->second.size() - 1 : 0;      // the one freed last: likeliest in L2
-    const CachedBlock b = it->second[at];
+    const CachedBlock b = std::move(it->second[at]);
     it->second.erase(it->second.begin() + at);
     pool->held -= b.bytes;
     pool->cached.erase(b.p);
@@ -149,7 +151,8 @@ prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out) {
     }
     pool->spare.push_back(b.freed);
     pool->spare.insert(pool->spare.end(), b.users.begin(), b.users.end());
-    g_live[b.p] = {want, ctx, !idle};
+    g_live[b.p] = {want, ctx, idle ? -1 : pool->fences};
+    pool->recycled = pool->recycled || !idle;
     *out = b.p;
     return PRAD_OK;
   }
@@ -160,7 +163,7 @@ prad_status pool_alloc(prad_ctx* ctx, size_t bytes, void** out) {
     set_error("prad_alloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? PRAD_ERR_OOM : PRAD_ERR_CUDA;
   }
-  g_live[*out] = {want, ctx, false};
+  g_live[*out] = {want, ctx, -1};
   return PRAD_OK;
 }
 
@@ -223,16 +226,28 @@ prad_status pool_free(prad_ctx* ctx, void* p) {
 
 prad_status pool_before_prefetch(prad_ctx* ctx, void* dst, size_t bytes) {
   std::lock_guard<std::mutex> lock(g_pool_mu);
-  auto it = g_live.upper_bound(dst);
-  if (it != g_live.begin()) --it;
-  for (; it != g_live.end() && (char*)it->first < (char*)dst + bytes; ++it) {
-    if (!it->second.recycled || (char*)it->first + it->second.bytes <= (char*)dst) continue;
-    it->second.recycled = false;
-    if (!it->second.owner) continue;          // its context is gone, and had waited for its work
-    PRAD_CUDA(cudaEventRecord(ctx->copy_done, it->second.owner->stream));
-    PRAD_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_done, 0));
-  }
+  DevicePool* pool = pool_of(ctx);
+  if (!pool->recycled) return PRAD_OK;
+  // (a block of another context has no old work pending: its owner is not alone, or is gone and had waited)
+  auto pending = [&](const void* p, const Live& l) {
+    return l.owner == ctx && l.recycled == pool->fences && (char*)p < (char*)dst + bytes && (char*)dst < (char*)p + l.bytes;
+  };
+  auto it = g_live.find(dst);
+  bool wait = it != g_live.end() && pending(it->first, it->second);
+  if (it == g_live.end() || it->second.bytes < bytes)        // inside a block
+    for (const auto& kv : g_live) wait = wait || pending(kv.first, kv.second);
+  if (!wait) return PRAD_OK;
+  PRAD_CUDA(cudaEventRecord(ctx->copy_done, ctx->stream));
+  PRAD_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_done, 0));
+  pool->fences++;
+  pool->recycled = false;
   return PRAD_OK;
+}
+void pool_fenced(prad_ctx* ctx) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  DevicePool* pool = pool_of(ctx);
+  pool->fences++;
+  pool->recycled = false;
 }
 
 void pool_limit(prad_ctx* ctx, size_t cap) {
@@ -254,7 +269,7 @@ void pool_enter(prad_ctx* ctx) {
     shrink(c, 0);
     if (!recording(c->stream)) cudaStreamSynchronize(c->stream);
     for (auto& kv : g_live)
-      if (kv.second.owner == c) kv.second.recycled = false;
+      if (kv.second.owner == c) kv.second.recycled = -1;
   }
   g_contexts.push_back(ctx);
 }
