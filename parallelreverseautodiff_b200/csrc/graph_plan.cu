@@ -395,7 +395,7 @@ struct GraphPlan {
   const unsigned char* blob = nullptr;
   const gp::Item* items = nullptr;
   const int* first = nullptr;
-  std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write, ascending, without overlaps
+  std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write: ascending, without overlaps
 };
 
 void GraphPlanFree::operator()(GraphPlan* p) const {
@@ -459,6 +459,7 @@ static void accesses(const Prim& p, size_t es, std::vector<Access>& out) {
 struct Region {
   uintptr_t lo, hi;
   bool local;                                // every access so far was element-local to the same interval
+  bool written;                              // by any operation
   std::vector<int> writers, readers;
 };
 
@@ -553,7 +554,8 @@ static double launch_cost(const Prim& p, int sms) {
 }
 
 template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& ops, int ctas, std::vector<unsigned char>& blob,
-                                        std::vector<std::vector<Item>>& lists, double* est_us, double* launch_us) {
+                                        std::vector<std::vector<Item>>& lists, std::vector<std::pair<uintptr_t, uintptr_t>>& written,
+                                        double* est_us, double* launch_us) {
   const size_t es = sizeof(T);
   const int N = (int)ops.size();
   std::vector<int> level(N, 0), group_of(N, -1);
@@ -567,12 +569,13 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       auto p = std::prev(it);
       if (p->second.hi > a.lo) it = p;
     }
-    if (it == mem.end() || it->first >= a.hi) return mem.emplace(a.lo, Region{a.lo, a.hi, true, {}, {}}).first->second;
+    if (it == mem.end() || it->first >= a.hi) return mem.emplace(a.lo, Region{a.lo, a.hi, true, false, {}, {}}).first->second;
     if (it->first == a.lo && it->second.hi == a.hi) return it->second;
-    Region joined{a.lo, a.hi, false, {}, {}};      // overlaps: one region for all of them
+    Region joined{a.lo, a.hi, false, false, {}, {}};      // overlaps: one region for all of them
     while (it != mem.end() && it->first < a.hi) {
       joined.lo = std::min(joined.lo, it->first);
       joined.hi = std::max(joined.hi, it->second.hi);
+      joined.written = joined.written || it->second.written;
       joined.writers.insert(joined.writers.end(), it->second.writers.begin(), it->second.writers.end());
       joined.readers.insert(joined.readers.end(), it->second.readers.begin(), it->second.readers.end());
       it = mem.erase(it);
@@ -622,10 +625,17 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       Region& r = region_at(a);
       r.local = r.local && a.local;
       if (!a.write) { r.readers.push_back(i); continue; }
+      r.written = true;
       if (r.lo == a.lo && r.hi == a.hi) { r.writers.clear(); r.readers.clear(); }
       r.writers.push_back(i);
     }
   }
+
+  for (const auto& m : mem)
+    if (m.second.written) {
+      if (!written.empty() && written.back().second == m.second.lo) written.back().second = m.second.hi;
+      else written.emplace_back(m.second.lo, m.second.hi);
+    }
 
   // programs, and the pieces of every level
   const int levels = N ? *std::max_element(level.begin(), level.end()) + 1 : 0;
@@ -813,7 +823,8 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
   std::vector<unsigned char> blob;
   std::vector<std::vector<Item>> lists;
   double est = 0, launches = 0;
-  build<T>(ctx, ops, ctas, blob, lists, &est, &launches);
+  std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write: ascending, without overlaps
+  build<T>(ctx, ops, ctas, blob, lists, written, &est, &launches);
   if (est >= launches) return nullptr;
   std::vector<Item> items;
   std::vector<int> first;
@@ -837,18 +848,7 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
     (void)cudaGetLastError();
     return nullptr;
   }
-  std::vector<Access> acc;
-  for (const Prim& p : ops) {
-    accesses(p, sizeof(T), acc);
-    for (const Access& a : acc)
-      if (a.write) plan->written.emplace_back(a.lo, a.hi);
-  }
-  std::sort(plan->written.begin(), plan->written.end());
-  size_t kept = 0;
-  for (const auto& w : plan->written)
-    if (kept && w.first <= plan->written[kept - 1].second) plan->written[kept - 1].second = std::max(plan->written[kept - 1].second, w.second);
-    else plan->written[kept++] = w;
-  plan->written.resize(kept);
+  plan->written = std::move(written);
   plan->items = (const Item*)plan->mem;
   plan->first = (const int*)((const unsigned char*)plan->mem + items_bytes);
   plan->blob = (const unsigned char*)plan->mem + items_bytes + first_bytes;
