@@ -176,8 +176,9 @@ prad_status prad_get_timings(prad_ctx* ctx, prad_timing_t* out, int capacity, in
 /* prad_free does not wait: the block is kept (see the option "pool_bytes") and a later prad_alloc of this context may return
  * it.  With one context on the device its new work runs behind everything enqueued so far on the context's stream and on the
  * legacy default stream.  With several, which may share their blocks, that prad_alloc waits until what every one of them had
- * enqueued before the free is done.  A caller that used the block on a non-blocking stream of its own waits for that before
- * the free. */
+ * enqueued before the free is done.  A caller that uses blocks on streams of its own orders that work itself: on a non-blocking
+ * stream it is done before the free, and on any stream it begins behind the context's stream (prad_sync) where the context is
+ * alone on its device. */
 prad_status prad_alloc(prad_ctx* ctx, size_t bytes, void** out_dptr);
 prad_status prad_free(prad_ctx* ctx, void* dptr);
 prad_status prad_zero(prad_ctx* ctx, void* dptr, size_t bytes);

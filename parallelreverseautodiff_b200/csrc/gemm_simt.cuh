@@ -609,13 +609,7 @@ template <> struct ShapeCosts<double> {
   static constexpr ShapeCost c[4] = {{16, 16, 25, 15.3}, {32, 32, 54, 45.5}, {64, 32, 92, 87}, {64, 64, 163, 163}};
 };
 struct ProductSize { int64_t M, N, K, batch; };
-#ifdef PRAD_TUNE
-extern "C" { extern int prad_tune_shape; }
-#endif
 template <typename T> static int pick_shape(const prad_ctx* ctx, const ProductSize* p, int count) {
-#ifdef PRAD_TUNE
-  if (prad_tune_shape >= 0) return prad_tune_shape;
-#endif
   int best = 0;
   double best_cost = 0;
   for (int s = 0; s < (int)(sizeof(ShapeCosts<T>::c) / sizeof(ShapeCost)); ++s) {

@@ -344,7 +344,9 @@ backward_kernel(const __grid_constant__ BackwardArgs<T> p) {
 
 // ---- host side: which tile, launch --------------------------------------------------------------------------
 // Padded hidden units per CTA (8, 12 or 16; float 8 or 16: two 16-byte groups at a time) and CTAs per cluster (a power of
-// two, at most 16 -- above 8 needs the device's consent): as few padded k as the clusters allow.  Up to 256 hidden units.
+// two, at most 16 -- above 8 needs the device's consent): as few padded k as the clusters allow, and on a tie the smaller
+// CTAs, i.e. the larger cluster.  Up to 256 hidden units.  (That tie is not measured: 56 float units run on eight CTAs, 1.9 us per
+// step, where their weights would fit one.)
 struct Plan { int jp = 0, cs = 0, jj = 0; };
 template <typename T> static Plan plan_of(int nh) {
   Plan best;
@@ -411,10 +413,10 @@ static prad_status launch(prad_ctx* ctx, int cs, int nt, size_t smem, int tiles,
 }
 
 // The batch tile.  A step takes a cluster little longer for four rows than for one (double, 256 units: 3.5 .. 5.7 us), and a
-// B200 runs 7 clusters of 16 at once, 15 of 8: so the smallest tile
-// with which all clusters run at once -- five rows exist for a batch of 29 .. 35 on those 7 -- or else five or four rows in the
-// fewest turns.  PRAD_ERR_UNSUPPORTED: more turns than one launch per operation is worth, or too many hidden units for a
-// cluster's shared memory.
+// B200 runs 7 clusters of 16 at once, 15 of 8: so the smallest tile with which all clusters run at once, or else the tile with the
+// fewest turns.  Tiles have 1, 2, 4 or 5 rows (five serve 35 rows at once on those 7 clusters; three run as four, which a step
+// hardly feels; more than five are not instantiated).  PRAD_ERR_UNSUPPORTED: more turns than one launch per operation is worth, or
+// too many hidden units for a cluster's shared memory.
 constexpr int MAX_TURNS = 8;
 template <typename T, bool FORWARD, int JP, typename Args>
 static prad_status run_jp(prad_ctx* ctx, const Plan& pl, Args& a) {

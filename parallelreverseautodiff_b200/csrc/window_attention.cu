@@ -9,7 +9,7 @@
 // 7 for 49 tokens, 14 reads of shared memory per 49 multiply-adds), a row's scores in eight neighbouring lanes, so the softmax is
 // three shuffles.  P is written once (the Backward reads it); the scores and their gradients never leave the SM.  Backward:
 // dV = P^T dO first, then dP = dO V^T in registers and dS = P (.) (dP - rowsum(dP (.) P)) over P's place, then K and Q over V's and
-// dO's places and dQ = scale dS K, dK = scale dS^T Q -- 30 KB per pair, seven or eight pairs per SM.  196 us forward and 297 us
+// dO's places and dQ = scale dS K, dK = scale dS^T Q -- 30 KB per pair, seven or eight pairs per SM.  193 us forward and 295 us
 // backward, three quarters of the issue slots used, half of them by multiply-adds.
 // Sums are fused multiply-adds, k ascending (the separate products round product and sum; both within the tolerance of the
 // composition they replace: BatchMatrixMultiplyOperation, MatrixMultiplyScalarOperation, SoftmaxOperation.cs:53-109).
@@ -285,6 +285,9 @@ template <int T, int HD> static prad_status launch(prad_ctx* ctx, const Call& c)
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
+// T = ceil(window / 8), or the next height there is: T = 1, 3 and 6 are not instantiated, so windows of 17 .. 24 and 41 .. 48 tokens
+// work on the scores of 32 and 56 (4096 windows, three heads of 32: 62 us forward with 24 tokens, 71 with 32; 186 with 48, 193 with
+// 49, 108 with 40).
 template <int HD> static prad_status pick(prad_ctx* ctx, const Call& c) {
   const int t = (c.ws + 7) / 8;
   if (t <= 2) return launch<2, HD>(ctx, c);

@@ -611,11 +611,8 @@ class LstmNetwork:
         self.IG = z(TB, n_hidden)                                 # i (.) g
         self._dpre_all, self.dpre = stacked(TB, n_hidden)
         self.dX = z(TB, n_in)
-        self._tmp = [z(batch, n_hidden) for _ in range(18)]
-        self._rec_all, rec = stacked(batch, n_hidden)             # dZ_g(t) U_g for the four gates
         self._seq_scratch = z(6 * batch, n_hidden)
-        for k, g in enumerate(self.GATES):
-            self._tmp[8 + k] = rec[g]
+        self._tmp = None                                          # see _backward_steps_by_operation
 
     def set_parameters(self, W, U, b):
         for g in self.GATES:
@@ -648,7 +645,6 @@ class LstmNetwork:
         """MSE per sample and step (MeanSquaredErrorLossOperation on each [hidden x 1] column),
         BPTT, then the time- and batch-reduced weight gradients."""
         e, T, B, nh = self.eng, self.T, self.B, self.n_h
-        tmp = self._tmp
         if not self.fused_cell:
             self._backward_steps_by_operation()
         else:
@@ -669,6 +665,10 @@ class LstmNetwork:
     def _backward_steps_by_operation(self):
         """The time loop of the backward with one library call per managed operation."""
         e, T, B, nh = self.eng, self.T, self.B, self.n_h
+        if self._tmp is None:
+            self._tmp = [e.empty((B, nh), self.dtype) for _ in range(18)]
+            self._rec_all = e.empty((len(self.GATES) * B, nh), self.dtype)      # dZ_g(t) U_g for the four gates
+            self._tmp[8:12] = [self._rec_all.view((B, nh), k * B * nh) for k in range(len(self.GATES))]
         tmp = self._tmp
         dh_rec = None           # four buffers: dZ_g(t+1) * U_g
         dc_next = None          # dc_{t+1} (.) f_{t+1}
