@@ -78,6 +78,10 @@ template <typename T> __device__ __forceinline__ T amplified_sigmoid_derivative(
   return div_rn(p, t_pow(add_rn((T)1, p), (T)2));
 }
 
+__device__ __forceinline__ double sum_of_8(const double (&s)[8]) {
+  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+
 // forward value of an activation
 template <typename T> __device__ __forceinline__ T act_value(prad_act act, T x, T alpha) {
   switch (act) {

@@ -221,10 +221,10 @@ colsum_short_kernel(const T* __restrict__ x, T* __restrict__ out, int rows, int 
   sm[w][lane] = acc;
   __syncthreads();
   if (w == 0 && col < cols) {
-    double s = 0.0;
+    double s[8] = {};         // (one chain of 32 additions loses up to half a bit against eight chains of eight warps)
 #pragma unroll
-    for (int k = 0; k < 32; ++k) s += sm[k][lane];
-    put_colsum(out + blockIdx.z * out_stride + col, s, scale, accumulate);
+    for (int k = 0; k < 32; ++k) s[k % 8] += sm[k][lane];
+    put_colsum(out + blockIdx.z * out_stride + col, sum_of_8(s), scale, accumulate);
   }
 }
 template <typename T>

@@ -261,17 +261,15 @@ __device__ void run_rows(const RowProg* p, int chunk, const StartTable<N>& start
   if (p->h.kind == PRIM_COLUMN_SUM) {        // out[j] = scalar * sum of rows (scalar 1: as is)
     const int64_t j = (int64_t)chunk * NT + tid;
     if (j >= cols) return;
-    double acc = 0.0;
-    int64_t r = 0;
-    for (; r + 4 <= p->rows; r += 4) {
-      T v[4];
+    double acc[8] = {};                      // eight chains, as many as the separate kernel has at the least
+    for (int64_t r = 0; r < p->rows; r += 8) {
+      T v[8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = x[(r + q) * cols + j];
+      for (int q = 0; q < 8; ++q) v[q] = r + q < p->rows ? x[(r + q) * cols + j] : (T)0;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc += (double)v[q];
+      for (int q = 0; q < 8; ++q) acc[q] += (double)v[q];
     }
-    for (; r < p->rows; ++r) acc += (double)x[r * cols + j];
-    out[j] = (T)acc;
+    out[j] = (T)sum_of_8(acc);
     return;
   }
   if (p->h.kind == PRIM_TRANSPOSE) {

@@ -1,8 +1,11 @@
 """Products summed over a batch (strideC = 0) and column sums of a batch, against one call per matrix."""
+import math
+
 import numpy as np
 import pytest
 
 from parallelreverseautodiff_b200 import engine as E
+from parallelreverseautodiff_b200.graph import Graph
 from util import rng
 
 pytestmark = pytest.mark.gpu
@@ -80,3 +83,35 @@ def test_partial_products_count_as_scratch():
         assert eng.device_info()["scratch_bytes"] - before >= batch * n * n * 4
         a.free()
         out.free()
+
+
+@pytest.mark.parametrize("rows,where", [(n, "operation") for n in (5, 20, 45, 64, 100, 200, 512)] + [(n, "graph") for n in (5, 20, 45, 64, 100)])
+def test_column_sums_lose_no_more_than_eight_chains(engine, rows, where):
+    """Column sums in double, on average over many columns as close to the exact sum as eight chains (row r in chain r mod 8) that
+    are added one after the other: the separate kernel's order in its first form."""
+    cols = 600 if where == "operation" else 96
+    x = rng(rows).standard_normal((rows, cols))
+    chains = np.zeros((8, cols))
+    for r in range(rows):
+        chains[r % 8] += x[r]
+    eight = np.zeros(cols)
+    for c in chains:
+        eight += c
+    if where == "operation":
+        got = engine.add_broadcast_backward(engine.upload(x)).numpy()[0]
+    else:
+        g = Graph(engine, np.float64)
+        d = engine.zeros((1, cols), np.float64)
+        y = g.input(engine.zeros((rows, cols), np.float64))
+        for _ in range(40):                              # enough operations for a plan
+            y = g.node("MatrixMultiplyScalarOperation", [y], scalar=1.0)
+        out = g.node("MatrixAddBroadcastingOperation", [y, g.weight(engine.zeros((1, cols), np.float64), d)])
+        g.forward()
+        n0 = engine.launch_count()
+        g.backward(out, engine.upload(x))
+        assert engine.launch_count() - n0 == 1
+        got = d.numpy()[0]
+        g.close()
+    exact = np.array([math.fsum(c) for c in x.T])
+    rms = lambda a: np.sqrt(np.mean((a - exact) ** 2))  # noqa: E731
+    assert rms(got) <= 1.1 * rms(eight) + 1e-17          # (a tenth: the scatter of the mean over the columns)
