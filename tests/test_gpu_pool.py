@@ -1,5 +1,6 @@
 """Reuse of freed device blocks (prad_alloc / prad_free): contents, size classes, recordings, limits."""
 import multiprocessing
+import threading
 
 import numpy as np
 import pytest
@@ -189,3 +190,54 @@ def test_a_packed_operand_dropped_while_recording_is_destroyed_afterwards():
         assert not out.numpy().any()
         np.testing.assert_allclose(want, a @ a, atol=1e-5 * np.abs(a).max() ** 2 * n)
         seq.close()
+
+
+def test_threads_with_a_context_each_share_a_matrix():
+    """Four threads, a context each, allocate, free and record at the same time; all read matrices of the first thread's context,
+    which it frees and replaces while the others' work is queued."""
+    n, rounds = 300, 40
+    errors = []
+    with E.Engine(0) as e0, E.Engine(0) as e1, E.Engine(0) as e2, E.Engine(0) as e3:
+        engines = (e0, e1, e2, e3)
+        barrier = threading.Barrier(len(engines), timeout=60)
+        shared = [None]
+
+        def work(me, eng):
+            try:
+                r = np.random.default_rng(me)
+                for k in range(rounds):
+                    if me == 0:
+                        shared[0] = e0.upload(np.full((n, n), float(k + 1)))
+                        e0.sync()
+                    barrier.wait()                # the matrix of this round is there
+                    src = E.DeviceMatrix(eng, shared[0].ptr, (n, n), np.float64, owned=False)
+                    y = [eng.scale(src, float(f)) for f in range(1, 6)]
+                    barrier.wait()                # everybody's work is queued
+                    if me == 0:
+                        shared[0].free()
+                        junk = e0.upload(np.full((n, n), -1.0))
+                    a = r.standard_normal(int(r.integers(1, 200000)))
+                    m = eng.upload(a)
+                    if k % 10 == me:
+                        out = eng.empty(a.shape, a.dtype)
+                        seq = eng.record(lambda: eng.scale(m, 2.0, out=out))
+                        seq.launch()
+                        np.testing.assert_array_equal(out.numpy(), 2.0 * a)
+                        seq.close()
+                    np.testing.assert_array_equal(eng.scale(m, 3.0).numpy(), 3.0 * a)
+                    for f, v in enumerate(y, 1):
+                        np.testing.assert_array_equal(v.numpy(), np.full((n, n), f * (k + 1.0)))
+                        v.free()
+                    m.free()
+                    if me == 0:
+                        junk.free()
+            except Exception as ex:               # noqa: BLE001  (the other threads must not wait for this one)
+                errors.append((me, repr(ex)))
+                barrier.abort()
+
+        threads = [threading.Thread(target=work, args=(i, eng)) for i, eng in enumerate(engines)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(120)
+        assert not errors and not any(t.is_alive() for t in threads)
