@@ -470,7 +470,8 @@ class FeedForwardNetwork:
             self.loss_value()
             self.backward(rows_total=rows_total)
 
-        replaced = type(self) is not FeedForwardNetwork or not {"forward", "loss_value", "backward"}.isdisjoint(vars(self))
+        own = vars(self)
+        replaced = type(self) is not FeedForwardNetwork or "forward" in own or "loss_value" in own or "backward" in own
         if self.world > 1 or self.packed or replaced:      # (somebody else's methods may do more than launch)
             return run()
         # everything the launches depend on: buffers, sizes, the activation slope, library options
