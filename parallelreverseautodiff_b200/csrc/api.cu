@@ -105,6 +105,7 @@ prad_status prad_init(int device, prad_ctx** out_ctx) {
     delete c;
     return PRAD_ERR_CUDA;
   }
+  memset(c->host_flag, 0, 64);
   pool_enter(c);
   *out_ctx = c;
   g_err[0] = 0;

@@ -49,7 +49,8 @@ struct prad_ctx {
   prad::DpState* dp = nullptr;
   prad::DevicePool* pool = nullptr;
   size_t total_mem = 0;               // device memory in bytes
-  int* host_flag = nullptr;   // page-locked int that kernels write and the host reads after a wait
+  int* host_flag = nullptr;   // page-locked ints that kernels write and the host reads: [0] a bad index, [1] the ticket of the call that looked
+  int flag_ticket = 0;
   cudaStream_t branch_stream = nullptr;   // second branch of a recording
   cudaEvent_t branch_event[2] = {nullptr, nullptr};
   cudaEvent_t flag_read = nullptr;    // recorded behind the kernel that writes host_flag where others follow it

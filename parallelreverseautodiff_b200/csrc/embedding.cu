@@ -12,22 +12,47 @@ template <> struct EmbVec<double> { using type = double2; static constexpr int N
 constexpr int EMB_THREADS = 256;
 constexpr int EMB_WARPS = EMB_THREADS / 32;
 
+// Where a call's host code learns of an index outside the table: flag[0] receives 1 + an offending position, and flag[1] the call's
+// ticket once every index has been looked at.  Both lie in page-locked host memory.
+__device__ __forceinline__ void emb_bad(int* flag, int i) {
+  *(volatile int*)flag = i + 1;
+  __threadfence_system();
+}
+__device__ __forceinline__ void emb_all_checked(int* flag, int ticket) {
+  __threadfence_system();
+  *(volatile int*)(flag + 1) = ticket;
+}
+
 // EmbeddingOperation.cs:56-60: out[i] = W[(int)input[i,0]].  One warp per row, four 128-bit loads in flight per lane
-// (16384 rows of 512 floats: 20 -> 12 us against one element per thread).  `bad` receives 1 + an offending position.
+// (16384 rows of 512 floats: 20 -> 12 us against one element per thread).  The first `checkers` CTAs look at all indices
+// instead, so that the host is back 3 us after the kernel has started instead of waiting for its 9 us and the stream.
 template <typename T, bool VECTORS>
 __global__ void __launch_bounds__(EMB_THREADS)
 embedding_gather_kernel(const T* __restrict__ index_col, const T* __restrict__ W, T* __restrict__ out, int n, int vocab, int dim,
-                        int* bad) {
+                        int* flag, int ticket, int checkers, int* checked) {
   chain_begin();
+  if ((int)blockIdx.x < checkers) {
+#pragma unroll 8
+    for (int i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += checkers * EMB_THREADS) {
+      const int idx = (int)index_col[i];
+      if (idx < 0 || idx >= vocab) emb_bad(flag, i);   // the managed code would throw IndexOutOfRange
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(checked, 1) == checkers - 1) {     // the last one: the counter is ready for the next call
+        *checked = 0;
+        emb_all_checked(flag, ticket);
+      }
+    }
+    return;
+  }
   using V = typename std::conditional<VECTORS, typename EmbVec<T>::type, T>::type;
   const int lane = threadIdx.x & 31;
   const int vecs = VECTORS ? dim / EmbVec<T>::N : dim;
-  for (int i = blockIdx.x * EMB_WARPS + (threadIdx.x >> 5); i < n; i += gridDim.x * EMB_WARPS) {
+  for (int i = ((int)blockIdx.x - checkers) * EMB_WARPS + (threadIdx.x >> 5); i < n; i += ((int)gridDim.x - checkers) * EMB_WARPS) {
     const int idx = (int)index_col[i];
-    if (idx < 0 || idx >= vocab) {  // the managed code would throw IndexOutOfRange
-      if (lane == 0) *(volatile int*)bad = i + 1;
-      continue;
-    }
+    if (idx < 0 || idx >= vocab) continue;
     const V* src = reinterpret_cast<const V*>(W + (int64_t)idx * dim);
     V* dst = reinterpret_cast<V*>(out + (int64_t)i * dim);
     for (int j0 = lane; j0 < vecs; j0 += 128) {
@@ -46,115 +71,161 @@ embedding_gather_kernel(const T* __restrict__ index_col, const T* __restrict__ W
 // EmbeddingOperation.cs:69-76: dW[idx[i]][j] += dOut[i][j] for i = 0..n-1 IN THAT ORDER, bit for bit, without
 // floating-point atomics; rows nobody hit become zeros.
 //
-// The positions are grouped by row first (a counting pass, a place for every row's list, a filling pass -- integer atomics,
-// so a list arrives in any order), and whoever sums a row puts its list into input order: a warp ranks up to 32 positions
-// against each other, a CTA sorts longer lists with a bitmap over the positions.  Then every row is read and written once.
-// (With every CTA scanning the whole index column for its rows instead, a pass over 16384 indices of a 50000 x 512 table took
-// 560 us, most of it for scanning; now 12 us for the grouping and 44 for the sums, 52 with a cold cache: the table's 102 MB are 16.)
-// Rows of many hits are the commonest words of a text: the commonest of 16384 appears a thousand times, and its additions are
-// a chain, so 32 vectors of such a row have a CTA to themselves whose eight teams of threads copy rows of dOut into a ring in
-// shared memory, 48 rows ahead of the team that adds them (with 16 rows in flight in registers that one row took 150 us).  The
-// ring is 32 KB because the CTAs of the other rows, which make up most of the pass, have room for it too.
+// The positions are grouped by row first (integer atomics, so a row's list arrives in any order) while the rest of the GPU writes
+// zeros over the table.  Then only the rows that were hit are summed: whoever sums a row puts its list into input order, a warp by
+// ranking up to 32 positions against each other, a CTA by a bitmap over the positions.  16384 word-like positions, a 50000 x 512
+// float table: with a grouping of four passes by a cluster of eight CTAs and sums that wrote the zeros in the place of rows without
+// hits, eight rows a warp one after another, gather and scatter took 82 us; now 70.  8677 positions, 157 x 858 doubles: 485 -> 96.
+// Rows of many hits are the commonest words of a text: the commonest of 16384 appears over a thousand times, and its additions
+// are a chain, so 8 vectors of such a row have a CTA to themselves whose 32 teams of threads copy rows of dOut into a ring
+// in shared memory, 96 rows ahead of the team that adds them: what bounds such a row is the latency of memory over the rows in
+// flight (with 16 rows in flight in registers that one row took 150 us).
 constexpr int EMB_FEW = 32;                       // hits a warp orders by itself
-constexpr int EMB_WINDOW = 65536;                 // positions of one bitmap
-constexpr int EMB_LIST = 2048;                    // ordered positions handed to the summing loop at a time
-constexpr int EMB_ROWS = 8;                       // table rows a warp takes at once
-constexpr int EMB_GROUP = 32;                     // vectors of a row of many hits that a CTA takes
-constexpr int EMB_CHUNK = 16, EMB_CHUNKS = 4;     // rows per step of the ring, steps in the ring
+constexpr int EMB_WINDOW = 32768;                 // positions of one bitmap
+constexpr int EMB_LIST = 1024;                    // ordered positions handed to the summing loop at a time
+constexpr int EMB_GROUP = 8;                      // vectors of a row of many hits that a CTA takes
+constexpr int EMB_CHUNK = 32, EMB_CHUNKS = 4;     // rows per step of the ring, steps in the ring
 
+// The rows with hits, in `segments` parts of `stride` entries: part q has few[q] rows of few hits from its front and many[q] rows of
+// many from its back.  An entry's hits are list[offset .. offset + count), with count and offset by entry, or by row.
 struct EmbPlan {
-  int *count, *offset, *slot, *list, *hot;        // per row, per row, per position, per position, rows of many hits
-  int* cursor;                                    // [0] list entries given away, [1] rows of many hits
+  int *count, *offset, *rows, *list;
+  const int *few, *many;
+  int segments, stride;
+  bool by_row;
 };
 
+// A large call: a counting pass, a place for every row's list, a filling pass.  cursor[0]: list entries given away, and in the high
+// word the rows of few hits; cursor[1]: rows of many.  One atomic addition per warp for the places.
 template <typename T>
 __global__ void __launch_bounds__(EMB_THREADS)
-emb_count_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab, int* bad) {
+emb_count_kernel(const T* __restrict__ index_col, EmbPlan p, int* __restrict__ slot, int n, int vocab, int* bad) {
   chain_begin();
   for (int i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += gridDim.x * EMB_THREADS) {
     const int idx = (int)index_col[i];
     if (idx < 0 || idx >= vocab) *(volatile int*)bad = i + 1;
-    else p.slot[i] = atomicAdd(p.count + idx, 1);
+    else slot[i] = atomicAdd(p.count + idx, 1);
   }
 }
 __global__ void __launch_bounds__(EMB_THREADS)
-emb_place_kernel(EmbPlan p, int vocab) {
+emb_place_kernel(EmbPlan p, unsigned long long* __restrict__ cursor, int vocab) {
   chain_begin();
   const int v = blockIdx.x * EMB_THREADS + threadIdx.x, lane = threadIdx.x & 31;
-  const int c = v < vocab ? p.count[v] : 0;
-  int incl = c;
+  const int c = v < vocab ? p.count[v] : 0, few = c > 0 && c <= EMB_FEW;
+  int incl = c, rank = few;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += u;
+    const int u = __shfl_up_sync(0xffffffffu, incl, o), r = __shfl_up_sync(0xffffffffu, rank, o);
+    if (lane >= o) incl += u, rank += r;
   }
-  int base = 0;
-  if (lane == 31 && incl) base = atomicAdd(p.cursor, incl);
-  base = __shfl_sync(0xffffffffu, base, 31);
-  if (v < vocab) p.offset[v] = base + incl - c;
-  if (c > EMB_FEW) p.hot[atomicAdd(p.cursor + 1, 1)] = v;
+  unsigned long long at = 0;
+  if (lane == 31 && incl) at = atomicAdd(cursor, ((unsigned long long)rank << 32) + incl);
+  at = __shfl_sync(0xffffffffu, at, 31);
+  if (v < vocab) p.offset[v] = (int)(unsigned)at + incl - c;
+  if (few) p.rows[(int)(at >> 32) + rank - 1] = v;
+  else if (c) p.rows[p.stride - 1 - (int)atomicAdd(cursor + 1, 1ull)] = v;
 }
 template <typename T>
 __global__ void __launch_bounds__(EMB_THREADS)
-emb_fill_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab) {
+emb_fill_kernel(const T* __restrict__ index_col, EmbPlan p, const int* __restrict__ slot, int n, int vocab) {
   chain_begin();
   for (int i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += gridDim.x * EMB_THREADS) {
     const int idx = (int)index_col[i];
-    if (idx >= 0 && idx < vocab) p.list[p.offset[idx] + p.slot[i]] = i;
+    if (idx >= 0 && idx < vocab) p.list[p.offset[idx] + slot[i]] = i;
   }
 }
 
-// Counting, places and filling of a small call in one cluster of eight CTAs, a cluster barrier between the passes: as a memset
-// and three launches the grouping of 16384 positions took 15 us, most of it launches.
+// A small call in one launch: each of `segments` CTAs reads all indices and groups those of its own rows in shared memory, and the
+// indices below its rows say where its lists begin, so no CTA waits for another (as passes of a cluster over counts in L2 the
+// grouping of 16384 positions took 12 us, and more beside the zeros that the other CTAs write meanwhile).
 constexpr int EMB_PLAN_MOST = 1 << 17;            // positions and rows together
-__device__ __forceinline__ void emb_plan_barrier() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
+constexpr int EMB_SEGMENTS = 16, EMB_PLAN_THREADS = 1024;
 template <typename T>
-__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(1024)
-emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int n, int vocab, int* bad) {
-  constexpr int THREADS = 8 * 1024;
-  const int t = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31;
-  if (t < 2) p.cursor[t] = 0;
-#pragma unroll 8
-  for (int v = t; v < vocab; v += THREADS) p.count[v] = 0;
-  emb_plan_barrier();
+__global__ void __launch_bounds__(EMB_PLAN_THREADS)
+emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int* __restrict__ few, int* __restrict__ many, int n, int vocab, int* flag,
+                int ticket, uint4* __restrict__ clear, int64_t clear_vecs) {
+  chain_begin();
+  constexpr int NT = EMB_PLAN_THREADS;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, q = blockIdx.x;
+  if (q >= p.segments) {
+    const int64_t stride = (int64_t)(gridDim.x - p.segments) * NT;
 #pragma unroll 4
-  for (int i = t; i < n; i += THREADS) {
-    const int idx = (int)index_col[i];
-    if (idx < 0 || idx >= vocab) *(volatile int*)bad = i + 1;
-    else p.slot[i] = atomicAdd(p.count + idx, 1);
+    for (int64_t i = (int64_t)(q - p.segments) * NT + tid; i < clear_vecs; i += stride) clear[i] = make_uint4(0, 0, 0, 0);
+    return;
   }
-  emb_plan_barrier();
-  constexpr int K = 8;                            // rows per thread and trip: one atomic round trip for 65536 rows
-  for (int v0 = t; v0 - lane < vocab; v0 += K * THREADS) {
-    int c[K], total = 0;
+  __shared__ int place[EMB_PLAN_MOST / EMB_SEGMENTS];        // of the CTA's rows: hits, then where the next one goes
+  __shared__ int sums[4][NT / 32];
+  __shared__ int totals[4];
+  const int lo = q * p.stride, mine = vocab - lo < p.stride ? vocab - lo : p.stride;
+  for (int v = tid; v < mine; v += NT) place[v] = 0;
+  __syncthreads();
+  int below = 0;
+#pragma unroll 8
+  for (int i = tid; i < n; i += NT) {
+    const int idx = (int)index_col[i];
+    if (idx < 0 || idx >= vocab) {
+      if (q == 0) emb_bad(flag, i);
+    } else if (idx < lo) {
+      ++below;
+    } else if (idx < lo + mine) {
+      atomicAdd(place + idx - lo, 1);
+    }
+  }
+  __syncthreads();
+  if (q == 0 && tid == 0 && ticket) emb_all_checked(flag, ticket);
+  // neighbouring rows to a thread; a scan over the threads of hits, rows of few and rows of many hits
+  const int per = (mine + NT - 1) / NT, r0 = tid * per, r1 = r0 + per < mine ? r0 + per : mine;
+  int v[4] = {below, 0, 0, 0};
+  for (int r = r0; r < r1; ++r) {
+    const int c = place[r];
+    v[1] += c;
+    v[2] += c > 0 && c <= EMB_FEW;
+    v[3] += c > EMB_FEW;
+  }
+  int incl[4];
 #pragma unroll
-    for (int k = 0; k < K; ++k) c[k] = v0 + k * THREADS < vocab ? __ldcg(p.count + v0 + k * THREADS) : 0;
-#pragma unroll
-    for (int k = 0; k < K; ++k) total += c[k];
-    int incl = total;
+  for (int k = 0; k < 4; ++k) {
+    incl[k] = v[k];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += u;
+      const int u = __shfl_up_sync(0xffffffffu, incl[k], o);
+      if (lane >= o) incl[k] += u;
     }
-    int at = 0;
-    if (lane == 31 && incl) at = atomicAdd(p.cursor, incl);
-    at = __shfl_sync(0xffffffffu, at, 31) + incl - total;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int v = v0 + k * THREADS;
-      if (v < vocab) p.offset[v] = at;
-      at += c[k];
-      if (c[k] > EMB_FEW) p.hot[atomicAdd(p.cursor + 1, 1)] = v;
-    }
+    if (lane == 31) sums[k][w] = incl[k];
   }
-  emb_plan_barrier();
-#pragma unroll 4
-  for (int i = t; i < n; i += THREADS) {
+  __syncthreads();
+  if (w < 4) {
+    int x = sums[w][lane], y = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) y += u;
+    }
+    sums[w][lane] = y - x;
+    if (lane == 31) totals[w] = y;
+  }
+  __syncthreads();
+  int at = totals[0] + sums[1][w] + incl[1] - v[1], front = lo + sums[2][w] + incl[2] - v[2], back = lo + p.stride - 1 - (sums[3][w] + incl[3] - v[3]);
+  for (int r = r0; r < r1; ++r) {
+    const int c = place[r];
+    place[r] = at;
+    if (c) {
+      const int e = c <= EMB_FEW ? front++ : back--;
+      p.rows[e] = lo + r;
+      p.count[e] = c;
+      p.offset[e] = at;
+    }
+    at += c;
+  }
+  if (tid == 0) {
+    few[q] = totals[2];
+    many[q] = totals[3];
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int i = tid; i < n; i += NT) {
     const int idx = (int)index_col[i];
-    if (idx >= 0 && idx < vocab) p.list[__ldcg(p.offset + idx) + p.slot[i]] = i;
+    if (idx >= lo && idx < lo + mine) p.list[atomicAdd(place + idx - lo, 1)] = i;
   }
 }
 
@@ -178,50 +249,81 @@ template <typename T, typename V> __device__ __forceinline__ V emb_zero() {
   return v;
 }
 
-// CTAs [0, hot_ctas) take (row of many hits, group of 32 vectors) pairs, the others eight table rows per warp.
+// CTAs [0, hot_ctas) take (row of many hits, group of 8 vectors) pairs, the warps of the others (row, 64 vectors) pairs, whose
+// loads of four hits are in flight together.  A pair is a chain of three loads, so a warp reads the next pair's entry and list
+// while it sums this one's (without that, the sums of the few took longer than those of the many).
 template <typename T, bool VECTORS>
-__global__ void __launch_bounds__(EMB_THREADS)
-emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n, int vocab, int dim, int hot_ctas) {
+__global__ void __launch_bounds__(EMB_THREADS, 4)
+emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n, int dim, int hot_ctas) {
   chain_begin();
   using V = typename std::conditional<VECTORS, typename EmbVec<T>::type, T>::type;
   const int vecs = VECTORS ? dim / EmbVec<T>::N : dim;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   __shared__ int ordered[EMB_LIST];
+  // entries of one kind before each part
+  const int here = lane < p.segments ? ((int)blockIdx.x >= hot_ctas ? p.few : p.many)[lane] : 0;
+  int before = here;
+#pragma unroll
+  for (int o = 1; o < EMB_SEGMENTS; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += u;
+  }
+  const int entries = __shfl_sync(0xffffffffu, before, EMB_SEGMENTS - 1);
+  // entry g in its part, counted from the front or the back (all lanes ask for the same one)
+  auto entry = [&](int g) {
+    const int q = __popc(__ballot_sync(0xffffffffu, lane < EMB_SEGMENTS && before <= g));
+    const int k = g - __shfl_sync(0xffffffffu, before - here, q);
+    return (int)blockIdx.x >= hot_ctas ? q * p.stride + k : (q + 1) * p.stride - 1 - k;
+  };
   if ((int)blockIdx.x >= hot_ctas) {
-    const int r0 = (((int)blockIdx.x - hot_ctas) * EMB_WARPS + w) * EMB_ROWS;
     int* mine = ordered + w * EMB_FEW;
-    int cnt = 0, off = 0;
-    if (lane < EMB_ROWS && r0 + lane < vocab) {
-      cnt = p.count[r0 + lane];
-      off = p.offset[r0 + lane];
-    }
-    for (int q = 0; q < EMB_ROWS && r0 + q < vocab; ++q) {
-      const int c = __shfl_sync(0xffffffffu, cnt, q), o = __shfl_sync(0xffffffffu, off, q);
-      if (c > EMB_FEW) continue;
-      V* row = reinterpret_cast<V*>(dW + (int64_t)(r0 + q) * dim);
-      if (c == 0) {
-        for (int j = lane; j < vecs; j += 32) __stcs(row + j, emb_zero<T, V>());
-        continue;
-      }
-      const int pos = lane < c ? p.list[o + lane] : 0x7fffffff;
+    const int blocks = (vecs + 63) / 64;
+    const int64_t units = (int64_t)entries * blocks, stride = (int64_t)(gridDim.x - hot_ctas) * EMB_WARPS;
+    auto of = [&](int64_t u, int& v, int& c, int& o) {
+      const int e = entry((int)(u / blocks));
+      v = p.rows[e];
+      c = p.count[p.by_row ? v : e];
+      o = p.offset[p.by_row ? v : e];
+    };
+    int64_t u0 = ((int64_t)blockIdx.x - hot_ctas) * EMB_WARPS + w;
+    if (u0 >= units) return;
+    int v, c, o, v1 = 0, c1 = 0, o1 = 0;
+    of(u0, v, c, o);
+    int pos = lane < c ? p.list[o + lane] : 0x7fffffff;
+    if (u0 + stride < units) of(u0 + stride, v1, c1, o1);
+    for (; u0 < units; u0 += stride) {
+      int v2 = 0, c2 = 0, o2 = 0;
+      if (u0 + 2 * stride < units) of(u0 + 2 * stride, v2, c2, o2);
+      const int pos1 = lane < c1 ? p.list[o1 + lane] : 0x7fffffff;
+      const int j = (int)(u0 % blocks) * 64 + lane;
       int rank = 0;
       for (int k = 0; k < c; ++k) rank += __shfl_sync(0xffffffffu, pos, k) < pos;
       __syncwarp();
       if (lane < c) mine[rank] = pos;
       __syncwarp();
-      for (int j = lane; j < vecs; j += 32) {
-        V acc = emb_zero<T, V>();
-        for (int k0 = 0; k0 < c; k0 += 4) {
-          V x[4];
+      const bool one = j < vecs, two = j + 32 < vecs;
+      V acc0 = emb_zero<T, V>(), acc1 = emb_zero<T, V>();
+      for (int k0 = 0; k0 < c; k0 += 4) {
+        V x[4], y[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (k0 + u < c) x[u] = __ldcs(reinterpret_cast<const V*>(dOut + (int64_t)mine[k0 + u] * dim) + j);
+        for (int u = 0; u < 4; ++u)
+          if (k0 + u < c) {
+            const V* from = reinterpret_cast<const V*>(dOut + (int64_t)mine[k0 + u] * dim) + j;
+            if (one) x[u] = __ldcs(from);
+            if (two) y[u] = __ldcs(from + 32);
+          }
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (k0 + u < c) emb_add<T, V>(acc, x[u]);
-        }
-        __stcs(row + j, acc);
+        for (int u = 0; u < 4; ++u)
+          if (k0 + u < c) {
+            if (one) emb_add<T, V>(acc0, x[u]);
+            if (two) emb_add<T, V>(acc1, y[u]);
+          }
       }
+      V* to = reinterpret_cast<V*>(dW + (int64_t)v * dim) + j;
+      if (one) __stcs(to, acc0);
+      if (two) __stcs(to + 32, acc1);
+      v = v1; c = c1; o = o1; pos = pos1;
+      v1 = v2; c1 = c2; o1 = o2;
     }
     return;
   }
@@ -233,10 +335,10 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
   constexpr int TEAMS = EMB_THREADS / EMB_GROUP;
   const int team = tid / EMB_GROUP, jl = tid % EMB_GROUP;
   const int groups = (vecs + EMB_GROUP - 1) / EMB_GROUP;
-  const int64_t tasks = (int64_t)p.cursor[1] * groups;
+  const int64_t tasks = (int64_t)entries * groups;
   for (int64_t h = blockIdx.x; h < tasks; h += hot_ctas) {
-    const int v = p.hot[h / groups], j = (int)(h % groups) * EMB_GROUP + jl;
-    const int c = p.count[v], o = p.offset[v];
+    const int e = entry((int)(h / groups)), v = p.rows[e], j = (int)(h % groups) * EMB_GROUP + jl;
+    const int c = p.count[p.by_row ? v : e], o = p.offset[p.by_row ? v : e];
     const V* col = reinterpret_cast<const V*>(dOut) + j;
     V acc = emb_zero<T, V>();
     for (int w0 = 0; w0 < n; w0 += EMB_WINDOW) {
@@ -248,10 +350,10 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
         if (q >= 0 && q < EMB_WINDOW) atomicOr(bits + (q >> 5), 1u << (q & 31));
       }
       __syncthreads();
-      int here = 0;
+      int set = 0;
 #pragma unroll
-      for (int k = 0; k < WORDS; ++k) here += __popc(bits[tid * WORDS + k]);
-      int incl = here;
+      for (int k = 0; k < WORDS; ++k) set += __popc(bits[tid * WORDS + k]);
+      int incl = set;
 #pragma unroll
       for (int s = 1; s < 32; s <<= 1) {
         const int u = __shfl_up_sync(0xffffffffu, incl, s);
@@ -259,7 +361,7 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
       }
       if (lane == 31) warp_sum[w] = incl;
       __syncthreads();
-      int base = incl - here, total = 0;
+      int base = incl - set, total = 0;
 #pragma unroll
       for (int k = 0; k < EMB_WARPS; ++k) {
         if (k < w) base += warp_sum[k];
@@ -302,49 +404,88 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
   }
 }
 
+static bool emb_small(int n, int vocab) { return (int64_t)n + vocab <= EMB_PLAN_MOST; }
+
+// ticket: the call's, where `bad` is the context's flag; 0: `bad` is a plain int.  `checked` is recorded (and *waits set) where
+// the indices have been looked at once a kernel is done rather than when the ticket arrives.
 template <typename T>
 static prad_status scatter_t(prad_ctx* ctx, const void* index_col, const void* dOut, void* dW, int n, int vocab, int dim, int* bad,
-                             cudaEvent_t checked = nullptr) {
-  const size_t words = 3 * (size_t)vocab + 2 * (size_t)n + 64;
-  prad_status s = ensure_stage(ctx, words * sizeof(int));
-  if (s) return s;
-  EmbPlan p;
-  p.cursor = (int*)ctx->stage;
-  p.count = p.cursor + 64;
-  p.offset = p.count + vocab;
-  p.hot = p.offset + vocab;
-  p.slot = p.hot + vocab;
-  p.list = p.slot + n;
-  const T* idx = (const T*)index_col;
-  const bool small = (int64_t)n + vocab <= EMB_PLAN_MOST && n > 0;
-  if (!small) PRAD_CUDA(cudaMemsetAsync(p.cursor, 0, (64 + (size_t)vocab) * sizeof(int), ctx->stream));
-  if (small) {
-    emb_plan_kernel<T><<<8, 1024, 0, ctx->stream>>>(idx, p, n, vocab, bad);
-    PRAD_LAUNCHED(ctx);
-    if (checked) PRAD_CUDA(cudaEventRecord(checked, ctx->stream));       // `bad` is known
-  } else if (n > 0) {
-    const int g = stream_grid(ctx, n, EMB_THREADS, 8);
-    launch_chained(emb_count_kernel<T>, g, EMB_THREADS, 0, ctx->stream, idx, p, n, vocab, bad);
-    PRAD_LAUNCHED(ctx);
-    if (checked) PRAD_CUDA(cudaEventRecord(checked, ctx->stream));       // `bad` is known
-    launch_chained(emb_place_kernel, (unsigned)ceil_div(vocab, EMB_THREADS), EMB_THREADS, 0, ctx->stream, p, vocab);
-    PRAD_LAUNCHED(ctx);
-    launch_chained(emb_fill_kernel<T>, g, EMB_THREADS, 0, ctx->stream, idx, p, n, vocab);
-    PRAD_LAUNCHED(ctx);
+                             int ticket = 0, cudaEvent_t checked = nullptr) {
+  const int64_t table = (int64_t)vocab * dim * sizeof(T);
+  if (n == 0) {
+    PRAD_CUDA(cudaMemsetAsync(dW, 0, table, ctx->stream));
+    return PRAD_OK;
   }
-  const int hot = n > EMB_FEW ? 2 * ctx->sm_count : 0;
-  const unsigned grid = (unsigned)(hot + ceil_div(vocab, EMB_WARPS * EMB_ROWS));
+  const T* idx = (const T*)index_col;
+  const int most = n < vocab ? n : vocab;        // rows that can have hits
+  EmbPlan p;
+  prad_status s;
+  if (emb_small(n, vocab)) {
+    // 512 rows a segment or more
+    p.segments = (int)ceil_div(vocab, 512);
+    if (p.segments > EMB_SEGMENTS) p.segments = EMB_SEGMENTS;
+    p.stride = (int)ceil_div(vocab, p.segments);
+    p.segments = (int)ceil_div(vocab, p.stride);
+    p.by_row = false;
+    const size_t all = (size_t)p.segments * p.stride;
+    if ((s = ensure_stage(ctx, (64 + 3 * all + n) * sizeof(int)))) return s;
+    int* head = (int*)ctx->stage;
+    p.few = head;
+    p.many = head + EMB_SEGMENTS;
+    p.count = head + 64;
+    p.offset = p.count + all;
+    p.rows = p.offset + all;
+    p.list = p.rows + all;
+    // a table that starts off a 16-byte boundary or lies over the indices is cleared by a launch of its own
+    const bool apart = (const char*)index_col + n * sizeof(T) <= (const char*)dW || (const char*)dW + table <= (const char*)index_col;
+    const bool beside = ((uintptr_t)dW & 15) == 0 && table % 16 == 0 && apart;
+    const int64_t vecs = beside ? table / 16 : 0;
+    int clearing = (int)ceil_div(vecs, 4 * EMB_PLAN_THREADS);
+    if (clearing > 2 * ctx->sm_count - p.segments) clearing = 2 * ctx->sm_count - p.segments;
+    launch_chained(emb_plan_kernel<T>, p.segments + clearing, EMB_PLAN_THREADS, 0, ctx->stream, idx, p, head, head + EMB_SEGMENTS, n, vocab, bad, ticket, (uint4*)dW, vecs);
+    PRAD_LAUNCHED(ctx);
+    if (!beside) PRAD_CUDA(cudaMemsetAsync(dW, 0, table, ctx->stream));
+  } else {
+    if ((s = ensure_stage(ctx, (64 + 2 * (size_t)vocab + most + 2 * (size_t)n) * sizeof(int)))) return s;
+    unsigned long long* cursor = (unsigned long long*)ctx->stage;
+    p.few = (const int*)ctx->stage + 1;
+    p.many = (const int*)ctx->stage + 2;
+    p.segments = 1;
+    p.stride = most;
+    p.by_row = true;
+    p.count = (int*)ctx->stage + 64;
+    p.offset = p.count + vocab;
+    p.rows = p.offset + vocab;
+    p.list = p.rows + most;
+    int* slot = p.list + n;
+    PRAD_CUDA(cudaMemsetAsync(cursor, 0, (64 + (size_t)vocab) * sizeof(int), ctx->stream));
+    const int g = stream_grid(ctx, n, EMB_THREADS, 8);
+    launch_chained(emb_count_kernel<T>, g, EMB_THREADS, 0, ctx->stream, idx, p, slot, n, vocab, bad);
+    PRAD_LAUNCHED(ctx);
+    if (checked) PRAD_CUDA(cudaEventRecord(checked, ctx->stream));       // `bad` is known
+    launch_chained(emb_place_kernel, (unsigned)ceil_div(vocab, EMB_THREADS), EMB_THREADS, 0, ctx->stream, p, cursor, vocab);
+    PRAD_LAUNCHED(ctx);
+    launch_chained(emb_fill_kernel<T>, g, EMB_THREADS, 0, ctx->stream, idx, p, slot, n, vocab);
+    PRAD_LAUNCHED(ctx);
+    PRAD_CUDA(cudaMemsetAsync(dW, 0, table, ctx->stream));
+  }
+  // as many CTAs as can have work, and no more than two an SM for either kind of row: all of them run at once
+  const bool vectors = dim % EmbVec<T>::N == 0 && (((uintptr_t)dOut | (uintptr_t)dW) & 15) == 0;
+  const int vecs = vectors ? dim / EmbVec<T>::N : dim;
+  auto at_most = [&](int64_t wanted, int per_sm) { return (int)(wanted < (int64_t)per_sm * ctx->sm_count ? wanted : (int64_t)per_sm * ctx->sm_count); };
+  const int hot = at_most(n / (EMB_FEW + 1) * ceil_div(vecs, EMB_GROUP), 2);
+  const int grid = hot + at_most(ceil_div((int64_t)most * ceil_div(vecs, 64), EMB_WARPS), 2);
   // shared memory for the ring only where a row can have many hits
-  if (dim % EmbVec<T>::N == 0 && (((uintptr_t)dOut | (uintptr_t)dW) & 15) == 0) {
+  if (vectors) {
     constexpr int ring = EMB_CHUNKS * EMB_CHUNK * EMB_GROUP * 16;
     s = allow_smem<emb_sum_kernel<T, true>>(ctx, ring);
     if (s) return s;
-    launch_chained(emb_sum_kernel<T, true>, grid, EMB_THREADS, hot ? ring : 0, ctx->stream, (const T*)dOut, (T*)dW, p, n, vocab, dim, hot);
+    launch_chained(emb_sum_kernel<T, true>, grid, EMB_THREADS, hot ? ring : 0, ctx->stream, (const T*)dOut, (T*)dW, p, n, dim, hot);
   } else {
     constexpr int ring = EMB_CHUNKS * EMB_CHUNK * EMB_GROUP * (int)sizeof(T);
     s = allow_smem<emb_sum_kernel<T, false>>(ctx, ring);
     if (s) return s;
-    launch_chained(emb_sum_kernel<T, false>, grid, EMB_THREADS, hot ? ring : 0, ctx->stream, (const T*)dOut, (T*)dW, p, n, vocab, dim, hot);
+    launch_chained(emb_sum_kernel<T, false>, grid, EMB_THREADS, hot ? ring : 0, ctx->stream, (const T*)dOut, (T*)dW, p, n, dim, hot);
   }
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
@@ -358,22 +499,41 @@ prad_status embedding_scatter_ordered(prad_ctx* ctx, prad_dtype dt, const void* 
                         : scatter_t<double>(ctx, index_col, dOut, dW, n, vocab, dim, bad);
 }
 
-// The offending position of a call arrives in page-locked host memory, so the check costs the wait alone.
-static prad_status check_bad_index(prad_ctx* ctx, const char* who, cudaEvent_t checked = nullptr) {
-  if (checked) PRAD_CUDA(cudaEventSynchronize(checked));
-  else PRAD_CUDA(cudaStreamSynchronize(ctx->stream));
+// A call's flag words, cleared for it; every call has another ticket.
+static int next_ticket(prad_ctx* ctx) {
+  *(volatile int*)ctx->host_flag = 0;
+  if (++ctx->flag_ticket <= 0) ctx->flag_ticket = 1;
+  return ctx->flag_ticket;
+}
+static prad_status check_bad_index(prad_ctx* ctx, const char* who) {
   const int h = *(volatile int*)ctx->host_flag;
   PRAD_REQUIRE(h == 0, PRAD_ERR_INVALID, "%s: index at input row %d is outside [0, vocab)", who, h - 1);
   return PRAD_OK;
 }
+// Waits until the call's ticket is in host memory, which the kernel writes before its other work is done, so that the host is
+// ahead of the GPU.  A stream that has stopped or come to its end without it ends the wait.
+static prad_status wait_ticket(prad_ctx* ctx, const char* who, int ticket) {
+  volatile int* arrived = ctx->host_flag + 1;
+  for (unsigned polls = 1; *arrived != ticket; ++polls) {
+    if (polls % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(ctx->stream);
+    if (e == cudaErrorNotReady) continue;
+    if (e == cudaSuccess && *arrived == ticket) break;
+    (void)cudaGetLastError();
+    PRAD_REQUIRE(false, PRAD_ERR_CUDA, "%s failed: %s", who, e == cudaSuccess ? "the indices were not looked at" : cudaGetErrorString(e));
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return check_bad_index(ctx, who);
+}
 
 template <typename T>
-static prad_status gather_t(prad_ctx* ctx, const void* index_col, const void* W, void* out, int n, int vocab, int dim) {
+static prad_status gather_t(prad_ctx* ctx, const void* index_col, const void* W, void* out, int n, int vocab, int dim, int ticket) {
   const int grid = stream_grid(ctx, n, EMB_WARPS, 8);
-  if (dim % EmbVec<T>::N == 0 && (((uintptr_t)W | (uintptr_t)out) & 15) == 0)
-    launch_chained(embedding_gather_kernel<T, true>, grid, EMB_THREADS, 0, ctx->stream, (const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag);
-  else
-    launch_chained(embedding_gather_kernel<T, false>, grid, EMB_THREADS, 0, ctx->stream, (const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag);
+  int checkers = (int)ceil_div(n, 8 * EMB_THREADS);        // eight loads in flight per thread
+  if (checkers > ctx->sm_count) checkers = ctx->sm_count;
+  const bool vectors = dim % EmbVec<T>::N == 0 && (((uintptr_t)W | (uintptr_t)out) & 15) == 0;
+  launch_chained(vectors ? embedding_gather_kernel<T, true> : embedding_gather_kernel<T, false>, checkers + grid, EMB_THREADS, 0, ctx->stream,
+                 (const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag, ticket, checkers, ctx->tc_err + 48);
   PRAD_LAUNCHED(ctx);
   return PRAD_OK;
 }
@@ -392,9 +552,10 @@ prad_status prad_embedding_forward(prad_ctx* ctx, prad_dtype dt, const void* ind
   if (n == 0 || dim == 0) return PRAD_OK;
   PRAD_REQUIRE(index_col && W && out, PRAD_ERR_INVALID, "prad_embedding_forward: null pointer");
   PRAD_NOT_CAPTURING(ctx, "prad_embedding_forward");   // the index check reads a flag back
-  *(volatile int*)ctx->host_flag = 0;
-  prad_status s = dt == PRAD_F32 ? gather_t<float>(ctx, index_col, W, out, n, vocab, dim) : gather_t<double>(ctx, index_col, W, out, n, vocab, dim);
-  return s ? s : check_bad_index(ctx, "prad_embedding_forward");
+  const int ticket = next_ticket(ctx);
+  prad_status s = dt == PRAD_F32 ? gather_t<float>(ctx, index_col, W, out, n, vocab, dim, ticket)
+                                 : gather_t<double>(ctx, index_col, W, out, n, vocab, dim, ticket);
+  return s ? s : wait_ticket(ctx, "prad_embedding_forward", ticket);
 }
 
 prad_status prad_embedding_backward(prad_ctx* ctx, prad_dtype dt, const void* index_col,
@@ -406,12 +567,15 @@ prad_status prad_embedding_backward(prad_ctx* ctx, prad_dtype dt, const void* in
   PRAD_REQUIRE(dW && (n == 0 || (index_col && dOut)), PRAD_ERR_INVALID,
                "prad_embedding_backward: null pointer");
   PRAD_NOT_CAPTURING(ctx, "prad_embedding_backward");
-  *(volatile int*)ctx->host_flag = 0;
+  const int ticket = next_ticket(ctx);
   // the indices have been looked at once the first kernel is done: the caller need not wait for the sums
   if (!ctx->flag_read) PRAD_CUDA(cudaEventCreateWithFlags(&ctx->flag_read, cudaEventDisableTiming));
-  prad_status s = dt == PRAD_F32 ? scatter_t<float>(ctx, index_col, dOut, dW, n, vocab, dim, ctx->host_flag, ctx->flag_read)
-                                 : scatter_t<double>(ctx, index_col, dOut, dW, n, vocab, dim, ctx->host_flag, ctx->flag_read);
-  return s || n == 0 ? s : check_bad_index(ctx, "prad_embedding_backward", ctx->flag_read);
+  prad_status s = dt == PRAD_F32 ? scatter_t<float>(ctx, index_col, dOut, dW, n, vocab, dim, ctx->host_flag, ticket, ctx->flag_read)
+                                 : scatter_t<double>(ctx, index_col, dOut, dW, n, vocab, dim, ctx->host_flag, ticket, ctx->flag_read);
+  if (s || n == 0) return s;
+  if (emb_small(n, vocab)) return wait_ticket(ctx, "prad_embedding_backward", ticket);
+  PRAD_CUDA(cudaEventSynchronize(ctx->flag_read));
+  return check_bad_index(ctx, "prad_embedding_backward");
 }
 
 }  // extern "C"

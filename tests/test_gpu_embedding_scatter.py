@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 
 import oracle as O
+from parallelreverseautodiff_b200._lib import PradError
 from util import rng
 
 pytestmark = pytest.mark.gpu
@@ -21,3 +22,38 @@ def test_scatter_in_input_order(engine, dtype, n, vocab, dim, hot):
     i, d = engine.upload(col), engine.upload(dOut)
     np.testing.assert_array_equal(engine.embedding_backward(i, d, vocab).numpy(), O.embedding_backward(col, dOut, vocab))
     np.testing.assert_array_equal(engine.embedding_forward(i, engine.upload(W)).numpy(), O.embedding_forward(col, W))
+
+
+@pytest.mark.parametrize("dtype,dim", [(np.float32, 20), (np.float64, 3)])
+@pytest.mark.parametrize("n,vocab", [(2500, 511), (2500, 512), (2500, 513), (3000, 7681), (3000, 8192), (3000, 8193), (40000, 91072), (40000, 91073)])
+def test_scatter_at_the_edges_of_the_grouping(engine, dtype, dim, n, vocab):
+    """Row counts on both sides of a segment, of sixteen of them and of what one launch groups; rows of 0, 1, 4, 5, 32, 33 and many
+    hits at both ends of the table; a table that does not start at a 16-byte boundary."""
+    r = rng(n + vocab + dim)
+    idx = r.integers(0, vocab, n)
+    at = 0
+    for row, hits in ((0, 33), (vocab - 1, 32), (1, 5), (vocab - 2, 4), (2, 1), (vocab // 2, 700)):
+        idx[at:at + hits] = row
+        at += hits
+    idx = r.permutation(idx)
+    col = idx.astype(dtype).reshape(n, 1)
+    dOut = (r.standard_normal((n, dim)) * 10.0 ** r.integers(-3, 4, (n, 1))).astype(dtype)
+    expected = O.embedding_backward(col, dOut, vocab)
+    i, d = engine.upload(col), engine.upload(dOut)
+    np.testing.assert_array_equal(engine.embedding_backward(i, d, vocab).numpy(), expected)
+    room = engine.upload(np.full((1, vocab * dim + 1), np.nan, dtype))
+    odd = room.view((vocab, dim), 1)
+    engine.embedding_backward(i, d, vocab, out=odd)
+    np.testing.assert_array_equal(odd.numpy(), expected)
+
+
+def test_bad_indices_are_told_apart_from_the_calls_after_them(engine):
+    W, d = engine.upload(np.ones((5, 4), np.float32)), engine.upload(np.ones((3, 4), np.float32))
+    good, bad = (engine.upload(np.array(v, np.float32).reshape(3, 1)) for v in ([0, 4, 4], [1, 5, 2]))
+    for _ in range(3):
+        with pytest.raises(PradError):
+            engine.embedding_forward(bad, W)
+        assert engine.embedding_forward(good, W).numpy().sum() == 12
+        with pytest.raises(PradError):
+            engine.embedding_backward(bad, d, 5)
+        np.testing.assert_array_equal(engine.embedding_backward(good, d, 5).numpy()[:, 0], [1, 0, 0, 0, 2])
