@@ -32,7 +32,7 @@ struct MultiTensor {
   int blk_start[MT_MAX + 1];
   int count;
   int chunk;  // elements a CTA covers, a multiple of MT_THREADS 16-byte vectors
-  bool fold;  // few partial sums per tensor: every CTA adds them up itself, in the order of mt_finalize_kernel
+  bool fold;  // few partial sums per tensor: every CTA adds them up itself, as mt_finalize_kernel would
 };
 
 __device__ __forceinline__ int find_tensor(const MultiTensor& t, int blk) {
@@ -48,37 +48,99 @@ __device__ __forceinline__ int find_tensor(const MultiTensor& t, int blk) {
 // [2*MT_MAX] global sum of squares, then the per-CTA partials.
 constexpr int ST_MEAN = 0, ST_STD = MT_MAX, ST_SS = 2 * MT_MAX, ST_PART = 2 * MT_MAX + 8;
 
-// Sum of a tensor's partial sums, in CTA order by a fixed tree; all threads get it.
-__device__ __forceinline__ double add_partials(const MultiTensor& t, int ti, const double* part) {
-  double acc = 0.0;
-  for (int b = t.blk_start[ti] + threadIdx.x; b < t.blk_start[ti + 1]; b += MT_THREADS) acc += part[b];
-  return block_sum_d<MT_THREADS>(acc);
-}
 template <typename T> __device__ __forceinline__ T mean_of(double s, int64_t size) { return div_rn((T)s, (T)size); }            // sum / count
 template <typename T> __device__ __forceinline__ T sigma_of(double s, int64_t size) { return sqrt_rn(div_rn((T)s, (T)size)); }  // Sqrt(varianceSum / count)
 
-// The partial sums of kind 1 follow those of kind 0 (the other kinds use the first place).
-__device__ __forceinline__ int part_at(const MultiTensor& t, int kind) { return ST_PART + (kind == 1 ? t.blk_start[t.count] : 0); }
+// Where the sums of squared deviations begin; the other partial sums are at ST_PART.
+__device__ __forceinline__ int squares_at(const MultiTensor& t) { return ST_PART + t.blk_start[t.count]; }
 
-// pass kinds: 0 = sum g ; 1 = sum (g-mean)^2 (T arithmetic for the square, as Pow(v-mean,2)
-// rounds to T in the float build) ; 2 = sum g^2 in double (global norm)
+// A tensor's mean and standard deviation from what its CTAs left: partial sums in CTA order by a fixed tree, and squares about
+// each CTA's own mean, moved to the common one: sum (x - mean)^2 = sum_b [sum (x - mean_b)^2 + n_b (mean_b - mean)^2].
+// All threads get them.
+template <typename T>
+__device__ __forceinline__ void tensor_stats(const MultiTensor& t, int ti, const double* __restrict__ stats, T* mean, T* sd) {
+  const int b0 = t.blk_start[ti], blocks = t.blk_start[ti + 1] - b0;
+  const double *sums = stats + ST_PART + b0, *squares = stats + squares_at(t) + b0;
+  const int64_t size = t.size[ti];
+  const bool mine = (int)threadIdx.x < blocks;
+  const double s0 = mine ? sums[threadIdx.x] : 0.0, q0 = mine ? squares[threadIdx.x] : 0.0;
+  double acc = s0;
+  for (int b = threadIdx.x + MT_THREADS; b < blocks; b += MT_THREADS) acc += sums[b];
+  const double total = block_sum_d<MT_THREADS>(acc);
+  *mean = mean_of<T>(total, size);
+  if (blocks == 1) {                       // about the mean itself already
+    *sd = sigma_of<T>(block_sum_d<MT_THREADS>(q0), size);
+    return;
+  }
+  const double mu = total / (double)size;
+  auto moved = [&](int b, double s, double q) {
+    const int64_t left = size - (int64_t)b * t.chunk;
+    const double n = (double)(left < t.chunk ? left : t.chunk), d = s / n - mu;
+    return q + n * d * d;
+  };
+  double var = mine ? moved(threadIdx.x, s0, q0) : 0.0;
+  for (int b = threadIdx.x + MT_THREADS; b < blocks; b += MT_THREADS) var += moved(b, sums[b], squares[b]);
+  *sd = sigma_of<T>(block_sum_d<MT_THREADS>(var), size);
+}
+
+// What the reference's clip has to know of a gradient (GradientClipper.cs:120-127), one pass over it: a CTA adds its values up
+// and then, from registers, the squares of their deviations from its own mean.  A tensor of one CTA takes the mean and the
+// squares as the float build does, rounded to T; else both are double.  (Mean and squares as a pass each: 4.3 + 5.5 us of a
+// 670 000-parameter step's 19.5 us for clip and Adam, and a second read of a large network's gradients.)
 template <typename T>
 __global__ void __launch_bounds__(MT_THREADS)
-mt_partial_kernel(MultiTensor t, double* __restrict__ stats, int kind) {
+mt_stats_kernel(MultiTensor t, double* __restrict__ stats) {
+  chain_begin();
+  constexpr int VEC = 16 / sizeof(T), TRIPS = MT_CHUNK / (MT_THREADS * VEC);
+  using V = typename MtVec<T>::type;
+  const int ti = find_tensor(t, blockIdx.x), blocks = t.blk_start[ti + 1] - t.blk_start[ti];
+  const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
+  int64_t end = start + t.chunk;
+  if (end > t.size[ti]) end = t.size[ti];
+  const T* g = (const T*)t.g[ti];
+  const int64_t vend = t.vec ? end - (end - start) % VEC : start;      // chunk starts are multiples of the vector width
+  const int64_t first = start + (int64_t)threadIdx.x * VEC;
+  V v[TRIPS];
+  double acc = 0.0;
+#pragma unroll
+  for (int k = 0; k < TRIPS; ++k)
+    if (first + k * MT_THREADS * VEC < vend) v[k] = *reinterpret_cast<const V*>(g + first + k * MT_THREADS * VEC);
+  auto each = [&](auto&& f) {
+#pragma unroll
+    for (int k = 0; k < TRIPS; ++k)
+      if (first + k * MT_THREADS * VEC < vend)
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) f(reinterpret_cast<const T*>(&v[k])[q]);
+    for (int64_t i = vend + threadIdx.x; i < end; i += MT_THREADS) f(g[i]);
+  };
+  each([&](T x) { acc += (double)x; });
+  const double s = block_sum_d<MT_THREADS>(acc);
+  double sq = 0.0;
+  if (blocks == 1) {
+    const T mean = mean_of<T>(s, t.size[ti]);
+    each([&](T x) { const T d = sub_rn(x, mean); sq += (double)mul_rn(d, d); });
+  } else {
+    const double mean = s / (double)(end - start);
+    each([&](T x) { const double d = (double)x - mean; sq = __fma_rn(d, d, sq); });
+  }
+  sq = block_sum_d<MT_THREADS>(sq);
+  if (threadIdx.x == 0) {
+    stats[ST_PART + blockIdx.x] = s;
+    stats[squares_at(t) + blockIdx.x] = sq;
+  }
+}
+
+// sum g^2 in double (global norm)
+template <typename T>
+__global__ void __launch_bounds__(MT_THREADS)
+mt_norm_kernel(MultiTensor t, double* __restrict__ stats) {
   chain_begin();
   const int ti = find_tensor(t, blockIdx.x);
   const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
   int64_t end = start + t.chunk;
   if (end > t.size[ti]) end = t.size[ti];
   const T* g = (const T*)t.g[ti];
-  T mean = (T)0;
-  if (kind == 1) mean = t.fold ? mean_of<T>(add_partials(t, ti, stats + ST_PART), t.size[ti]) : (T)stats[ST_MEAN + ti];
   double acc = 0.0;
-  auto term = [&](T x) {
-    if (kind == 0) acc += (double)x;
-    else if (kind == 1) { T d = sub_rn(x, mean); acc += (double)mul_rn(d, d); }
-    else acc += (double)x * (double)x;
-  };
   int64_t i0 = start;
   if (t.vec) {    // 128-bit loads; chunk starts are multiples of the vector width
     constexpr int VEC = 16 / sizeof(T);
@@ -87,24 +149,24 @@ mt_partial_kernel(MultiTensor t, double* __restrict__ stats, int kind) {
     for (int64_t i = start + (int64_t)threadIdx.x * VEC; i < vend; i += MT_THREADS * VEC) {
       V v = *reinterpret_cast<const V*>(g + i);
 #pragma unroll
-      for (int q = 0; q < VEC; ++q) term(reinterpret_cast<const T*>(&v)[q]);
+      for (int q = 0; q < VEC; ++q) { const double x = (double)reinterpret_cast<const T*>(&v)[q]; acc += x * x; }
     }
     i0 = vend;
   }
-  for (int64_t i = i0 + threadIdx.x; i < end; i += MT_THREADS) term(g[i]);
+  for (int64_t i = i0 + threadIdx.x; i < end; i += MT_THREADS) acc += (double)g[i] * (double)g[i];
   double s = block_sum_d<MT_THREADS>(acc);
-  if (threadIdx.x == 0) stats[part_at(t, kind) + blockIdx.x] = s;
+  if (threadIdx.x == 0) stats[ST_PART + blockIdx.x] = s;
 }
 
-// one CTA per tensor adds that tensor's partials in CTA order (fixed tree)
+// one CTA per tensor of many partial sums
 template <typename T>
 __global__ void __launch_bounds__(MT_THREADS)
-mt_finalize_kernel(MultiTensor t, double* __restrict__ stats, int kind) {
-  const int ti = blockIdx.x;
-  const double s = add_partials(t, ti, stats + part_at(t, kind));
+mt_finalize_kernel(MultiTensor t, double* __restrict__ stats) {
+  T mean, sd;
+  tensor_stats<T>(t, blockIdx.x, stats, &mean, &sd);
   if (threadIdx.x == 0) {
-    if (kind == 0) stats[ST_MEAN + ti] = (double)mean_of<T>(s, t.size[ti]);
-    else stats[ST_STD + ti] = (double)sigma_of<T>(s, t.size[ti]);
+    stats[ST_MEAN + blockIdx.x] = (double)mean;
+    stats[ST_STD + blockIdx.x] = (double)sd;
   }
 }
 // global norm: every partial of every tensor, one CTA
@@ -174,7 +236,7 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
   // A tensor-core product on this context ran out of a bounded wait: the gradients on the stream are
   // not valid, so weights, moments and gradients are left exactly as they are (one load per CTA; the
   // host learns of it at its next prad_sync / prad_download, which returns PRAD_ERR_TIMEOUT).
-  if (gemm_gave_up && *gemm_gave_up != 0) return;
+  const int gave_up = gemm_gave_up ? *gemm_gave_up : 0;
   const int ti = find_tensor(t, blockIdx.x);
   const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
   int64_t end = start + t.chunk;
@@ -185,15 +247,30 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
   T* v = (T*)t.v[ti];
   T mean = 0, sd = 1, gscale = 1;
   bool scale_on = false;
+  constexpr int VEC = 16 / sizeof(T);
+  using V = typename MtVec<T>::type;
+  const int64_t vend = t.vec ? end - (end - start) % VEC : start;
+  // the first trip's values are on their way while the statistics are put together
+  V gv, wv, mv, vv;
+  auto load = [&](int64_t i) {
+    gv = *reinterpret_cast<const V*>(g + i);
+    if (do_adam) {
+      wv = *reinterpret_cast<const V*>(w + i);
+      mv = *reinterpret_cast<const V*>(m + i);
+      vv = *reinterpret_cast<const V*>(v + i);
+    }
+  };
+  int64_t i = start + (int64_t)threadIdx.x * VEC;
+  if (i < vend) load(i);
   if (clip_mode == 1) {
     if (t.fold) {
-      mean = mean_of<T>(add_partials(t, ti, stats + ST_PART), t.size[ti]);
-      sd = sigma_of<T>(add_partials(t, ti, stats + part_at(t, 1)), t.size[ti]);
+      tensor_stats<T>(t, ti, stats, &mean, &sd);
     } else {
       mean = (T)stats[ST_MEAN + ti];
       sd = (T)stats[ST_STD + ti];
     }
   }
+  if (gave_up) return;
   if (clip_mode == 2) {
     double norm = sqrt(stats[ST_SS]);
     if (norm > max_norm) { gscale = (T)(max_norm / norm); scale_on = true; }
@@ -203,36 +280,24 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
     if (scale_on) return mul_rn(gi, gscale);
     return gi;
   };
-  int64_t i0 = start;
-  if (t.vec) {
-    constexpr int VEC = 16 / sizeof(T);
-    using V = typename MtVec<T>::type;
-    const int64_t vend = end - ((end - start) % VEC);
-    for (int64_t i = start + (int64_t)threadIdx.x * VEC; i < vend; i += MT_THREADS * VEC) {
-      V gv = *reinterpret_cast<const V*>(g + i);
-      V wv, mv, vv;
-      if (do_adam) {
-        wv = *reinterpret_cast<const V*>(w + i);
-        mv = *reinterpret_cast<const V*>(m + i);
-        vv = *reinterpret_cast<const V*>(v + i);
-      }
+  while (i < vend) {
 #pragma unroll
-      for (int q = 0; q < VEC; ++q) {
-        T gi = clip_one(reinterpret_cast<T*>(&gv)[q]);
-        if (do_adam)
-          adam_value<T>(a, gi, reinterpret_cast<T*>(&wv)[q], reinterpret_cast<T*>(&mv)[q], reinterpret_cast<T*>(&vv)[q]);
-        reinterpret_cast<T*>(&gv)[q] = zero_grad ? (T)0 : gi;
-      }
-      if (do_adam) {
-        *reinterpret_cast<V*>(w + i) = wv;
-        *reinterpret_cast<V*>(m + i) = mv;
-        *reinterpret_cast<V*>(v + i) = vv;
-      }
-      if (zero_grad || clip_mode != 0) *reinterpret_cast<V*>(g + i) = gv;
+    for (int q = 0; q < VEC; ++q) {
+      T gi = clip_one(reinterpret_cast<T*>(&gv)[q]);
+      if (do_adam)
+        adam_value<T>(a, gi, reinterpret_cast<T*>(&wv)[q], reinterpret_cast<T*>(&mv)[q], reinterpret_cast<T*>(&vv)[q]);
+      reinterpret_cast<T*>(&gv)[q] = zero_grad ? (T)0 : gi;
     }
-    i0 = vend;
+    if (do_adam) {
+      *reinterpret_cast<V*>(w + i) = wv;
+      *reinterpret_cast<V*>(m + i) = mv;
+      *reinterpret_cast<V*>(v + i) = vv;
+    }
+    if (zero_grad || clip_mode != 0) *reinterpret_cast<V*>(g + i) = gv;
+    i += MT_THREADS * VEC;
+    if (i < vend) load(i);
   }
-  for (int64_t i = i0 + threadIdx.x; i < end; i += MT_THREADS) {
+  for (int64_t i = vend + threadIdx.x; i < end; i += MT_THREADS) {
     T gi = clip_one(g[i]);
     if (do_adam) {
       T wi = w[i], mi = m[i], vi = v[i];
@@ -319,7 +384,7 @@ static prad_status clip_adam_t(prad_ctx* ctx, void* const* w, void* const* g, vo
     for (int first = 0; first < count; first += MT_MAX) {
       int cnt = count - first < MT_MAX ? count - first : MT_MAX;
       int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
-      launch_chained(mt_partial_kernel<T>, nb, MT_THREADS, 0, ctx->stream, t, stats, 2);
+      launch_chained(mt_norm_kernel<T>, nb, MT_THREADS, 0, ctx->stream, t, stats);
       PRAD_LAUNCHED(ctx);
       mt_finalize_ss_kernel<<<1, MT_THREADS, 0, ctx->stream>>>(nb, stats, first > 0);
       PRAD_LAUNCHED(ctx);
@@ -329,11 +394,10 @@ static prad_status clip_adam_t(prad_ctx* ctx, void* const* w, void* const* g, vo
     int cnt = count - first < MT_MAX ? count - first : MT_MAX;
     int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
     if (clip_mode == 1) {
-      for (int kind = 0; kind < 2; ++kind) {
-        launch_chained(mt_partial_kernel<T>, nb, MT_THREADS, 0, ctx->stream, t, stats, kind);
-        PRAD_LAUNCHED(ctx);
-        if (t.fold) continue;
-        mt_finalize_kernel<T><<<cnt, MT_THREADS, 0, ctx->stream>>>(t, stats, kind);
+      launch_chained(mt_stats_kernel<T>, nb, MT_THREADS, 0, ctx->stream, t, stats);
+      PRAD_LAUNCHED(ctx);
+      if (!t.fold) {
+        mt_finalize_kernel<T><<<cnt, MT_THREADS, 0, ctx->stream>>>(t, stats);
         PRAD_LAUNCHED(ctx);
       }
     }

@@ -12,24 +12,19 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// all threads of the block must call; result valid in thread 0 (and broadcast to all)
+// all threads of the block must call; all of them get the result
 template <int THREADS>
 __device__ __forceinline__ double block_sum_d(double v) {
   __shared__ double warp_tot[THREADS / 32];
-  __shared__ double total;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   v = warp_sum_d(v);
-  __syncthreads();  // protects warp_tot/total across back-to-back calls
+  __syncthreads();  // protects warp_tot across back-to-back calls
   if (lane == 0) warp_tot[w] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
+  double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < THREADS / 32; ++k) s += warp_tot[k];
-    total = s;
-  }
-  __syncthreads();
-  return total;
+  for (int k = 0; k < THREADS / 32; ++k) s += warp_tot[k];
+  return s;
 }
 
 }  // namespace prad
