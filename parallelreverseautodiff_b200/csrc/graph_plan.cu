@@ -6,11 +6,15 @@
 // Here the walk is recorded once as a list of primitive operations.  A level of the plan holds operations that depend on
 // earlier levels only; chains of elementwise operations on the same elements (a gate's sum and activation, a cell update, the
 // += of a shared weight's gradients over the time steps) share a level too, as a small program that keeps every value of one
-// element in shared memory from its load to its store.  One cluster of 16 CTAs runs the levels with the cluster's hardware
-// barrier between them (no waiting loops, no other CTA to wait for).  A level is latency: a barrier, a program, loads from L2,
-// a chain of 64 additions.  So the pieces of a level -- 64 or 256 elements, 256 or 1024 outputs -- are dealt to 64 workers when
-// the plan is made, four to an SM, and a worker fetches its next program while it runs this one. 
-// (One worker per SM took 240 us per walk of that LSTM, four take 150 us.)
+// element in shared memory from its load to its store, and such a program computes the products that it reads, where they are
+// small, for its own elements: a cell of an LSTM is one level instead of a level of products and one of programs.  One cluster of
+// 16 CTAs runs the levels with the cluster's hardware barrier between them (no waiting loops, no other CTA to wait for).  What
+// nothing waits for (weight gradients, outputs) comes as late as it can, and large levels at the end run on all SMs, as launches of
+// their own.  A level is latency: a barrier (1.1 us), a program (1.7), operands from L2 (1.2), a chain of 64 additions (1.5).  So
+// the pieces of a level -- 32, 64 or 256 elements, 256 or 1024 outputs -- are dealt to 32 workers when the plan is made, two to an
+// SM, and a worker fetches its next program while it runs this one.  The eight-step two-layer LSTM of 64 units and 8 columns, both
+// walks, losses and optimiser: 297 us with 22 levels each way and four workers of 64 registers (their spilled values went through
+// L2 after every barrier, which emptied the L1), 172 us now.
 //
 // Values are those of the separate kernels bit for bit for elementwise operations and products (k ascending, product and sum
 // rounded separately); row reductions and column sums add in double or in the same lane order.  (Compiled with -fmad=false.)
@@ -25,23 +29,32 @@ namespace prad {
 namespace gp {
 
 constexpr int NT = 256;                   // threads of a worker
-constexpr int WORKERS = 4;                // workers of a CTA: a piece is mostly latency, so several share an SM
+constexpr int WORKERS = 2;                // workers of a CTA: a piece is mostly latency, so two share an SM; 126 registers, no spills
 constexpr int SLOTS = 64;                 // values of one element a program keeps
 constexpr int MAX_INS = 96;
-constexpr int PROG_BYTES = 32 + SLOTS * 16 + MAX_INS * 24 + SLOTS * 16;
-constexpr int WORK_BYTES = 44 * 1024;     // a worker's shared memory: the slots of its elements, or the operands of a product
+constexpr int MAX_DOTS = 16;              // products a program computes for its own elements
+constexpr int MAX_TASKS = 64;             // copies their operands are cut into
+constexpr int PROG_BYTES = 64 + SLOTS * 16 + MAX_INS * 24 + SLOTS * 16 + MAX_TASKS * 32 + MAX_DOTS * 24;
+constexpr int WORK_BYTES = 88 * 1024;     // a worker's shared memory: the slots of its elements, or the operands of a product
 
 // a piece of one worker
 struct Item { uint32_t prog, bytes, chunk, barrier; };
 
-// team: 4 where four threads share an element's instructions (a piece is 64 elements then), else 1
-struct Head { int32_t kind, n_load, n_ins, n_store; int64_t n; int64_t team; };
+// team: how many threads share an element's instructions: 8 (a piece is 32 elements then) where it has products, 4 or 1
+// n_dot products of rows x dot_n outputs, ks values of k of their n_opd operands at a time, from work_at values on
+struct Head { int32_t kind, n_load, n_ins, n_store; int64_t n; int32_t team, n_opd, n_dot, dot_n, most_k, ks, work_at, pad; };
 struct Load { const void* p; uint32_t cols, slot; };        // cols: 0 = element i, else element i % cols
 // phase: in the first instruction of a phase (instructions that do not touch one another's values), how many it has
 struct Ins { uint8_t op, act, n_in, phase; uint8_t dst[2], pad2[2]; uint8_t src[8]; double scalar; };
 constexpr uint8_t INS_FOLD = 64;          // ((src0 + src1) + src2) + ... in T: a run of dst += src
 struct Store { void* p; uint32_t slot, pad; };
-static_assert(sizeof(Head) == 32 && sizeof(Load) == 16 && sizeof(Ins) == 24 && sizeof(Store) == 16, "program layout");
+// An operand of a program's products.  kind 0: the piece's rows of an [M][K] matrix, 1: of a [K][M] one (X = M),
+// 2: all columns of a [K][N] matrix, 3: of an [N][K] one (X = N); at: where it goes, behind work_at, as [row or column][k]
+// (values k_lo .. k_hi of k: an operand is several tasks)
+struct Opd { const void* p; int32_t kind, X, K, at, k_lo, k_hi; };
+struct Dot { double alpha; int32_t K, slot, a_at, b_at; };
+static_assert(sizeof(Head) == 56 && sizeof(Load) == 16 && sizeof(Ins) == 24 && sizeof(Store) == 16 && sizeof(Opd) == 32 && sizeof(Dot) == 24,
+              "program layout");
 struct ProductProg {
   Head h;                                                    // kind = PRIM_PRODUCT
   const void *A, *B;
@@ -52,8 +65,12 @@ struct ProductProg {
 };
 struct RowProg { Head h; const void* in[4]; void* out[3]; int64_t rows; int32_t cols, depth; double scalar; };
 
+// The cluster meets, and what its threads wrote is visible to all of them: a CTA's stores are published by one fence of one
+// thread behind a barrier of the CTA (a release by every thread took 1800 cycles, most of it 32 fences one after another).
 __device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0) __threadfence();
+  asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 template <int BYTES> __device__ __forceinline__ void copy_async(void* dst, const void* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -106,22 +123,139 @@ __device__ __forceinline__ void execute(const Ins& c, T* v, int stride) {
   v[c.dst[0] * stride] = r;
 }
 
-// A piece: 256 elements, one per thread, or 64 elements with four threads each, which take the loads, the instructions of a
-// phase and the stores in turn (four gates' exponentials side by side instead of one after another).
+// ---- products: operands as [row][k] in shared memory
+// rows of 16-byte vectors plus one: the rows of neighbouring threads fall into different banks
+template <typename T> __host__ __device__ constexpr int product_pitch(int ks) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  return (ks + VEC - 1) / VEC * VEC + VEC;
+}
+// R x R sums over kc values of k, ascending, product and sum rounded separately; a thread's rows (columns) are `da` (`db`) values
+// apart.  16-byte reads (with a read per value, reading was most of a piece), the next ones on their way while these are added.
+template <typename T, int R>
+__device__ __forceinline__ void multiply(const T* a, int da, const T* b, int db, int kc, T (&acc)[R][R]) {
+  constexpr int VEC = 16 / (int)sizeof(T), G = R == 1 ? 2 : 1, KG = G * VEC;      // k at a time: what 64 registers have room for
+  alignas(16) T x[R][KG], y[R][KG];
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        *reinterpret_cast<uint4*>(&x[i][g * VEC]) = *reinterpret_cast<const uint4*>(a + i * da + k + g * VEC);
+        *reinterpret_cast<uint4*>(&y[i][g * VEC]) = *reinterpret_cast<const uint4*>(b + i * db + k + g * VEC);
+      }
+  };
+  int k = 0;
+  if (kc >= KG) fetch(0);
+#pragma unroll 1
+  for (; k + KG <= kc; k += KG) {
+    T pr[R][R][KG];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+#pragma unroll
+        for (int q = 0; q < KG; ++q) pr[i][j][q] = mul_rn(x[i][q], y[j][q]);
+    if (k + 2 * KG <= kc) fetch(k + KG);
+#pragma unroll
+    for (int q = 0; q < KG; ++q)
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) acc[i][j] = add_rn(acc[i][j], pr[i][j][q]);
+  }
+#pragma unroll 1
+  for (; k < kc; ++k)
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < R; ++j) acc[i][j] = add_rn(acc[i][j], mul_rn(a[i * da + k], b[j * db + k]));
+}
+
+// The worker copies ks values of k, from k0 on, of a program's operands.  The plan has cut them into tasks of about the same size,
+// which the warps take in turn.  (A loop of all warps over all operands took longer than all the arithmetic: it is a chain of
+// instructions per operand, not bytes, that takes the time.)
 template <typename T, int N>
-__device__ void run_elementwise(const Head* h, int chunk, T* v, const StartTable<N>& starts) {
-  const int tid = threadIdx.x % NT, team = (int)h->team;
-  const int per = NT / team, e = tid % per, q0 = tid / per;
+__device__ __forceinline__ void copy_program_operands(const Opd* op, int n_opd, T* work, int pitch, int row0, int rows, int dot_n, int k0,
+                                                      int ks, const StartTable<N>& starts) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  const int lane = threadIdx.x & 31;
+  for (int o = threadIdx.x % NT / 32; o < n_opd; o += NT / 32) {
+    const Opd d = op[o];
+    int k_lo = d.k_lo > k0 ? d.k_lo : k0, k_hi = d.k_hi < k0 + ks ? d.k_hi : k0 + ks;
+    if (k_lo >= k_hi) continue;
+    const bool a = d.kind < 2;
+    const int first = a ? row0 : 0, left = d.X - first, most = a ? rows : dot_n, count = left < most ? left : most;
+    const T* g = source<T>(d.p, starts);
+    T* s = work + d.at - k0;
+    if (d.kind == 0 || d.kind == 3) {                        // [row][k]
+      g += (int64_t)first * d.K;
+      if (k_lo % VEC == 0 && k_hi % VEC == 0 && k0 % VEC == 0 && d.K % VEC == 0 && ((uintptr_t)g & 15) == 0) {
+#pragma unroll 4
+        for (int r = 0; r < count; ++r)
+          for (int k = k_lo + lane * VEC; k < k_hi; k += 32 * VEC) {
+            const uint32_t to = (uint32_t)__cvta_generic_to_shared(s + r * pitch + k);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(g + r * d.K + k) : "memory");
+          }
+      } else {
+#pragma unroll 4
+        for (int r = 0; r < count; ++r)
+          for (int k = k_lo + lane; k < k_hi; k += 32) copy_async<sizeof(T)>(s + r * pitch + k, g + r * d.K + k);
+      }
+    } else {                                                 // [k][row]
+      const int k_lane = lane / most, r = lane - k_lane * most, step = 32 / most;
+      if (r < count && k_lane < step) {                      // (at most 32 rows; lanes beyond a whole number of k stay out)
+        g += first + r;
+        s += r * pitch;
+#pragma unroll 4
+        for (int k = k_lo + k_lane; k < k_hi; k += step) copy_async<sizeof(T)>(s + k, g + k * d.X);
+      }
+    }
+  }
+}
+
+// A piece: 256 elements, one per thread, or 64 (32) elements with four (eight) threads each, which take the loads, the products,
+// the instructions of a phase and the stores in turn (four gates' exponentials side by side instead of one after another).
+template <typename T, int N>
+__device__ void run_elementwise(const Head* h, int chunk, T* work, const StartTable<N>& starts) {
+  const int tid = threadIdx.x % NT, team = h->team, n_dot = h->n_dot;
+  // (a piece of 32: columns by the lanes' upper bits and rows by bits 0 and 4, so that reads of either operand of a product have
+  // lane pairs one or two apart on one address: 2 cycles instead of 4)
+  const int per = NT / team, q0 = tid / per, e = team == 8 ? (tid >> 1 & 15) | (tid & 1) << 4 : tid % per;
   const Load* ld = reinterpret_cast<const Load*>(h + 1);
   const Ins* ins = reinterpret_cast<const Ins*>(ld + h->n_load);
   const Store* st = reinterpret_cast<const Store*>(ins + h->n_ins);
   const int64_t i = (int64_t)chunk * per + e;
   const bool on = i < h->n;
-  v += e;
+  T* v = work + e;
   if (on)
     for (int k = q0; k < h->n_load; k += team)      // all on their way at once
       copy_async<sizeof(T)>(v + ld[k].slot * per, source<T>(ld[k].p, starts) + (ld[k].cols ? i % ld[k].cols : i));
-  copy_wait();
+  if (n_dot) {
+    const Opd* op = reinterpret_cast<const Opd*>(st + h->n_store);
+    const Dot* dots = reinterpret_cast<const Dot*>(op + h->n_opd);
+    const int ks = h->ks, pitch = product_pitch<T>(ks), dot_n = h->dot_n, i0 = chunk * per, most = h->most_k;
+    const int row0 = i0 / dot_n, rows = (i0 + per - 1) / dot_n - row0 + 1;
+    const int m = (i0 + e) / dot_n - row0, c = (i0 + e) % dot_n;
+    T* operands = work + h->work_at;
+    for (int k0 = 0; k0 < most; k0 += ks) {
+      if (k0) worker_sync();
+      copy_program_operands<T>(op, h->n_opd, operands, pitch, row0, rows, dot_n, k0, ks, starts);
+      copy_wait();
+      worker_sync();
+      if (on)
+        for (int d = q0; d < n_dot; d += team) {
+          const Dot& t = dots[d];
+          const int kc = t.K - k0 < ks ? t.K - k0 : ks;
+          if (kc <= 0) continue;
+          T acc[1][1];
+          acc[0][0] = k0 ? v[t.slot * per] : (T)0;
+          multiply<T, 1>(operands + t.a_at + m * pitch, 0, operands + t.b_at + c * pitch, 0, kc, acc);
+          v[t.slot * per] = k0 + ks < t.K ? acc[0][0] : mul_rn((T)t.alpha, acc[0][0]);
+        }
+    }
+  } else {
+    copy_wait();
+  }
   if (team > 1) {
     worker_sync();
     for (int k0 = 0; k0 < h->n_ins;) {
@@ -138,12 +272,7 @@ __device__ void run_elementwise(const Head* h, int chunk, T* v, const StartTable
     for (int k = q0; k < h->n_store; k += team) ((T*)st[k].p)[i] = v[st[k].slot * per];
 }
 
-// ---- products: a tm x tn tile, R x R outputs per thread, both operands of ks values of k in shared memory
-// rows of 16-byte vectors plus one: the rows of neighbouring threads fall into different banks
-template <typename T> __host__ __device__ constexpr int product_pitch(int ks) {
-  constexpr int VEC = 16 / (int)sizeof(T);
-  return (ks + VEC - 1) / VEC * VEC + VEC;
-}
+// ---- products of their own: a tm x tn tile, R x R outputs per thread, both operands of ks values of k in shared memory
 // `rows` operand rows of kc values of k into s[row][pitch]; KC: memory is [row][k], otherwise [k][row] (rows a power of two)
 template <typename T, bool KC>
 __device__ __forceinline__ void copy_operand(T* s, int pitch, const T* g, int64_t ld, int row0, int X, int rows, int kc) {
@@ -195,43 +324,7 @@ __device__ void run_product(const ProductProg* p, int chunk, T* smem, const Star
     else copy_operand<T, false>(Bs, pa, B + (int64_t)k0 * N, N, n0, N, tn, kc);
     copy_wait();
     worker_sync();
-    if (on) {
-      const T* a = As + mi * pa;
-      const T* b = Bs + ni * pa;
-      T x[R][R], y[R][R];
-      auto products = [&](T (&d)[R][R], int k) {
-        T av[R], bv[R];
-#pragma unroll
-        for (int i = 0; i < R; ++i) { av[i] = a[i * ty * pa + k]; bv[i] = b[i * tx * pa + k]; }
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-          for (int j = 0; j < R; ++j) d[i][j] = mul_rn(av[i], bv[j]);
-      };
-      auto sums = [&](const T (&d)[R][R]) {
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-          for (int j = 0; j < R; ++j) acc[i][j] = add_rn(acc[i][j], d[i][j]);
-      };
-      // the products of the next k are formed ahead of the sums of this one
-      products(x, 0);
-      int k = 1;
-#pragma unroll 4
-      for (; k + 1 < kc; k += 2) {
-        products(y, k);
-        sums(x);
-        products(x, k + 1);
-        sums(y);
-      }
-      if (k < kc) {
-        products(y, k);
-        sums(x);
-        sums(y);
-      } else {
-        sums(x);
-      }
-    }
+    if (on) multiply<T, R>(As + mi * pa, ty * pa, Bs + ni * pa, tx * pa, kc, acc);
   }
   if (on)
 #pragma unroll
@@ -352,6 +445,7 @@ template <typename T, int N>
 __global__ void __launch_bounds__(WORKERS * NT)
 walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ items, const int* __restrict__ first,
             const __grid_constant__ StartTable<N> starts) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char gp_smem[];
   const int tid = threadIdx.x % NT, worker = blockIdx.x * WORKERS + threadIdx.x / NT;
   unsigned char* prog = gp_smem + (threadIdx.x / NT) * (2 * PROG_BYTES + WORK_BYTES);
@@ -359,7 +453,10 @@ walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ ite
   items += first[worker];
   const int n = first[worker + 1] - first[worker];
   auto fetch = [&](const Item& it, int i) {
-    for (uint32_t b = tid * 8; b < it.bytes; b += NT * 8) copy_async<8>(prog + (i & 1) * PROG_BYTES + b, blob + it.prog + b);
+    for (uint32_t b = tid * 16; b < it.bytes; b += NT * 16) {
+      const uint32_t d = (uint32_t)__cvta_generic_to_shared(prog + (i & 1) * PROG_BYTES + b);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(blob + it.prog + b) : "memory");
+    }
   };
   Item cur{0, 0, 0, 0}, nxt{0, 0, 0, 0};
   if (n > 0) { cur = items[0]; fetch(cur, 0); }
@@ -387,12 +484,14 @@ walk_kernel(const unsigned char* __restrict__ blob, const Item* __restrict__ ite
 }  // namespace gp
 
 struct GraphPlan {
-  int device = 0, ctas = 0;
+  // a launch: one cluster with barriers between the levels, or one level on all SMs
+  struct Part { int ctas; bool cluster; const int* first; };
+  int device = 0;
   prad_dtype dt = PRAD_F32;
-  void* mem = nullptr;                       // [items][first item of each worker][blob]
+  void* mem = nullptr;                       // [items][first item of each worker, part by part][blob]
   const unsigned char* blob = nullptr;
   const gp::Item* items = nullptr;
-  const int* first = nullptr;
+  std::vector<Part> parts;
   std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write: ascending, without overlaps
 };
 
@@ -410,7 +509,8 @@ namespace gp {
 static bool elementwise(const Prim& p) { return p.kind <= PRIM_LAST_ELEMENTWISE; }
 
 // What an operation reads and writes.  `local`: value i of the operation touches element i of the buffer only.
-struct Access { uintptr_t lo, hi; bool write, local; };
+// `fresh`: written by a product that a program computes for its own elements, ahead of whatever else the program does.
+struct Access { uintptr_t lo, hi; bool write, local, fresh = false; };
 
 static void accesses(const Prim& p, size_t es, std::vector<Access>& out) {
   out.clear();
@@ -467,13 +567,51 @@ struct Group {
   std::vector<int> ops;                      // ascending
 };
 
+// Products that programs can compute for themselves.  A product of few outputs whose first reader is an elementwise operation on
+// them needs no level of its own, with its barrier and its way through memory: dots[e] are the products that operation e takes
+// along, fused[i] says that product i is one.  The product moves to the place of its reader, so nothing in between may write what
+// it reads or touch what it writes.
+constexpr int DOT_COLUMNS = 32, DOT_LOOK = 256;
+constexpr int64_t TEAM_ELEMENTS = 2048;      // up to here several threads can share an element
+static void find_dots(const std::vector<Prim>& ops, const std::vector<std::vector<Access>>& acc, std::vector<std::vector<int>>& dots,
+                      std::vector<char>& fused) {
+  const int N = (int)ops.size();
+  auto meets = [](const Access& a, const Access& b) { return a.lo < b.hi && b.lo < a.hi; };
+  for (int i = 0; i < N; ++i) {
+    const Prim& p = ops[i];
+    if (p.kind != PRIM_PRODUCT || p.batch != 1 || p.K < 1 || p.N < 1 || p.N > DOT_COLUMNS || (int64_t)p.M * p.N > TEAM_ELEMENTS || acc[i].size() != 3) continue;
+    const Access &A = acc[i][0], &B = acc[i][1], &X = acc[i][2];
+    if (meets(X, A) || meets(X, B)) continue;
+    for (int e = i + 1; e < N && e <= i + DOT_LOOK; ++e) {
+      bool touched = false, good = elementwise(ops[e]) && ops[e].n == (int64_t)p.M * p.N, harm = false;
+      for (const Access& a : acc[e]) {
+        if (meets(a, X)) {
+          touched = true;
+          good = good && !a.write && a.local && a.lo == X.lo && a.hi == X.hi;
+        }
+        harm = harm || (a.write && (meets(a, A) || meets(a, B)));
+      }
+      if (!touched && !harm) continue;
+      int same = 0;                          // programs have one shape of product each
+      for (int d : dots[e]) same += ops[d].N == p.N;
+      if (touched && good && !harm && same == (int)dots[e].size()) {
+        dots[e].push_back(i);
+        fused[i] = 1;
+      }
+      break;
+    }
+  }
+}
+
 // (buffer, columns of a row operand or 0): what has a place of its own in a program
 using Place = std::pair<const void*, int>;
 static Place place_of(const Prim& p, size_t k) { return {p.in[k], p.kind == PRIM_ADD_ROW && k == 1 ? p.cols : 0}; }
-constexpr int64_t TEAM_ELEMENTS = 2048;      // up to here four threads can share an element
 template <typename T> static int slot_limit(int64_t n) {
   return n <= TEAM_ELEMENTS ? SLOTS : std::min(SLOTS, WORK_BYTES / (NT * (int)sizeof(T)));
 }
+// operand rows a product in a program keeps in shared memory, at the most
+constexpr int DOT_PIECE = NT / 8, DOT_ROWS = 320;
+static int dot_rows(const Prim& p) { return (p.N <= DOT_PIECE && DOT_PIECE % p.N == 0 ? DOT_PIECE / p.N : (DOT_PIECE - 1) / p.N + 2) + p.N; }
 static int places(const std::vector<Prim>& all, const std::vector<int>& ops) {
   std::vector<Place> seen;
   for (int o : ops) {
@@ -551,14 +689,22 @@ static double launch_cost(const Prim& p, int sms) {
   return base + n / 400e3;
 }
 
+// One launch of a plan: its workers' lists.
+struct Part { int ctas; bool cluster; std::vector<std::vector<Item>> lists; };
+
 template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& ops, int ctas, std::vector<unsigned char>& blob,
-                                        std::vector<std::vector<Item>>& lists, std::vector<std::pair<uintptr_t, uintptr_t>>& written,
+                                        std::vector<Part>& parts, std::vector<std::pair<uintptr_t, uintptr_t>>& written,
                                         double* est_us, double* launch_us) {
   const size_t es = sizeof(T);
   const int N = (int)ops.size();
   std::vector<int> level(N, 0), group_of(N, -1);
   std::vector<Group> groups;
   std::map<uintptr_t, Region> mem;
+  std::vector<std::vector<Access>> all_acc(N);
+  std::vector<std::vector<int>> dots(N), after(N);           // after[d]: operations that wait for d
+  std::vector<char> fused(N, 0);
+  for (int i = 0; i < N; ++i) accesses(ops[i], es, all_acc[i]);
+  find_dots(ops, all_acc, dots, fused);
   std::vector<Access> acc;
   *launch_us = 0;
   auto region_at = [&](const Access& a) -> Region& {
@@ -583,16 +729,24 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
   };
   for (int i = 0; i < N; ++i) {
     *launch_us += launch_cost(ops[i], ctx->sm_count);
-    accesses(ops[i], es, acc);
+    if (fused[i]) continue;                  // with its reader
+    acc.clear();
+    for (int d : dots[i])
+      for (Access a : all_acc[d]) {
+        if (a.write) a.local = a.fresh = true;
+        acc.push_back(a);
+      }
+    acc.insert(acc.end(), all_acc[i].begin(), all_acc[i].end());
     int lv = 0;
     std::vector<int> near;                   // operations this one may share a program with
     for (const Access& a : acc) {
       Region& r = region_at(a);
       auto depend = [&](int d) {
         if (d == i) return;
-        const bool local = a.local && r.local && elementwise(ops[i]) && elementwise(ops[d]) && ops[i].n == ops[d].n;
+        const bool local = a.local && !a.fresh && r.local && elementwise(ops[i]) && elementwise(ops[d]) && ops[i].n == ops[d].n;
         lv = std::max(lv, local ? level[d] : level[d] + 1);
         if (local) near.push_back(d);
+        after[d].push_back(i);
       };
       for (int d : r.writers) depend(d);
       if (a.write)
@@ -608,7 +762,17 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       for (int g : join) merged.ops.insert(merged.ops.end(), groups[g].ops.begin(), groups[g].ops.end());
       std::sort(merged.ops.begin(), merged.ops.end());
       merged.ops.push_back(i);
-      if (!join.empty() && ((int)merged.ops.size() > MAX_INS || places(ops, merged.ops) > slot_limit<T>(merged.n))) {
+      int n_dot = 0, rows = 0;
+      bool one_shape = true;
+      for (int o : merged.ops)
+        for (int d : dots[o]) {
+          ++n_dot;
+          rows += dot_rows(ops[d]);
+          for (int o2 : merged.ops)
+            for (int d2 : dots[o2]) one_shape = one_shape && ops[d].N == ops[d2].N;
+        }
+      if (!join.empty() && ((int)merged.ops.size() > MAX_INS || places(ops, merged.ops) > slot_limit<T>(merged.n) || n_dot > MAX_DOTS ||
+                            rows > DOT_ROWS || !one_shape)) {
         ++lv;                                // a program of its own, behind a barrier
         join.clear();
         merged.ops.assign(1, i);
@@ -635,8 +799,30 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       else written.emplace_back(m.second.lo, m.second.hi);
     }
 
-  // programs, and the pieces of every level
+  // As late as possible: what nothing waits for yet (the embedding of the next time steps, weight gradients and their sums,
+  // outputs) would take workers from what the next level waits for.  Whole programs move, to the level before their first user.
   const int levels = N ? *std::max_element(level.begin(), level.end()) + 1 : 0;
+  {
+    auto unit = [&](int i) { return group_of[i] >= 0 ? groups[group_of[i]].ops.front() : i; };
+    std::vector<int> order, latest(N, levels - 1);
+    for (int i = 0; i < N; ++i)
+      if (!fused[i] && unit(i) == i) order.push_back(i);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return level[x] > level[y]; });
+    std::vector<std::vector<int>> users(N);                  // of a unit: units behind it
+    for (int d = 0; d < N; ++d)
+      for (int i : after[d])
+        if (unit(i) != unit(d)) users[unit(d)].push_back(unit(i));
+    for (int u : order) {                                    // users have a higher level, so they have been here
+      int lv = levels - 1;
+      for (int v : users[u]) lv = std::min(lv, latest[v] - 1);
+      latest[u] = lv;
+    }
+    std::vector<int> moved(N);
+    for (int i = 0; i < N; ++i) moved[i] = fused[i] ? 0 : latest[unit(i)];
+    level.swap(moved);
+  }
+
+  // programs, and the pieces of every level
   std::vector<std::vector<Piece>> pieces(levels);
   auto put = [&](const void* p, size_t bytes) {
     const size_t at = blob.size();
@@ -646,6 +832,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
   };
   for (int i = 0; i < N; ++i) {
     const Prim& p = ops[i];
+    if (fused[i]) continue;
     if (elementwise(p)) {
       const Group& g = groups[group_of[i]];
       if (g.ops.front() != i) continue;
@@ -654,8 +841,14 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       std::vector<Store> stores;
       std::map<Place, int> slot;
       int slots = 0;
+      std::vector<int> taken;                // products, with their places
       for (int o : g.ops) {
         const Prim& q = ops[o];
+        for (int d : dots[o]) {
+          taken.push_back(d);
+          slot[Place{ops[d].out[0], 0}] = slots;
+          stores.push_back({ops[d].out[0], (uint32_t)slots++, 0});
+        }
         Ins c;
         memset(&c, 0, sizeof(c));
         c.op = (uint8_t)q.kind;
@@ -688,22 +881,80 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       h.n_ins = (int)ins.size();
       h.n_store = (int)stores.size();
       h.n = g.n;
-      h.team = g.n <= TEAM_ELEMENTS && (ins.size() >= 4 || slots > WORK_BYTES / (NT * (int)es)) ? 4 : 1;
-      std::vector<unsigned char> prog(sizeof(Head) + loads.size() * sizeof(Load) + ins.size() * sizeof(Ins) + stores.size() * sizeof(Store));
+      h.team = !taken.empty() ? NT / DOT_PIECE : g.n <= TEAM_ELEMENTS && (ins.size() >= 4 || slots > WORK_BYTES / (NT * (int)es)) ? 4 : 1;
+      std::vector<Opd> opds;
+      std::vector<Dot> dot;
+      int most_k = 0;
+      if (!taken.empty()) {
+        std::vector<int> opd_rows;
+        auto operand = [&](const void* q, int kind, int X, int K, int rows) {
+          for (size_t k = 0; k < opds.size(); ++k)
+            if (opds[k].p == q && opds[k].kind == kind && opds[k].X == X && opds[k].K == K) return (int)k;
+          opds.push_back({q, kind, X, K, 0, 0, K});
+          opd_rows.push_back(rows);
+          return (int)opds.size() - 1;
+        };
+        for (int d : taken) {
+          const Prim& q = ops[d];
+          const int a = operand(q.in[0], q.tA ? 1 : 0, q.M, q.K, dot_rows(q) - q.N), b = operand(q.in[1], q.tB ? 3 : 2, q.N, q.K, q.N);
+          dot.push_back({q.scalar, q.K, slot[Place{q.out[0], 0}], a, b});
+          most_k = std::max(most_k, q.K);
+        }
+        int rows = 0;
+        for (int r : opd_rows) rows += r;
+        const int slot_values = (slots * DOT_PIECE * (int)es + 15) / 16 * 16 / (int)es;
+        h.ks = most_k;
+        while (rows * product_pitch<T>(h.ks) * (int)es > WORK_BYTES - slot_values * (int)es) h.ks = (int)ceil_div(h.ks / 2, 8) * 8;
+        h.most_k = most_k;
+        h.n_dot = (int)dot.size();
+        h.dot_n = ops[taken[0]].N;
+        h.work_at = slot_values;
+        int at = 0;
+        for (size_t k = 0; k < opds.size(); ++k) {
+          opds[k].at = at;
+          at += opd_rows[k] * product_pitch<T>(h.ks);
+        }
+        for (Dot& t : dot) {
+          t.a_at = opds[t.a_at].at;
+          t.b_at = opds[t.b_at].at;
+        }
+        // operands of more than 256 copies are cut along k, while there is room for tasks; whole vectors of k
+        const int copy_of[4] = {16, (int)es, (int)es, 16};
+        std::vector<Opd> tasks;
+        for (size_t k = 0; k < opds.size(); ++k) {
+          const int copies = opd_rows[k] * opds[k].K * (int)es / copy_of[opds[k].kind];
+          const int room = (MAX_TASKS - (int)tasks.size()) / (int)(opds.size() - k);
+          const int cut = std::max(1, std::min(room, copies / 192));
+          const int len = (int)ceil_div(ceil_div(opds[k].K, cut), 8) * 8;
+          for (int lo = 0; lo < opds[k].K; lo += len) {
+            tasks.push_back(opds[k]);
+            tasks.back().k_lo = lo;
+            tasks.back().k_hi = std::min(opds[k].K, lo + len);
+          }
+        }
+        opds.swap(tasks);
+      }
+      h.n_opd = (int)opds.size();
+      std::vector<unsigned char> prog(sizeof(Head) + loads.size() * sizeof(Load) + ins.size() * sizeof(Ins) + stores.size() * sizeof(Store) +
+                                      opds.size() * sizeof(Opd) + dot.size() * sizeof(Dot));
       unsigned char* w = prog.data();
       memcpy(w, &h, sizeof(h)); w += sizeof(h);
       memcpy(w, loads.data(), loads.size() * sizeof(Load)); w += loads.size() * sizeof(Load);
       memcpy(w, ins.data(), ins.size() * sizeof(Ins)); w += ins.size() * sizeof(Ins);
-      memcpy(w, stores.data(), stores.size() * sizeof(Store));
+      memcpy(w, stores.data(), stores.size() * sizeof(Store)); w += stores.size() * sizeof(Store);
+      memcpy(w, opds.data(), opds.size() * sizeof(Opd)); w += opds.size() * sizeof(Opd);
+      memcpy(w, dot.data(), dot.size() * sizeof(Dot));
       const uint32_t at = put(prog.data(), prog.size());
       double cost = 1.0 + 0.02 * (double)loads.size() / (double)h.team;
+      if (!dot.empty())
+        cost += 0.4 + most_k * (es == 8 ? 0.012 : 0.008) * (double)ceil_div((int64_t)dot.size(), h.team) + 0.6 * (double)(ceil_div(most_k, h.ks) - 1);
       if (h.team > 1) {
-        cost += 0.35 * phases;
+        cost += 0.25 * phases;
       } else {
         cost += 0.1 * (double)ins.size();
         for (const Ins& c : ins) cost += c.op == PRIM_ACT_FORWARD || c.op == PRIM_ACT_BACKWARD ? 0.3 : 0;
       }
-      for (int64_t c = 0; c < ceil_div(g.n, NT / h.team); ++c) pieces[level[i]].push_back({at, (uint32_t)((prog.size() + 7) & ~(size_t)7), (uint32_t)c, cost});
+      for (int64_t c = 0; c < ceil_div(g.n, NT / h.team); ++c) pieces[level[i]].push_back({at, (uint32_t)((prog.size() + 15) & ~(size_t)15), (uint32_t)c, cost});
       continue;
     }
     if (p.kind == PRIM_PRODUCT) {
@@ -727,7 +978,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       q.tiles_mn = (int)ceil_div(p.M, q.tm) * q.tiles_n;
       const uint32_t at = put(&q, sizeof(q));
       const double cost = 1.2 + p.K * (es == 8 ? 0.017 : 0.012) * (q.r == 2 ? 2 : 1) + 0.6 * (double)(ceil_div(p.K, q.ks) - 1);
-      for (int64_t c = 0; c < (int64_t)q.tiles_mn * p.batch; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 7) & ~(size_t)7), (uint32_t)c, cost});
+      for (int64_t c = 0; c < (int64_t)q.tiles_mn * p.batch; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 15) & ~(size_t)15), (uint32_t)c, cost});
       continue;
     }
     RowProg q{};
@@ -742,30 +993,50 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     else if (p.kind == PRIM_TRANSPOSE) { chunks = ceil_div(p.rows * p.cols * p.depth, NT); cost = 0.9; }
     else { q.rows = p.rows * p.depth; chunks = ceil_div(q.rows, NT / 32); cost = 2.0 + 0.1 * (double)p.cols; }
     const uint32_t at = put(&q, sizeof(q));
-    for (int64_t c = 0; c < chunks; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 7) & ~(size_t)7), (uint32_t)c, cost});
+    for (int64_t c = 0; c < chunks; ++c) pieces[level[i]].push_back({at, (uint32_t)((sizeof(q) + 15) & ~(size_t)15), (uint32_t)c, cost});
   }
 
-  // deal the pieces of a level to the workers, the longest first to whoever has least (and to another SM before the same one
-  // again); a barrier behind every level
-  const int workers = ctas * WORKERS;
-  lists.assign(workers, {});
-  *est_us = 4.0;
-  std::vector<double> busy(workers);         // worker k of the dealing order is number k / ctas of CTA k % ctas
-  for (int lv = 0; lv < levels; ++lv) {
-    std::stable_sort(pieces[lv].begin(), pieces[lv].end(), [](const Piece& a, const Piece& b) { return a.cost > b.cost; });
-    std::fill(busy.begin(), busy.end(), 0.0);
-    std::vector<size_t> before(workers);
-    for (int c = 0; c < workers; ++c) before[c] = lists[c].size();
+  // Deal the pieces of a level to the workers of `c` CTAs, the longest first to whoever has least (and to another SM before the
+  // same one again); worker k of the dealing order is number k / c of CTA k % c.  Returns the time of the busiest.
+  auto deal = [&](int lv, int c, std::vector<std::vector<Item>>* lists) {
+    std::vector<std::pair<double, int>> heap;                // least busy first
+    for (int k = 0; k < c * WORKERS; ++k) heap.push_back({0.0, k});
+    auto later = [](const std::pair<double, int>& x, const std::pair<double, int>& y) { return x > y; };
+    double most = 0;
     for (const Piece& p : pieces[lv]) {
-      const int k = (int)(std::min_element(busy.begin(), busy.end()) - busy.begin());
-      busy[k] += p.cost;
-      lists[k % ctas * WORKERS + k / ctas].push_back({p.prog, p.bytes, p.chunk, 0});
+      std::pop_heap(heap.begin(), heap.end(), later);
+      const int k = heap.back().second;
+      most = std::max(most, heap.back().first += p.cost);
+      std::push_heap(heap.begin(), heap.end(), later);
+      if (lists) (*lists)[k % c * WORKERS + k / c].push_back({p.prog, p.bytes, p.chunk, 0});
     }
-    for (int c = 0; c < workers; ++c) {
-      if (lists[c].size() == before[c]) lists[c].push_back({0, 0, 0, 1});
-      else lists[c].back().barrier = 1;
+    return most;
+  };
+  for (auto& lv : pieces) std::stable_sort(lv.begin(), lv.end(), [](const Piece& a, const Piece& b) { return a.cost > b.cost; });
+  // The last levels run on all SMs, a launch each, where sixteen SMs would need 6 us longer for them (a launch, its program's way
+  // into every SM and the pieces are 4 us at the least).
+  int narrow = levels;
+  while (narrow > 0 && deal(narrow - 1, ctas, nullptr) - deal(narrow - 1, ctx->sm_count, nullptr) > 6.0) --narrow;
+  *est_us = 4.0;
+  if (narrow > 0) {
+    Part part{ctas, true, {}};
+    part.lists.assign(ctas * WORKERS, {});
+    for (int lv = 0; lv < narrow; ++lv) {
+      std::vector<size_t> before(part.lists.size());
+      for (size_t c = 0; c < before.size(); ++c) before[c] = part.lists[c].size();
+      *est_us += 0.8 + deal(lv, ctas, &part.lists);
+      for (size_t c = 0; c < before.size(); ++c) {           // a barrier behind every level
+        if (part.lists[c].size() == before[c]) part.lists[c].push_back({0, 0, 0, 1});
+        else part.lists[c].back().barrier = 1;
+      }
     }
-    *est_us += 0.8 + *std::max_element(busy.begin(), busy.end());
+    parts.push_back(std::move(part));
+  }
+  for (int lv = narrow; lv < levels; ++lv) {
+    Part part{ctx->sm_count, false, {}};
+    part.lists.assign(ctx->sm_count * WORKERS, {});
+    *est_us += 3.0 + deal(lv, ctx->sm_count, &part.lists);
+    parts.push_back(std::move(part));
   }
 }
 
@@ -819,18 +1090,20 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
     if (p.in.size() > 8) return nullptr;
   }
   std::vector<unsigned char> blob;
-  std::vector<std::vector<Item>> lists;
+  std::vector<Part> parts;
   double est = 0, launches = 0;
   std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write: ascending, without overlaps
-  build<T>(ctx, ops, ctas, blob, lists, written, &est, &launches);
+  build<T>(ctx, ops, ctas, blob, parts, written, &est, &launches);
   if (est >= launches) return nullptr;
   std::vector<Item> items;
   std::vector<int> first;
-  for (auto& l : lists) {
+  for (auto& part : parts) {
+    for (auto& l : part.lists) {
+      first.push_back((int)items.size());
+      items.insert(items.end(), l.begin(), l.end());
+    }
     first.push_back((int)items.size());
-    items.insert(items.end(), l.begin(), l.end());
   }
-  first.push_back((int)items.size());
   const size_t items_bytes = items.size() * sizeof(Item), first_bytes = (first.size() * sizeof(int) + 15) & ~(size_t)15;
   std::vector<unsigned char> host(items_bytes + first_bytes + blob.size());
   memcpy(host.data(), items.data(), items_bytes);
@@ -838,7 +1111,6 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
   memcpy(host.data() + items_bytes + first_bytes, blob.data(), blob.size());
   GraphPlanPtr plan(new GraphPlan());
   plan->device = ctx->device;
-  plan->ctas = ctas;
   plan->dt = dt;
   if (device_malloc(&plan->mem, host.size()) != cudaSuccess ||
       cudaMemcpyAsync(plan->mem, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
@@ -848,7 +1120,11 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
   }
   plan->written = std::move(written);
   plan->items = (const Item*)plan->mem;
-  plan->first = (const int*)((const unsigned char*)plan->mem + items_bytes);
+  const int* at = (const int*)((const unsigned char*)plan->mem + items_bytes);
+  for (const auto& part : parts) {
+    plan->parts.push_back({part.ctas, part.cluster, at});
+    at += part.lists.size() + 1;
+  }
   plan->blob = (const unsigned char*)plan->mem + items_bytes + first_bytes;
   return plan;
 }
@@ -866,30 +1142,34 @@ bool graph_plan_writes(const GraphPlan* plan, const void* p, size_t bytes) {
 }
 
 template <typename T, int N>
-static prad_status run_walk(prad_ctx* ctx, const cudaLaunchConfig_t& cfg, const GraphPlan* plan, const void* const* starts, int count) {
+static prad_status run_walk(prad_ctx* ctx, const GraphPlan* plan, const void* const* starts, int count) {
   gp::StartTable<N> table;
   for (int i = 0; i < count; ++i) table.p[i] = starts[i];
-  PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<T, N>, plan->blob, plan->items, plan->first, table));
-  PRAD_LAUNCHED(ctx);
+  for (const GraphPlan::Part& part : plan->parts) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = part.ctas;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)part.ctas);
+    cfg.blockDim = dim3(gp::WORKERS * gp::NT);
+    cfg.dynamicSmemBytes = gp::SMEM_BYTES;
+    cfg.stream = ctx->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = part.cluster ? 2 : 1;
+    PRAD_CUDA(cudaLaunchKernelEx(&cfg, gp::walk_kernel<T, N>, plan->blob, plan->items, part.first, table));
+    PRAD_LAUNCHED(ctx);
+  }
   return PRAD_OK;
 }
 
 prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan, const void* const* starts, int count) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = plan->ctas;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)plan->ctas);
-  cfg.blockDim = dim3(gp::WORKERS * gp::NT);
-  cfg.dynamicSmemBytes = gp::SMEM_BYTES;
-  cfg.stream = ctx->stream;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
   const bool few = count <= gp::FEW_STARTS;
   if (plan->dt == PRAD_F32)
-    return few ? run_walk<float, gp::FEW_STARTS>(ctx, cfg, plan, starts, count) : run_walk<float, MOST_STARTS>(ctx, cfg, plan, starts, count);
-  return few ? run_walk<double, gp::FEW_STARTS>(ctx, cfg, plan, starts, count) : run_walk<double, MOST_STARTS>(ctx, cfg, plan, starts, count);
+    return few ? run_walk<float, gp::FEW_STARTS>(ctx, plan, starts, count) : run_walk<float, MOST_STARTS>(ctx, plan, starts, count);
+  return few ? run_walk<double, gp::FEW_STARTS>(ctx, plan, starts, count) : run_walk<double, MOST_STARTS>(ctx, plan, starts, count);
 }
 
 }  // namespace prad
