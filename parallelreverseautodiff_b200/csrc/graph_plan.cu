@@ -34,15 +34,16 @@ constexpr int SLOTS = 64;                 // values of one element a program kee
 constexpr int MAX_INS = 96;
 constexpr int MAX_DOTS = 16;              // products a program computes for its own elements
 constexpr int MAX_TASKS = 64;             // copies their operands are cut into
-constexpr int PROG_BYTES = 64 + SLOTS * 16 + MAX_INS * 24 + SLOTS * 16 + MAX_TASKS * 32 + MAX_DOTS * 24;
+constexpr int PROG_BYTES = 64 + SLOTS * 16 + MAX_INS * 24 + SLOTS * 16 + MAX_TASKS * 40 + MAX_DOTS * 24;
 constexpr int WORK_BYTES = 88 * 1024;     // a worker's shared memory: the slots of its elements, or the operands of a product
 
 // a piece of one worker
 struct Item { uint32_t prog, bytes, chunk, barrier; };
 
 // team: how many threads share an element's instructions: 8 (a piece is 32 elements then) where it has products, 4 or 1
-// n_dot products of rows x dot_n outputs, ks values of k of their n_opd operands at a time, from work_at values on
-struct Head { int32_t kind, n_load, n_ins, n_store; int64_t n; int32_t team, n_opd, n_dot, dot_n, most_k, ks, work_at, pad; };
+// n_dot products of rows x dot_n outputs, ks values of k of their n_opd operands at a time, from work_at values on; dot_inv and
+// Opd::inv divide by dot_n and Opd::most
+struct Head { int32_t kind, n_load, n_ins, n_store; int64_t n; int32_t team, n_opd, n_dot, dot_n, most_k, ks, work_at; uint32_t dot_inv; };
 struct Load { const void* p; uint32_t cols, slot; };        // cols: 0 = element i, else element i % cols
 // phase: in the first instruction of a phase (instructions that do not touch one another's values), how many it has
 struct Ins { uint8_t op, act, n_in, phase; uint8_t dst[2], pad2[2]; uint8_t src[8]; double scalar; };
@@ -51,9 +52,9 @@ struct Store { void* p; uint32_t slot, pad; };
 // An operand of a program's products.  kind 0: the piece's rows of an [M][K] matrix, 1: of a [K][M] one (X = M),
 // 2: all columns of a [K][N] matrix, 3: of an [N][K] one (X = N); at: where it goes, behind work_at, as [row or column][k]
 // (values k_lo .. k_hi of k: an operand is several tasks)
-struct Opd { const void* p; int32_t kind, X, K, at, k_lo, k_hi; };
+struct Opd { const void* p; int32_t kind, X, K, at, k_lo, k_hi, most, inv; };     // most: rows or columns of a piece
 struct Dot { double alpha; int32_t K, slot, a_at, b_at; };
-static_assert(sizeof(Head) == 56 && sizeof(Load) == 16 && sizeof(Ins) == 24 && sizeof(Store) == 16 && sizeof(Opd) == 32 && sizeof(Dot) == 24,
+static_assert(sizeof(Head) == 56 && sizeof(Load) == 16 && sizeof(Ins) == 24 && sizeof(Store) == 16 && sizeof(Opd) == 40 && sizeof(Dot) == 24,
               "program layout");
 struct ProductProg {
   Head h;                                                    // kind = PRIM_PRODUCT
@@ -175,16 +176,15 @@ __device__ __forceinline__ void multiply(const T* a, int da, const T* b, int db,
 // which the warps take in turn.  (A loop of all warps over all operands took longer than all the arithmetic: it is a chain of
 // instructions per operand, not bytes, that takes the time.)
 template <typename T, int N>
-__device__ __forceinline__ void copy_program_operands(const Opd* op, int n_opd, T* work, int pitch, int row0, int rows, int dot_n, int k0,
-                                                      int ks, const StartTable<N>& starts) {
+__device__ __forceinline__ void copy_program_operands(const Opd* op, int n_opd, T* work, int pitch, int row0, int k0, int ks,
+                                                      const StartTable<N>& starts) {
   constexpr int VEC = 16 / (int)sizeof(T);
   const int lane = threadIdx.x & 31;
   for (int o = threadIdx.x % NT / 32; o < n_opd; o += NT / 32) {
     const Opd d = op[o];
     int k_lo = d.k_lo > k0 ? d.k_lo : k0, k_hi = d.k_hi < k0 + ks ? d.k_hi : k0 + ks;
     if (k_lo >= k_hi) continue;
-    const bool a = d.kind < 2;
-    const int first = a ? row0 : 0, left = d.X - first, most = a ? rows : dot_n, count = left < most ? left : most;
+    const int first = d.kind < 2 ? row0 : 0, left = d.X - first, count = left < d.most ? left : d.most;
     const T* g = source<T>(d.p, starts);
     T* s = work + d.at - k0;
     if (d.kind == 0 || d.kind == 3) {                        // [row][k]
@@ -202,7 +202,7 @@ __device__ __forceinline__ void copy_program_operands(const Opd* op, int n_opd, 
           for (int k = k_lo + lane; k < k_hi; k += 32) copy_async<sizeof(T)>(s + r * pitch + k, g + r * d.K + k);
       }
     } else {                                                 // [k][row]
-      const int k_lane = lane / most, r = lane - k_lane * most, step = 32 / most;
+      const int k_lane = lane * d.inv >> 16, r = lane - k_lane * d.most, step = 32 * d.inv >> 16;
       if (r < count && k_lane < step) {                      // (at most 32 rows; lanes beyond a whole number of k stay out)
         g += first + r;
         s += r * pitch;
@@ -220,7 +220,8 @@ __device__ void run_elementwise(const Head* h, int chunk, T* work, const StartTa
   const int tid = threadIdx.x % NT, team = h->team, n_dot = h->n_dot;
   // (a piece of 32: columns by the lanes' upper bits and rows by bits 0 and 4, so that reads of either operand of a product have
   // lane pairs one or two apart on one address: 2 cycles instead of 4)
-  const int per = NT / team, q0 = tid / per, e = team == 8 ? (tid >> 1 & 15) | (tid & 1) << 4 : tid % per;
+  const int per = team == 8 ? NT / 8 : team == 4 ? NT / 4 : NT, q0 = team == 8 ? tid >> 5 : team == 4 ? tid >> 6 : 0;
+  const int e = team == 8 ? (tid >> 1 & 15) | (tid & 1) << 4 : tid & (per - 1);
   const Load* ld = reinterpret_cast<const Load*>(h + 1);
   const Ins* ins = reinterpret_cast<const Ins*>(ld + h->n_load);
   const Store* st = reinterpret_cast<const Store*>(ins + h->n_ins);
@@ -229,17 +230,17 @@ __device__ void run_elementwise(const Head* h, int chunk, T* work, const StartTa
   T* v = work + e;
   if (on)
     for (int k = q0; k < h->n_load; k += team)      // all on their way at once
-      copy_async<sizeof(T)>(v + ld[k].slot * per, source<T>(ld[k].p, starts) + (ld[k].cols ? i % ld[k].cols : i));
+      copy_async<sizeof(T)>(v + ld[k].slot * per, source<T>(ld[k].p, starts) + (ld[k].cols ? (uint32_t)i % ld[k].cols : (uint32_t)i));
   if (n_dot) {
     const Opd* op = reinterpret_cast<const Opd*>(st + h->n_store);
     const Dot* dots = reinterpret_cast<const Dot*>(op + h->n_opd);
     const int ks = h->ks, pitch = product_pitch<T>(ks), dot_n = h->dot_n, i0 = chunk * per, most = h->most_k;
-    const int row0 = i0 / dot_n, rows = (i0 + per - 1) / dot_n - row0 + 1;
-    const int m = (i0 + e) / dot_n - row0, c = (i0 + e) % dot_n;
+    auto row_of = [&](int x) { return (int)((uint32_t)x * h->dot_inv >> 20); };      // x < 2048 + 32, dot_n <= 32
+    const int row0 = row_of(i0), row = row_of(i0 + e), m = row - row0, c = i0 + e - row * dot_n;
     T* operands = work + h->work_at;
     for (int k0 = 0; k0 < most; k0 += ks) {
       if (k0) worker_sync();
-      copy_program_operands<T>(op, h->n_opd, operands, pitch, row0, rows, dot_n, k0, ks, starts);
+      copy_program_operands<T>(op, h->n_opd, operands, pitch, row0, k0, ks, starts);
       copy_wait();
       worker_sync();
       if (on)
@@ -817,6 +818,55 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       for (int v : users[u]) lv = std::min(lv, latest[v] - 1);
       latest[u] = lv;
     }
+    // Of the rest, what may be anywhere between two levels goes where it prolongs a level least: the embeddings of all time steps
+    // as early as they can be, or all as late, take workers from the cells.
+    if (order.size() <= 500 && levels > 2) {
+      const int workers = ctas * WORKERS;
+      std::vector<std::vector<double>> busy(levels, std::vector<double>(workers, 0.0));
+      auto add = [&](std::vector<double> b, int u, double* most) {
+        const Prim& p = ops[u];
+        double cost;
+        int64_t n;
+        if (group_of[u] >= 0) {
+          const Group& g = groups[group_of[u]];
+          int k = 0;
+          for (int o : g.ops)
+            for (int d : dots[o]) k = std::max(k, ops[d].K);
+          const bool team = k || (g.n <= TEAM_ELEMENTS && g.ops.size() >= 4);
+          n = ceil_div(g.n, k ? DOT_PIECE : team ? NT / 4 : NT);
+          cost = (k ? 1.8 + 0.02 * k : 1.0) + (team ? 0.25 * (double)std::min<size_t>(g.ops.size(), 7) : 0.3 * (double)g.ops.size());
+        } else if (p.kind == PRIM_PRODUCT) {
+          n = ceil_div((int64_t)p.M * p.N, p.K <= 32 && p.M > 16 && p.N > 16 ? 1024 : NT) * p.batch;
+          cost = 1.5 + 0.02 * p.K;
+        } else {
+          n = ceil_div(p.rows * p.depth, NT / 32);
+          cost = 2.0 + 0.1 * p.cols;
+        }
+        for (int64_t k = 0; k < std::min<int64_t>(n, 4 * workers); ++k) *std::min_element(b.begin(), b.end()) += cost;
+        *most = *std::max_element(b.begin(), b.end());
+        return b;
+      };
+      double ignored;
+      std::vector<int> lowest(N, 0);
+      for (int u : order)
+        if (level[u] == latest[u]) busy[latest[u]] = add(busy[latest[u]], u, &ignored);
+      for (size_t x = order.size(); x-- > 0;) {              // those with a lower level first
+        const int u = order[x];
+        if (lowest[u] < latest[u] && latest[u] < levels - 2) {
+          int best = latest[u];
+          double least = 1e30;
+          for (int lv = latest[u]; lv >= lowest[u]; --lv) {
+            double most;
+            add(busy[lv], u, &most);
+            const double more = most - *std::max_element(busy[lv].begin(), busy[lv].end());
+            if (more < least - 1e-9) { least = more; best = lv; }
+          }
+          latest[u] = best;
+          busy[best] = add(busy[best], u, &ignored);
+        }
+        for (int v : users[u]) lowest[v] = std::max(lowest[v], latest[u] + 1);
+      }
+    }
     std::vector<int> moved(N);
     for (int i = 0; i < N; ++i) moved[i] = fused[i] ? 0 : latest[unit(i)];
     level.swap(moved);
@@ -890,7 +940,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
         auto operand = [&](const void* q, int kind, int X, int K, int rows) {
           for (size_t k = 0; k < opds.size(); ++k)
             if (opds[k].p == q && opds[k].kind == kind && opds[k].X == X && opds[k].K == K) return (int)k;
-          opds.push_back({q, kind, X, K, 0, 0, K});
+          opds.push_back({q, kind, X, K, 0, 0, K, rows, 65536 / rows + 1});
           opd_rows.push_back(rows);
           return (int)opds.size() - 1;
         };
@@ -908,6 +958,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
         h.most_k = most_k;
         h.n_dot = (int)dot.size();
         h.dot_n = ops[taken[0]].N;
+        h.dot_inv = (1u << 20) / h.dot_n + 1;
         h.work_at = slot_values;
         int at = 0;
         for (size_t k = 0; k < opds.size(); ++k) {
