@@ -151,12 +151,12 @@ template <typename T> struct Product {
   EpiParams<T> epi;
 };
 
-// tile shapes: BM x BN outputs, TM x TN per thread, BK k per stage
-template <typename T, int BM_, int BN_, int BK_, int TM_, int TN_, int STAGES_>
+// tile shapes: BM x BN outputs, TM x TN per thread, BK k per stage, NC threads that copy
+template <typename T, int BM_, int BN_, int BK_, int TM_, int TN_, int STAGES_, int NC_>
 struct TileShape {
   static constexpr int BM = BM_, BN = BN_, BK = BK_, TM = TM_, TN = TN_, STAGES = STAGES_;
   static constexpr int NT = (BM / TM) * (BN / TN);      // threads that multiply
-  static constexpr int NC = 64;                         // threads that copy
+  static constexpr int NC = NC_;
   static constexpr int THREADS = NT + NC;
   // either layout of either operand
   static constexpr int STAGE_A = OperandTile<T, BM, BK, NC, true>::SIZE > OperandTile<T, BM, BK, NC, false>::SIZE
@@ -510,19 +510,26 @@ static prad_status launch_small(prad_ctx* ctx, bool exact, bool tA, bool tB, int
 
 template <typename T> static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
+// Small tiles, of which an SM has one or two: the copies' instructions are spread over all four schedulers, for the four multiplying
+// warps meet after every stage and wait for the slowest (512 x 784 x 256 in double, forward and backward, 67 us with copying warps
+// on two schedulers, 59 on four).  Where an operand's rows do not start at 16-byte boundaries (SmallOdd) there are twice or four
+// times as many copies, and four warps of them get in the way: a double step of 887 x 98-217-217-217-9 takes 301 us with them,
+// 212 with two.  Double: stages of 32 k, for half the barriers and half the ends of rows (that step took 350 us with 16).
 template <typename T> struct SimtShapes;
 template <> struct SimtShapes<float> {
-  using Tiny = TileShape<float, 16, 16, 32, 2, 2, 4>;
-  using Small = TileShape<float, 32, 32, 32, 4, 2, 4>;
-  using Wide = TileShape<float, 64, 32, 32, 4, 4, 3>;
-  using Medium = TileShape<float, 64, 64, 32, 4, 4, 3>;
-  using Large = TileShape<float, 128, 128, 16, 8, 8, 4>;
+  using Tiny = TileShape<float, 16, 16, 32, 2, 2, 4, 64>;
+  using Small = TileShape<float, 32, 32, 32, 4, 2, 4, 128>;
+  using SmallOdd = TileShape<float, 32, 32, 32, 4, 2, 4, 64>;
+  using Wide = TileShape<float, 64, 32, 32, 4, 4, 3, 64>;
+  using Medium = TileShape<float, 64, 64, 32, 4, 4, 3, 64>;
+  using Large = TileShape<float, 128, 128, 16, 8, 8, 4, 64>;
 };
 template <> struct SimtShapes<double> {
-  using Tiny = TileShape<double, 16, 16, 16, 2, 2, 4>;
-  using Small = TileShape<double, 32, 32, 16, 4, 2, 4>;
-  using Wide = TileShape<double, 64, 32, 16, 4, 4, 3>;
-  using Medium = TileShape<double, 64, 64, 16, 4, 4, 3>;
+  using Tiny = TileShape<double, 16, 16, 32, 2, 2, 4, 64>;
+  using Small = TileShape<double, 32, 32, 32, 4, 2, 3, 128>;
+  using SmallOdd = TileShape<double, 32, 32, 32, 4, 2, 3, 64>;
+  using Wide = TileShape<double, 64, 32, 16, 4, 4, 3, 64>;
+  using Medium = TileShape<double, 64, 64, 16, 4, 4, 3, 64>;
   using Large = Medium;
 };
 
@@ -663,7 +670,9 @@ prad_status gemm_simt(prad_ctx* ctx, bool exact, bool tA, bool tB, int M, int N,
   using Shapes = SimtShapes<T>;
   switch (pick_shape<T>(ctx, &size, 1)) {
     case 0: return launch_shape<T, typename Shapes::Tiny>(ctx, exact, tA, tB, batch, p);
-    case 1: return launch_shape<T, typename Shapes::Small>(ctx, exact, tA, tB, batch, p);
+    case 1:
+      return p.vecA && p.vecB ? launch_shape<T, typename Shapes::Small>(ctx, exact, tA, tB, batch, p)
+                              : launch_shape<T, typename Shapes::SmallOdd>(ctx, exact, tA, tB, batch, p);
     case 2: return launch_shape<T, typename Shapes::Wide>(ctx, exact, tA, tB, batch, p);
     case 3: return launch_shape<T, typename Shapes::Medium>(ctx, exact, tA, tB, batch, p);
     default: return launch_shape<T, typename Shapes::Large>(ctx, exact, tA, tB, batch, p);
@@ -680,7 +689,9 @@ prad_status gemm_simt_backward(prad_ctx* ctx, bool exact, const void* A, const v
   using Shapes = SimtShapes<T>;
   switch (pick_shape<T>(ctx, size, 2)) {
     case 0: return launch_backward<T, typename Shapes::Tiny>(ctx, exact, nt, tn);
-    case 1: return launch_backward<T, typename Shapes::Small>(ctx, exact, nt, tn);
+    case 1:
+      return nt.vecA && nt.vecB && tn.vecA && tn.vecB ? launch_backward<T, typename Shapes::Small>(ctx, exact, nt, tn)
+                                                      : launch_backward<T, typename Shapes::SmallOdd>(ctx, exact, nt, tn);
     case 2: return launch_backward<T, typename Shapes::Wide>(ctx, exact, nt, tn);
     case 3: return launch_backward<T, typename Shapes::Medium>(ctx, exact, nt, tn);
     default: return launch_backward<T, typename Shapes::Large>(ctx, exact, nt, tn);
