@@ -75,16 +75,18 @@ embedding_gather_kernel(const T* __restrict__ index_col, const T* __restrict__ W
 // zeros over the table.  Then only the rows that were hit are summed: whoever sums a row puts its list into input order, a warp by
 // ranking up to 32 positions against each other, a CTA by a bitmap over the positions.  16384 word-like positions, a 50000 x 512
 // float table: with a grouping of four passes by a cluster of eight CTAs and sums that wrote the zeros in the place of rows without
-// hits, eight rows a warp one after another, gather and scatter took 82 us; now 70.  8677 positions, 157 x 858 doubles: 485 -> 96.
+// hits, eight rows a warp one after another, gather and scatter took 82 us; now 64 (the sums 49 -> 23 with a cold cache).  5962
+// positions, 130 x 394 floats: 250 -> 61; 8677 positions, 157 x 858 doubles: 487 -> 97.
 // Rows of many hits are the commonest words of a text: the commonest of 16384 appears over a thousand times, and its additions
 // are a chain, so 8 vectors of such a row have a CTA to themselves whose 32 teams of threads copy rows of dOut into a ring
-// in shared memory, 96 rows ahead of the team that adds them: what bounds such a row is the latency of memory over the rows in
-// flight (with 16 rows in flight in registers that one row took 150 us).
+// in shared memory, 192 rows ahead of the warp that adds them, and the longest chains begin first: that row took 38 000 cycles,
+// after two others, with the additions of four values per lane waiting for every read, and the whole pass waited for it.
 constexpr int EMB_FEW = 32;                       // hits a warp orders by itself
+constexpr int EMB_VERY_MANY = 256;                // hits of rows that have to be begun first
 constexpr int EMB_WINDOW = 32768;                 // positions of one bitmap
-constexpr int EMB_LIST = 1024;                    // ordered positions handed to the summing loop at a time
+constexpr int EMB_LIST = 2048;                    // ordered positions handed to the summing loop at a time
 constexpr int EMB_GROUP = 8;                      // vectors of a row of many hits that a CTA takes
-constexpr int EMB_CHUNK = 32, EMB_CHUNKS = 4;     // rows per step of the ring, steps in the ring
+constexpr int EMB_CHUNK = 64, EMB_CHUNKS = 4;     // rows per step of the ring, steps in the ring
 
 // The rows with hits, in `segments` parts of `stride` entries: part q has few[q] rows of few hits from its front and many[q] rows of
 // many from its back.  An entry's hits are list[offset .. offset + count), with count and offset by entry, or by row.
@@ -154,8 +156,8 @@ emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int* __restrict__ fe
     return;
   }
   __shared__ int place[EMB_PLAN_MOST / EMB_SEGMENTS];        // of the CTA's rows: hits, then where the next one goes
-  __shared__ int sums[4][NT / 32];
-  __shared__ int totals[4];
+  __shared__ int sums[5][NT / 32];
+  __shared__ int totals[5];
   const int lo = q * p.stride, mine = vocab - lo < p.stride ? vocab - lo : p.stride;
   for (int v = tid; v < mine; v += NT) place[v] = 0;
   __syncthreads();
@@ -173,18 +175,19 @@ emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int* __restrict__ fe
   }
   __syncthreads();
   if (q == 0 && tid == 0 && ticket) emb_all_checked(flag, ticket);
-  // neighbouring rows to a thread; a scan over the threads of hits, rows of few and rows of many hits
+  // neighbouring rows to a thread; a scan over the threads of hits, rows of few, of many and of very many hits
   const int per = (mine + NT - 1) / NT, r0 = tid * per, r1 = r0 + per < mine ? r0 + per : mine;
-  int v[4] = {below, 0, 0, 0};
+  int v[5] = {below, 0, 0, 0, 0};
   for (int r = r0; r < r1; ++r) {
     const int c = place[r];
     v[1] += c;
     v[2] += c > 0 && c <= EMB_FEW;
-    v[3] += c > EMB_FEW;
+    v[3] += c > EMB_FEW && c <= EMB_VERY_MANY;
+    v[4] += c > EMB_VERY_MANY;
   }
-  int incl[4];
+  int incl[5];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < 5; ++k) {
     incl[k] = v[k];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -194,7 +197,7 @@ emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int* __restrict__ fe
     if (lane == 31) sums[k][w] = incl[k];
   }
   __syncthreads();
-  if (w < 4) {
+  if (w < 5) {
     int x = sums[w][lane], y = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -205,12 +208,13 @@ emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int* __restrict__ fe
     if (lane == 31) totals[w] = y;
   }
   __syncthreads();
-  int at = totals[0] + sums[1][w] + incl[1] - v[1], front = lo + sums[2][w] + incl[2] - v[2], back = lo + p.stride - 1 - (sums[3][w] + incl[3] - v[3]);
+  int at = totals[0] + sums[1][w] + incl[1] - v[1], front = lo + sums[2][w] + incl[2] - v[2], back = lo + p.stride - 1 - (totals[4] + sums[3][w] + incl[3] - v[3]);
+  int first = lo + p.stride - 1 - (sums[4][w] + incl[4] - v[4]);
   for (int r = r0; r < r1; ++r) {
     const int c = place[r];
     place[r] = at;
     if (c) {
-      const int e = c <= EMB_FEW ? front++ : back--;
+      const int e = c <= EMB_FEW ? front++ : c <= EMB_VERY_MANY ? back-- : first--;
       p.rows[e] = lo + r;
       p.count[e] = c;
       p.offset[e] = at;
@@ -219,7 +223,7 @@ emb_plan_kernel(const T* __restrict__ index_col, EmbPlan p, int* __restrict__ fe
   }
   if (tid == 0) {
     few[q] = totals[2];
-    many[q] = totals[3];
+    many[q] = totals[3] + totals[4];
   }
   __syncthreads();
 #pragma unroll 8
@@ -272,8 +276,19 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
   // entry g in its part, counted from the front or the back (all lanes ask for the same one)
   auto entry = [&](int g) {
     const int q = __popc(__ballot_sync(0xffffffffu, lane < EMB_SEGMENTS && before <= g));
-    const int k = g - __shfl_sync(0xffffffffu, before - here, q);
-    return (int)blockIdx.x >= hot_ctas ? q * p.stride + k : (q + 1) * p.stride - 1 - k;
+    return q * p.stride + g - __shfl_sync(0xffffffffu, before - here, q);
+  };
+  // rows of many: every part's first one, then the second ones and so on, for the parts have their largest rows first
+  auto entry_of_many = [&](int g) {
+    for (int k = 0;; ++k) {
+      unsigned with = __ballot_sync(0xffffffffu, here > k);
+      if (g >= __popc(with)) {
+        g -= __popc(with);
+        continue;
+      }
+      for (; g > 0; --g) with &= with - 1;
+      return __ffs(with) * p.stride - 1 - k;
+    }
   };
   if ((int)blockIdx.x >= hot_ctas) {
     int* mine = ordered + w * EMB_FEW;
@@ -332,19 +347,20 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
   constexpr int WORDS = EMB_WINDOW / 32 / EMB_THREADS;       // bitmap words per thread
   extern __shared__ __align__(16) unsigned char emb_smem[];
   V* ring = reinterpret_cast<V*>(emb_smem);                  // [EMB_CHUNKS][EMB_CHUNK][EMB_GROUP]
-  constexpr int TEAMS = EMB_THREADS / EMB_GROUP;
+  constexpr int TEAMS = EMB_THREADS / EMB_GROUP, VALUES = EMB_GROUP * (int)(sizeof(V) / sizeof(T));
   const int team = tid / EMB_GROUP, jl = tid % EMB_GROUP;
   const int groups = (vecs + EMB_GROUP - 1) / EMB_GROUP;
   const int64_t tasks = (int64_t)entries * groups;
   for (int64_t h = blockIdx.x; h < tasks; h += hot_ctas) {
-    const int e = entry((int)(h / groups)), v = p.rows[e], j = (int)(h % groups) * EMB_GROUP + jl;
+    const int e = entry_of_many((int)(h / groups)), v = p.rows[e], j = (int)(h % groups) * EMB_GROUP + jl;
     const int c = p.count[p.by_row ? v : e], o = p.offset[p.by_row ? v : e];
     const V* col = reinterpret_cast<const V*>(dOut) + j;
-    V acc = emb_zero<T, V>();
+    T sum = (T)0;
     for (int w0 = 0; w0 < n; w0 += EMB_WINDOW) {
 #pragma unroll
       for (int k = 0; k < WORDS; ++k) bits[k * EMB_THREADS + tid] = 0;
       __syncthreads();
+#pragma unroll 4
       for (int k = tid; k < c; k += EMB_THREADS) {
         const int q = p.list[o + k] - w0;
         if (q >= 0 && q < EMB_WINDOW) atomicOr(bits + (q >> 5), 1u << (q & 31));
@@ -390,17 +406,37 @@ emb_sum_kernel(const T* __restrict__ dOut, T* __restrict__ dW, EmbPlan p, int n,
           asm volatile("cp.async.wait_group %0;" ::"n"(EMB_CHUNKS - 2) : "memory");
           __syncthreads();                                   // chunk i is there; chunk i - 1 has been added
           fetch(i + EMB_CHUNKS - 1);
-          if (team == 0) {
-            const V* x = ring + i % EMB_CHUNKS * EMB_CHUNK * EMB_GROUP + jl;
-            const int here2 = m - i * EMB_CHUNK < EMB_CHUNK ? m - i * EMB_CHUNK : EMB_CHUNK;
-#pragma unroll 8
-            for (int k = 0; k < here2; ++k) emb_add<T, V>(acc, x[k * EMB_GROUP]);
+          if (w == 0 && lane < VALUES) {
+            // a value per lane, B rows read ahead of the B that are added (vectors by eight lanes, one after another: 50 cycles a row)
+            const T* x = reinterpret_cast<const T*>(ring + i % EMB_CHUNKS * EMB_CHUNK * EMB_GROUP) + lane;
+            const int rows = m - i * EMB_CHUNK < EMB_CHUNK ? m - i * EMB_CHUNK : EMB_CHUNK;
+            constexpr int B = sizeof(T) == 4 ? 16 : 8;
+            int k = 0;
+            if (rows >= B) {
+              T y[B];
+#pragma unroll
+              for (int u = 0; u < B; ++u) y[u] = x[u * VALUES];
+#pragma unroll 1
+              for (k = B; k + B <= rows; k += B) {
+                T z[B];
+#pragma unroll
+                for (int u = 0; u < B; ++u) z[u] = x[(k + u) * VALUES];
+#pragma unroll
+                for (int u = 0; u < B; ++u) sum = add_rn(sum, y[u]);
+#pragma unroll
+                for (int u = 0; u < B; ++u) y[u] = z[u];
+              }
+#pragma unroll
+              for (int u = 0; u < B; ++u) sum = add_rn(sum, y[u]);
+            }
+            for (; k < rows; ++k) sum = add_rn(sum, x[k * VALUES]);
           }
         }
         __syncthreads();
       }
     }
-    if (team == 0 && j < vecs) __stcs(reinterpret_cast<V*>(dW + (int64_t)v * dim) + j, acc);
+    const int64_t column = h % groups * VALUES + lane;
+    if (w == 0 && lane < VALUES && column < dim) dW[(int64_t)v * dim + column] = sum;
   }
 }
 
@@ -474,7 +510,7 @@ static prad_status scatter_t(prad_ctx* ctx, const void* index_col, const void* d
   const int vecs = vectors ? dim / EmbVec<T>::N : dim;
   auto at_most = [&](int64_t wanted, int per_sm) { return (int)(wanted < (int64_t)per_sm * ctx->sm_count ? wanted : (int64_t)per_sm * ctx->sm_count); };
   const int hot = at_most(n / (EMB_FEW + 1) * ceil_div(vecs, EMB_GROUP), 2);
-  const int grid = hot + at_most(ceil_div((int64_t)most * ceil_div(vecs, 64), EMB_WARPS), 2);
+  const int grid = hot + at_most(ceil_div((int64_t)most * ceil_div(vecs, 64), EMB_WARPS), hot ? 2 : 4);
   // shared memory for the ring only where a row can have many hits
   if (vectors) {
     constexpr int ring = EMB_CHUNKS * EMB_CHUNK * EMB_GROUP * 16;
