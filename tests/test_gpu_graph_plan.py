@@ -254,3 +254,42 @@ def test_plans_of_many_sets_of_start_values(engine):
     assert launches[:16] == [1] * 16 and min(launches[16:20]) > 6
     assert launches[20:40] == launches[:20] == launches[40:]
     g.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("units,cols,inner,steps", [(5, 1, 3, 2), (13, 7, 9, 3), (16, 8, 64, 6), (33, 15, 130, 2), (64, 16, 33, 5),
+                                                    (20, 32, 7, 3), (20, 33, 7, 3), (64, 8, 700, 2), (96, 4, 96, 7)])
+def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, inner, steps):
+    """Cells whose products are taken along by the programs that read them, forward and backward: column counts that divide a piece
+    and that do not, the last that fits and the first that does not, more k than shared memory has room for, gradients of shared
+    weights added up over the steps."""
+    results = []
+    for plan in ("1", "0"):
+        r = rng(units + cols + inner)
+        up = lambda *s: engine.upload((r.standard_normal(s) * 0.4).astype(dtype))  # noqa: E731
+        engine.set_option("graph_plan", plan)
+        try:
+            g = Graph(engine, dtype)
+            grads, w = [], {}
+            for name, shape in (("We", (units, inner)), ("Wa", (units, units)), ("Wb", (units, units)), ("b", (units, cols))):
+                grads.append(engine.zeros(shape, dtype))
+                w[name] = (up(*shape), grads[-1])
+            h, outs = g.input(up(units, cols)), []
+            for _ in range(steps):
+                x = g.node("MatrixMultiplyOperation", [g.weight(*w["We"]), g.input(up(inner, cols))])
+                a = g.node("MatrixAddThreeOperation", [x, g.node("MatrixMultiplyOperation", [g.weight(*w["Wa"]), h]), g.weight(*w["b"])])
+                c = g.node("SigmoidOperation", [g.node("MatrixMultiplyOperation", [g.weight(*w["Wb"]), h])])
+                h = g.node("HadamardProductOperation", [g.node("TanhOperation", [a]), c])
+                outs.append(g.node("MatrixAddOperation", [h, x]))
+            got = []
+            for k in range(2):
+                g.forward()
+                got += [g.data(o).numpy() for o in outs]
+                g.backward(outs[-1 - k], up(units, cols))
+                got += [d.numpy() for d in grads]
+            results.append(got)
+            g.close()
+        finally:
+            engine.set_option("graph_plan", "1")
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
