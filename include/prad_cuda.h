@@ -546,7 +546,9 @@ prad_status prad_cce_backward(prad_ctx* ctx, prad_dtype dt, const void* out, con
 /* ---------------------------------------------------------------- embedding
  * EmbeddingOperation.cs:49-86.  index_col holds the row indices as values of the matrix
  * type (column 0 of the input matrix, cast with (int)).  The backward adds duplicate
- * indices in input-row order, so the result is bit-identical to the sequential loop. */
+ * indices in input-row order, so the result is bit-identical to the sequential loop.  Both
+ * return once the indices have been looked at (PRAD_ERR_INVALID for one outside the table);
+ * the rows may then still be on their way, in stream order like everything else. */
 prad_status prad_embedding_forward(prad_ctx* ctx, prad_dtype dt, const void* index_col,
                                    const void* W, void* out, int n, int vocab, int dim);
 prad_status prad_embedding_backward(prad_ctx* ctx, prad_dtype dt, const void* index_col,

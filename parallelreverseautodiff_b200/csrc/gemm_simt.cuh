@@ -14,12 +14,12 @@
 // shared memory at 128 bytes per cycle and SM: with TM x TN outputs per thread a tile needs (TM + TN) / (TM TN) values per
 // multiply-add.  Products below 2^27 multiply-adds leave an SM one or two small tiles, a warp its scheduler to itself, so
 // nothing may ever wait for something that could have been started before:
-//  - k advances through a ring of shared-memory stages filled with cp.async by two warps of their own (the address
+//  - k advances through a ring of shared-memory stages filled with cp.async by warps of their own (the address
 //    arithmetic of the copies took the multiplying warps 8 of 26 cycles per k);
 //  - the fragments of the next 16 bytes of k are read while these are multiplied;
 //  - the products of the next k are formed before the sums of this one (26 -> 16 cycles per k in float, 49 -> 25 in double
 //    for a 16 x 16 tile).
-// 256 x 512 over k = 784: float 47 -> 14.5 us, double (as 512 x 256) 39 -> 22 us, against one register-staged tile ahead.
+// 256 x 512 over k = 784: float 47 -> 14.5 us, double (as 512 x 256) 39 -> 21 us, against one register-staged tile ahead.
 //
 // Each operand keeps the orientation it has in global memory -- [row][k] when k is contiguous, [k][row] when the row index
 // is -- because a copy cannot transpose.  A thread reads its fragments as 128-bit vectors along whichever is contiguous:
@@ -606,7 +606,8 @@ static prad_status launch_backward(prad_ctx* ctx, bool exact, Product<T> nt, Pro
 
 // Which tile shape.  A CTA that has its SM to itself takes `alone` cycles per k (its chain of additions, and the shared
 // memory's 128 bytes per cycle), n CTAs of one SM take n * `shared`: measured for the exact variants on products of
-// 128^2 x 2048, 256 x 512 x 784, 1024^2 x 120 and 2048^2 x 31.  The estimate is the busiest SM's time; the 24 stands for
+// 128^2 x 2048, 256 x 512 x 784, 1024^2 x 120 and 2048^2 x 31, before lanes and copies were laid out as they are now (16 x 16
+// alone: 14.5 float, 23 double); where the shapes cross has not been measured again.  The estimate is the busiest SM's time; the 24 stands for
 // filling the stages and writing the tile.  Small tiles win while there are fewer tiles than SMs, large ones once
 // every SM has several.
 struct ShapeCost { int bm, bn; double alone, shared; };

@@ -855,7 +855,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
         if (lowest[u] < latest[u] && latest[u] < levels - 2) {
           int best = latest[u];
           double least = 1e30;
-          for (int lv = latest[u]; lv >= lowest[u]; --lv) {
+          for (int lv = latest[u]; lv >= lowest[u] && least > 0; --lv) {
             double most;
             add(busy[lv], u, &most);
             const double more = most - *std::max_element(busy[lv].begin(), busy[lv].end());
@@ -1050,6 +1050,14 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
   // Deal the pieces of a level to the workers of `c` CTAs, the longest first to whoever has least (and to another SM before the
   // same one again); worker k of the dealing order is number k / c of CTA k % c.  Returns the time of the busiest.
   auto deal = [&](int lv, int c, std::vector<std::vector<Item>>* lists) {
+    if (pieces[lv].size() <= (size_t)c * WORKERS) {          // one each
+      if (lists)
+        for (int k = 0; k < (int)pieces[lv].size(); ++k) {
+          const Piece& p = pieces[lv][k];
+          (*lists)[k % c * WORKERS + k / c].push_back({p.prog, p.bytes, p.chunk, 0});
+        }
+      return pieces[lv].empty() ? 0.0 : pieces[lv][0].cost;
+    }
     std::vector<std::pair<double, int>> heap;                // least busy first
     for (int k = 0; k < c * WORKERS; ++k) heap.push_back({0.0, k});
     auto later = [](const std::pair<double, int>& x, const std::pair<double, int>& y) { return x > y; };
@@ -1067,7 +1075,11 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
   // The last levels run on all SMs, a launch each, where sixteen SMs would need 6 us longer for them (a launch, its program's way
   // into every SM and the pieces are 4 us at the least).
   int narrow = levels;
-  while (narrow > 0 && deal(narrow - 1, ctas, nullptr) - deal(narrow - 1, ctx->sm_count, nullptr) > 6.0) --narrow;
+  auto gain = [&](int lv) {
+    const double here = deal(lv, ctas, nullptr);
+    return here > 6.0 ? here - deal(lv, ctx->sm_count, nullptr) : 0.0;
+  };
+  while (narrow > 0 && gain(narrow - 1) > 6.0) --narrow;
   *est_us = 4.0;
   if (narrow > 0) {
     Part part{ctas, true, {}};
