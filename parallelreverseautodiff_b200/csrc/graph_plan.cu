@@ -571,16 +571,20 @@ struct Group {
 // Products that programs can compute for themselves.  A product of few outputs whose first reader is an elementwise operation on
 // them needs no level of its own, with its barrier and its way through memory: dots[e] are the products that operation e takes
 // along, fused[i] says that product i is one.  The product moves to the place of its reader, so nothing in between may write what
-// it reads or touch what it writes.
-constexpr int DOT_COLUMNS = 32, DOT_LOOK = 256;
+// it reads or touch what it writes.  Every piece reads all columns of a product's second operand, so that may have DOT_OPERAND
+// bytes: three layers of 64 double units over twelve steps take 526 us with 16 columns (8 KB) as levels of their own and 592 us inside
+// programs, with 32 columns 890 and 1433 us; eight steps of two layers with 8 columns (4 KB) 169 us inside, 298 as before.
+constexpr int DOT_COLUMNS = 32, DOT_LOOK = 256, DOT_OPERAND = 4 * 1024;
 constexpr int64_t TEAM_ELEMENTS = 2048;      // up to here several threads can share an element
-static void find_dots(const std::vector<Prim>& ops, const std::vector<std::vector<Access>>& acc, std::vector<std::vector<int>>& dots,
+static void find_dots(const std::vector<Prim>& ops, size_t es, const std::vector<std::vector<Access>>& acc, std::vector<std::vector<int>>& dots,
                       std::vector<char>& fused) {
   const int N = (int)ops.size();
   auto meets = [](const Access& a, const Access& b) { return a.lo < b.hi && b.lo < a.hi; };
   for (int i = 0; i < N; ++i) {
     const Prim& p = ops[i];
-    if (p.kind != PRIM_PRODUCT || p.batch != 1 || p.K < 1 || p.N < 1 || p.N > DOT_COLUMNS || (int64_t)p.M * p.N > TEAM_ELEMENTS || acc[i].size() != 3) continue;
+    if (p.kind != PRIM_PRODUCT || p.batch != 1 || p.K < 1 || p.N < 1 || p.N > DOT_COLUMNS || (int64_t)p.M * p.N > TEAM_ELEMENTS || acc[i].size() != 3 ||
+        (int64_t)p.K * p.N * (int64_t)es > DOT_OPERAND)
+      continue;
     const Access &A = acc[i][0], &B = acc[i][1], &X = acc[i][2];
     if (meets(X, A) || meets(X, B)) continue;
     for (int e = i + 1; e < N && e <= i + DOT_LOOK; ++e) {
@@ -705,7 +709,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
   std::vector<std::vector<int>> dots(N), after(N);           // after[d]: operations that wait for d
   std::vector<char> fused(N, 0);
   for (int i = 0; i < N; ++i) accesses(ops[i], es, all_acc[i]);
-  find_dots(ops, all_acc, dots, fused);
+  find_dots(ops, es, all_acc, dots, fused);
   std::vector<Access> acc;
   *launch_us = 0;
   auto region_at = [&](const Access& a) -> Region& {

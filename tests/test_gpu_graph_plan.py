@@ -258,7 +258,7 @@ def test_plans_of_many_sets_of_start_values(engine):
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("units,cols,inner,steps", [(5, 1, 3, 2), (13, 7, 9, 3), (16, 8, 64, 6), (33, 15, 130, 2), (64, 16, 33, 5),
-                                                    (20, 32, 7, 3), (20, 33, 7, 3), (64, 8, 700, 2), (96, 4, 96, 7)])
+                                                    (20, 32, 7, 3), (20, 33, 7, 3), (64, 8, 700, 2), (64, 8, 65, 2), (96, 4, 96, 7), (400, 1, 500, 2)])
 def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, inner, steps):
     """Cells whose products are taken along by the programs that read them, forward and backward: column counts that divide a piece
     and that do not, the last that fits and the first that does not, more k than shared memory has room for, gradients of shared
