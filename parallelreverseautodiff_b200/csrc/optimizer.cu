@@ -88,7 +88,7 @@ __device__ __forceinline__ void tensor_stats(const MultiTensor& t, int ti, const
 // squares as the float build does, rounded to T; else both are double.  (Mean and squares as a pass each: 4.3 + 5.5 us of a
 // 670 000-parameter step's 19.5 us for clip and Adam, and a second read of a large network's gradients.)
 template <typename T>
-__global__ void __launch_bounds__(MT_THREADS)
+__global__ void __launch_bounds__(MT_THREADS, sizeof(T) == 4 ? 4 : 2)
 mt_stats_kernel(MultiTensor t, double* __restrict__ stats) {
   chain_begin();
   constexpr int VEC = 16 / sizeof(T), TRIPS = MT_CHUNK / (MT_THREADS * VEC);
@@ -228,8 +228,10 @@ __device__ __forceinline__ void adam_value(const AdamScalars<T>& a, T g, T& w, T
 
 // The streaming pass.  clip_mode 0 none / 1 reference / 2 global norm (scale from stats);
 // do_adam 0 = clip only (writes g), 1 = also update w, m, v; zero_grad clears g afterwards.
+// (Registers: five CTAs an SM in float, four in double, as many as without the loads ahead.  With that, eight layers of 4096 x 4096
+// over 1024 rows take 3580 -> 3480 us a step; with three CTAs an SM large networks took longer than before.)
 template <typename T>
-__global__ void __launch_bounds__(MT_THREADS)
+__global__ void __launch_bounds__(MT_THREADS, sizeof(T) == 4 ? 5 : 4)
 mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, T clip, T minv,
                 double max_norm, int do_adam, AdamScalars<T> a, int zero_grad, const int* __restrict__ gemm_gave_up) {
   chain_begin();
