@@ -51,82 +51,87 @@ constexpr int ST_MEAN = 0, ST_STD = MT_MAX, ST_SS = 2 * MT_MAX, ST_PART = 2 * MT
 template <typename T> __device__ __forceinline__ T mean_of(double s, int64_t size) { return div_rn((T)s, (T)size); }            // sum / count
 template <typename T> __device__ __forceinline__ T sigma_of(double s, int64_t size) { return sqrt_rn(div_rn((T)s, (T)size)); }  // Sqrt(varianceSum / count)
 
-// Where the sums of squared deviations begin; the other partial sums are at ST_PART.
-__device__ __forceinline__ int squares_at(const MultiTensor& t) { return ST_PART + t.blk_start[t.count]; }
+// What a CTA leaves of its values: their sum, the sum of their deviations from a mean of its own, and that of the deviations' squares.
+enum { ST_SUMS, ST_DEVS, ST_SQUARES, ST_KINDS };
+__device__ __forceinline__ int part_at(const MultiTensor& t, int kind) { return ST_PART + kind * t.blk_start[t.count]; }
 
-// A tensor's mean and standard deviation from what its CTAs left: partial sums in CTA order by a fixed tree, and squares about
-// each CTA's own mean, moved to the common one: sum (x - mean)^2 = sum_b [sum (x - mean_b)^2 + n_b (mean_b - mean)^2].
-// All threads get them.
+// The mean that a CTA of n values, of the sum s, takes them about: the tensor's where it has all of them, its own otherwise.
+template <typename T> __device__ __forceinline__ double pivot_of(double s, int64_t n, int64_t size) {
+  return n == size ? (double)mean_of<T>(s, size) : s / (double)n;
+}
+
+// A tensor's mean and standard deviation from what its CTAs left: partial sums in CTA order by a fixed tree.  The mean is the one
+// that clip_reference_value subtracts, rounded to T, and the squares are moved to it: with p a CTA's pivot, r = sum (x - p) and
+// d = p - mean, sum (x - mean)^2 = sum (x - p)^2 + d (2 r + n d).  r is rounding only (p is s / n rounded), but where all values are
+// about the same, so are the squares, and z = (x - mean) / sigma is 1, not 0 or infinity.  All threads get them.
 template <typename T>
 __device__ __forceinline__ void tensor_stats(const MultiTensor& t, int ti, const double* __restrict__ stats, T* mean, T* sd) {
   const int b0 = t.blk_start[ti], blocks = t.blk_start[ti + 1] - b0;
-  const double *sums = stats + ST_PART + b0, *squares = stats + squares_at(t) + b0;
+  const double *sums = stats + part_at(t, ST_SUMS) + b0, *devs = stats + part_at(t, ST_DEVS) + b0, *squares = stats + part_at(t, ST_SQUARES) + b0;
   const int64_t size = t.size[ti];
   const bool mine = (int)threadIdx.x < blocks;
-  const double s0 = mine ? sums[threadIdx.x] : 0.0, q0 = mine ? squares[threadIdx.x] : 0.0;
+  const double s0 = mine ? sums[threadIdx.x] : 0.0, r0 = mine ? devs[threadIdx.x] : 0.0, q0 = mine ? squares[threadIdx.x] : 0.0;
   double acc = s0;
   for (int b = threadIdx.x + MT_THREADS; b < blocks; b += MT_THREADS) acc += sums[b];
-  const double total = block_sum_d<MT_THREADS>(acc);
-  *mean = mean_of<T>(total, size);
-  if (blocks == 1) {                       // about the mean itself already
-    *sd = sigma_of<T>(block_sum_d<MT_THREADS>(q0), size);
-    return;
-  }
-  const double mu = total / (double)size;
-  auto moved = [&](int b, double s, double q) {
-    const int64_t left = size - (int64_t)b * t.chunk;
-    const double n = (double)(left < t.chunk ? left : t.chunk), d = s / n - mu;
-    return q + n * d * d;
+  const T mu = mean_of<T>(block_sum_d<MT_THREADS>(acc), size);
+  auto moved = [&](int b, double s, double r, double q) {
+    if (isinf(q)) return q;                  // (the rest may be infinite too, with the other sign)
+    const int64_t left = size - (int64_t)b * t.chunk, n = left < t.chunk ? left : t.chunk;
+    const double d = pivot_of<T>(s, n, size) - (double)mu;
+    return q + d * (2.0 * r + (double)n * d);
   };
-  double var = mine ? moved(threadIdx.x, s0, q0) : 0.0;
-  for (int b = threadIdx.x + MT_THREADS; b < blocks; b += MT_THREADS) var += moved(b, sums[b], squares[b]);
+  double var = mine ? moved(threadIdx.x, s0, r0, q0) : 0.0;
+  for (int b = threadIdx.x + MT_THREADS; b < blocks; b += MT_THREADS) var += moved(b, sums[b], devs[b], squares[b]);
+  *mean = mu;
   *sd = sigma_of<T>(block_sum_d<MT_THREADS>(var), size);
 }
 
 // What the reference's clip has to know of a gradient (GradientClipper.cs:120-127), one pass over it: a CTA adds its values up
-// and then, from registers, the squares of their deviations from its own mean.  A tensor of one CTA takes the mean and the
-// squares as the float build does, rounded to T; else both are double.  (Mean and squares as a pass each: 4.3 + 5.5 us of a
-// 670 000-parameter step's 19.5 us for clip and Adam, and a second read of a large network's gradients.)
+// and then, from registers, their deviations from its pivot and the squares of these, in double.  (Mean and squares as a pass each:
+// 4.3 + 5.5 us of a 670 000-parameter step's 19.5 us for clip and Adam, and a second read of a large network's gradients.)
 template <typename T>
 __global__ void __launch_bounds__(MT_THREADS, sizeof(T) == 4 ? 4 : 2)
 mt_stats_kernel(MultiTensor t, double* __restrict__ stats) {
   chain_begin();
   constexpr int VEC = 16 / sizeof(T), TRIPS = MT_CHUNK / (MT_THREADS * VEC);
   using V = typename MtVec<T>::type;
-  const int ti = find_tensor(t, blockIdx.x), blocks = t.blk_start[ti + 1] - t.blk_start[ti];
-  const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
-  int64_t end = start + t.chunk;
-  if (end > t.size[ti]) end = t.size[ti];
-  const T* g = (const T*)t.g[ti];
-  const int64_t vend = t.vec ? end - (end - start) % VEC : start;      // chunk starts are multiples of the vector width
-  const int64_t first = start + (int64_t)threadIdx.x * VEC;
+  const int ti = find_tensor(t, blockIdx.x);
+  const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk, left = t.size[ti] - start;
+  const int n = left < t.chunk ? (int)left : t.chunk;
+  const T* g = (const T*)t.g[ti] + start;
+  const int vecs = t.vec ? n / VEC : 0;      // chunk starts are multiples of the vector width
   V v[TRIPS];
   double acc = 0.0;
 #pragma unroll
   for (int k = 0; k < TRIPS; ++k)
-    if (first + k * MT_THREADS * VEC < vend) v[k] = *reinterpret_cast<const V*>(g + first + k * MT_THREADS * VEC);
+    if ((int)threadIdx.x + k * MT_THREADS < vecs) v[k] = reinterpret_cast<const V*>(g)[threadIdx.x + k * MT_THREADS];
   auto each = [&](auto&& f) {
 #pragma unroll
     for (int k = 0; k < TRIPS; ++k)
-      if (first + k * MT_THREADS * VEC < vend)
+      if ((int)threadIdx.x + k * MT_THREADS < vecs)
 #pragma unroll
         for (int q = 0; q < VEC; ++q) f(reinterpret_cast<const T*>(&v[k])[q]);
-    for (int64_t i = vend + threadIdx.x; i < end; i += MT_THREADS) f(g[i]);
+    for (int i = vecs * VEC + threadIdx.x; i < n; i += MT_THREADS) f(g[i]);
   };
   each([&](T x) { acc += (double)x; });
   const double s = block_sum_d<MT_THREADS>(acc);
-  double sq = 0.0;
-  if (blocks == 1) {
-    const T mean = mean_of<T>(s, t.size[ti]);
-    each([&](T x) { const T d = sub_rn(x, mean); sq += (double)mul_rn(d, d); });
-  } else {
-    const double mean = s / (double)(end - start);
-    each([&](T x) { const double d = (double)x - mean; sq = __fma_rn(d, d, sq); });
+  const double pivot = pivot_of<T>(s, n, t.size[ti]);
+  double sums[2] = {0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < TRIPS; ++k) {          // not converted once for both passes: 32 doubles do not fit the registers
+    uint4& x = reinterpret_cast<uint4&>(v[k]);
+    asm volatile("" : "+r"(x.x), "+r"(x.y), "+r"(x.z), "+r"(x.w));
   }
-  sq = block_sum_d<MT_THREADS>(sq);
+  each([&](T x) {
+    const double d = (double)x - pivot;
+    sums[0] += d;
+    sums[1] = __fma_rn(d, d, sums[1]);
+  });
+  block_sums_d<MT_THREADS>(sums);
   if (threadIdx.x == 0) {
-    stats[ST_PART + blockIdx.x] = s;
-    stats[squares_at(t) + blockIdx.x] = sq;
+    stats[part_at(t, ST_SUMS) + blockIdx.x] = s;
+    stats[part_at(t, ST_DEVS) + blockIdx.x] = sums[0];
+    stats[part_at(t, ST_SQUARES) + blockIdx.x] = sums[1];
   }
 }
 
@@ -378,7 +383,7 @@ static prad_status clip_adam_t(prad_ctx* ctx, void* const* w, void* const* g, vo
     int nb = build_table<T>(ctx, t, w, g, m, v, sizes, first, cnt);
     if (nb > max_blocks) max_blocks = nb;
   }
-  prad_status s = ensure_workspace(ctx, (size_t)(ST_PART + 2 * max_blocks) * sizeof(double));
+  prad_status s = ensure_workspace(ctx, (ST_PART + ST_KINDS * (size_t)max_blocks) * sizeof(double));
   if (s) return s;
   double* stats = (double*)ctx->ws;
 
