@@ -1,4 +1,6 @@
 """Ordered scatter-add where rows collect no, one, a warp's worth and many hits, against the sequential loop, bit for bit."""
+import time
+
 import numpy as np
 import pytest
 
@@ -57,3 +59,42 @@ def test_bad_indices_are_told_apart_from_the_calls_after_them(engine):
         with pytest.raises(PradError):
             engine.embedding_backward(bad, d, 5)
         np.testing.assert_array_equal(engine.embedding_backward(good, d, 5).numpy()[:, 0], [1, 0, 0, 0, 2])
+
+
+@pytest.mark.parametrize("dtype,dim", [(np.float32, 1), (np.float32, 33), (np.float32, 132), (np.float32, 260), (np.float64, 18), (np.float64, 67)])
+@pytest.mark.parametrize("n,vocab", [(9000, 60), (60000, 500), (60000, 2500), (140000, 700), (140000, 540), (530000, 3000)])
+def test_rows_of_many_and_of_very_many_hits(engine, dtype, dim, n, vocab):
+    """Most rows beyond what a warp orders: lists of 33, 255, 256, 257, 2048 and 2049 hits beside those of the calls' own lengths, over one
+    segment of rows, over several, and in calls that are too large for one launch, where a list runs over several windows."""
+    r = rng(n + vocab + dim)
+    idx = r.integers(0, vocab, n)
+    at = 0
+    for row, hits in ((0, 33), (vocab - 1, 256), (1, 257), (vocab - 2, 255), (2, 2048), (vocab // 2, 2049)):
+        idx[idx == row] = (vocab - 3) - row % 7
+        idx[at:at + hits] = row
+        at += hits
+    idx = r.permutation(idx)
+    col = idx.astype(dtype).reshape(n, 1)
+    dOut = (r.standard_normal((n, dim)) * 10.0 ** r.integers(-3, 4, (n, 1))).astype(dtype)
+    got = engine.embedding_backward(engine.upload(col), engine.upload(dOut), vocab).numpy()
+    np.testing.assert_array_equal(got, O.embedding_backward(col, dOut, vocab))
+
+
+def test_rows_of_many_hits_cost_what_their_data_costs(engine):
+    """The same rows of dOut, added up over 50000 rows of about 21 hits and over 25000 of about 42: two ways through the sums, the same
+    bytes.  (A search per task that grew with the number of such rows made the second one 60 times as slow.)"""
+    n, dim = 1 << 20, 64
+    dOut = engine.zeros((n, dim), np.float32)
+    times = []
+    for vocab in (50000, 25000):
+        idx = engine.upload(rng(vocab).integers(0, vocab, (n, 1)).astype(np.float32))
+        out = engine.empty((vocab, dim), np.float32)
+        best = 1e9
+        for _ in range(4):
+            engine.sync()
+            t = time.perf_counter()
+            engine.embedding_backward(idx, dOut, vocab, out=out)
+            engine.sync()
+            best = min(best, time.perf_counter() - t)
+        times.append(best)
+    assert times[1] < 10 * times[0], times
