@@ -233,17 +233,15 @@ __device__ __forceinline__ void adam_value(const AdamScalars<T>& a, T g, T& w, T
 
 // The streaming pass.  clip_mode 0 none / 1 reference / 2 global norm (scale from stats);
 // do_adam 0 = clip only (writes g), 1 = also update w, m, v; zero_grad clears g afterwards.
-// (Registers: five CTAs an SM in float, four in double, as many as without the loads ahead.  With that, eight layers of 4096 x 4096
-// over 1024 rows take 3580 -> 3480 us a step; with three CTAs an SM large networks took longer than before.)
 template <typename T>
-__global__ void __launch_bounds__(MT_THREADS, sizeof(T) == 4 ? 5 : 4)
+__global__ void __launch_bounds__(MT_THREADS)
 mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, T clip, T minv,
                 double max_norm, int do_adam, AdamScalars<T> a, int zero_grad, const int* __restrict__ gemm_gave_up) {
   chain_begin();
   // A tensor-core product on this context ran out of a bounded wait: the gradients on the stream are
   // not valid, so weights, moments and gradients are left exactly as they are (one load per CTA; the
   // host learns of it at its next prad_sync / prad_download, which returns PRAD_ERR_TIMEOUT).
-  const int gave_up = gemm_gave_up ? *gemm_gave_up : 0;
+  if (gemm_gave_up && *gemm_gave_up != 0) return;
   const int ti = find_tensor(t, blockIdx.x);
   const int64_t start = (int64_t)(blockIdx.x - t.blk_start[ti]) * t.chunk;
   int64_t end = start + t.chunk;
@@ -257,18 +255,6 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
   constexpr int VEC = 16 / sizeof(T);
   using V = typename MtVec<T>::type;
   const int64_t vend = t.vec ? end - (end - start) % VEC : start;
-  // the first trip's values are on their way while the statistics are put together
-  V gv, wv, mv, vv;
-  auto load = [&](int64_t i) {
-    gv = *reinterpret_cast<const V*>(g + i);
-    if (do_adam) {
-      wv = *reinterpret_cast<const V*>(w + i);
-      mv = *reinterpret_cast<const V*>(m + i);
-      vv = *reinterpret_cast<const V*>(v + i);
-    }
-  };
-  int64_t i = start + (int64_t)threadIdx.x * VEC;
-  if (i < vend) load(i);
   if (clip_mode == 1) {
     if (t.fold) {
       tensor_stats<T>(t, ti, stats, &mean, &sd);
@@ -277,7 +263,6 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
       sd = (T)stats[ST_STD + ti];
     }
   }
-  if (gave_up) return;
   if (clip_mode == 2) {
     double norm = sqrt(stats[ST_SS]);
     if (norm > max_norm) { gscale = (T)(max_norm / norm); scale_on = true; }
@@ -287,7 +272,14 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
     if (scale_on) return mul_rn(gi, gscale);
     return gi;
   };
-  while (i < vend) {
+  for (int64_t i = start + (int64_t)threadIdx.x * VEC; i < vend; i += MT_THREADS * VEC) {
+    V gv = *reinterpret_cast<const V*>(g + i);
+    V wv, mv, vv;
+    if (do_adam) {
+      wv = *reinterpret_cast<const V*>(w + i);
+      mv = *reinterpret_cast<const V*>(m + i);
+      vv = *reinterpret_cast<const V*>(v + i);
+    }
 #pragma unroll
     for (int q = 0; q < VEC; ++q) {
       T gi = clip_one(reinterpret_cast<T*>(&gv)[q]);
@@ -301,8 +293,6 @@ mt_apply_kernel(MultiTensor t, const double* __restrict__ stats, int clip_mode, 
       *reinterpret_cast<V*>(v + i) = vv;
     }
     if (zero_grad || clip_mode != 0) *reinterpret_cast<V*>(g + i) = gv;
-    i += MT_THREADS * VEC;
-    if (i < vend) load(i);
   }
   for (int64_t i = vend + threadIdx.x; i < end; i += MT_THREADS) {
     T gi = clip_one(g[i]);
