@@ -740,10 +740,18 @@ static prad_status gather_t(prad_ctx* ctx, const void* index_col, const void* W,
   int checkers = (int)ceil_div(n, 8 * EMB_THREADS);        // eight loads in flight per thread
   if (checkers > ctx->sm_count) checkers = ctx->sm_count;
   const bool vectors = dim % EmbVec<T>::N == 0 && (((uintptr_t)W | (uintptr_t)out) & 15) == 0;
-  launch_chained(vectors ? embedding_gather_kernel<T, true> : embedding_gather_kernel<T, false>, checkers + grid, EMB_THREADS, 0, ctx->stream,
-                 (const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag, ticket, checkers, ctx->tc_err + 48);
-  PRAD_LAUNCHED(ctx);
-  return PRAD_OK;
+  auto launch = [&](int first, int rest) -> prad_status {
+    launch_chained(vectors ? embedding_gather_kernel<T, true> : embedding_gather_kernel<T, false>, first + rest, EMB_THREADS, 0, ctx->stream,
+                   (const T*)index_col, (const T*)W, (T*)out, n, vocab, dim, ctx->host_flag, ticket, first, ctx->tc_err + 48);
+    PRAD_LAUNCHED(ctx);
+    return PRAD_OK;
+  };
+  // rows written over the indices (a table of one column, in place): looked at before the first one is
+  const char *i0 = (const char*)index_col, *o0 = (const char*)out;
+  const bool over = i0 < o0 + (int64_t)n * dim * sizeof(T) && o0 < i0 + (int64_t)n * sizeof(T);
+  if (!over) return launch(checkers, grid);
+  const prad_status s = launch(checkers, 0);
+  return s ? s : launch(0, grid);
 }
 
 }  // namespace prad

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 
 import oracle as O
-from parallelreverseautodiff_b200._lib import PradError
+from parallelreverseautodiff_b200._lib import PradError, check
+from parallelreverseautodiff_b200.engine import dtype_code
 from util import rng
 
 pytestmark = pytest.mark.gpu
@@ -98,3 +99,17 @@ def test_rows_of_many_hits_cost_what_their_data_costs(engine):
             best = min(best, time.perf_counter() - t)
         times.append(best)
     assert times[1] < 10 * times[0], times
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_gather_of_one_column_in_the_place_of_its_indices(engine, dtype):
+    """A row is written after its own index has been read, so a one-column gather may replace its indices.  The table's values are no
+    indices: whoever looked at them there would find rows outside the table."""
+    n, vocab = 1 << 20, 1000
+    idx = rng(3).integers(0, vocab, (n, 1))
+    W = -1.0 - np.arange(vocab, dtype=dtype).reshape(vocab, 1)
+    table = engine.upload(W)
+    for _ in range(5):
+        m = engine.upload(idx.astype(dtype))
+        check(engine.lib.prad_embedding_forward(engine.ctx, dtype_code(dtype), m.ptr, table.ptr, m.ptr, n, vocab, 1))
+        np.testing.assert_array_equal(m.numpy(), W[idx[:, 0]])
