@@ -562,10 +562,15 @@ struct Region {
   std::vector<int> writers, readers;
 };
 
+// (buffer, columns of a row operand or 0): what has a place of its own in a program
+using Place = std::pair<const void*, int>;
+
 // An elementwise program in the making.
 struct Group {
   int64_t n = 0;
   std::vector<int> ops;                      // ascending
+  std::vector<Place> places;                 // of their operands, ascending
+  int dots = 0, rows = 0, dot_n = 0;         // products taken along, rows of their operands, their columns
 };
 
 // Products that programs can compute for themselves.  A product of few outputs whose first reader is an elementwise operation on
@@ -608,8 +613,6 @@ static void find_dots(const std::vector<Prim>& ops, size_t es, const std::vector
   }
 }
 
-// (buffer, columns of a row operand or 0): what has a place of its own in a program
-using Place = std::pair<const void*, int>;
 static Place place_of(const Prim& p, size_t k) { return {p.in[k], p.kind == PRIM_ADD_ROW && k == 1 ? p.cols : 0}; }
 template <typename T> static int slot_limit(int64_t n) {
   return n <= TEAM_ELEMENTS ? SLOTS : std::min(SLOTS, WORK_BYTES / (NT * (int)sizeof(T)));
@@ -617,14 +620,21 @@ template <typename T> static int slot_limit(int64_t n) {
 // operand rows a product in a program keeps in shared memory, at the most
 constexpr int DOT_PIECE = NT / 8, DOT_ROWS = 320;
 static int dot_rows(const Prim& p) { return (p.N <= DOT_PIECE && DOT_PIECE % p.N == 0 ? DOT_PIECE / p.N : (DOT_PIECE - 1) / p.N + 2) + p.N; }
-static int places(const std::vector<Prim>& all, const std::vector<int>& ops) {
-  std::vector<Place> seen;
-  for (int o : ops) {
-    for (size_t k = 0; k < all[o].in.size(); ++k) seen.push_back(place_of(all[o], k));
-    for (void* q : all[o].out) seen.push_back({q, 0});
+// a program of one operation
+static void program_of(const std::vector<Prim>& all, int i, const std::vector<int>& dots, Group& g) {
+  g.n = all[i].n;
+  g.ops.assign(1, i);
+  g.places.clear();
+  for (size_t k = 0; k < all[i].in.size(); ++k) g.places.push_back(place_of(all[i], k));
+  for (void* q : all[i].out) g.places.push_back({q, 0});
+  std::sort(g.places.begin(), g.places.end());
+  g.places.erase(std::unique(g.places.begin(), g.places.end()), g.places.end());
+  g.dots = g.rows = g.dot_n = 0;
+  for (int d : dots) {
+    ++g.dots;
+    g.rows += dot_rows(all[d]);
+    g.dot_n = all[d].N;
   }
-  std::sort(seen.begin(), seen.end());
-  return (int)(std::unique(seen.begin(), seen.end()) - seen.begin());
 }
 
 struct Piece { uint32_t prog, bytes, chunk; double cost; };
@@ -662,15 +672,18 @@ static void fold_into(std::vector<Ins>& ins, const Ins& c) {
 // Sorts a program into phases: an instruction comes behind those whose values it reads or replaces.  Returns how many.
 static int order_by_phase(std::vector<Ins>& ins) {
   std::vector<int> phase(ins.size(), 0);
-  int phases = 0;
+  int phases = 0, written[SLOTS], read[SLOTS];               // by a slot: the first phase behind its writers, behind its readers
+  std::fill(written, written + SLOTS, 0);
+  std::fill(read, read + SLOTS, 0);
   for (size_t x = 0; x < ins.size(); ++x) {
-    for (size_t y = 0; y < x; ++y) {
-      bool after = false;
-      for (int k = 0; k < ins[x].n_in; ++k) after = after || writes(ins[y], ins[x].src[k]);
-      for (int k = 0; k < outputs(ins[x]); ++k) after = after || writes(ins[y], ins[x].dst[k]) || reads(ins[y], ins[x].dst[k]);
-      if (after) phase[x] = std::max(phase[x], phase[y] + 1);
-    }
-    phases = std::max(phases, phase[x] + 1);
+    const Ins& c = ins[x];
+    int ph = 0;
+    for (int k = 0; k < c.n_in; ++k) ph = std::max(ph, written[c.src[k]]);
+    for (int k = 0; k < outputs(c); ++k) ph = std::max(ph, std::max(written[c.dst[k]], read[c.dst[k]]));
+    phase[x] = ph;
+    for (int k = 0; k < c.n_in; ++k) read[c.src[k]] = std::max(read[c.src[k]], ph + 1);
+    for (int k = 0; k < outputs(c); ++k) written[c.dst[k]] = ph + 1;
+    phases = std::max(phases, ph + 1);
   }
   std::vector<Ins> sorted;
   for (int ph = 0; ph < phases; ++ph) {
@@ -712,6 +725,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
   find_dots(ops, es, all_acc, dots, fused);
   std::vector<Access> acc;
   *launch_us = 0;
+  int joins = 0;
   auto region_at = [&](const Access& a) -> Region& {
     auto it = mem.upper_bound(a.lo);
     if (it != mem.begin()) {
@@ -721,6 +735,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     if (it == mem.end() || it->first >= a.hi) return mem.emplace(a.lo, Region{a.lo, a.hi, true, false, {}, {}}).first->second;
     if (it->first == a.lo && it->second.hi == a.hi) return it->second;
     Region joined{a.lo, a.hi, false, false, {}, {}};      // overlaps: one region for all of them
+    ++joins;
     while (it != mem.end() && it->first < a.hi) {
       joined.lo = std::min(joined.lo, it->first);
       joined.hi = std::max(joined.hi, it->second.hi);
@@ -732,6 +747,10 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     const uintptr_t lo = joined.lo;
     return mem.emplace(lo, std::move(joined)).first->second;
   };
+  std::vector<int> near, join;               // operations that one may share a program with, their programs
+  Group one;
+  std::vector<Place> united, both;
+  std::vector<Region*> regions;              // of its accesses
   for (int i = 0; i < N; ++i) {
     *launch_us += launch_cost(ops[i], ctx->sm_count);
     if (fused[i]) continue;                  // with its reader
@@ -743,15 +762,18 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       }
     acc.insert(acc.end(), all_acc[i].begin(), all_acc[i].end());
     int lv = 0;
-    std::vector<int> near;                   // operations this one may share a program with
+    near.clear();
+    regions.clear();
+    const int joins_before = joins;
     for (const Access& a : acc) {
       Region& r = region_at(a);
+      regions.push_back(&r);
       auto depend = [&](int d) {
         if (d == i) return;
         const bool local = a.local && !a.fresh && r.local && elementwise(ops[i]) && elementwise(ops[d]) && ops[i].n == ops[d].n;
         lv = std::max(lv, local ? level[d] : level[d] + 1);
         if (local) near.push_back(d);
-        after[d].push_back(i);
+        if (after[d].empty() || after[d].back() != i) after[d].push_back(i);
       };
       for (int d : r.writers) depend(d);
       if (a.write)
@@ -759,37 +781,56 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     }
     if (elementwise(ops[i])) {
       // join the programs of the local neighbours at this level, if one program can hold them all
-      Group merged;
-      merged.n = ops[i].n;
-      std::vector<int> join;
+      join.clear();
       for (int d : near)
         if (level[d] == lv && std::find(join.begin(), join.end(), group_of[d]) == join.end()) join.push_back(group_of[d]);
-      for (int g : join) merged.ops.insert(merged.ops.end(), groups[g].ops.begin(), groups[g].ops.end());
-      std::sort(merged.ops.begin(), merged.ops.end());
-      merged.ops.push_back(i);
-      int n_dot = 0, rows = 0;
-      bool one_shape = true;
-      for (int o : merged.ops)
-        for (int d : dots[o]) {
-          ++n_dot;
-          rows += dot_rows(ops[d]);
-          for (int o2 : merged.ops)
-            for (int d2 : dots[o2]) one_shape = one_shape && ops[d].N == ops[d2].N;
+      program_of(ops, i, dots[i], one);
+      if (!join.empty()) {
+        size_t count = 1;
+        int n_dot = one.dots, rows = one.rows, columns = one.dot_n;
+        bool fits = true;
+        united = one.places;
+        for (int g : join) {
+          const Group& o = groups[g];
+          count += o.ops.size();
+          n_dot += o.dots;
+          rows += o.rows;
+          fits = fits && (!o.dots || !columns || columns == o.dot_n);      // programs have one shape of product each
+          if (o.dots) columns = o.dot_n;
+          both.clear();
+          std::set_union(united.begin(), united.end(), o.places.begin(), o.places.end(), std::back_inserter(both));
+          united.swap(both);
         }
-      if (!join.empty() && ((int)merged.ops.size() > MAX_INS || places(ops, merged.ops) > slot_limit<T>(merged.n) || n_dot > MAX_DOTS ||
-                            rows > DOT_ROWS || !one_shape)) {
-        ++lv;                                // a program of its own, behind a barrier
-        join.clear();
-        merged.ops.assign(1, i);
+        if (fits && count <= MAX_INS && (int)united.size() <= slot_limit<T>(one.n) && n_dot <= MAX_DOTS && rows <= DOT_ROWS) {
+          Group& g = groups[join[0]];
+          for (size_t k = 1; k < join.size(); ++k) {
+            Group& o = groups[join[k]];
+            for (int op : o.ops) group_of[op] = join[0];
+            const size_t mid = g.ops.size();
+            g.ops.insert(g.ops.end(), o.ops.begin(), o.ops.end());
+            std::inplace_merge(g.ops.begin(), g.ops.begin() + mid, g.ops.end());
+            o = Group();
+          }
+          g.ops.push_back(i);
+          g.places = united;
+          g.dots = n_dot;
+          g.rows = rows;
+          g.dot_n = columns;
+          group_of[i] = join[0];
+        } else {
+          ++lv;                              // a program of its own, behind a barrier
+          join.clear();
+        }
       }
-      for (int g : join) groups[g].ops.clear();
-      const int id = (int)groups.size();
-      for (int o : merged.ops) group_of[o] = id;
-      groups.push_back(std::move(merged));
+      if (join.empty()) {
+        group_of[i] = (int)groups.size();
+        groups.push_back(one);
+      }
     }
     level[i] = lv;
-    for (const Access& a : acc) {
-      Region& r = region_at(a);
+    for (size_t k = 0; k < acc.size(); ++k) {
+      const Access& a = acc[k];
+      Region& r = joins == joins_before ? *regions[k] : region_at(a);
       r.local = r.local && a.local;
       if (!a.write) { r.readers.push_back(i); continue; }
       r.written = true;
@@ -826,10 +867,10 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     // as early as they can be, or all as late, take workers from the cells.
     if (order.size() <= 500 && levels > 2) {
       const int workers = ctas * WORKERS;
-      std::vector<std::vector<double>> busy(levels, std::vector<double>(workers, 0.0));
-      auto add = [&](std::vector<double> b, int u, double* most) {
+      std::vector<double> times((size_t)levels * workers, 0.0), total(levels, 0.0), copy(workers);
+      auto busy = [&](int lv) { return times.data() + (size_t)lv * workers; };       // ascending
+      auto pieces_of = [&](int u, double* cost) {            // how many, and a piece's time
         const Prim& p = ops[u];
-        double cost;
         int64_t n;
         if (group_of[u] >= 0) {
           const Group& g = groups[group_of[u]];
@@ -838,35 +879,58 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
             for (int d : dots[o]) k = std::max(k, ops[d].K);
           const bool team = k || (g.n <= TEAM_ELEMENTS && g.ops.size() >= 4);
           n = ceil_div(g.n, k ? DOT_PIECE : team ? NT / 4 : NT);
-          cost = (k ? 1.8 + 0.02 * k : 1.0) + (team ? 0.25 * (double)std::min<size_t>(g.ops.size(), 7) : 0.3 * (double)g.ops.size());
+          *cost = (k ? 1.8 + 0.02 * k : 1.0) + (team ? 0.25 * (double)std::min<size_t>(g.ops.size(), 7) : 0.3 * (double)g.ops.size());
         } else if (p.kind == PRIM_PRODUCT) {
           n = ceil_div((int64_t)p.M * p.N, p.K <= 32 && p.M > 16 && p.N > 16 ? 1024 : NT) * p.batch;
-          cost = 1.5 + 0.02 * p.K;
+          *cost = 1.5 + 0.02 * p.K;
         } else {
           n = ceil_div(p.rows * p.depth, NT / 32);
-          cost = 2.0 + 0.1 * p.cols;
+          *cost = 2.0 + 0.1 * p.cols;
         }
-        for (int64_t k = 0; k < std::min<int64_t>(n, 4 * workers); ++k) *std::min_element(b.begin(), b.end()) += cost;
-        *most = *std::max_element(b.begin(), b.end());
-        return b;
+        return std::min<int64_t>(n, 4 * workers);
       };
-      double ignored;
+      auto add = [&](double* b, int64_t n, double cost) {    // every piece to whoever has least
+        for (; n > 0 && b[workers - 1] - b[0] > cost; --n) {
+          const double x = b[0] + cost;
+          int k = 0;
+          for (; k + 1 < workers && b[k + 1] < x; ++k) b[k] = b[k + 1];
+          b[k] = x;
+        }
+        const int each = (int)(n / workers), more = (int)(n % workers);              // in turn from here on
+        for (int k = 0; k < workers; ++k) b[k] += (each + (k < more)) * cost;
+        std::rotate(b, b + more, b + workers);
+      };
+      auto longer = [&](int lv, int64_t n, double cost, double least) {              // by how much the level would be, if less than `least`
+        const double* b = busy(lv);
+        const double most = b[workers - 1], mean = (total[lv] + (double)n * cost) / workers;
+        if (mean - most >= least) return least;
+        std::copy(b, b + workers, copy.begin());
+        add(copy.data(), n, cost);
+        return std::max(0.0, copy[workers - 1] - most);
+      };
+      auto put = [&](int lv, int64_t n, double cost) {
+        add(busy(lv), n, cost);
+        total[lv] += (double)n * cost;
+      };
       std::vector<int> lowest(N, 0);
+      double cost;
       for (int u : order)
-        if (level[u] == latest[u]) busy[latest[u]] = add(busy[latest[u]], u, &ignored);
+        if (level[u] == latest[u]) {
+          const int64_t n = pieces_of(u, &cost);
+          put(latest[u], n, cost);
+        }
       for (size_t x = order.size(); x-- > 0;) {              // those with a lower level first
         const int u = order[x];
         if (lowest[u] < latest[u] && latest[u] < levels - 2) {
+          const int64_t n = pieces_of(u, &cost);
           int best = latest[u];
           double least = 1e30;
           for (int lv = latest[u]; lv >= lowest[u] && least > 0; --lv) {
-            double most;
-            add(busy[lv], u, &most);
-            const double more = most - *std::max_element(busy[lv].begin(), busy[lv].end());
+            const double more = longer(lv, n, cost, least);
             if (more < least - 1e-9) { least = more; best = lv; }
           }
           latest[u] = best;
-          busy[best] = add(busy[best], u, &ignored);
+          put(best, n, cost);
         }
         for (int v : users[u]) lowest[v] = std::max(lowest[v], latest[u] + 1);
       }
@@ -893,14 +957,15 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       std::vector<Load> loads;
       std::vector<Ins> ins;
       std::vector<Store> stores;
-      std::map<Place, int> slot;
-      int slots = 0;
+      int slot_of[SLOTS + 1], slots = 0;
+      std::fill(slot_of, slot_of + SLOTS + 1, -1);
+      auto slot = [&](const Place& at) -> int& { return slot_of[std::lower_bound(g.places.begin(), g.places.end(), at) - g.places.begin()]; };
       std::vector<int> taken;                // products, with their places
       for (int o : g.ops) {
         const Prim& q = ops[o];
         for (int d : dots[o]) {
           taken.push_back(d);
-          slot[Place{ops[d].out[0], 0}] = slots;
+          slot(Place{ops[d].out[0], 0}) = slots;
           stores.push_back({ops[d].out[0], (uint32_t)slots++, 0});
         }
         Ins c;
@@ -911,20 +976,20 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
         c.scalar = q.scalar;
         for (size_t k = 0; k < q.in.size(); ++k) {
           const Place at = place_of(q, k);
-          auto it = slot.find(at);
-          if (it == slot.end()) {
-            it = slot.emplace(at, slots++).first;
-            loads.push_back({at.first, (uint32_t)at.second, (uint32_t)it->second});
+          int& it = slot(at);
+          if (it < 0) {
+            it = slots++;
+            loads.push_back({at.first, (uint32_t)at.second, (uint32_t)it});
           }
-          c.src[k] = (uint8_t)it->second;
+          c.src[k] = (uint8_t)it;
         }
         for (size_t k = 0; k < q.out.size(); ++k) {
-          auto it = slot.find(Place{q.out[k], 0});
-          if (it == slot.end()) it = slot.emplace(Place{q.out[k], 0}, slots++).first;
-          c.dst[k] = (uint8_t)it->second;
+          int& it = slot(Place{q.out[k], 0});
+          if (it < 0) it = slots++;
+          c.dst[k] = (uint8_t)it;
           bool stored = false;
           for (const Store& s : stores) stored = stored || s.p == q.out[k];
-          if (!stored) stores.push_back({q.out[k], (uint32_t)it->second, 0});
+          if (!stored) stores.push_back({q.out[k], (uint32_t)it, 0});
         }
         fold_into(ins, c);
       }
@@ -951,7 +1016,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
         for (int d : taken) {
           const Prim& q = ops[d];
           const int a = operand(q.in[0], q.tA ? 1 : 0, q.M, q.K, dot_rows(q) - q.N), b = operand(q.in[1], q.tB ? 3 : 2, q.N, q.K, q.N);
-          dot.push_back({q.scalar, q.K, slot[Place{q.out[0], 0}], a, b});
+          dot.push_back({q.scalar, q.K, slot(Place{q.out[0], 0}), a, b});
           most_k = std::max(most_k, q.K);
         }
         int rows = 0;
@@ -1065,25 +1130,56 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     std::vector<std::pair<double, int>> heap;                // least busy first
     for (int k = 0; k < c * WORKERS; ++k) heap.push_back({0.0, k});
     auto later = [](const std::pair<double, int>& x, const std::pair<double, int>& y) { return x > y; };
-    double most = 0;
-    for (const Piece& p : pieces[lv]) {
-      std::pop_heap(heap.begin(), heap.end(), later);
-      const int k = heap.back().second;
-      most = std::max(most, heap.back().first += p.cost);
-      std::push_heap(heap.begin(), heap.end(), later);
-      if (lists) (*lists)[k % c * WORKERS + k / c].push_back({p.prog, p.bytes, p.chunk, 0});
+    auto give = [&](std::pair<double, int>& to, const Piece& p) {
+      to.first += p.cost;
+      if (lists) (*lists)[to.second % c * WORKERS + to.second / c].push_back({p.prog, p.bytes, p.chunk, 0});
+    };
+    const std::vector<Piece>& all = pieces[lv];
+    if (lists)
+      for (auto& l : *lists) l.reserve(l.size() + all.size() / (size_t)(c * WORKERS) + 1);
+    for (size_t k = 0; k < all.size();) {
+      size_t end = k + 1;                                    // pieces of one cost, many: in turn, once nobody is a piece ahead
+      while (end < all.size() && all[end].cost == all[k].cost) ++end;
+      if (end - k > 16) {
+        std::sort(heap.begin(), heap.end());                 // (a heap too)
+        if (heap.back().first - heap[0].first <= all[k].cost) {
+          for (size_t at = 0; k < end; ++k, at = at + 1 == heap.size() ? 0 : at + 1) give(heap[at], all[k]);
+          std::make_heap(heap.begin(), heap.end(), later);
+          continue;
+        }
+      }
+      for (; k < end; ++k) {
+        std::pop_heap(heap.begin(), heap.end(), later);
+        give(heap.back(), all[k]);
+        std::push_heap(heap.begin(), heap.end(), later);
+      }
     }
+    double most = 0;
+    for (const auto& w : heap) most = std::max(most, w.first);
     return most;
   };
   for (auto& lv : pieces) std::stable_sort(lv.begin(), lv.end(), [](const Piece& a, const Piece& b) { return a.cost > b.cost; });
   // The last levels run on all SMs, a launch each, where sixteen SMs would need 6 us longer for them (a launch, its program's way
   // into every SM and the pieces are 4 us at the least).
   int narrow = levels;
-  auto gain = [&](int lv) {
-    const double here = deal(lv, ctas, nullptr);
-    return here > 6.0 ? here - deal(lv, ctx->sm_count, nullptr) : 0.0;
-  };
-  while (narrow > 0 && gain(narrow - 1) > 6.0) --narrow;
+  std::vector<Part> wide;
+  std::vector<double> wide_us;
+  while (narrow > 0) {
+    double all = 0, longest = 0;
+    for (const Piece& p : pieces[narrow - 1]) { all += p.cost; longest = std::max(longest, p.cost); }
+    const double at_least = std::max(longest, all / (ctx->sm_count * WORKERS));      // on all SMs
+    if (all / (ctas * WORKERS) + longest - at_least <= 6.0) break;                   // (no worker is a piece ahead of the mean)
+    const bool sure = all / (ctas * WORKERS) - all / (ctx->sm_count * WORKERS) - longest > 6.0;
+    const double here = sure ? 1e30 : deal(narrow - 1, ctas, nullptr);
+    if (here - at_least <= 6.0) break;
+    Part part{ctx->sm_count, false, {}};
+    part.lists.assign(ctx->sm_count * WORKERS, {});
+    const double there = deal(narrow - 1, ctx->sm_count, &part.lists);
+    if (here - there <= 6.0) break;
+    wide.push_back(std::move(part));
+    wide_us.push_back(there);
+    --narrow;
+  }
   *est_us = 4.0;
   if (narrow > 0) {
     Part part{ctas, true, {}};
@@ -1099,11 +1195,9 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     }
     parts.push_back(std::move(part));
   }
-  for (int lv = narrow; lv < levels; ++lv) {
-    Part part{ctx->sm_count, false, {}};
-    part.lists.assign(ctx->sm_count * WORKERS, {});
-    *est_us += 3.0 + deal(lv, ctx->sm_count, &part.lists);
-    parts.push_back(std::move(part));
+  for (size_t k = wide.size(); k-- > 0;) {
+    *est_us += 3.0 + wide_us[k];
+    parts.push_back(std::move(wide[k]));
   }
 }
 
