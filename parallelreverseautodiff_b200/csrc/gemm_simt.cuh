@@ -514,12 +514,20 @@ template <typename T> static bool aligned16(const void* p) { return ((uintptr_t)
 // warps meet after every stage and wait for the slowest (512 x 784 x 256 in double, forward and backward, 67 us with copying warps
 // on two schedulers, 59 on four).  Where an operand's rows do not start at 16-byte boundaries (SmallOdd) there are twice or four
 // times as many copies, and four warps of them get in the way: a double step of 887 x 98-217-217-217-9 takes 301 us with them,
-// 212 with two.  Double: stages of 32 k, for half the barriers and half the ends of rows (that step took 350 us with 16).
+// 212 with two.  So do they in float where an SM has more than four tiles (256 x 784 x 512, backward, 4.05 tiles an SM: 25.5 us with
+// four, 23.2 with two; 128 x 784 x 512, 3.4 tiles: 14.3 and 15.0), for one less of the larger CTAs has room there.  (A Small without the
+// element-wise copies that it does not need is no better: 256 x 784 x 512 in double 24.0 instead of 19.3 us.)
+// Double: stages of 32 k, for half the barriers and half the ends of rows (that step took 350 us with 16), but of 16 (SmallShort), with
+// as many values on their way, for one product whose last stage of 32 would be zeros for a sixteenth of the work: 512 x 33 x 512 4.8
+// and 4.15 us, 184 x 80 x 1008 6.1 and 5.7, 1000 x 100 x 1000 21.5 and 20.1, but 176 x 144 x 656 5.4 and 5.8.  For the two products of a
+// Backward longer stages are the better ones all the same (41 x 230 x 896 13.2 and 14.4), and for 16 x 16 tiles in a network's step
+// (500 x 33-128-128-10 from the host 108 and 122).
 template <typename T> struct SimtShapes;
 template <> struct SimtShapes<float> {
   using Tiny = TileShape<float, 16, 16, 32, 2, 2, 4, 64>;
   using Small = TileShape<float, 32, 32, 32, 4, 2, 4, 128>;
   using SmallOdd = TileShape<float, 32, 32, 32, 4, 2, 4, 64>;
+  using SmallShort = SmallOdd;
   using Wide = TileShape<float, 64, 32, 32, 4, 4, 3, 64>;
   using Medium = TileShape<float, 64, 64, 32, 4, 4, 3, 64>;
   using Large = TileShape<float, 128, 128, 16, 8, 8, 4, 64>;
@@ -528,6 +536,7 @@ template <> struct SimtShapes<double> {
   using Tiny = TileShape<double, 16, 16, 32, 2, 2, 4, 64>;
   using Small = TileShape<double, 32, 32, 32, 4, 2, 3, 128>;
   using SmallOdd = TileShape<double, 32, 32, 32, 4, 2, 3, 64>;
+  using SmallShort = TileShape<double, 32, 32, 16, 4, 2, 6, 64>;
   using Wide = TileShape<double, 64, 32, 16, 4, 4, 3, 64>;
   using Medium = TileShape<double, 64, 64, 16, 4, 4, 3, 64>;
   using Large = Medium;
@@ -639,6 +648,14 @@ template <typename T> static int pick_shape(const prad_ctx* ctx, const ProductSi
   return best;
 }
 
+// The two rules of SimtShapes: whether small tiles are copied by four warps, and in stages of 16 k.
+template <typename T> static bool four_copying_warps(const prad_ctx* ctx, const ProductSize* p, int count) {
+  int64_t tiles = 0;
+  for (int i = 0; i < count; ++i) tiles += ceil_div(p[i].M, 32) * ceil_div(p[i].N, 32) * p[i].batch;
+  return sizeof(T) == 8 || tiles <= 4 * (int64_t)ctx->sm_count;
+}
+template <typename T> static bool short_stages(int64_t K) { return sizeof(T) == 8 && 16 * (ceil_div(K, 32) * 32) > 17 * (ceil_div(K, 16) * 16); }
+
 template <typename T>
 static Product<T> make_product(int M, int N, int K, double alpha, const void* A, int64_t lda, const void* B, int64_t ldb, double beta,
                                void* C, int64_t ldc, int64_t sA, int64_t sB, int64_t sC, const GemmEpilogue& e) {
@@ -672,8 +689,9 @@ prad_status gemm_simt(prad_ctx* ctx, bool exact, bool tA, bool tB, int M, int N,
   switch (pick_shape<T>(ctx, &size, 1)) {
     case 0: return launch_shape<T, typename Shapes::Tiny>(ctx, exact, tA, tB, batch, p);
     case 1:
-      return p.vecA && p.vecB ? launch_shape<T, typename Shapes::Small>(ctx, exact, tA, tB, batch, p)
-                              : launch_shape<T, typename Shapes::SmallOdd>(ctx, exact, tA, tB, batch, p);
+      if (short_stages<T>(K)) return launch_shape<T, typename Shapes::SmallShort>(ctx, exact, tA, tB, batch, p);
+      return p.vecA && p.vecB && four_copying_warps<T>(ctx, &size, 1) ? launch_shape<T, typename Shapes::Small>(ctx, exact, tA, tB, batch, p)
+                                                                      : launch_shape<T, typename Shapes::SmallOdd>(ctx, exact, tA, tB, batch, p);
     case 2: return launch_shape<T, typename Shapes::Wide>(ctx, exact, tA, tB, batch, p);
     case 3: return launch_shape<T, typename Shapes::Medium>(ctx, exact, tA, tB, batch, p);
     default: return launch_shape<T, typename Shapes::Large>(ctx, exact, tA, tB, batch, p);
@@ -691,8 +709,9 @@ prad_status gemm_simt_backward(prad_ctx* ctx, bool exact, const void* A, const v
   switch (pick_shape<T>(ctx, size, 2)) {
     case 0: return launch_backward<T, typename Shapes::Tiny>(ctx, exact, nt, tn);
     case 1:
-      return nt.vecA && nt.vecB && tn.vecA && tn.vecB ? launch_backward<T, typename Shapes::Small>(ctx, exact, nt, tn)
-                                                      : launch_backward<T, typename Shapes::SmallOdd>(ctx, exact, nt, tn);
+      return nt.vecA && nt.vecB && tn.vecA && tn.vecB && four_copying_warps<T>(ctx, size, 2)
+                 ? launch_backward<T, typename Shapes::Small>(ctx, exact, nt, tn)
+                 : launch_backward<T, typename Shapes::SmallOdd>(ctx, exact, nt, tn);
     case 2: return launch_backward<T, typename Shapes::Wide>(ctx, exact, nt, tn);
     case 3: return launch_backward<T, typename Shapes::Medium>(ctx, exact, nt, tn);
     default: return launch_backward<T, typename Shapes::Large>(ctx, exact, nt, tn);

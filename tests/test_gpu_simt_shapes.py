@@ -48,3 +48,12 @@ def test_pitches_and_epilogues(engine, dtype, pad):
     y = engine.matmul_forward(a, b, bias=engine.upload(bias), Z_out=z, act=E.ACT_LEAKY_RELU, act_alpha=0.01)
     np.testing.assert_array_equal(z.numpy(), ref + bias)
     np.testing.assert_array_equal(y.numpy(), O.leaky_relu_forward(ref + bias, 0.01))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("M,K,N", [(512, 32, 512), (512, 33, 512), (512, 48, 508), (510, 49, 510), (184, 80, 1008), (1000, 271, 96), (1000, 273, 96),
+                                   (256, 512, 512), (256, 764, 512), (256, 784, 512)])
+def test_ways_to_copy_small_tiles(engine, dtype, M, K, N):
+    """32 x 32 tiles on both sides of the rules for their copies: the last stage of k half full or fuller, aligned rows or not, up to four
+    tiles an SM and more."""
+    test_products_equal_the_sequential_loops(engine, dtype, M, K, N)
