@@ -673,6 +673,9 @@ prad_status prad_graph_value_data(prad_graph* g, int value, void** out_data);
 prad_status prad_graph_value_gradient(prad_graph* g, int value, void** out_grad);
 /* How many consumers each value had in the last backward (BackwardDependencyCounts). */
 prad_status prad_graph_consumer_count(prad_graph* g, int value, int* out_count);
+/* For diagnosis: how many matrix products the one-kernel walks of the graph ("graph_plan") take along with the elementwise
+ * operations that read them, in the forward walk and in all backward walks so far. */
+prad_status prad_graph_plan_products(prad_graph* g, int64_t* out_forward, int64_t* out_backward);
 
 /* ---------------------------------------------------------------- Tensor elementwise operations
  * The reference's second public API (PRAD `Tensor` / `TensorReverse`, src/PRAD/Tensor.Common.cs and

@@ -141,6 +141,7 @@ SIGNATURES = {
     "prad_graph_value_data": [vp, i32, pvp],
     "prad_graph_value_gradient": [vp, i32, pvp],
     "prad_graph_consumer_count": [vp, i32, C.POINTER(C.c_int)],
+    "prad_graph_plan_products": [vp, pi64, pi64],
     "prad_dp_unique_id": [vp],
     "prad_dp_init": [vp, vp, i32, i32],
     "prad_dp_allreduce": [vp, i32, vp, i64],

@@ -704,6 +704,16 @@ static prad_status backward_walk(prad_graph* g, const int* start_values, const v
   return PRAD_OK;
 }
 
+prad_status prad_graph_plan_products(prad_graph* g, int64_t* out_forward, int64_t* out_backward) {
+  PRAD_CHECK_GRAPH(g);
+  PRAD_REQUIRE(out_forward && out_backward, PRAD_ERR_INVALID, "prad_graph_plan_products: null output");
+  *out_forward = g->forward_walk.plan ? graph_plan_products(g->forward_walk.plan.get()) : 0;
+  *out_backward = 0;
+  for (const auto& w : g->backward_walks)
+    if (w.plan) *out_backward += graph_plan_products(w.plan.get());
+  return PRAD_OK;
+}
+
 prad_status prad_graph_backward(prad_graph* g, int start_value, const void* d_start) {
   return prad_graph_backward_multi(g, &start_value, &d_start, 1);
 }

@@ -493,6 +493,7 @@ struct GraphPlan {
   const unsigned char* blob = nullptr;
   const gp::Item* items = nullptr;
   std::vector<Part> parts;
+  int products = 0;                          // that programs compute for themselves
   std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write: ascending, without overlaps
 };
 
@@ -576,20 +577,31 @@ struct Group {
 // Products that programs can compute for themselves.  A product of few outputs whose first reader is an elementwise operation on
 // them needs no level of its own, with its barrier and its way through memory: dots[e] are the products that operation e takes
 // along, fused[i] says that product i is one.  The product moves to the place of its reader, so nothing in between may write what
-// it reads or touch what it writes.  Every piece reads all columns of a product's second operand, so that may have DOT_OPERAND
-// bytes: three layers of 64 double units over twelve steps take 526 us with 16 columns (8 KB) as levels of their own and 592 us inside
-// programs, with 32 columns 890 and 1433 us; eight steps of two layers with 8 columns (4 KB) 169 us inside, 298 as before.
-constexpr int DOT_COLUMNS = 32, DOT_LOOK = 256, DOT_OPERAND = 4 * 1024;
+// it reads or touch what it writes.
+//
+// Which ones pay (us of both walks, losses and update; products as levels of their own, then inside programs; six steps of two layers).
+// Inside, every piece of 32 elements reads its rows of one operand and all columns of the other, so:
+//  - up to 512 outputs, a piece for each of the cluster's SMs: 64 units and 8 columns 157, 129 in double, 142, 112 in float, 100 and 5
+//    249, 198 and 231, 171, 16 and 32 116, 94 and 110, 87.  More pieces share an SM and take turns: 64 and 16 196, 207 in double, 32 and 32
+//    153, 180 in float; long chains beside short rows still pay in float (100 and 8 225, 202, 64 and 10 174, 167, but 64 and 12 174, 180);
+//  - weight gradients of a few more: those of all time steps and their sum become one program (24 units, 21 columns 166, 145);
+//  - operands that fit a worker's memory at once, or in two parts where nearly every SM has a piece (150 and 3 335, 267, but 128 and 2
+//    202, 242, 200 and 1 378, 758 and 300 and 1 1112, 2312).  What a program will hold is known when it is complete: then everything is
+//    grouped once more without its products.
+constexpr int DOT_COLUMNS = 32, DOT_LOOK = 256;
 constexpr int64_t TEAM_ELEMENTS = 2048;      // up to here several threads can share an element
-static void find_dots(const std::vector<Prim>& ops, size_t es, const std::vector<std::vector<Access>>& acc, std::vector<std::vector<int>>& dots,
-                      std::vector<char>& fused) {
+static bool dot_pays(const Prim& p, size_t es) {
+  const int64_t n = (int64_t)p.M * p.N;
+  if (p.kind != PRIM_PRODUCT || p.batch != 1 || p.K < 1 || p.N < 1 || p.N > DOT_COLUMNS || n > TEAM_ELEMENTS || (int64_t)p.K * p.N * (int64_t)es > 8192) return false;
+  return n <= 512 || (p.tB && (n <= 1024 || p.K <= 10)) || (es == 4 && n <= 1024 && p.N <= 10 && p.K >= 64);
+}
+static void find_dots(const std::vector<Prim>& ops, size_t es, const std::vector<std::vector<Access>>& acc, const std::vector<char>& barred,
+                      std::vector<std::vector<int>>& dots, std::vector<char>& fused) {
   const int N = (int)ops.size();
   auto meets = [](const Access& a, const Access& b) { return a.lo < b.hi && b.lo < a.hi; };
   for (int i = 0; i < N; ++i) {
     const Prim& p = ops[i];
-    if (p.kind != PRIM_PRODUCT || p.batch != 1 || p.K < 1 || p.N < 1 || p.N > DOT_COLUMNS || (int64_t)p.M * p.N > TEAM_ELEMENTS || acc[i].size() != 3 ||
-        (int64_t)p.K * p.N * (int64_t)es > DOT_OPERAND)
-      continue;
+    if (!dot_pays(p, es) || acc[i].size() != 3 || (!barred.empty() && barred[i])) continue;
     const Access &A = acc[i][0], &B = acc[i][1], &X = acc[i][2];
     if (meets(X, A) || meets(X, B)) continue;
     for (int e = i + 1; e < N && e <= i + DOT_LOOK; ++e) {
@@ -635,6 +647,39 @@ static void program_of(const std::vector<Prim>& all, int i, const std::vector<in
     g.rows += dot_rows(all[d]);
     g.dot_n = all[d].N;
   }
+}
+
+// The operands of the products that a program takes along, and how many k of them fit beside its slots.
+struct DotLayout {
+  struct Operand { const void* p; int kind, X, K, rows; };
+  std::vector<Operand> operands;
+  std::vector<std::pair<int, int>> of;       // by product: the numbers of its two
+  int rows = 0, most_k = 0, ks = 0, slot_values = 0;
+};
+template <typename T> static void dot_layout(const std::vector<Prim>& ops, const Group& g, const std::vector<std::vector<int>>& dots, DotLayout& l) {
+  l.operands.clear();
+  l.of.clear();
+  l.rows = l.most_k = 0;
+  auto operand = [&](const void* q, int kind, int X, int K, int rows) {
+    for (size_t k = 0; k < l.operands.size(); ++k) {
+      const auto& o = l.operands[k];
+      if (o.p == q && o.kind == kind && o.X == X && o.K == K) return (int)k;
+    }
+    l.operands.push_back({q, kind, X, K, rows});
+    l.rows += rows;
+    return (int)l.operands.size() - 1;
+  };
+  for (int o : g.ops)
+    for (int d : dots[o]) {
+      const Prim& q = ops[d];
+      const int a = operand(q.in[0], q.tA ? 1 : 0, q.M, q.K, dot_rows(q) - q.N);
+      l.of.push_back({a, operand(q.in[1], q.tB ? 3 : 2, q.N, q.K, q.N)});
+      l.most_k = std::max(l.most_k, q.K);
+    }
+  const int es = (int)sizeof(T);
+  l.slot_values = ((int)g.places.size() * DOT_PIECE * es + 15) / 16 * 16 / es;
+  l.ks = l.most_k;
+  while (l.rows * product_pitch<T>(l.ks) * es > WORK_BYTES - l.slot_values * es) l.ks = (int)ceil_div(l.ks / 2, 8) * 8;
 }
 
 struct Piece { uint32_t prog, bytes, chunk; double cost; };
@@ -712,7 +757,7 @@ struct Part { int ctas; bool cluster; std::vector<std::vector<Item>> lists; };
 
 template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& ops, int ctas, std::vector<unsigned char>& blob,
                                         std::vector<Part>& parts, std::vector<std::pair<uintptr_t, uintptr_t>>& written,
-                                        double* est_us, double* launch_us) {
+                                        double* est_us, double* launch_us, int* products, std::vector<char> barred = {}) {
   const size_t es = sizeof(T);
   const int N = (int)ops.size();
   std::vector<int> level(N, 0), group_of(N, -1);
@@ -722,7 +767,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
   std::vector<std::vector<int>> dots(N), after(N);           // after[d]: operations that wait for d
   std::vector<char> fused(N, 0);
   for (int i = 0; i < N; ++i) accesses(ops[i], es, all_acc[i]);
-  find_dots(ops, es, all_acc, dots, fused);
+  find_dots(ops, es, all_acc, barred, dots, fused);
   std::vector<Access> acc;
   *launch_us = 0;
   int joins = 0;
@@ -837,6 +882,29 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       if (r.lo == a.lo && r.hi == a.hi) { r.writers.clear(); r.readers.clear(); }
       r.writers.push_back(i);
     }
+  }
+
+  *products = (int)std::count(fused.begin(), fused.end(), 1);
+  // once more without the products whose operands make a program go over k several times (dot_pays)
+  DotLayout layout;
+  bool again = false;
+  for (const Group& g : groups) {
+    if (!g.dots) continue;
+    dot_layout<T>(ops, g, dots, layout);
+    const int64_t passes = ceil_div(layout.most_k, layout.ks);
+    if (passes == 1 || (passes == 2 && g.n > 14 * DOT_PIECE)) continue;
+    barred.resize(N, 0);
+    again = true;
+    for (int o : g.ops)
+      for (int d : dots[o])
+        for (int i = 0; i < N; ++i) {
+          const Prim &p = ops[d], &q = ops[i];
+          if (q.kind == PRIM_PRODUCT && p.M == q.M && p.N == q.N && p.K == q.K && p.tA == q.tA && p.tB == q.tB) barred[i] = 1;
+        }
+  }
+  if (again) {
+    build<T>(ctx, ops, ctas, blob, parts, written, est_us, launch_us, products, std::move(barred));
+    return;
   }
 
   for (const auto& m : mem)
@@ -1005,34 +1073,23 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
       std::vector<Dot> dot;
       int most_k = 0;
       if (!taken.empty()) {
-        std::vector<int> opd_rows;
-        auto operand = [&](const void* q, int kind, int X, int K, int rows) {
-          for (size_t k = 0; k < opds.size(); ++k)
-            if (opds[k].p == q && opds[k].kind == kind && opds[k].X == X && opds[k].K == K) return (int)k;
-          opds.push_back({q, kind, X, K, 0, 0, K, rows, 65536 / rows + 1});
-          opd_rows.push_back(rows);
-          return (int)opds.size() - 1;
-        };
-        for (int d : taken) {
-          const Prim& q = ops[d];
-          const int a = operand(q.in[0], q.tA ? 1 : 0, q.M, q.K, dot_rows(q) - q.N), b = operand(q.in[1], q.tB ? 3 : 2, q.N, q.K, q.N);
-          dot.push_back({q.scalar, q.K, slot(Place{q.out[0], 0}), a, b});
-          most_k = std::max(most_k, q.K);
+        dot_layout<T>(ops, g, dots, layout);
+        for (const auto& o : layout.operands) opds.push_back({o.p, o.kind, o.X, o.K, 0, 0, o.K, o.rows, 65536 / o.rows + 1});
+        for (size_t k = 0; k < taken.size(); ++k) {
+          const Prim& q = ops[taken[k]];
+          dot.push_back({q.scalar, q.K, slot(Place{q.out[0], 0}), layout.of[k].first, layout.of[k].second});
         }
-        int rows = 0;
-        for (int r : opd_rows) rows += r;
-        const int slot_values = (slots * DOT_PIECE * (int)es + 15) / 16 * 16 / (int)es;
-        h.ks = most_k;
-        while (rows * product_pitch<T>(h.ks) * (int)es > WORK_BYTES - slot_values * (int)es) h.ks = (int)ceil_div(h.ks / 2, 8) * 8;
+        most_k = layout.most_k;
+        h.ks = layout.ks;
         h.most_k = most_k;
         h.n_dot = (int)dot.size();
         h.dot_n = ops[taken[0]].N;
         h.dot_inv = (1u << 20) / h.dot_n + 1;
-        h.work_at = slot_values;
+        h.work_at = layout.slot_values;
         int at = 0;
         for (size_t k = 0; k < opds.size(); ++k) {
           opds[k].at = at;
-          at += opd_rows[k] * product_pitch<T>(h.ks);
+          at += layout.operands[k].rows * product_pitch<T>(h.ks);
         }
         for (Dot& t : dot) {
           t.a_at = opds[t.a_at].at;
@@ -1042,7 +1099,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
         const int copy_of[4] = {16, (int)es, (int)es, 16};
         std::vector<Opd> tasks;
         for (size_t k = 0; k < opds.size(); ++k) {
-          const int copies = opd_rows[k] * opds[k].K * (int)es / copy_of[opds[k].kind];
+          const int copies = opds[k].most * opds[k].K * (int)es / copy_of[opds[k].kind];
           const int room = (MAX_TASKS - (int)tasks.size()) / (int)(opds.size() - k);
           const int cut = std::max(1, std::min(room, copies / 192));
           const int len = (int)ceil_div(ceil_div(opds[k].K, cut), 8) * 8;
@@ -1254,7 +1311,8 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
   std::vector<Part> parts;
   double est = 0, launches = 0;
   std::vector<std::pair<uintptr_t, uintptr_t>> written;      // where the operations write: ascending, without overlaps
-  build<T>(ctx, ops, ctas, blob, parts, written, &est, &launches);
+  int products = 0;
+  build<T>(ctx, ops, ctas, blob, parts, written, &est, &launches, &products);
   if (est >= launches) return nullptr;
   std::vector<Item> items;
   std::vector<int> first;
@@ -1280,6 +1338,7 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
     return nullptr;
   }
   plan->written = std::move(written);
+  plan->products = products;
   plan->items = (const Item*)plan->mem;
   const int* at = (const int*)((const unsigned char*)plan->mem + items_bytes);
   for (const auto& part : parts) {
@@ -1295,6 +1354,8 @@ template <typename T> static GraphPlanPtr build_plan(prad_ctx* ctx, prad_dtype d
 GraphPlanPtr graph_plan_build(prad_ctx* ctx, prad_dtype dt, const std::vector<Prim>& ops) {
   return dt == PRAD_F32 ? gp::build_plan<float>(ctx, dt, ops) : gp::build_plan<double>(ctx, dt, ops);
 }
+
+int graph_plan_products(const GraphPlan* plan) { return plan->products; }
 
 bool graph_plan_writes(const GraphPlan* plan, const void* p, size_t bytes) {
   const uintptr_t lo = (uintptr_t)p, hi = lo + bytes;

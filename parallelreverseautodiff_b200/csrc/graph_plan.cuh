@@ -47,6 +47,8 @@ using GraphPlanPtr = std::unique_ptr<GraphPlan, GraphPlanFree>;
 // or a device that cannot run the cluster).
 GraphPlanPtr graph_plan_build(prad_ctx* ctx, prad_dtype dt, const std::vector<Prim>& ops);
 prad_status graph_plan_run(prad_ctx* ctx, GraphPlan* plan, const void* const* starts = nullptr, int count = 0);
+// how many products its programs compute for themselves
+int graph_plan_products(const GraphPlan* plan);
 // whether the plan's operations write anywhere in [p, p + bytes)
 bool graph_plan_writes(const GraphPlan* plan, const void* p, size_t bytes);
 

@@ -88,6 +88,12 @@ class Graph:
     def gradient(self, v: int):
         return self._matrix(self.eng.lib.prad_graph_value_gradient, v)
 
+    def plan_products(self):
+        """Products that the one-kernel walks take along, (forward, backward)."""
+        n = (C.c_int64(), C.c_int64())
+        check(self.eng.lib.prad_graph_plan_products(self.h, C.byref(n[0]), C.byref(n[1])))
+        return n[0].value, n[1].value
+
     def consumers(self, v: int) -> int:
         n = C.c_int()
         check(self.eng.lib.prad_graph_consumer_count(self.h, v, C.byref(n)))

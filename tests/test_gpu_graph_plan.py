@@ -256,13 +256,23 @@ def test_plans_of_many_sets_of_start_values(engine):
     g.close()
 
 
+# units, columns, inputs, steps, and how many of a step's three products (of the inputs, twice of the state) the forward program takes
+# along, in double and in float
+FUSED = [(5, 1, 3, 2, 3, 3), (13, 7, 9, 3, 3, 3), (16, 8, 64, 6, 3, 3), (64, 8, 65, 2, 3, 3), (96, 4, 96, 7, 3, 3), (24, 21, 12, 4, 3, 3),
+         (16, 32, 7, 3, 3, 3), (15, 33, 7, 3, 0, 0),              # columns: the last that fit, the first that do not
+         (64, 9, 33, 3, 0, 2), (64, 9, 64, 3, 0, 3), (63, 9, 33, 3, 0, 0), (102, 10, 64, 2, 0, 3), (103, 10, 64, 2, 0, 0),
+         (64, 11, 64, 2, 0, 0), (20, 32, 7, 3, 0, 0),             # beyond 512 outputs
+         (16, 32, 33, 2, 2, 3), (16, 32, 65, 2, 2, 2),            # a second operand of 8 KB
+         (230, 2, 230, 2, 3, 3), (230, 2, 600, 2, 2, 3),          # k in two parts, in double and in float
+         (220, 2, 230, 2, 0, 3), (400, 1, 500, 2, 0, 0)]          # two parts for too few pieces; many parts
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-@pytest.mark.parametrize("units,cols,inner,steps", [(5, 1, 3, 2), (13, 7, 9, 3), (16, 8, 64, 6), (33, 15, 130, 2), (64, 16, 33, 5),
-                                                    (20, 32, 7, 3), (20, 33, 7, 3), (64, 8, 700, 2), (64, 8, 65, 2), (96, 4, 96, 7), (400, 1, 500, 2)])
-def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, inner, steps):
-    """Cells whose products are taken along by the programs that read them, forward and backward: column counts that divide a piece
-    and that do not, the last that fits and the first that does not, more k than shared memory has room for, gradients of shared
-    weights added up over the steps."""
+@pytest.mark.parametrize("units,cols,inner,steps,in_double,in_float", FUSED)
+def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, inner, steps, in_double, in_float):
+    """Cells whose products are taken along by the programs that read them, forward and backward, and cells beyond every limit of
+    that: column counts that divide a piece and that do not, more k than shared memory has room for, gradients of shared weights added
+    up over the steps."""
     results = []
     for plan in ("1", "0"):
         r = rng(units + cols + inner)
@@ -283,11 +293,19 @@ def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, 
                 outs.append(g.node("MatrixAddOperation", [h, x]))
             got = []
             for k in range(2):
+                n0 = engine.launch_count()
                 g.forward()
+                launches = engine.launch_count() - n0
+                assert launches == 1 if plan == "1" else launches >= 8 * steps
                 got += [g.data(o).numpy() for o in outs]
                 g.backward(outs[-1 - k], up(units, cols))
                 got += [d.numpy() for d in grads]
             results.append(got)
+            forward, backward = g.plan_products()
+            expected = in_double if dtype == np.float64 else in_float
+            assert forward == (plan == "1") * steps * expected
+            # (no plan for the backward of a weight beyond 65536 values)
+            assert backward == 0 if plan == "0" or units * inner > 65536 else backward > 0 or expected < 3
             g.close()
         finally:
             engine.set_option("graph_plan", "1")
