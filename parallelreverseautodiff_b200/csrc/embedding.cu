@@ -33,9 +33,9 @@ embedding_gather_kernel(const T* __restrict__ index_col, const T* __restrict__ W
   chain_begin();
   if ((int)blockIdx.x < checkers) {
 #pragma unroll 8
-    for (int i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += checkers * EMB_THREADS) {
+    for (int64_t i = blockIdx.x * EMB_THREADS + threadIdx.x; i < n; i += checkers * EMB_THREADS) {      // (n up to the last int)
       const int idx = (int)index_col[i];
-      if (idx < 0 || idx >= vocab) emb_bad(flag, i);   // the managed code would throw IndexOutOfRange
+      if (idx < 0 || idx >= vocab) emb_bad(flag, (int)i);   // the managed code would throw IndexOutOfRange
     }
     __syncthreads();
     if (threadIdx.x == 0) {
