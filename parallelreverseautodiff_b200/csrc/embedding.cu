@@ -710,7 +710,7 @@ prad_status embedding_scatter_ordered(prad_ctx* ctx, prad_dtype dt, const void* 
 // A call's flag words, cleared for it; every call has another ticket.
 static int next_ticket(prad_ctx* ctx) {
   *(volatile int*)ctx->host_flag = 0;
-  if (++ctx->flag_ticket <= 0) ctx->flag_ticket = 1;
+  ctx->flag_ticket = ctx->flag_ticket < 0x7fffffff ? ctx->flag_ticket + 1 : 1;
   return ctx->flag_ticket;
 }
 static prad_status check_bad_index(prad_ctx* ctx, const char* who) {
