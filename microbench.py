@@ -89,7 +89,7 @@ def hbm_kernels(eng, only=None, rows=65536, cols=4096):
         ("softmax_backward_49", 3 * srows * 49 * 4, lambda: eng.softmax_backward(S, dS, out=oS)),
         ("layernorm_backward_96", 3 * lrows * 96 * 4, lambda: eng.layernorm_backward(Lx, mu, sd, dL, out=oL)),
         ("adam", 7 * npar * 4, lambda: eng.adam(P[0], P[1], P[2], P[3], 1e-3, .9, .999, 1e-8, 1.0)),
-        ("clip_reference_adam_zero", 11 * npar * 4,
+        ("clip_reference_adam_zero", 9 * npar * 4,
          lambda: eng.clip_adam(P[0], P[1], P[2], P[3], 1, 4.0, 1e-8, 1e-3, .9, .999, 1e-8, 1.0, zero_grad=True)),
         ("clip_global_norm_adam_zero", 9 * npar * 4,
          lambda: eng.clip_adam(P[0], P[1], P[2], P[3], 2, 4.0, 1e-8, 1e-3, .9, .999, 1e-8, 1.0, zero_grad=True)),

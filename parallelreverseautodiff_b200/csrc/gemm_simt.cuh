@@ -615,8 +615,9 @@ static prad_status launch_backward(prad_ctx* ctx, bool exact, Product<T> nt, Pro
 
 // Which tile shape.  A CTA that has its SM to itself takes `alone` cycles per k (its chain of additions, and the shared
 // memory's 128 bytes per cycle), n CTAs of one SM take n * `shared`: measured for the exact variants on products of
-// 128^2 x 2048, 256 x 512 x 784, 1024^2 x 120 and 2048^2 x 31, before lanes and copies were laid out as they are now (16 x 16
-// alone: 14.5 float, 23 double); where the shapes cross has not been measured again.  The estimate is the busiest SM's time; the 24 stands for
+// 128^2 x 2048, 256 x 512 x 784, 1024^2 x 120 and 2048^2 x 31, with the lanes, copies and stages of that time (16 x 16 alone takes
+// 14.5 and 23 since).  With the shapes that they choose, 69 other sizes of either type are as fast as with those kernels or faster, but for
+// those named at SimtShapes; where the shapes would cross now has not been measured.  The estimate is the busiest SM's time; the 24 stands for
 // filling the stages and writing the tile.  Small tiles win while there are fewer tiles than SMs, large ones once
 // every SM has several.
 struct ShapeCost { int bm, bn; double alone, shared; };

@@ -14,7 +14,7 @@
 // the pieces of a level -- 32, 64 or 256 elements, 256 or 1024 outputs -- are dealt to 32 workers when the plan is made, two to an
 // SM, and a worker fetches its next program while it runs this one.  The eight-step two-layer LSTM of 64 units and 8 columns, both
 // walks, losses and optimiser: 297 us with 22 levels each way and four workers of 64 registers (their spilled values went through
-// L2 after every barrier, which emptied the L1), 172 us now.
+// L2 after every barrier, which emptied the L1), 166 us now.
 //
 // Values are those of the separate kernels bit for bit for elementwise operations and products (k ascending, product and sum
 // rounded separately); row reductions and column sums add in double or in the same lane order.  (Compiled with -fmad=false.)
@@ -29,7 +29,7 @@ namespace prad {
 namespace gp {
 
 constexpr int NT = 256;                   // threads of a worker
-constexpr int WORKERS = 2;                // workers of a CTA: a piece is mostly latency, so two share an SM; 126 registers, no spills
+constexpr int WORKERS = 2;                // workers of a CTA: a piece is mostly latency, so two share an SM; up to 128 registers, no spills
 constexpr int SLOTS = 64;                 // values of one element a program keeps
 constexpr int MAX_INS = 96;
 constexpr int MAX_DOTS = 16;              // products a program computes for its own elements
@@ -134,7 +134,7 @@ template <typename T> __host__ __device__ constexpr int product_pitch(int ks) {
 // apart.  16-byte reads (with a read per value, reading was most of a piece), the next ones on their way while these are added.
 template <typename T, int R>
 __device__ __forceinline__ void multiply(const T* a, int da, const T* b, int db, int kc, T (&acc)[R][R]) {
-  constexpr int VEC = 16 / (int)sizeof(T), G = R == 1 ? 2 : 1, KG = G * VEC;      // k at a time: what 64 registers have room for
+  constexpr int VEC = 16 / (int)sizeof(T), G = R == 1 ? 2 : 1, KG = G * VEC;      // k at a time
   alignas(16) T x[R][KG], y[R][KG];
   auto fetch = [&](int k) {
 #pragma unroll
