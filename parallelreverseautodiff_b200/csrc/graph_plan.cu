@@ -1175,13 +1175,12 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
 
   // Deal the pieces of a level to the workers of `c` CTAs, the longest first to whoever has least (and to another SM before the
   // same one again); worker k of the dealing order is number k / c of CTA k % c.  Returns the time of the busiest.
-  auto deal = [&](int lv, int c, std::vector<std::vector<Item>>* lists) {
+  auto deal = [&](int lv, int c, std::vector<std::vector<Item>>& lists) {
     if (pieces[lv].size() <= (size_t)c * WORKERS) {          // one each
-      if (lists)
-        for (int k = 0; k < (int)pieces[lv].size(); ++k) {
-          const Piece& p = pieces[lv][k];
-          (*lists)[k % c * WORKERS + k / c].push_back({p.prog, p.bytes, p.chunk, 0});
-        }
+      for (int k = 0; k < (int)pieces[lv].size(); ++k) {
+        const Piece& p = pieces[lv][k];
+        lists[k % c * WORKERS + k / c].push_back({p.prog, p.bytes, p.chunk, 0});
+      }
       return pieces[lv].empty() ? 0.0 : pieces[lv][0].cost;
     }
     std::vector<std::pair<double, int>> heap;                // least busy first
@@ -1189,11 +1188,10 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     auto later = [](const std::pair<double, int>& x, const std::pair<double, int>& y) { return x > y; };
     auto give = [&](std::pair<double, int>& to, const Piece& p) {
       to.first += p.cost;
-      if (lists) (*lists)[to.second % c * WORKERS + to.second / c].push_back({p.prog, p.bytes, p.chunk, 0});
+      lists[to.second % c * WORKERS + to.second / c].push_back({p.prog, p.bytes, p.chunk, 0});
     };
     const std::vector<Piece>& all = pieces[lv];
-    if (lists)
-      for (auto& l : *lists) l.reserve(l.size() + all.size() / (size_t)(c * WORKERS) + 1);
+    for (auto& l : lists) l.reserve(l.size() + all.size() / (size_t)(c * WORKERS) + 1);
     for (size_t k = 0; k < all.size();) {
       size_t end = k + 1;                                    // pieces of one cost, many: in turn, once nobody is a piece ahead
       while (end < all.size() && all[end].cost == all[k].cost) ++end;
@@ -1216,26 +1214,27 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     return most;
   };
   for (auto& lv : pieces) std::stable_sort(lv.begin(), lv.end(), [](const Piece& a, const Piece& b) { return a.cost > b.cost; });
-  // The last levels run on all SMs, a launch each, where sixteen SMs would need 6 us longer for them (a launch, its program's way
-  // into every SM and the pieces are 4 us at the least).
+  // The last levels run on all SMs, a launch each (its program's way into every SM and the launch: 2.8 us more than a level of the
+  // cluster), from the level on where that gains most: a level of many pieces may be followed by one that loses by it.  (Ended at the first
+  // level from behind that would gain less than 6 us, twenty elementwise operations on 128 x 128 floats took 40 us backward, and
+  // a step of three layers of 128 units, 16 columns, twelve time steps, double, 1246; now 21 and 469.)
   int narrow = levels;
-  std::vector<Part> wide;
-  std::vector<double> wide_us;
-  while (narrow > 0) {
-    double all = 0, longest = 0;
-    for (const Piece& p : pieces[narrow - 1]) { all += p.cost; longest = std::max(longest, p.cost); }
-    const double at_least = std::max(longest, all / (ctx->sm_count * WORKERS));      // on all SMs
-    if (all / (ctas * WORKERS) + longest - at_least <= 6.0) break;                   // (no worker is a piece ahead of the mean)
-    const bool sure = all / (ctas * WORKERS) - all / (ctx->sm_count * WORKERS) - longest > 6.0;
-    const double here = sure ? 1e30 : deal(narrow - 1, ctas, nullptr);
-    if (here - at_least <= 6.0) break;
-    Part part{ctx->sm_count, false, {}};
-    part.lists.assign(ctx->sm_count * WORKERS, {});
-    const double there = deal(narrow - 1, ctx->sm_count, &part.lists);
-    if (here - there <= 6.0) break;
-    wide.push_back(std::move(part));
-    wide_us.push_back(there);
-    --narrow;
+  double gained = 0, most_gained = 0;
+  for (int lv = levels; lv-- > 0;) {
+    const std::vector<Piece>& level_pieces = pieces[lv];
+    if (level_pieces.empty()) continue;
+    const double longest = level_pieces.front().cost;
+    double all = 0;
+    for (const Piece& p : level_pieces) all += p.cost;
+    auto time = [&](int workers) {
+      if (longest == level_pieces.back().cost) return (double)ceil_div((int64_t)level_pieces.size(), workers) * longest;
+      return std::max(longest, all / workers);
+    };
+    gained += time(ctas * WORKERS) - time(ctx->sm_count * WORKERS) - 2.8;
+    if (gained > most_gained) {
+      most_gained = gained;
+      narrow = lv;
+    }
   }
   *est_us = 4.0;
   if (narrow > 0) {
@@ -1244,7 +1243,7 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     for (int lv = 0; lv < narrow; ++lv) {
       std::vector<size_t> before(part.lists.size());
       for (size_t c = 0; c < before.size(); ++c) before[c] = part.lists[c].size();
-      *est_us += 0.8 + deal(lv, ctas, &part.lists);
+      *est_us += 0.8 + deal(lv, ctas, part.lists);
       for (size_t c = 0; c < before.size(); ++c) {           // a barrier behind every level
         if (part.lists[c].size() == before[c]) part.lists[c].push_back({0, 0, 0, 1});
         else part.lists[c].back().barrier = 1;
@@ -1252,9 +1251,12 @@ template <typename T> static void build(prad_ctx* ctx, const std::vector<Prim>& 
     }
     parts.push_back(std::move(part));
   }
-  for (size_t k = wide.size(); k-- > 0;) {
-    *est_us += 3.0 + wide_us[k];
-    parts.push_back(std::move(wide[k]));
+  for (int lv = narrow; lv < levels; ++lv) {
+    if (pieces[lv].empty()) continue;
+    Part part{ctx->sm_count, false, {}};
+    part.lists.assign(ctx->sm_count * WORKERS, {});
+    *est_us += 3.0 + deal(lv, ctx->sm_count, part.lists);
+    parts.push_back(std::move(part));
   }
 }
 

@@ -311,3 +311,36 @@ def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, 
             engine.set_option("graph_plan", "1")
     for a, b in zip(*results):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("rows,cols,depth", [(100, 100, 20), (128, 128, 20), (90, 100, 30), (128, 128, 40), (255, 257, 12)])
+def test_long_elementwise_chains_on_all_SMs_are_the_same_bits(engine, dtype, rows, cols, depth):
+    """More pieces a level than the cluster has workers, over several levels: from the best one on, a launch on all SMs each, also where
+    the last level alone would gain nothing by that."""
+    results = []
+    for plan in ("1", "0"):
+        r = rng(rows + depth)
+        up = lambda: engine.upload((r.standard_normal((rows, cols)) * 0.3).astype(dtype))  # noqa: E731
+        engine.set_option("graph_plan", plan)
+        try:
+            g = Graph(engine, dtype)
+            dx = engine.zeros((rows, cols), dtype)
+            h, x = g.input(up()), g.weight(up(), dx)
+            for k in range(depth):
+                h = g.node(("SigmoidOperation", "TanhOperation", "GELUOperation", "LeakyReLUOperation")[k % 4], [h], scalar=0.01)
+                h = g.node("HadamardProductOperation" if k % 2 else "MatrixAddOperation", [h, x])
+            got, d = [], up()
+            for _ in range(2):
+                g.forward()
+                n0 = engine.launch_count()
+                g.backward(h, d)
+                launches = engine.launch_count() - n0
+                assert launches > depth if plan == "0" else launches < 6
+                got += [g.data(h).numpy(), dx.numpy()]
+            results.append(got)
+            g.close()
+        finally:
+            engine.set_option("graph_plan", "1")
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
