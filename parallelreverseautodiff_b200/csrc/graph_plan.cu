@@ -9,12 +9,12 @@
 // element in shared memory from its load to its store, and such a program computes the products that it reads, where they are
 // small, for its own elements: a cell of an LSTM is one level instead of a level of products and one of programs.  One cluster of
 // 16 CTAs runs the levels with the cluster's hardware barrier between them (no waiting loops, no other CTA to wait for).  What
-// nothing waits for (weight gradients, outputs) comes as late as it can, and large levels at the end run on all SMs, as launches of
-// their own.  A level is latency: a barrier (1.1 us), a program (1.7), operands from L2 (1.2), a chain of 64 additions (1.5).  So
+// nothing waits for (weight gradients, outputs) comes as late as it can, and from the level on where that gains most the levels run
+// on all SMs, as launches of their own.  A level is latency: a barrier (1.1 us), a program (1.7), operands from L2 (1.2), a chain of 64 additions (1.5).  So
 // the pieces of a level -- 32, 64 or 256 elements, 256 or 1024 outputs -- are dealt to 32 workers when the plan is made, two to an
 // SM, and a worker fetches its next program while it runs this one.  The eight-step two-layer LSTM of 64 units and 8 columns, both
 // walks, losses and optimiser: 297 us with 22 levels each way and four workers of 64 registers (their spilled values went through
-// L2 after every barrier, which emptied the L1), 166 us now.
+// L2 after every barrier, which emptied the L1), 160 us now.
 //
 // Values are those of the separate kernels bit for bit for elementwise operations and products (k ascending, product and sum
 // rounded separately); row reductions and column sums add in double or in the same lane order.  (Compiled with -fmad=false.)
@@ -579,21 +579,19 @@ struct Group {
 // along, fused[i] says that product i is one.  The product moves to the place of its reader, so nothing in between may write what
 // it reads or touch what it writes.
 //
-// Which ones pay (us of both walks, losses and update; products as levels of their own, then inside programs; six steps of two layers).
-// Inside, every piece of 32 elements reads its rows of one operand and all columns of the other, so:
-//  - up to 512 outputs, a piece for each of the cluster's SMs: 64 units and 8 columns 157, 129 in double, 142, 112 in float, 100 and 5
-//    249, 198 and 231, 171, 16 and 32 116, 94 and 110, 87.  More pieces share an SM and take turns: 64 and 16 196, 207 in double, 32 and 32
-//    153, 180 in float; long chains beside short rows still pay in float (100 and 8 225, 202, 64 and 10 174, 167, but 64 and 12 174, 180);
-//  - weight gradients of a few more: those of all time steps and their sum become one program (24 units, 21 columns 166, 145);
-//  - operands that fit a worker's memory at once, or in two parts where nearly every SM has a piece (150 and 3 335, 267, but 128 and 2
-//    202, 242, 200 and 1 378, 758 and 300 and 1 1112, 2312).  What a program will hold is known when it is complete: then everything is
-//    grouped once more without its products.
-constexpr int DOT_COLUMNS = 32, DOT_LOOK = 256;
+// Which ones pay (us of both walks, losses and update of an LSTM of two layers and six steps, or as many as said; products as levels of
+// their own, then inside programs): up to 2048 outputs, where several threads share an element -- 64 units and 8 columns 157, 129 in
+// double and 142, 112 in float, 64 and 16 196, 130 and 172, 116, 32 and 32 148, 126 and 137, 115, 100 and 12 238, 186 and 222, 158, 30 and
+// 20 over twelve steps of three layers 463, 309 and 260, 216, though 20 and 32 131, 154 and 124, 145, 48 and 11 165, 179 and 150, 154; a
+// second operand of up to 16 KB, for every piece of 32 elements reads all its columns (with up to 8 KB 100 and 20 221, 160 and 12 249 in
+// double, now 205 and 229); and operands that fit a worker's memory at once, or in two parts where nearly every SM of the cluster has
+// a piece (150 and 3 335, 267, but 128 and 2 in two parts 244, as levels 192).  What a program will hold is known when it is complete: then
+// everything is grouped once more without its products.
+constexpr int DOT_COLUMNS = 32, DOT_LOOK = 256, DOT_OPERAND = 16 * 1024;
 constexpr int64_t TEAM_ELEMENTS = 2048;      // up to here several threads can share an element
 static bool dot_pays(const Prim& p, size_t es) {
-  const int64_t n = (int64_t)p.M * p.N;
-  if (p.kind != PRIM_PRODUCT || p.batch != 1 || p.K < 1 || p.N < 1 || p.N > DOT_COLUMNS || n > TEAM_ELEMENTS || (int64_t)p.K * p.N * (int64_t)es > 8192) return false;
-  return n <= 512 || (p.tB && (n <= 1024 || p.K <= 10)) || (es == 4 && n <= 1024 && p.N <= 10 && p.K >= 64);
+  return p.kind == PRIM_PRODUCT && p.batch == 1 && p.K >= 1 && p.N >= 1 && p.N <= DOT_COLUMNS && (int64_t)p.M * p.N <= TEAM_ELEMENTS &&
+         (int64_t)p.K * p.N * (int64_t)es <= DOT_OPERAND;
 }
 static void find_dots(const std::vector<Prim>& ops, size_t es, const std::vector<std::vector<Access>>& acc, const std::vector<char>& barred,
                       std::vector<std::vector<int>>& dots, std::vector<char>& fused) {

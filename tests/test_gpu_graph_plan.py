@@ -260,10 +260,9 @@ def test_plans_of_many_sets_of_start_values(engine):
 # along, in double and in float
 FUSED = [(5, 1, 3, 2, 3, 3), (13, 7, 9, 3, 3, 3), (16, 8, 64, 6, 3, 3), (64, 8, 65, 2, 3, 3), (96, 4, 96, 7, 3, 3), (24, 21, 12, 4, 3, 3),
          (16, 32, 7, 3, 3, 3), (15, 33, 7, 3, 0, 0),              # columns: the last that fit, the first that do not
-         (64, 9, 33, 3, 0, 2), (64, 9, 64, 3, 0, 3), (63, 9, 33, 3, 0, 0), (102, 10, 64, 2, 0, 3), (103, 10, 64, 2, 0, 0),
-         (64, 11, 64, 2, 0, 0), (20, 32, 7, 3, 0, 0),             # beyond 512 outputs
-         (16, 32, 33, 2, 2, 3), (16, 32, 65, 2, 2, 2),            # a second operand of 8 KB
-         (230, 2, 230, 2, 3, 3), (230, 2, 600, 2, 2, 3),          # k in two parts, in double and in float
+         (64, 32, 33, 2, 3, 3), (65, 32, 7, 2, 0, 0),             # outputs
+         (16, 32, 64, 2, 3, 3), (16, 32, 65, 2, 2, 3), (16, 32, 129, 2, 2, 2),      # the second operand
+         (230, 2, 230, 2, 3, 3), (230, 2, 600, 2, 0, 3),          # k in two parts, in double and in float
          (220, 2, 230, 2, 0, 3), (400, 1, 500, 2, 0, 0)]          # two parts for too few pieces; many parts
 
 
@@ -273,7 +272,7 @@ def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, 
     """Cells whose products are taken along by the programs that read them, forward and backward, and cells beyond every limit of
     that: column counts that divide a piece and that do not, more k than shared memory has room for, gradients of shared weights added
     up over the steps."""
-    results = []
+    results, launches = [], []
     for plan in ("1", "0"):
         r = rng(units + cols + inner)
         up = lambda *s: engine.upload((r.standard_normal(s) * 0.4).astype(dtype))  # noqa: E731
@@ -295,8 +294,7 @@ def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, 
             for k in range(2):
                 n0 = engine.launch_count()
                 g.forward()
-                launches = engine.launch_count() - n0
-                assert launches == 1 if plan == "1" else launches >= 8 * steps
+                launches.append(engine.launch_count() - n0)
                 got += [g.data(o).numpy() for o in outs]
                 g.backward(outs[-1 - k], up(units, cols))
                 got += [d.numpy() for d in grads]
@@ -309,6 +307,7 @@ def test_products_inside_programs_are_the_same_bits(engine, dtype, units, cols, 
             g.close()
         finally:
             engine.set_option("graph_plan", "1")
+    assert launches[0] * 2 < launches[2] and launches[0] == launches[1] and launches[2] == launches[3] >= 8 * steps
     for a, b in zip(*results):
         np.testing.assert_array_equal(a, b)
 
